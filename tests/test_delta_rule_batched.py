@@ -137,3 +137,69 @@ def test_gated_delta_net_mixer_on_cuda_runs_the_state_kernel_and_matches_the_cpu
     assert (got.cpu() - want).abs().max() <= 2e-2 * max(1.0, want.abs().max())
     for (n, a), b in zip(dev.named_parameters(), ref.parameters()):
         assert (a.grad.cpu() - b.grad).abs().max() <= 3e-2 * max(1.0, b.grad.abs().max()), n
+
+
+def test_chunk_tables_cover_every_row_once():
+    from torchturbo_b200.ops.providers.b200_linear_attention import _chunk_tables
+
+    segs = [(0, 0, 1), (0, 1, 1), (0, 1, 66), (0, 66, 194)]
+    if torch.cuda.is_available():
+        seq, rows, last, first = (t.cpu() for t in _chunk_tables(segs, 64, "cuda"))
+    else:
+        pin = torch.Tensor.pin_memory
+        torch.Tensor.pin_memory = lambda self: self
+        try:
+            seq, rows, last, first = _chunk_tables(segs, 64, "cpu")
+        finally:
+            torch.Tensor.pin_memory = pin
+    assert seq.tolist() == [[0, 1], [1, 0], [1, 2], [3, 2]]
+    assert rows.tolist() == [[0, 1, 0], [1, 64, 2], [65, 1, 2], [66, 64, 3], [130, 64, 3]]
+    covered = [r for a, n, _ in rows.tolist() for r in range(a, a + n)]
+    assert covered == list(range(194))
+    assert first.tolist() == [0, 2, 3, 6] and last.tolist() == [1, 2, 5, 8]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vec", [False, True])
+@pytest.mark.parametrize("cu, T, H, l2, strided", [
+    ([0, 1], 1, 1, True, False),                       # one row
+    ([0, 63, 127, 192], 192, 3, False, False),         # one short of a chunk, a whole chunk, one over
+    ([0, 70, 70, 199], 260, 2, True, True),            # an empty sequence, a padded tail, rows inside a wider projection
+    (None, 128, 2, True, False),                       # two whole-chunk rows of a batch
+])
+def test_fused_chunk_kernels_on_bf16_rows_match_the_fp32_formulation(vec, cu, T, H, l2, strided):
+    """The fused kernels against the batched formulation in fp32 on the CPU, same bf16 inputs, values and all gradients.
+    Bound: the recurrence multiplies bf16-rounded operands (2^-9 each) and outputs are rounded to bf16, so a few units of
+    2^-9 of the largest entry; 2e-2 is five of them and the bound of the recurrence's own test above."""
+    from torchturbo_b200 import kernels as K
+    from torchturbo_b200.ops.providers import b200_linear_attention as L
+
+    B = 2 if cu is None else 1
+    gen = torch.Generator().manual_seed(T)
+    D = 128
+    wide = torch.randn(B, T, 3, H, D, generator=gen).to(torch.bfloat16)
+    g = -torch.rand(B, T, H, *([D] if vec else []), generator=gen) * 0.3
+    beta = torch.rand(B, T, H, generator=gen)
+    n = B if cu is None else len(cu) - 1 + (cu[-1] < T)
+    init = torch.randn(n, H, D, D, generator=gen) * 0.05
+
+    def run(dev, dtype):
+        w = wide.to(dev, dtype)
+        qkv = [w[:, :, i] if strided else w[:, :, i].contiguous() for i in range(3)]
+        if not l2:
+            qkv[0], qkv[1] = qkv[0] * 0.0625, qkv[1] * 0.0625
+        leaves = [t.detach().requires_grad_(True) for t in (*qkv, g.to(dev), beta.to(dev), init.to(dev))]
+        o, fin = L.chunk_delta_rule_batched(*leaves[:5], initial_state=leaves[5], output_final_state=True, cu_seqlens=cu, use_qk_l2norm=l2)
+        w1 = torch.sin(torch.arange(o.numel(), device=dev, dtype=torch.float32)).view(o.shape).to(o.dtype)
+        (o.float() * w1.float()).sum().add(fin.sum() * 0.1).backward()
+        return [o, fin] + [t.grad for t in leaves]
+
+    before = K.launch_count()
+    got = run("cuda", torch.bfloat16)
+    torch.cuda.synchronize()
+    assert K.launch_count() - before == (7 if vec else 6) and K.status() == (0, 0)   # no torch formulation in between
+    for name, a, b in zip(("o", "final", "dq", "dk", "dv", "dg", "dbeta", "dinit"), got, run("cpu", torch.float32)):
+        a, b = a.float().cpu(), b.float()
+        assert a.shape == b.shape
+        assert (a - b).abs().max() <= 2e-2 * max(1.0, b.abs().max()), (name, (a - b).abs().max(), b.abs().max())
+        assert (a - b).norm() <= 2e-2 * b.norm() + 1e-6, (name, (a - b).norm() / b.norm())

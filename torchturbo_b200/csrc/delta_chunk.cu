@@ -1,0 +1,681 @@
+// Kernels of the gated delta rule with one decay per head (GatedDeltaNet); the formulas, the arithmetic and the reasons
+// are at the top of delta_chunk.cuh.
+#include "delta_chunk.cuh"
+
+namespace ttb {
+
+// ------------------------------------------------------------------------------------------------
+// prep
+// ------------------------------------------------------------------------------------------------
+struct DpSmem {
+  static constexpr int Q = 0, K = Q + DC_C * DC_QS * 2, V = K + DC_C * DC_QS * 2;
+  static constexpr int L = V + DC_C * DC_QS * 2, T = L + DC_C * DP_LT * 4;
+  static constexpr int ROWS = T + DC_C * DP_LT * 4;     // G, beta, 1/|k|, 1/|q|, beta e^G / |k|
+  static constexpr int TOTAL = ROWS + 5 * DC_C * 4;
+};
+
+__global__ void __launch_bounds__(256, 2)
+delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restrict__ Ag, float* __restrict__ U,
+                  __nv_bfloat16* __restrict__ W, __nv_bfloat16* __restrict__ Ko, float* __restrict__ decay) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sm + DpSmem::Q);
+  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(sm + DpSmem::K);
+  __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(sm + DpSmem::V);
+  float* sL = reinterpret_cast<float*>(sm + DpSmem::L);
+  float* sT = reinterpret_cast<float*>(sm + DpSmem::T);
+  float* sG = reinterpret_cast<float*>(sm + DpSmem::ROWS);
+  float *sB = sG + DC_C, *sRk = sB + DC_C, *sRq = sRk + DC_C, *sW = sRq + DC_C;
+  const int c = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int row0 = p.chunk_rows[3 * c], n = p.chunk_rows[3 * c + 1];
+  const long long hc = static_cast<long long>(h) * p.NC + c;
+
+  dc_load_rows<256>(sQ, p.q + row0 * p.q_t + h * p.q_h, p.q_t, n);
+  dc_load_rows<256>(sK, p.k + row0 * p.k_t + h * p.k_h, p.k_t, n);
+  dc_load_rows<256>(sV, p.v + row0 * p.v_t + h * p.v_h, p.v_t, n);
+  dc_load_gates(p, row0, n, h, sG, sB);
+  __syncthreads();
+  dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
+  dc_row_norms<256>(sK, sRk, p.l2, 1.f);
+  if (warp == 0) dc_cumsum(sG, lane);
+  __syncthreads();
+  if (tid < DC_C) sW[tid] = sB[tid] * sRk[tid] * dc_exp(sG[tid]);
+  if (tid == 0) decay[hc] = dc_exp(sG[DC_C - 1]);
+
+  const int mi = warp & 3, m0 = mi * 16, g = lane >> 2, t2 = (lane & 3) * 2;
+  {
+    // scores: warps 0-3 k k^T -> L, warps 4-7 q k^T -> A, 16 rows each
+    const bool is_q = warp >= 4;
+    float acc[8][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      uint32_t a[4];
+      dc_a(a, is_q ? sQ : sK, m0, kk * 16, lane);
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        if (np > mi) continue;
+        uint32_t b[4];
+        dc_b(b, sK, np * 16, kk * 16, lane);
+        dc_mma(acc[2 * np], a, b[0], b[1]);
+        dc_mma(acc[2 * np + 1], a, b[2], b[3]);
+      }
+    }
+    float* Aout = Ag + hc * DC_C * DC_C;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int i = m0 + g + rr * 8, j = nt * 8 + t2;
+        float2 o = make_float2(0.f, 0.f);
+        const float ri = is_q ? sRq[i] : sRk[i] * sB[i];
+        if (is_q ? (j <= i) : (j < i)) o.x = acc[nt][2 * rr] * (ri * sRk[j]) * dc_exp(sG[i] - sG[j]);
+        if (is_q ? (j + 1 <= i) : (j + 1 < i)) o.y = acc[nt][2 * rr + 1] * (ri * sRk[j + 1]) * dc_exp(sG[i] - sG[j + 1]);
+        *reinterpret_cast<float2*>(is_q ? Aout + i * DC_C + j : sL + i * DP_LT + j) = o;
+      }
+    }
+  }
+  __syncthreads();
+  dc_invert(sL, sT);
+  {
+    float* Tout = Tg + hc * DC_C * DC_C;
+#pragma unroll
+    for (int e = tid; e < DC_C * 16; e += 256) {
+      const int i = e >> 4, j = (e & 15) * 4;
+      *reinterpret_cast<float4*>(Tout + i * DC_C + j) = *reinterpret_cast<const float4*>(sT + i * DP_LT + j);
+    }
+  }
+  // ---- u = (T beta) v, w = (T beta e^G / |k|) k: 16 rows x 64 columns per warp, T lower triangular
+  const int n0 = (warp >> 2) * 64;
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    float acc[8][4] = {};
+    for (int kk = 0; kk <= mi; ++kk) {
+      uint32_t a[3][4];
+      dc_af<3>(a, sT, DP_LT, m0, kk * 16, lane, which ? sW : sB);
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        uint32_t b[4];
+        dc_b_t(b, which ? sK : sV, n0 + np * 16, kk * 16, lane);
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          dc_mma(acc[2 * np], a[i], b[0], b[1]);
+          dc_mma(acc[2 * np + 1], a[i], b[2], b[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const long long at = (hc * DC_C + m0 + g + rr * 8) * DC_D + n0 + nt * 8 + t2;
+        if (which) *reinterpret_cast<uint32_t*>(W + at) = pack_bf16(acc[nt][2 * rr], acc[nt][2 * rr + 1]);
+        else *reinterpret_cast<float2*>(U + at) = make_float2(acc[nt][2 * rr], acc[nt][2 * rr + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = tid; e < DC_C * 16; e += 256) {
+    const int i = e >> 4, j = (e & 15) * 8;
+    const float f = dc_exp(sG[DC_C - 1] - sG[i]) * sRk[i];
+    uint4 u = *reinterpret_cast<const uint4*>(sK + i * DC_QS + j);
+    uint32_t* w = reinterpret_cast<uint32_t*>(&u);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float2 v = unpack_bf16(w[x]);
+      w[x] = pack_bf16(v.x * f, v.y * f);
+    }
+    *reinterpret_cast<uint4*>(Ko + (hc * DC_C + i) * DC_D + j) = u;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// out: o = (q e^G / |q|) S + A x, 64 of the 128 value columns per CTA
+// ------------------------------------------------------------------------------------------------
+struct DoSmem {
+  static constexpr int Q = 0, S = Q + DC_C * DC_QS * 2, X = S + DC_D * DO_LD * 4, A = X + DC_C * DO_LD * 4;
+  static constexpr int ROWS = A + DC_C * DP_LT * 4;
+  static constexpr int TOTAL = ROWS + 2 * DC_C * 4;
+};
+
+__global__ void __launch_bounds__(256, 2)
+delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float* __restrict__ X, const float* __restrict__ St,
+                 int nseq, __nv_bfloat16* __restrict__ O) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sm + DoSmem::Q);
+  float* sS = reinterpret_cast<float*>(sm + DoSmem::S);
+  float* sX = reinterpret_cast<float*>(sm + DoSmem::X);
+  float* sA = reinterpret_cast<float*>(sm + DoSmem::A);
+  float* sG = reinterpret_cast<float*>(sm + DoSmem::ROWS);
+  float* sRq = sG + DC_C;
+  const int c = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * 64, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = p.chunk_rows[3 * c], n = p.chunk_rows[3 * c + 1], slot = c + p.chunk_rows[3 * c + 2];
+  const long long hc = static_cast<long long>(h) * p.NC + c;
+  dc_load_rows<256>(sQ, p.q + row0 * p.q_t + h * p.q_h, p.q_t, n);
+  dc_load_f32<256, DC_D, 64>(sS, DO_LD, St + ((static_cast<long long>(h) * (p.NC + nseq) + slot) * DC_D) * DC_D + v0, DC_D);
+  dc_load_f32<256, DC_C, 64>(sX, DO_LD, X + hc * DC_C * DC_D + v0, DC_D);
+  dc_load_f32<256, DC_C, 64>(sA, DP_LT, Ag + hc * DC_C * DC_C, DC_C);
+  if (threadIdx.x < DC_C) sG[threadIdx.x] = threadIdx.x < n ? __ldg(p.g + static_cast<long long>(row0 + threadIdx.x) * p.H + h) : 0.f;
+  __syncthreads();
+  dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
+  if (warp == 0) dc_cumsum(sG, lane);
+  __syncthreads();
+  const int g = lane >> 2, t2 = (lane & 3) * 2, n0 = warp * 8;
+  float acc[4][4] = {};
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    uint32_t b[3][2];
+    dc_bf_t<3>(b, sS, DO_LD, n0, kk * 16, lane);
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi) {
+      uint32_t a[4];
+      dc_a(a, sQ, mi * 16, kk * 16, lane);
+#pragma unroll
+      for (int i = 2; i >= 0; --i) dc_mma(acc[mi], a, b[i][0], b[i][1]);
+    }
+  }
+#pragma unroll
+  for (int mi = 0; mi < 4; ++mi) {
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const int i = mi * 16 + g + rr * 8;
+      const float f = sRq[i] * dc_exp(sG[i]);
+      acc[mi][2 * rr] *= f;
+      acc[mi][2 * rr + 1] *= f;
+    }
+  }
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    uint32_t b[2][2];
+    dc_bf_t<2>(b, sX, DO_LD, n0, kk * 16, lane);
+#pragma unroll
+    for (int mi = kk; mi < 4; ++mi) {
+      uint32_t a[2][4];
+      dc_af<2>(a, sA, DP_LT, mi * 16, kk * 16, lane);
+      dc_mma22(acc[mi], a[0], a[1], b[0], b[1]);
+    }
+  }
+  __syncthreads();
+  __nv_bfloat16* sO = sQ;                      // [64][72]: whole 128-byte rows go out
+#pragma unroll
+  for (int mi = 0; mi < 4; ++mi) {
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr)
+      *reinterpret_cast<uint32_t*>(sO + (mi * 16 + g + rr * 8) * 72 + n0 + t2) = pack_bf16(acc[mi][2 * rr], acc[mi][2 * rr + 1]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = threadIdx.x; e < DC_C * 8; e += 256) {
+    const int i = e >> 3, j = (e & 7) * 8;
+    if (i < n)
+      *reinterpret_cast<uint4*>(O + (static_cast<long long>(row0 + i) * p.H + h) * DC_D + v0 + j) = *reinterpret_cast<const uint4*>(sO + i * 72 + j);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// bwd_pre: gx = A^T do, gS = (q e^G / |q|)^T do, written to the slot of the chunk's start state
+// ------------------------------------------------------------------------------------------------
+struct DbSmem {
+  static constexpr int Q = 0, DO = Q + DC_C * DC_QS * 2, A = DO + DC_C * DC_QS * 2;
+  static constexpr int ROWS = A + DC_C * DO_LD * 4;
+  static constexpr int TOTAL = ROWS + 3 * DC_C * 4;
+};
+
+__global__ void __launch_bounds__(256, 2)
+delta_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO, const float* __restrict__ Ag, int nseq,
+                     float* __restrict__ GX, float* __restrict__ GS) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sm + DbSmem::Q);
+  __nv_bfloat16* sDO = reinterpret_cast<__nv_bfloat16*>(sm + DbSmem::DO);
+  float* sA = reinterpret_cast<float*>(sm + DbSmem::A);
+  float* sG = reinterpret_cast<float*>(sm + DbSmem::ROWS);
+  float *sRq = sG + DC_C, *sF = sRq + DC_C;
+  const int c = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = p.chunk_rows[3 * c], n = p.chunk_rows[3 * c + 1], slot = c + p.chunk_rows[3 * c + 2];
+  const long long hc = static_cast<long long>(h) * p.NC + c;
+  dc_load_rows<256>(sQ, p.q + row0 * p.q_t + h * p.q_h, p.q_t, n);
+  dc_load_rows<256>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
+  dc_load_f32<256, DC_C, 64>(sA, DO_LD, Ag + hc * DC_C * DC_C, DC_C);
+  if (threadIdx.x < DC_C) sG[threadIdx.x] = threadIdx.x < n ? __ldg(p.g + static_cast<long long>(row0 + threadIdx.x) * p.H + h) : 0.f;
+  __syncthreads();
+  dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
+  if (warp == 0) dc_cumsum(sG, lane);
+  __syncthreads();
+  if (threadIdx.x < DC_C) sF[threadIdx.x] = sRq[threadIdx.x] * dc_exp(sG[threadIdx.x]);
+  __syncthreads();
+  const int g = lane >> 2, t2 = (lane & 3) * 2, n0 = warp * 16;
+  {
+    float acc[4][2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t b[4];
+      dc_b_t(b, sDO, n0, kk * 16, lane);
+#pragma unroll
+      for (int mi = 0; mi <= kk; ++mi) {           // rows j of A^T meet rows i >= j only
+        uint32_t a[3][4];
+        dc_af_t<3>(a, sA, DO_LD, mi * 16, kk * 16, lane);
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          dc_mma(acc[mi][0], a[i], b[0], b[1]);
+          dc_mma(acc[mi][1], a[i], b[2], b[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr)
+          *reinterpret_cast<float2*>(GX + (hc * DC_C + mi * 16 + g + rr * 8) * DC_D + n0 + nt * 8 + t2) =
+              make_float2(acc[mi][nt][2 * rr], acc[mi][nt][2 * rr + 1]);
+  }
+  {
+    // the row factor runs along the contraction, so it rides on do (split in three) and q stays exact
+    float acc[8][2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t b[4], bs[3][4];
+      dc_b_t(b, sDO, n0, kk * 16, lane);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int k = kk * 16 + t2 + (r & 1) * 8;
+        const float2 v = unpack_bf16(b[r]);
+        uint32_t w[3];
+        dc_split<3>(v.x * sF[k], v.y * sF[k + 1], w);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) bs[i][r] = w[i];
+      }
+#pragma unroll
+      for (int mi = 0; mi < 8; ++mi) {
+        uint32_t a[4];
+        dc_a_t(a, sQ, mi * 16, kk * 16, lane);
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          dc_mma(acc[mi][0], a, bs[i][0], bs[i][1]);
+          dc_mma(acc[mi][1], a, bs[i][2], bs[i][3]);
+        }
+      }
+    }
+    float* out = GS + ((static_cast<long long>(h) * (p.NC + nseq) + slot) * DC_D) * DC_D;
+#pragma unroll
+    for (int mi = 0; mi < 8; ++mi)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr)
+          *reinterpret_cast<float2*>(out + (mi * 16 + g + rr * 8) * DC_D + n0 + nt * 8 + t2) =
+              make_float2(acc[mi][nt][2 * rr], acc[mi][nt][2 * rr + 1]);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// bwd_post: dq, dk, dv, dg, dbeta of one chunk and head
+// ------------------------------------------------------------------------------------------------
+constexpr int DQ_LD = 136;   // row stride of fp32 tiles read in pairs along a row
+constexpr int DQ_DX = 132;   // row stride of dx, read down its columns
+constexpr int DQ_P = 68;     // row stride of T / P and R
+struct DqSmem {
+  static constexpr int Q = 0, K = Q + DC_C * DC_QS * 2, DO = K + DC_C * DC_QS * 2;
+  static constexpr int S = DO + DC_C * DC_QS * 2;                    // dx, then S, then dS
+  static constexpr int X = S + DC_D * DQ_LD * 4, DB = X + DC_C * DQ_LD * 4;
+  static constexpr int P = DB + DC_C * DQ_LD * 4, R = P + DC_C * DQ_P * 4;
+  static constexpr int ROWS = R + DC_C * DQ_P * 4;                   // G, beta, 1/|k|, scale/|q|, e^G, e^(Gl-G), beta/|k|
+  static constexpr int PART = P;                                     // [6][4][64] row sums per column quarter (after P, R)
+  static constexpr int RED = ROWS + 7 * DC_C * 4;
+  static constexpr int TOTAL = RED + 32 * 4;
+};
+static_assert(DqSmem::TOTAL <= 232448, "one CTA per SM");
+
+__global__ void __launch_bounds__(512, 1)
+delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO, const float* __restrict__ Tg,
+                      const float* __restrict__ X, const float* __restrict__ dX, const float* __restrict__ St,
+                      const float* __restrict__ dSt, int nseq, __nv_bfloat16* __restrict__ dQ, __nv_bfloat16* __restrict__ dK,
+                      __nv_bfloat16* __restrict__ dV, float* __restrict__ dG, float* __restrict__ dBeta) {
+  constexpr int NT = 512;
+  extern __shared__ __align__(16) uint8_t sm[];
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::Q);
+  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::K);
+  __nv_bfloat16* sDO = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::DO);
+  float* sS = reinterpret_cast<float*>(sm + DqSmem::S);
+  float* sX = reinterpret_cast<float*>(sm + DqSmem::X);
+  float* sDB = reinterpret_cast<float*>(sm + DqSmem::DB);
+  float* sP = reinterpret_cast<float*>(sm + DqSmem::P);
+  float* sR = reinterpret_cast<float*>(sm + DqSmem::R);
+  float* sPart = reinterpret_cast<float*>(sm + DqSmem::PART);
+  float* sG = reinterpret_cast<float*>(sm + DqSmem::ROWS);
+  float *sB = sG + DC_C, *sRk = sB + DC_C, *sRq = sRk + DC_C, *sE = sRq + DC_C, *sL = sE + DC_C, *sBk = sL + DC_C;
+  float* sRed = reinterpret_cast<float*>(sm + DqSmem::RED);
+  const int c = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int row0 = p.chunk_rows[3 * c], n = p.chunk_rows[3 * c + 1], slot = c + p.chunk_rows[3 * c + 2];
+  const long long hc = static_cast<long long>(h) * p.NC + c;
+  const long long st_at = ((static_cast<long long>(h) * (p.NC + nseq) + slot) * DC_D) * DC_D;
+
+  dc_load_f32<NT, DC_C, DC_D>(sS, DQ_DX, dX + hc * DC_C * DC_D, DC_D);
+  dc_load_f32<NT, DC_C, 64>(sP, DQ_P, Tg + hc * DC_C * DC_C, DC_C);
+  dc_load_rows<NT>(sQ, p.q + row0 * p.q_t + h * p.q_h, p.q_t, n);
+  dc_load_rows<NT>(sK, p.k + row0 * p.k_t + h * p.k_h, p.k_t, n);
+  dc_load_rows<NT>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
+  dc_load_f32<NT, DC_C, DC_D>(sX, DQ_LD, X + hc * DC_C * DC_D, DC_D);
+  dc_load_gates(p, row0, n, h, sG, sB);
+  __syncthreads();
+  dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
+  dc_row_norms<NT>(sK, sRk, p.l2, 1.f);
+  if (warp == 0) dc_cumsum(sG, lane);
+  __syncthreads();
+  if (tid < DC_C) {
+    sE[tid] = dc_exp(sG[tid]);
+    sL[tid] = dc_exp(sG[DC_C - 1] - sG[tid]);
+    sBk[tid] = sB[tid] * sRk[tid];
+  }
+  // warp tile: 16 rows x 32 columns
+  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int i0 = m0 + g, i1 = i0 + 8;
+  // sums over a row's 128 channels: four lanes, then four warps (added in a fixed order at the end)
+  float part[6][2];
+#pragma unroll
+  for (int x = 0; x < 6; ++x) part[x][0] = part[x][1] = 0.f;
+  // ---- db = T^T dx; dv = beta db
+  {
+    float acc[4][4] = {};
+    for (int kk = mi; kk < 4; ++kk) {
+      uint32_t a[2][4];
+      dc_af_t<2>(a, sP, DQ_P, m0, kk * 16, lane);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        uint32_t b[2][2];
+        dc_bf_t<2>(b, sS, DQ_DX, n0 + nt * 8, kk * 16, lane);
+        dc_mma22(acc[nt], a[0], a[1], b[0], b[1]);
+      }
+    }
+    const float be0 = sB[i0], be1 = sB[i1];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int col = n0 + nt * 8 + t2;
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int i = rr ? i1 : i0;
+        const float x = acc[nt][2 * rr], y = acc[nt][2 * rr + 1], be = rr ? be1 : be0;
+        *reinterpret_cast<float2*>(sDB + i * DQ_LD + col) = make_float2(x, y);
+        if (i < n) {
+          const float2 v = unpack_bf16(__ldg(reinterpret_cast<const uint32_t*>(p.v + (row0 + i) * p.v_t + h * p.v_h + col)));
+          part[0][rr] += x * v.x + y * v.y;
+          *reinterpret_cast<uint32_t*>(dV + (static_cast<long long>(row0 + i) * p.H + h) * DC_D + col) = pack_bf16(x * be, y * be);
+        }
+      }
+    }
+  }
+  __syncthreads();                               // db is complete, dx and T are no longer read
+  dc_load_f32<NT, DC_D, DC_D>(sS, DQ_LD, St + st_at, DC_D);
+  // ---- P = dL . D with dL = -strict_lower(db x^T), R = dA . D with dA = lower(do x^T); 16 x 16 per warp
+  {
+    float accP[2][4] = {}, accR[2][4] = {};
+    if (cq <= mi) {
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        uint32_t ad[4], ab[2][4];
+        dc_a(ad, sDO, m0, kk * 16, lane);
+        dc_af<2>(ab, sDB, DQ_LD, m0, kk * 16, lane);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          uint32_t b[3][2];
+          dc_bf<3>(b, sX, DQ_LD, cq * 16 + nt * 8, kk * 16, lane);
+#pragma unroll
+          for (int i = 2; i >= 0; --i) dc_mma(accR[nt], ad, b[i][0], b[i][1]);
+          dc_mma22(accP[nt], ab[0], ab[1], b[0], b[1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int i = rr ? i1 : i0, j = cq * 16 + nt * 8 + t2;
+        float2 pv = make_float2(0.f, 0.f), rv = make_float2(0.f, 0.f);
+        if (j <= i) {
+          const float d = dc_exp(sG[i] - sG[j]);
+          rv.x = accR[nt][2 * rr] * d;
+          if (j < i) pv.x = -accP[nt][2 * rr] * d;
+        }
+        if (j + 1 <= i) {
+          const float d = dc_exp(sG[i] - sG[j + 1]);
+          rv.y = accR[nt][2 * rr + 1] * d;
+          if (j + 1 < i) pv.y = -accP[nt][2 * rr + 1] * d;
+        }
+        *reinterpret_cast<float2*>(sP + i * DQ_P + j) = pv;
+        *reinterpret_cast<float2*>(sR + i * DQ_P + j) = rv;
+      }
+    }
+  }
+  __syncthreads();                               // S, P and R are complete
+  // ---- d(q^ e^G) = do S^T, d(beta k^ e^G) = -db S^T, then the score terms R k^, P k^ on the same accumulators
+  float dq[4][4] = {}, dk[4][4] = {};
+#pragma unroll 2
+  for (int kk = 0; kk < 8; ++kk) {
+    uint32_t ad[4], ab[2][4];
+    dc_a(ad, sDO, m0, kk * 16, lane);
+    dc_af<2>(ab, sDB, DQ_LD, m0, kk * 16, lane);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      uint32_t b[3][2];
+      dc_bf<3>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
+#pragma unroll
+      for (int i = 2; i >= 0; --i) dc_mma(dq[nt], ad, b[i][0], b[i][1]);
+      dc_mma22(dk[nt], ab[0], ab[1], b[0], b[1]);
+    }
+  }
+  // the gradient of the chunk's end state is fetched while the score terms run
+  float4 ds[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) ds[e] = __ldg(reinterpret_cast<const float4*>(dSt + st_at + DC_D * DC_D) + tid + e * NT);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float e = sE[x < 2 ? i0 : i1];
+      dq[nt][x] *= e;
+      dk[nt][x] *= -e;
+    }
+  }
+  for (int kk = 0; kk <= mi; ++kk) {
+    uint32_t ar[3][4], ap[3][4];
+    dc_af<3>(ar, sR, DQ_P, m0, kk * 16, lane, sRk);
+    dc_af<3>(ap, sP, DQ_P, m0, kk * 16, lane, sRk);
+#pragma unroll
+    for (int np = 0; np < 2; ++np) {
+      uint32_t b[4];
+      dc_b_t(b, sK, n0 + np * 16, kk * 16, lane);
+#pragma unroll
+      for (int i = 2; i >= 0; --i) {
+        dc_mma(dq[2 * np], ar[i], b[0], b[1]);
+        dc_mma(dq[2 * np + 1], ar[i], b[2], b[3]);
+        dc_mma(dk[2 * np], ap[i], b[0], b[1]);
+        dc_mma(dk[2 * np + 1], ap[i], b[2], b[3]);
+      }
+    }
+  }
+  uint32_t kv[4][2];                             // this thread's k values (bf16 pairs)
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const int at = (rr ? i1 : i0) * DC_QS + n0 + nt * 8 + t2;
+      kv[nt][rr] = *reinterpret_cast<const uint32_t*>(sK + at);
+      const float2 kf = unpack_bf16(kv[nt][rr]), qf = unpack_bf16(*reinterpret_cast<const uint32_t*>(sQ + at));
+      part[1][rr] += qf.x * dq[nt][2 * rr] + qf.y * dq[nt][2 * rr + 1];
+      part[2][rr] += kf.x * dk[nt][2 * rr] + kf.y * dk[nt][2 * rr + 1];
+      const float be = sB[rr ? i1 : i0];
+      dk[nt][2 * rr] *= be;
+      dk[nt][2 * rr + 1] *= be;
+    }
+  }
+  // ---- k in the role of the earlier row: P^T (beta k^) + R^T q^
+  {
+    float acc[4][4] = {};
+    for (int kk = mi; kk < 4; ++kk) {
+      uint32_t ar[3][4], ap[3][4];
+      dc_af_t<3>(ar, sR, DQ_P, m0, kk * 16, lane, sRq);
+      dc_af_t<3>(ap, sP, DQ_P, m0, kk * 16, lane, sBk);
+#pragma unroll
+      for (int np = 0; np < 2; ++np) {
+        uint32_t bk[4], bq[4];
+        dc_b_t(bk, sK, n0 + np * 16, kk * 16, lane);
+        dc_b_t(bq, sQ, n0 + np * 16, kk * 16, lane);
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          dc_mma(acc[2 * np], ap[i], bk[0], bk[1]);
+          dc_mma(acc[2 * np + 1], ap[i], bk[2], bk[3]);
+          dc_mma(acc[2 * np], ar[i], bq[0], bq[1]);
+          dc_mma(acc[2 * np + 1], ar[i], bq[2], bq[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const float2 kf = unpack_bf16(kv[nt][rr]);
+        part[3][rr] += kf.x * acc[nt][2 * rr] + kf.y * acc[nt][2 * rr + 1];
+        dk[nt][2 * rr] += acc[nt][2 * rr];
+        dk[nt][2 * rr + 1] += acc[nt][2 * rr + 1];
+      }
+  }
+  __syncthreads();                               // S is no longer read
+  float dot = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {                  // <dS, S> on the way in
+    const int f = tid + e * NT, r = f >> 5, col = (f & 31) * 4;
+    float4* at = reinterpret_cast<float4*>(sS + r * DQ_LD + col);
+    const float4 s = *at;
+    dot += s.x * ds[e].x + s.y * ds[e].y + s.z * ds[e].z + s.w * ds[e].w;
+    *at = ds[e];
+  }
+  dot = warp_sum(dot);
+  if (lane == 0) sRed[warp] = dot;
+  __syncthreads();
+  // ---- d(k_out) = x dS^T
+  {
+    float acc[4][4] = {};
+#pragma unroll 2
+    for (int kk = 0; kk < 8; ++kk) {
+      uint32_t a[2][4];
+      dc_af<2>(a, sX, DQ_LD, m0, kk * 16, lane);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        uint32_t b[2][2];
+        dc_bf<2>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
+        dc_mma22(acc[nt], a[0], a[1], b[0], b[1]);
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const float2 kf = unpack_bf16(kv[nt][rr]);
+        const float e = sL[rr ? i1 : i0], x = acc[nt][2 * rr] * e, y = acc[nt][2 * rr + 1] * e;
+        part[4][rr] += kf.x * x + kf.y * y;
+        dk[nt][2 * rr] += x;
+        dk[nt][2 * rr + 1] += y;
+        part[5][rr] += kf.x * dk[nt][2 * rr] + kf.y * dk[nt][2 * rr + 1];
+      }
+  }
+  // (P and R were last read before the two barriers above: their space takes the row sums)
+#pragma unroll
+  for (int x = 0; x < 6; ++x)
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      float v = part[x][rr];
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      if ((lane & 3) == 0) sPart[(x * 4 + cq) * DC_C + (rr ? i1 : i0)] = v;
+    }
+  __syncthreads();
+  auto row_sum = [&](int x, int i) {
+    const float* a = sPart + x * 4 * DC_C + i;
+    return (a[0] + a[DC_C]) + (a[2 * DC_C] + a[3 * DC_C]);
+  };
+#pragma unroll
+  for (int rr = 0; rr < 2; ++rr) {
+    const int i = rr ? i1 : i0;
+    if (i >= n) continue;
+    const float rk = sRk[i], rq = sRq[i], r0 = rq / p.scale;     // 1/|k|, scale/|q|, 1/|q|
+    const float tq = p.l2 ? r0 * r0 * row_sum(1, i) : 0.f, tk = p.l2 ? rk * rk * row_sum(5, i) : 0.f;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int col = n0 + nt * 8 + t2;
+      const long long at = (static_cast<long long>(row0 + i) * p.H + h) * DC_D + col;
+      const float2 kf = unpack_bf16(kv[nt][rr]), qf = unpack_bf16(*reinterpret_cast<const uint32_t*>(sQ + i * DC_QS + col));
+      *reinterpret_cast<uint32_t*>(dQ + at) = pack_bf16(rq * (dq[nt][2 * rr] - qf.x * tq), rq * (dq[nt][2 * rr + 1] - qf.y * tq));
+      *reinterpret_cast<uint32_t*>(dK + at) = pack_bf16(rk * (dk[nt][2 * rr] - kf.x * tk), rk * (dk[nt][2 * rr + 1] - kf.y * tk));
+    }
+  }
+  // ---- gates: dG_i = kb.dkb + q^.dq^ - k^.(score + out terms); the chunk's last G also carries e^(G_last - G) and decay
+  if (warp < 2) {
+    const int i = tid;
+    const float kb = row_sum(2, i) * sRk[i], out = row_sum(4, i) * sRk[i];
+    sPart[24 * DC_C + i] = sB[i] * kb + row_sum(1, i) * sRq[i] - row_sum(3, i) * sRk[i] - out;
+    sPart[25 * DC_C + i] = out;
+    if (i < n) dBeta[static_cast<long long>(row0 + i) * p.H + h] = row_sum(0, i) + kb;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float total = 0.f;
+    if (lane < 16) total = sRed[lane];
+    total = warp_sum(total) * sE[DC_C - 1];
+    total += warp_sum(sPart[25 * DC_C + lane] + sPart[25 * DC_C + 32 + lane]);
+    const float a = sPart[24 * DC_C + 2 * lane], b = sPart[24 * DC_C + 2 * lane + 1];
+    float run = a + b;                           // sum from this pair to the chunk's end
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float dn = __shfl_down_sync(0xffffffffu, run, o);
+      if (lane + o < 32) run += dn;
+    }
+    if (2 * lane < n) dG[static_cast<long long>(row0 + 2 * lane) * p.H + h] = run + total;
+    if (2 * lane + 1 < n) dG[static_cast<long long>(row0 + 2 * lane + 1) * p.H + h] = run - a + total;
+  }
+}
+
+}  // namespace ttb
+
+using namespace ttb;
+
+// T, A: fp32 [H, NC, 64, 64]; U: fp32 [H, NC, 64, 128]; W, K_out: bf16 [H, NC, 64, 128]; decay: fp32 [H, NC]
+TTB_EXPORT int ttb_delta_prep(const DeltaChunkIn* in, float* T, float* A, float* U, void* W, void* Ko, float* decay, void* stream) {
+  if (dc_bad(*in)) return 921;
+  static bool done[16] = {};
+  if (int e = dc_ready(delta_prep_kernel, DpSmem::TOTAL, done)) return e;
+  delta_prep_kernel<<<dim3(in->NC, in->H), 256, DpSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
+      *in, T, A, U, reinterpret_cast<__nv_bfloat16*>(W), reinterpret_cast<__nv_bfloat16*>(Ko), decay);
+  return dc_launched();
+}
+
+// X: fp32 [H, NC, 64, 128]; states: fp32 [H, NC + nseq, 128, 128]; O: bf16 [rows, H, 128]
+TTB_EXPORT int ttb_delta_out(const DeltaChunkIn* in, const float* A, const float* X, const float* states, int nseq, void* O, void* stream) {
+  if (dc_bad(*in)) return 921;
+  static bool done[16] = {};
+  if (int e = dc_ready(delta_out_kernel, DoSmem::TOTAL, done)) return e;
+  delta_out_kernel<<<dim3(in->NC, in->H, 2), 256, DoSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
+      *in, A, X, states, nseq, reinterpret_cast<__nv_bfloat16*>(O));
+  return dc_launched();
+}
+
+// dO: bf16 [rows, H, 128] contiguous; GX like X; GS like states (only the slots of chunk starts are written)
+TTB_EXPORT int ttb_delta_bwd_pre(const DeltaChunkIn* in, const void* dO, const float* A, int nseq, float* GX, float* GS, void* stream) {
+  if (dc_bad(*in) || (reinterpret_cast<uintptr_t>(dO) & 15)) return 921;
+  static bool done[16] = {};
+  if (int e = dc_ready(delta_bwd_pre_kernel, DbSmem::TOTAL, done)) return e;
+  delta_bwd_pre_kernel<<<dim3(in->NC, in->H), 256, DbSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
+      *in, reinterpret_cast<const __nv_bfloat16*>(dO), A, nseq, GX, GS);
+  return dc_launched();
+}
+
+// dQ, dK, dV: bf16 [rows, H, 128]; dG, dBeta: fp32 [rows, H]
+TTB_EXPORT int ttb_delta_bwd_post(const DeltaChunkIn* in, const void* dO, const float* T, const float* X, const float* dX,
+                                  const float* states, const float* dstates, int nseq, void* dQ, void* dK, void* dV, float* dG,
+                                  float* dBeta, void* stream) {
+  if (dc_bad(*in) || (reinterpret_cast<uintptr_t>(dO) & 15)) return 921;
+  static bool done[16] = {};
+  if (int e = dc_ready(delta_bwd_post_kernel, DqSmem::TOTAL, done)) return e;
+  delta_bwd_post_kernel<<<dim3(in->NC, in->H), 512, DqSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
+      *in, reinterpret_cast<const __nv_bfloat16*>(dO), T, X, dX, states, dstates, nseq, reinterpret_cast<__nv_bfloat16*>(dQ),
+      reinterpret_cast<__nv_bfloat16*>(dK), reinterpret_cast<__nv_bfloat16*>(dV), dG, dBeta);
+  return dc_launched();
+}

@@ -100,7 +100,7 @@ def lib():
 # kernels launched per C entry point (used to report how many of this library's kernels ran in a region)
 _LAUNCHES_PER_CALL = {"ttb_rmsnorm_bwd": 2, "ttb_layernorm_bwd": 2, "ttb_bias_act_bwd": 2, "ttb_causal_conv1d_bwd": 3,
                       "ttb_causal_conv1d_row_blocks": 0, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
-                      "ttb_ep_combine_all": 3, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
+                      "ttb_ep_combine_all": 3, "ttb_delta_vec_bwd_post": 2, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
                       "ttb_gemm_status": 0}
 LAUNCH_COUNT = 0
 
@@ -689,6 +689,79 @@ def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, r
                                       C.c_int(NC), C.c_int(int(reverse)), C.c_float(s1), C.c_float(s2), _stream()),
            "ttb_delta_state_scan")
     return x, states
+
+
+class _DeltaChunkIn(C.Structure):
+    """`struct DeltaChunkIn` of csrc/delta_chunk.cu."""
+
+    _fields_ = [("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p),
+                ("q_t", C.c_longlong), ("q_h", C.c_longlong), ("k_t", C.c_longlong), ("k_h", C.c_longlong),
+                ("v_t", C.c_longlong), ("v_h", C.c_longlong),
+                ("g", C.c_void_p), ("beta", C.c_void_p), ("chunk_rows", C.c_void_p),
+                ("H", C.c_int), ("NC", C.c_int), ("l2", C.c_int), ("scale", C.c_float)]
+
+
+def _delta_in(q, k, v, g, beta, chunk_rows, l2: bool, scale: float) -> _DeltaChunkIn:
+    """q, k, v: bf16 [rows, H, 128] (any row / head stride that keeps 16-byte alignment); g: fp32 [rows, H]
+    or [rows, H, 128] (one decay per head, or per head and channel); beta: fp32 [rows, H]; chunk_rows: int32 [NC, 3] on the device (first row, number of rows, sequence of every chunk)."""
+    R, H, D = q.shape
+    check_device(q)
+    for t in (q, k, v):
+        assert t.dtype == torch.bfloat16 and t.shape == (R, H, 128) and t.stride(2) == 1
+    assert g.dtype == torch.float32 and g.shape in ((R, H), (R, H, 128)) and g.is_contiguous()
+    assert beta.dtype == torch.float32 and beta.shape == (R, H) and beta.is_contiguous()
+    assert chunk_rows.dtype == torch.int32 and chunk_rows.is_contiguous() and chunk_rows.shape[1] == 3
+    return _DeltaChunkIn(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0), k.stride(1),
+                         v.stride(0), v.stride(1), g.data_ptr(), beta.data_ptr(), chunk_rows.data_ptr(), H,
+                         chunk_rows.shape[0], int(l2), scale)
+
+
+def _delta_call(step: str, g, *args) -> None:
+    name = f"ttb_delta_{'vec_' if g.dim() == 3 else ''}{step}"
+    _check(getattr(lib(), name)(*args), name)
+
+
+def delta_prep(q, k, v, g, beta, chunk_rows, *, l2: bool, scale: float):
+    """Chunk-parallel operands of the gated delta rule (csrc/delta_chunk.cu).  Returns (T, A fp32 [H, NC, 64, 64],
+    u fp32 [H, NC, 64, 128], w, k_out bf16 [H, NC, 64, 128], decay fp32 [H, NC] or [H, NC, 128])."""
+    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
+    H, NC, dev = a.H, a.NC, q.device
+    tri = torch.empty(2, H, NC, 64, 64, dtype=torch.float32, device=dev)
+    u = torch.empty(H, NC, 64, 128, dtype=torch.float32, device=dev)
+    wk = torch.empty(2, H, NC, 64, 128, dtype=torch.bfloat16, device=dev)
+    decay = torch.empty(H, NC, *g.shape[2:], dtype=torch.float32, device=dev)
+    _delta_call("prep", g, C.byref(a), _p(tri[0]), _p(tri[1]), _p(u), _p(wk[0]), _p(wk[1]), _p(decay), _stream())
+    return tri[0], tri[1], u, wk[0], wk[1], decay
+
+
+def delta_out(q, k, v, g, beta, chunk_rows, A, x, states, *, l2: bool, scale: float):
+    """o bf16 [rows, H, 128] from the new values `x` and the chunk-start states of the recurrence."""
+    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
+    o = torch.empty(q.shape, dtype=torch.bfloat16, device=q.device)
+    _delta_call("out", g, C.byref(a), _p(A), _p(x), _p(states), C.c_int(states.shape[1] - a.NC), _p(o), _stream())
+    return o
+
+
+def delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq: int, *, l2: bool, scale: float):
+    """Gradients that reach the recurrence directly: (gx like x, gS [H, NC + nseq, 128, 128]; the slots behind the last
+    chunk of a sequence are left to the caller)."""
+    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
+    assert do.is_contiguous() and do.dtype == torch.bfloat16 and do.shape == q.shape
+    gx = torch.empty(a.H, a.NC, 64, 128, dtype=torch.float32, device=q.device)
+    gs = torch.empty(a.H, a.NC + nseq, 128, 128, dtype=torch.float32, device=q.device)
+    _delta_call("bwd_pre", g, C.byref(a), _p(do), _p(A), C.c_int(nseq), _p(gx), _p(gs), _stream())
+    return gx, gs
+
+
+def delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, *, l2: bool, scale: float):
+    """(dq, dk, dv bf16 [rows, H, 128], dg like g, dbeta fp32 [rows, H])."""
+    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
+    dq, dk, dv = (torch.empty(q.shape, dtype=torch.bfloat16, device=q.device) for _ in range(3))
+    dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
+    scratch = [_p(torch.empty(4, *x.shape, dtype=torch.float32, device=q.device))] if g.dim() == 3 else []
+    _delta_call("bwd_post", g, C.byref(a), _p(do), _p(T), _p(x), _p(dx), _p(states), _p(dstates), C.c_int(states.shape[1] - a.NC),
+                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta), *scratch, _stream())
+    return dq, dk, dv, dg, dbeta
 
 
 # --------------------------------------------------------------------------------------

@@ -11,6 +11,10 @@ The chunked evaluation splits into work that is parallel over chunks and one rec
   chunk-parallel again:
       o_c = q_in_c S_c + tril(q k^T . D) v_new_c
 
+On bf16 rows with 128-wide heads the chunk-parallel work runs in fused kernels, one CTA per chunk and head (`ChunkDelta`,
+csrc/delta_chunk.cu and csrc/delta_chunk_vec.cu).  Everything else (fp32 rows, other widths, boundaries that leave rows
+uncovered, CPU) takes the formulation below out of torch operations:
+
 `StateScan` is the autograd function around the recurrence: its backward is the same kernel run over the chunks in
 reverse (dS_c = d_c (.) dS_{c+1} - w_c^T dv_new_c + gS_c, dv_new_c = g_c + k_out_c dS_{c+1}) followed by batched products
 for the operand gradients; everything chunk-parallel is differentiated by autograd.  Without CUDA (or for head
@@ -100,6 +104,78 @@ class StateScan(torch.autograd.Function):
         return dx, dw.to(ctx.w_dtype), dk_out.to(ctx.k_dtype), ddecay, dinit, None, None
 
 
+class ChunkDelta(torch.autograd.Function):
+    """(Gated) delta rule on bf16 rows: a few kernels around the recurrence instead of batched fp32
+    products over materialised chunk tensors.  q, k, v [rows, H, 128]; g fp32 [rows, H] or [rows, H, 128]; beta fp32 [rows, H]; init [H, nseq, 128, 128]
+    or None; `tables` = (seq_chunks, chunk_rows, last slots, first slots) on the device."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2):
+        seq, chunk_rows, last, first = tables
+        kw = dict(l2=l2, scale=scale)
+        T, A, u, w, k_out, decay = K.delta_prep(q, k, v, g, beta, chunk_rows, **kw)
+        x, states = K.delta_state_scan(w, k_out, u, decay, init, None, seq, reverse=False, s1=-1.0, s2=1.0)
+        o = K.delta_out(q, k, v, g, beta, chunk_rows, A, x, states, **kw)
+        ctx.save_for_backward(q, k, v, g, beta, T, A, w, k_out, decay, x, states, seq, chunk_rows, last, first)
+        ctx.meta = (kw, init is not None)
+        ctx.set_materialize_grads(False)
+        return o, states.index_select(1, last)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, do, dfinal):
+        q, k, v, g, beta, T, A, w, k_out, decay, x, states, seq, chunk_rows, last, first = ctx.saved_tensors
+        kw, has_init = ctx.meta
+        do = do.contiguous() if do is not None else torch.zeros(q.shape, dtype=q.dtype, device=q.device)
+        gx, gs = K.delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, seq.shape[0], **kw)
+        if dfinal is None:
+            gs.index_fill_(1, last, 0.0)
+        else:
+            gs.index_copy_(1, last, dfinal.contiguous())
+        dx, ds = K.delta_state_scan(k_out, w, gx, decay, None, gs, seq, reverse=True, s1=1.0, s2=-1.0)
+        dq, dk, dv, dg, dbeta = K.delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, ds, **kw)
+        return dq, dk, dv, dg, dbeta, (ds.index_select(1, first) if has_init else None), None, None, None
+
+
+def _rows_for_kernel(t: torch.Tensor, R: int) -> torch.Tensor:
+    """[B, T, H, 128] -> [rows, H, 128]; copied only where a row would not start on a 16-byte boundary."""
+    t = t.reshape(R, *t.shape[2:])
+    if t.stride(2) != 1 or t.stride(0) % 8 or t.stride(1) % 8 or t.data_ptr() % 16:
+        t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+def _chunk_tables(segs, C: int, device):
+    """Device tables of the chunked layout, sent in one copy: per sequence (first chunk, chunks), per chunk (first row, rows,
+    sequence), and the state slots behind the last / before the first chunk of every sequence."""
+    seq, rows, last, first, c = [], [], [], [], 0
+    for s, (base, a, b) in enumerate(segs):
+        n = (b - a + C - 1) // C
+        seq += [c, n]
+        for r in range(a, b, C):
+            rows += [base + r, min(C, b - r), s]
+        first.append(c + s)
+        c += n
+        last.append(c + s)
+    nseq = len(segs)
+    host = torch.tensor(seq + rows + last + first, dtype=torch.int32).pin_memory()
+    dev = host.to(device, non_blocking=True)
+    seq_d, rows_d, slots_d = dev.split([2 * nseq, 3 * c, 2 * nseq])
+    last_d, first_d = slots_d.long().split(nseq)
+    return seq_d.view(nseq, 2), rows_d.view(c, 3), last_d, first_d
+
+
+def _fused_usable(q, k, v, g, beta, segs, scale) -> bool:
+    """The fused kernels take bf16 q / k / v of 128-wide heads and sequences that cover every row (fp32 rows would lose
+    mantissa bits as tensor-core operands; they keep the batched fp32 products)."""
+    R = q.shape[0] * q.shape[1]
+    return (_kernel_ok(q, q.shape[-1], v.shape[-1]) and all(t.dtype == torch.bfloat16 and t.is_cuda for t in (q, k, v))
+            and k.shape == q.shape and v.shape == q.shape and g.shape in (q.shape, q.shape[:3])
+            and beta.shape == q.shape[:3] and scale != 0
+            and 0 < q.shape[2] <= 65535 and R > 0 and sum(b - a for _, a, b in segs) == R
+            and all(0 <= a <= b <= q.shape[1] for _, a, b in segs))
+
+
 def _layout(segs, T_total: int, C: int, device):
     """Gather / scatter indices between packed tokens and the zero-padded `[chunk, C]` layout."""
     gather, seq_chunks, inv = [], [], torch.full((T_total,), -1, dtype=torch.long)
@@ -162,12 +238,19 @@ def chunk_delta_rule_batched(q, k, v, g, beta, scale=None, initial_state=None, o
     dev = q.device
     C = CHUNK
     scale = Kd ** -0.5 if scale is None else scale
-    qf, kf, vf, gf, bf = (t.float() for t in (q, k, v, g, beta))
-    if use_qk_l2norm:
-        qf, kf = l2norm(qf), l2norm(kf)
     if cu_seqlens is not None and B != 1:
         raise ValueError("packed delta rule expects a single row")
     segs = [(0, a, b) for a, b in _bounds(cu_seqlens, T)] if cu_seqlens is not None else [(r * T, 0, T) for r in range(B)]
+    if _fused_usable(q, k, v, g, beta, segs, scale):
+        R = B * T
+        tables = _chunk_tables(segs, C, dev)
+        init = initial_state.float().transpose(0, 1).contiguous() if initial_state is not None else None
+        o, final = ChunkDelta.apply(*(_rows_for_kernel(t, R) for t in (q, k, v)), g.float().reshape(R, *g.shape[2:]).contiguous(),
+                                    beta.float().reshape(R, H).contiguous(), init, tables, float(scale), bool(use_qk_l2norm))
+        return o.view(B, T, H, V), (final.transpose(0, 1).contiguous() if output_final_state else None)
+    qf, kf, vf, gf, bf = (t.float() for t in (q, k, v, g, beta))
+    if use_qk_l2norm:
+        qf, kf = l2norm(qf), l2norm(kf)
     vec = gf.dim() == 4
     # sequences that are whole chunks and tile the rows need no gather: the chunk layout is a view of the packed rows
     aligned = all((b - a) % C == 0 for _, a, b in segs) and sum(b - a for _, a, b in segs) == B * T
