@@ -10,11 +10,15 @@
 //     dS     <- d_c (.) dS - w_c^T dX_c + GS_c   (s2 = -1, B = w, GS = gradient that reaches the chunk's start state)
 // so one kernel runs both directions.  d_c is a scalar per chunk (GatedDeltaNet) or a vector over K (KDA).
 //
-// One CTA owns one (sequence, head).  The state lives transposed in registers, one thread per value column v holding
-// its 128 K-entries in fp32 (TMEM lane = v), and as a bf16 K-major tile in shared memory for the tensor cores:
+// One CTA owns one (sequence, head).  The state lives transposed in registers, two threads per value column v holding
+// 64 of its 128 K-entries each in fp32 (TMEM lane = v), and as a bf16 K-major tile in shared memory for the tensor cores:
 //     acc1 [V, 64]  = S^T  A_c^T       tcgen05, M = 128, N = 64   (K-major x K-major)
 //     acc2 [V, 128] = X^T  B_c         tcgen05, M = 128, N = 128  (K-major x MN-major)
-// Warp roles: 0 TMA producer (A_c / B_c tiles, two stages), 1 MMA issuer, 2-5 state warps.  Every wait is bounded; on a
+// Warp roles: 0 TMA producer (A_c / B_c tiles, two stages), 1 MMA issuer, 2-9 state warps: warps 2-5 take K-entries 0-63
+// and tokens 0-31, warps 6-9 the others.  A chunk is a chain of two small products with 160 - 224 KB of states and rows
+// moved around it, so what counts is how much of that traffic is off the chain: the added gradient and the next chunk's U
+// are requested while the products run, and eight warps share the loads and stores (four documents of 16 chunks on average x 32 heads, both directions: 394 us with four
+// state warps that fetched everything on the chain, 309 now).  Every wait is bounded; on a
 // timeout the roles drain to the final barrier, TMEM is freed and the status word records kernel / site.
 //
 // Counterpart of the `chunk_gated_delta_rule` / `chunk_kda` operators that the reference takes from
@@ -26,6 +30,7 @@ namespace ttb {
 constexpr unsigned KID_DELTA_STATE = 9;
 constexpr int DS_C = 64;     // tokens per chunk
 constexpr int DS_D = 128;    // K = V = 128
+constexpr int DS_THREADS = 64 + 256;
 
 struct DeltaStateParams {
   const float* U;        // [H, NC, 64, 128]
@@ -50,7 +55,7 @@ struct DsSmem {
   static constexpr int TOTAL = BARS + 256 + 1024;
 };
 
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(DS_THREADS, 1)
 delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const DeltaStateParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -75,9 +80,9 @@ delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&ab_full[i], 1); mbar_init(&ab_empty[i], 1); }
-    mbar_init(st_ready, 4);
+    mbar_init(st_ready, 8);
     mbar_init(acc1_full, 1);
-    mbar_init(x_ready, 4);
+    mbar_init(x_ready, 8);
     mbar_init(acc2_full, 1);
     *s_dead = 0;
     mbar_fence_init();
@@ -142,114 +147,115 @@ delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       }
     }
   } else {
-    // ---------------------------------------------------------------- state warps (thread = value column v)
-    const int lg = warp & 3;
-    const int v = lg * 32 + lane;
+    // ---------------------------------------------------------------- state warps (two threads per value column v)
+    const int lg = warp & 3, half = (warp - 2) >> 2;
+    const int v = lg * 32 + lane, k0 = half * 64, t0 = half * 32;   // this thread's K-entries and tokens
     const uint32_t lane_off = static_cast<uint32_t>(lg * 32) << 16;
     const int tid = threadIdx.x - 64;
-    float S[DS_D];
-    uint8_t* sST = smem + DsSmem::ST;
+    float S[64], u[32], av[64];
+    uint8_t* sST = smem + DsSmem::ST + half * 16384;
     uint8_t* sXT = smem + DsSmem::XT;
-    auto state_ptr = [&](const float* base, int slot) {
-      return base + ((static_cast<long long>(h) * slots + slot) * DS_D) * DS_D + v;
-    };
-    // S^T row v -> bf16 K-major tile (two 64-wide panels, 128-byte swizzle)
+    auto state_at = [&](int slot) { return ((static_cast<long long>(h) * slots + slot) * DS_D + k0) * DS_D + v; };
+    // this half of row v of S^T -> bf16 K-major panel (128-byte swizzle)
     auto publish = [&]() {
 #pragma unroll
-      for (int ch = 0; ch < 16; ++ch) {
+      for (int ch = 0; ch < 8; ++ch) {
         uint4 w;
         w.x = pack_bf16(S[ch * 8 + 0], S[ch * 8 + 1]); w.y = pack_bf16(S[ch * 8 + 2], S[ch * 8 + 3]);
         w.z = pack_bf16(S[ch * 8 + 4], S[ch * 8 + 5]); w.w = pack_bf16(S[ch * 8 + 6], S[ch * 8 + 7]);
-        *reinterpret_cast<uint4*>(sST + (ch >> 3) * 16384 + v * 128 + (((ch & 7) ^ (v & 7)) * 16)) = w;
+        *reinterpret_cast<uint4*>(sST + v * 128 + ((ch ^ (v & 7)) * 16)) = w;
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(st_ready);
     };
+    auto row_at = [&](int i) { return ((static_cast<long long>(h) * p.NC + chunk_of(i)) * DS_C + t0) * DS_D + v; };
+    auto fetch_u = [&](int i) {
+      const float* src = p.U + row_at(i);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) u[j] = __ldg(src + j * DS_D);
+    };
     // initial state, also recorded in the slot that precedes the first processed chunk
     {
       const int slot0 = (p.reverse ? c0 + n : c0) + seq;
-      const float* src = p.reverse ? (p.add ? state_ptr(p.add, slot0) : nullptr)
-                                   : (p.init ? p.init + ((static_cast<long long>(h) * p.nseq + seq) * DS_D) * DS_D + v : nullptr);
-      float* dst = const_cast<float*>(state_ptr(p.states, slot0));
-      // all loads before the first store: the compiler may not move a load above a store that could alias it
+      const float* src = p.reverse ? (p.add ? p.add + state_at(slot0) : nullptr)
+                                   : (p.init ? p.init + ((static_cast<long long>(h) * p.nseq + seq) * DS_D + k0) * DS_D + v : nullptr);
+      float* dst = p.states + state_at(slot0);
 #pragma unroll
-      for (int k = 0; k < DS_D; ++k) S[k] = src ? src[k * DS_D] : 0.f;
+      for (int k = 0; k < 64; ++k) S[k] = src ? __ldg(src + k * DS_D) : 0.f;
 #pragma unroll
-      for (int k = 0; k < DS_D; ++k) dst[k * DS_D] = S[k];
+      for (int k = 0; k < 64; ++k) dst[k * DS_D] = S[k];
     }
-    if (n > 0) publish();
+    if (n > 0) {
+      publish();
+      fetch_u(0);
+    }
     bool ok = true;
-    auto step = [&](int i) -> bool {
+    for (int i = 0; i < n; ++i) {
       const int c = chunk_of(i);
-      const long long xoff = ((static_cast<long long>(h) * p.NC + c) * DS_C) * DS_D + v;
-      // the chunk in two halves of 32 tokens: U is fetched ahead of the product it is added to
-      float u[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) u[j] = p.U[xoff + j * DS_D];
-      if (!mbar_wait(acc1_full, i & 1, KID_DELTA_STATE, 5)) return false;
-      tc_fence_after();
-#pragma unroll
-      for (int cb = 0; cb < 2; ++cb) {
+      const int slot = (p.reverse ? c : c + 1) + seq;
+      if (ok && mbar_wait(acc1_full, i & 1, KID_DELTA_STATE, 5)) {
+        tc_fence_after();
         uint32_t r[32];
-        tmem_ld_32x32b_x32(tm1 + cb * 32 + lane_off, r);
+        tmem_ld_32x32b_x32(tm1 + t0 + lane_off, r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) u[j] = fmaf(p.s1, __uint_as_float(r[j]), u[j]);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) p.X[xoff + (cb * 32 + j) * DS_D] = u[j];
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
           uint4 w;
           w.x = pack_bf16(p.s2 * u[ch * 8 + 0], p.s2 * u[ch * 8 + 1]); w.y = pack_bf16(p.s2 * u[ch * 8 + 2], p.s2 * u[ch * 8 + 3]);
           w.z = pack_bf16(p.s2 * u[ch * 8 + 4], p.s2 * u[ch * 8 + 5]); w.w = pack_bf16(p.s2 * u[ch * 8 + 6], p.s2 * u[ch * 8 + 7]);
-          *reinterpret_cast<uint4*>(sXT + v * 128 + (((cb * 4 + ch) ^ (v & 7)) * 16)) = w;
+          *reinterpret_cast<uint4*>(sXT + v * 128 + (((half * 4 + ch) ^ (v & 7)) * 16)) = w;
         }
-        if (cb == 0) {
+        tc_fence_before();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(x_ready);
+        // off the chain, while the second product runs: X goes out, the added gradient comes in, and a vector
+        // decay is staged for all threads (its last readers have published the state that this chunk's first product waited for)
+        float* xout = p.X + row_at(i);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) u[j] = p.U[xoff + (32 + j) * DS_D];
+        for (int j = 0; j < 32; ++j) xout[j * DS_D] = u[j];
+        if (p.add) {
+          const float* src = p.add + state_at(slot);
+#pragma unroll
+          for (int k = 0; k < 64; ++k) av[k] = __ldg(src + k * DS_D);
         }
+        if (p.vec && tid < DS_D) s_dec[tid] = __ldg(p.decay + (static_cast<long long>(h) * p.NC + c) * DS_D + tid);
+      } else {
+        *s_dead = 1;
+        ok = false;
       }
-      tc_fence_before();
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(x_ready);
-      // a vector decay is staged for all threads while the second product runs
-      if (p.vec) s_dec[tid] = p.decay[(static_cast<long long>(h) * p.NC + c) * DS_D + tid];
-      return true;
-    };
-    for (int i = 0; i < n; ++i) {
-      const int c = chunk_of(i);
-      if (!ok || !step(i)) { *s_dead = 1; ok = false; }
-      asm volatile("bar.sync 1, 128;" ::: "memory");     // the decay vector is staged; a failed wait is published
+      asm volatile("bar.sync 1, 256;" ::: "memory");     // the decay vector is staged; a failed wait is published
       if (*s_dead) { ok = false; break; }
       if (!mbar_wait(acc2_full, i & 1, KID_DELTA_STATE, 6)) { ok = false; continue; }
       tc_fence_after();
-      const float dsc = p.vec ? 1.f : p.decay[static_cast<long long>(h) * p.NC + c];
-      const int slot = (p.reverse ? c : c + 1) + seq;
-      const float* addp = p.add ? state_ptr(p.add, slot) : nullptr;
-      float* dst = const_cast<float*>(state_ptr(p.states, slot));
+      const float dsc = p.vec ? 1.f : __ldg(p.decay + static_cast<long long>(h) * p.NC + c);
 #pragma unroll
-      for (int cb = 0; cb < 4; ++cb) {
-        // the 32 added values are fetched together, ahead of the stores of this block (a load may not pass a store
-        // that could alias it, and one exposed memory round trip per value would dominate the chunk)
-        float av[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) av[j] = addp ? addp[(cb * 32 + j) * DS_D] : 0.f;
+      for (int cb = 0; cb < 2; ++cb) {
         uint32_t r[32];
-        tmem_ld_32x32b_x32(tm2 + cb * 32 + lane_off, r);
+        tmem_ld_32x32b_x32(tm2 + k0 + cb * 32 + lane_off, r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const int k = cb * 32 + j;
-          const float d = p.vec ? s_dec[k] : dsc;
-          S[k] = fmaf(d, S[k], __uint_as_float(r[j])) + av[j];
+          const float d = p.vec ? s_dec[k0 + k] : dsc;
+          S[k] = fmaf(d, S[k], __uint_as_float(r[j]));
         }
+      }
+      if (p.add) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) dst[(cb * 32 + j) * DS_D] = S[cb * 32 + j];
+        for (int k = 0; k < 64; ++k) S[k] += av[k];
       }
       tc_fence_before();
-      if (i + 1 < n) publish();
+      if (i + 1 < n) {
+        publish();
+        fetch_u(i + 1);
+      }
+      float* dst = p.states + state_at(slot);
+#pragma unroll
+      for (int k = 0; k < 64; ++k) dst[k * DS_D] = S[k];
     }
     if (!ok) *s_dead = 1;
   }
@@ -290,7 +296,7 @@ TTB_EXPORT int ttb_delta_state_scan(const void* A, const void* B, const float* U
   }
   DeltaStateParams p{U, X, decay, init, add, states, seq_chunks, nseq, H, NC, vec, reverse, s1, s2};
   dim3 grid(nseq, H);
-  delta_state_kernel<<<grid, 192, DsSmem::TOTAL, stream>>>(ta, tb, p);
+  delta_state_kernel<<<grid, DS_THREADS, DsSmem::TOTAL, stream>>>(ta, tb, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
