@@ -85,6 +85,7 @@ struct GemmParams {
   const float* row_scale; // optional [M]
   __nv_bfloat16* preact;  // optional [M, ld_preact] receives gate|up
   long long ld_preact;
+  const float* alpha;     // optional device scalar multiplied into the product (plain stores)
 };
 
 template <int BN, bool A_MN, bool B_MN>
@@ -384,6 +385,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
         constexpr int CH = BN / 32 / (EPI_WARPS / 4);
+        const float alpha = p.alpha ? __ldg(p.alpha) : 1.f;
 #pragma unroll 1
         for (int c = col_half * CH; c < (col_half + 1) * CH; ++c) {
           const int col0 = n0 + c * 32;
@@ -392,6 +394,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           if (nkb > 0) {
             tmem_ld_32x32b_x32(t_row + c * 32, v);
             tmem_ld_wait();
+            if (p.alpha) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+            }
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
@@ -742,6 +748,7 @@ struct GemmArgs {
   long long ld_preact;
   int num_sms;
   const struct EpFuseArgs* ep;   // optional expert-parallel fusion (grouped-M launches only)
+  const float* alpha;            // optional device scalar multiplied into the product (plain stores only)
 };
 
 // Host description of the expert-parallel fusion of one launch (C ABI; see `EpFuse` for the meaning of the fields).
@@ -854,7 +861,7 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
   p.c_fp32 = a.c_fp32; p.accumulate = a.accumulate;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual); p.ldr = a.ldr;
   p.tile_group = a.tile_group; p.group_rows = a.group_rows;
-  p.F = a.F; p.row_scale = a.row_scale;
+  p.F = a.F; p.row_scale = a.row_scale; p.alpha = a.alpha;
   p.preact = reinterpret_cast<__nv_bfloat16*>(a.preact); p.ld_preact = a.ld_preact;
 
   auto kfn = gemm_kernel<BN, A_MN, B_MN, EPI>;
@@ -886,6 +893,7 @@ TTB_EXPORT int ttb_gemm_bf16(const ttb::GemmArgs* args, void* stream_ptr) {
   if (reinterpret_cast<uintptr_t>(a.C) & 15) return 903;
   if (a.residual && ((a.ldr % 8) || (reinterpret_cast<uintptr_t>(a.residual) & 15))) return 904;
   if (a.epi == EPI_SWIGLU && ((a.F % 8) || a.c_fp32 || (a.preact && (a.ld_preact % 8)))) return 905;
+  if (a.alpha && a.epi != EPI_STORE) return 905;
   if (a.ep) {
     const EpFuseArgs& e = *a.ep;
     if (!a.tile_group || a.groups_k > 0 || e.W < 1 || e.W > MAX_RANKS || e.El < 1 || e.El * e.W > 1024 || !e.status) return 906;

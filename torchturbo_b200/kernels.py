@@ -43,6 +43,7 @@ class _GemmArgs(C.Structure):
         ("row_scale", C.c_void_p), ("preact", C.c_void_p), ("ld_preact", C.c_longlong),
         ("num_sms", C.c_int),
         ("ep", C.c_void_p),
+        ("alpha", C.c_void_p),
     ]
 
 
@@ -169,6 +170,7 @@ def gemm(
     row_scale: torch.Tensor | None = None,
     preact: torch.Tensor | None = None,
     ep: "EpFuseArgs | None" = None,
+    alpha: torch.Tensor | None = None,
 ) -> torch.Tensor:
     """tcgen05 GEMM ``C = op(A) @ op(B)`` on bf16 operands with fp32 accumulation.
 
@@ -181,6 +183,7 @@ def gemm(
         with ``group_rows`` an int32 ``[G+1]`` device tensor of 64-aligned row offsets.
       * ``swiglu=True``: ``b`` holds ``[gate | up]`` output columns (``2F``); the result is
         ``silu(gate) * up * row_scale`` of width ``F``; ``preact`` (``[M, 2F]``) optionally keeps gate|up.
+      * ``alpha`` (one fp32 value on the device) is multiplied into the fp32 product before it is rounded or added.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     assert a.stride(-1) == 1 and b.stride(-1) == 1
@@ -241,6 +244,9 @@ def gemm(
         assert preact.dtype == torch.bfloat16
         args.preact, args.ld_preact = preact.data_ptr(), preact.stride(0)
     args.num_sms = num_sms(a.device.index)
+    if alpha is not None:
+        assert alpha.dtype == torch.float32 and alpha.numel() == 1 and alpha.device == a.device and not swiglu
+        args.alpha = alpha.data_ptr()
     if ep is not None:
         args.ep = C.addressof(ep)
     _check(lib().ttb_gemm_bf16(C.byref(args), _stream()), "ttb_gemm_bf16")
