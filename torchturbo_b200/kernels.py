@@ -99,7 +99,7 @@ def lib():
 
 
 # kernels launched per C entry point (used to report how many of this library's kernels ran in a region)
-_LAUNCHES_PER_CALL = {"ttb_rmsnorm_bwd": 2, "ttb_layernorm_bwd": 2, "ttb_bias_act_bwd": 2, "ttb_causal_conv1d_bwd": 3,
+_LAUNCHES_PER_CALL = {"ttb_rmsnorm_bwd": 2, "ttb_gated_rmsnorm_bwd": 2, "ttb_layernorm_bwd": 2, "ttb_bias_act_bwd": 2, "ttb_causal_conv1d_bwd": 3,
                       "ttb_causal_conv1d_row_blocks": 0, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
                       "ttb_ep_combine_all": 3, "ttb_delta_vec_bwd_post": 2, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
                       "ttb_gemm_status": 0}
@@ -273,20 +273,48 @@ def rmsnorm_fwd(x, weight, eps, residual=None, one_plus_w=False):
     return y.view(x.shape), rstd, (xsum.view(x.shape) if xsum is not None else x)
 
 
-def rmsnorm_bwd(dy, x_sum, weight, rstd, dres=None, one_plus_w=False):
-    """Returns (dx, dw_fp32); ``dres`` (gradient arriving on the residual stream) is added into dx."""
+def rmsnorm_bwd(dy, x_sum, weight, rstd, dres=None, one_plus_w=False, dw_dtype=torch.float32):
+    """Returns (dx, dw in ``dw_dtype``: fp32 or bf16); ``dres`` (gradient arriving on the residual stream) is added into dx."""
     H = x_sum.shape[-1]
     x2, dy2 = x_sum.reshape(-1, H), dy.reshape(-1, H)
     T = x2.shape[0]
     grid = max(1, min(T, 2 * num_sms(x_sum.device.index)))
     dx = torch.empty_like(x2)
     partial = torch.empty(grid, H, dtype=torch.float32, device=x_sum.device)
-    dw = torch.empty(H, dtype=torch.float32, device=x_sum.device)
+    dw = torch.empty(H, dtype=dw_dtype, device=x_sum.device)
     d2 = dres.reshape(-1, H) if dres is not None else None
     _check(lib().ttb_rmsnorm_bwd(_p(dy2), _p(x2), _p(weight), _p(rstd), _p(d2), _p(dx), _p(partial), _p(dw),
-                                 C.c_longlong(T), C.c_int(H), C.c_int(int(one_plus_w)), C.c_int(grid), _stream()),
+                                 C.c_int(int(dw_dtype == torch.bfloat16)), C.c_longlong(T), C.c_int(H), C.c_int(int(one_plus_w)), C.c_int(grid), _stream()),
            "ttb_rmsnorm_bwd")
     return dx.view(x_sum.shape), dw
+
+
+def _gated_grid(R: int, H: int, device) -> int:
+    rows = 2048 // H                       # rows of one 256-thread block
+    return max(1, min((R + rows - 1) // rows, 8 * num_sms(device.index)))
+
+
+def gated_rmsnorm_fwd(x, gate, weight, eps, silu: bool):
+    """``bf16(rmsnorm(x) * weight) * act(gate)`` on bf16 rows of 64, 128 or 256 channels.  Returns (y, rstd)."""
+    R, H = x.shape
+    y = torch.empty_like(x)
+    rstd = torch.empty(R, dtype=torch.float32, device=x.device)
+    _check(lib().ttb_gated_rmsnorm_fwd(_p(x), _p(gate), _p(weight), _p(y), _p(rstd), C.c_longlong(R), C.c_int(H), C.c_float(eps),
+                                       C.c_int(int(silu)), C.c_int(_gated_grid(R, H, x.device)), _stream()), "ttb_gated_rmsnorm_fwd")
+    return y, rstd
+
+
+def gated_rmsnorm_bwd(dy, x, gate, weight, rstd, silu: bool):
+    """Returns (dx, dgate, dw), all bf16."""
+    R, H = x.shape
+    grid = _gated_grid(R, H, x.device)
+    dx, dgate = torch.empty_like(x), torch.empty_like(x)
+    dw = torch.empty_like(weight) if R else torch.zeros_like(weight)
+    partial = torch.empty(grid, H, dtype=torch.float32, device=x.device)
+    _check(lib().ttb_gated_rmsnorm_bwd(_p(dy), _p(x), _p(gate), _p(weight), _p(rstd), _p(dx), _p(dgate), _p(partial), _p(dw),
+                                       C.c_longlong(R), C.c_int(H), C.c_int(int(silu)), C.c_int(grid), _stream()),
+           "ttb_gated_rmsnorm_bwd")
+    return dx, dgate, dw
 
 
 # --------------------------------------------------------------------------------------
@@ -308,17 +336,17 @@ def layernorm_fwd(x, weight, bias, eps):
     return y.view(x.shape), mean, rstd
 
 
-def layernorm_bwd(dy, x, weight, mean, rstd):
-    """Returns (dx, dw_fp32, db_fp32)."""
+def layernorm_bwd(dy, x, weight, mean, rstd, dw_dtype=torch.float32):
+    """Returns (dx, dw, db), the last two in ``dw_dtype`` (fp32 or bf16)."""
     H = x.shape[-1]
     x2, dy2 = x.reshape(-1, H), dy.reshape(-1, H)
     T = x2.shape[0]
     grid = max(1, min(T, 2 * num_sms(x.device.index)))
     dx = torch.empty_like(x2)
     part = torch.empty(grid, 2 * H, dtype=torch.float32, device=x.device)
-    dwdb = torch.empty(2, H, dtype=torch.float32, device=x.device)
+    dwdb = torch.empty(2, H, dtype=dw_dtype, device=x.device)
     _check(lib().ttb_layernorm_bwd(_p(dy2), _p(x2), _p(weight), _p(mean), _p(rstd), _p(dx), _p(part), _p(dwdb),
-                                   C.c_longlong(T), C.c_int(H), C.c_int(grid), _stream()), "ttb_layernorm_bwd")
+                                   C.c_int(int(dw_dtype == torch.bfloat16)), C.c_longlong(T), C.c_int(H), C.c_int(grid), _stream()), "ttb_layernorm_bwd")
     return dx.view(x.shape), dwdb[0], dwdb[1]
 
 
@@ -333,8 +361,8 @@ def bias_act_fwd(x, bias, act, residual=None):
     return y.view(x.shape)
 
 
-def bias_act_bwd(dy, x, bias, act):
-    """Returns (dx, dbias_fp32); with the identity activation dx is dy itself."""
+def bias_act_bwd(dy, x, bias, act, db_dtype=torch.float32):
+    """Returns (dx, dbias in ``db_dtype``: fp32 or bf16); with the identity activation dx is dy itself."""
     Cn = x.shape[-1]
     x2, dy2 = x.reshape(-1, Cn), dy.reshape(-1, Cn)
     R = x2.shape[0]
@@ -342,8 +370,9 @@ def bias_act_bwd(dy, x, bias, act):
     grid = max(1, min(R, 2 * num_sms(x.device.index)))
     dx = torch.empty_like(x2) if code else None
     part = torch.empty(grid, Cn, dtype=torch.float32, device=x.device)
-    db = torch.empty(Cn, dtype=torch.float32, device=x.device)
-    _check(lib().ttb_bias_act_bwd(_p(dy2), _p(x2), _p(bias), _p(dx), _p(part), _p(db), C.c_longlong(R), C.c_int(Cn),
+    db = torch.empty(Cn, dtype=db_dtype, device=x.device)
+    _check(lib().ttb_bias_act_bwd(_p(dy2), _p(x2), _p(bias), _p(dx), _p(part), _p(db),
+                                  C.c_int(int(db_dtype == torch.bfloat16)), C.c_longlong(R), C.c_int(Cn),
                                   C.c_int(code), C.c_int(grid), _stream()), "ttb_bias_act_bwd")
     return (dx.view(x.shape) if dx is not None else dy), db
 

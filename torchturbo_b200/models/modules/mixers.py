@@ -63,10 +63,7 @@ class GatedRMSNorm(nn.Module):
         self.eps, self.activation = eps, activation
 
     def forward(self, x, gate):
-        y = ops.rms_norm(x, self.weight, self.eps)
-        g = gate.float()
-        g = F.silu(g) if self.activation == "silu" else torch.sigmoid(g)
-        return (y.float() * g).to(x.dtype)
+        return ops.gated_rms_norm(x, gate, self.weight, self.eps, activation="silu" if self.activation == "silu" else "sigmoid")
 
 
 # ------------------------------------------------------------------------------------------------
@@ -166,28 +163,30 @@ class GatedDeltaNet(nn.Module):
         z = ops.linear(x, self.in_proj_z.weight).view(T, self.n_v, self.dv)
         b = ops.linear(x, self.in_proj_b.weight)
         a = ops.linear(x, self.in_proj_a.weight)
-        q, k, v = qkv.split([self.key_dim, self.key_dim, self.value_dim], dim=-1)
-        q, k, v = q.reshape(T, self.n_k, self.dk), k.reshape(T, self.n_k, self.dk), v.reshape(T, self.n_v, self.dv)
         w = self.conv1d.weight.squeeze(1)
-        wq, wk, wv = w.split([self.key_dim, self.key_dim, self.value_dim], dim=0)
         A_log, dt_bias = self.A_log, self.dt_bias
+        Tg, hk, hv = T, self.n_k, self.n_v
         if sp > 1:
             # full sequence of the local heads; per-head parameters sliced to match
+            q, k, v = qkv.split([self.key_dim, self.key_dim, self.value_dim], dim=-1)
+            q, k, v = q.reshape(T, self.n_k, self.dk), k.reshape(T, self.n_k, self.dk), v.reshape(T, self.n_v, self.dv)
+            wq, wk, wv = w.split([self.key_dim, self.key_dim, self.value_dim], dim=0)
             q, k, v = (gather_seq_scatter_heads(t.contiguous(), ctx.sp_group, sp) for t in (q, k, v))
             ba = gather_seq_scatter_heads(torch.stack((b, a), -1).contiguous(), ctx.sp_group, sp)
             b, a = ba[..., 0], ba[..., 1]
             wq, wk, wv = (_head_slice(t, h, sp, r) for t, h in ((wq, self.n_k), (wk, self.n_k), (wv, self.n_v)))
             A_log, dt_bias = _head_slice(A_log, self.n_v, sp, r), _head_slice(dt_bias, self.n_v, sp, r)
-        Tg, hk, hv = q.shape[0], q.shape[1], v.shape[1]
+            Tg, hk, hv = q.shape[0], q.shape[1], v.shape[1]
+            qkv, w = torch.cat((q.reshape(Tg, -1), k.reshape(Tg, -1), v.reshape(Tg, -1)), -1), torch.cat((wq, wk, wv), 0)
         cu = ctx.cu_seqlens
-        mixed = torch.cat((q.reshape(Tg, -1), k.reshape(Tg, -1), v.reshape(Tg, -1)), -1).unsqueeze(0)
-        mixed, _ = ops.causal_conv1d(mixed, torch.cat((wq, wk, wv), 0), None, activation="silu", cu_seqlens=cu)
+        mixed, _ = ops.causal_conv1d(qkv.unsqueeze(0), w, None, activation="silu", cu_seqlens=cu)
         q, k, v = mixed[0].split([hk * self.dk, hk * self.dk, hv * self.dv], dim=-1)
         q, k, v = q.reshape(1, Tg, hk, self.dk), k.reshape(1, Tg, hk, self.dk), v.reshape(1, Tg, hv, self.dv)
         beta = torch.sigmoid(b.float()).unsqueeze(0)
         g = (-A_log.float().exp() * F.softplus(a.float() + dt_bias.float())).unsqueeze(0)
         if hv // hk > 1:
-            q, k = q.repeat_interleave(hv // hk, dim=2), k.repeat_interleave(hv // hk, dim=2)
+            # every key head serves hv / hk value heads; as a broadcast its gradient is a plain sum over them
+            q, k = (t.unsqueeze(3).expand(1, Tg, hk, hv // hk, self.dk).reshape(1, Tg, hv, self.dk) for t in (q, k))
         o, _ = ops.gated_delta_rule(q, k, v, g, beta, use_qk_l2norm_in_kernel=True, cu_seqlens=cu)
         o = o[0]                                                            # [Tg, hv, dv]
         if sp > 1:

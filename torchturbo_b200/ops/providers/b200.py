@@ -160,8 +160,8 @@ class RMSNormFn(torch.autograd.Function):
     def backward(ctx, dy, dsum=None):
         xsum, w, rstd = ctx.saved_tensors
         dx, dw = K.rmsnorm_bwd(dy.contiguous(), xsum, w, rstd, dres=dsum.contiguous() if dsum is not None else None,
-                               one_plus_w=ctx.one_plus_w)
-        return dx, dw.to(w.dtype), None, (dx if ctx.has_res else None), None
+                               one_plus_w=ctx.one_plus_w, dw_dtype=w.dtype)
+        return dx, dw, None, (dx if ctx.has_res else None), None
 
 
 @_custom("rms_norm", "b200_rms_norm")
@@ -176,6 +176,40 @@ class B200RMSNorm(_B200Op):
         return RMSNormFn.apply(x, weight, eps, residual, one_plus_weight)
 
 
+class GatedRMSNormFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, gate, w, eps, silu):
+        y, rstd = K.gated_rmsnorm_fwd(x, gate, w, eps, silu)
+        ctx.save_for_backward(x, gate, w, rstd)
+        ctx.silu = silu
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, gate, w, rstd = ctx.saved_tensors
+        return (*K.gated_rmsnorm_bwd(dy.contiguous(), x, gate, w, rstd, ctx.silu), None, None)
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on a 16-byte boundary (the kernels read and write eight bf16 values at a time)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+@_custom("gated_rms_norm", "b200_gated_rms_norm")
+class B200GatedRMSNorm(_B200Op):
+    """Norm, activation of the gate and their product in one pass each way; head widths other than 64 / 128 / 256 take the
+    norm kernel and torch products."""
+
+    def __call__(self, x, gate, weight, eps=1e-6, *, activation="silu"):
+        H = x.shape[-1]
+        if not _ok(x, gate, weight) or H not in (64, 128, 256) or x.shape != gate.shape or activation not in ("silu", "sigmoid"):
+            return N.TorchGatedRMSNorm()(x, gate, weight, eps, activation=activation)
+        y = GatedRMSNormFn.apply(_aligned(x.reshape(-1, H)), _aligned(gate.reshape(-1, H)), _aligned(weight), float(eps),
+                                 activation == "silu")
+        return y.view(x.shape)
+
+
 class LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps):
@@ -187,8 +221,8 @@ class LayerNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, mean, rstd = ctx.saved_tensors
-        dx, dw, db = K.layernorm_bwd(dy.contiguous(), x, w, mean, rstd)
-        return dx, dw.to(w.dtype), db.to(w.dtype), None
+        dx, dw, db = K.layernorm_bwd(dy.contiguous(), x, w, mean, rstd, dw_dtype=w.dtype)
+        return dx, dw, db, None
 
 
 @_custom("layer_norm", "b200_layer_norm")
@@ -215,8 +249,8 @@ class BiasActFn(torch.autograd.Function):
     def backward(ctx, dy):
         x, bias = ctx.saved_tensors
         dy = dy.contiguous()
-        dx, db = K.bias_act_bwd(dy, x, bias, ctx.act)
-        return dx, db.to(bias.dtype), None, (dy if ctx.has_res else None)
+        dx, db = K.bias_act_bwd(dy, x, bias, ctx.act, db_dtype=bias.dtype)
+        return dx, db, None, (dy if ctx.has_res else None)
 
 
 @_custom("bias_act", "b200_bias_act")

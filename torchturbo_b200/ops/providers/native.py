@@ -43,6 +43,18 @@ class TorchRMSNorm(OpImpl):
         return rms_norm_ref(x, weight, eps, residual, one_plus_weight)
 
 
+@_native("gated_rms_norm")
+class TorchGatedRMSNorm(OpImpl):
+    """`weight * rmsnorm(x) * act(gate)` over the last dimension; the norm is the selected `rms_norm`, the product fp32."""
+
+    def __call__(self, x, gate, weight, eps=1e-6, *, activation="silu"):
+        from ..ops import ops
+
+        y, g = ops.rms_norm(x, weight, eps), gate.float()
+        g = F.silu(g) if activation == "silu" else torch.sigmoid(g)
+        return (y.float() * g).to(x.dtype)
+
+
 def layer_norm_ref(x, weight, bias, eps=1e-6):
     return F.layer_norm(x.float(), (x.shape[-1],), weight.float(), bias.float(), eps).to(x.dtype)
 
