@@ -447,14 +447,16 @@ def swiglu_fwd(x, row_scale=None, nrows=None):
     return y
 
 
-def swiglu_bwd(dy, x, row_scale=None, want_dscale=False, nrows=None):
-    """`nrows` (int32 device scalar, optional): rows from `nrows[0]` on are left untouched (padded buffers)."""
+def swiglu_bwd(dy, x, row_scale=None, want_dscale=False, nrows=None, y_out=None):
+    """`nrows` (int32 device scalar, optional): rows from `nrows[0]` on are left untouched (padded buffers).  `y_out` (bf16
+    [R, F], optional) receives the forward result, as `swiglu_fwd` computes it."""
     R, F2 = x.shape
     F = F2 // 2
     dx = torch.empty_like(x)
     dscale = torch.empty(R, dtype=torch.float32, device=x.device) if want_dscale else None
     _check(lib().ttb_swiglu_bwd(_p(dy), C.c_longlong(dy.stride(0)), _p(x), C.c_longlong(x.stride(0)), _p(row_scale),
-                                _p(dx), C.c_longlong(dx.stride(0)), _p(dscale), C.c_longlong(R), C.c_int(F), _p(nrows),
+                                _p(dx), C.c_longlong(dx.stride(0)), _p(dscale), _p(y_out),
+                                C.c_longlong(y_out.stride(0) if y_out is not None else 0), C.c_longlong(R), C.c_int(F), _p(nrows),
                                 _stream()), "ttb_swiglu_bwd")
     return dx, dscale
 

@@ -518,10 +518,12 @@ class MoEExpertsFn(torch.autograd.Function):
         dy = dy.contiguous()
         # d(act) = dY @ W2[e]^T  (W2[e] is [F, H] = [N, K] K-major)
         dact = K.gemm(dy, w2, tile_group=tile_group)
-        dpre, dprob = K.swiglu_bwd(dact, pre, row_prob, want_dscale=row_prob is not None)
+        # the buffer holds `seg_start[-1]` rows; what lies behind them is capacity that no tile reads.  The activation that
+        # the second weight gradient needs comes out of the same pass over the pre-activations.
+        act = torch.empty_like(dact) if ctx.needs_input_grad[3] else None
+        dpre, dprob = K.swiglu_bwd(dact, pre, row_prob, want_dscale=row_prob is not None, nrows=seg_start[-1:], y_out=act)
         dw1 = dw2 = None
         if ctx.needs_input_grad[3]:
-            act = K.swiglu_fwd(pre, row_prob)
             dw2 = _weight_grad(w2, act, dy, group_rows=seg_start)
         if ctx.needs_input_grad[2]:
             dw1 = _weight_grad(w1, xp, dpre, group_rows=seg_start)
