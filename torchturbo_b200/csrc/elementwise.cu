@@ -759,6 +759,35 @@ __global__ void qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, con
 }
 
 // ============================================================================
+// Half-rotation RoPE of [T, heads, 2 * half] with any token / head stride; y contiguous.  sign = -1 is the transpose (the
+// backward).  Four pairs per thread, fp32 arithmetic, one rounding.  3000 patches x 16 heads of 72: 5.5 us each, in place of about
+// ten torch launches forward and more backward.
+//   y1 = x1 c - sign x2 s,  y2 = x2 c + sign x1 s
+// ============================================================================
+__global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, long long x_t, long long x_h, const float* __restrict__ cos_t,
+                            const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ y, long long total, int heads, int half,
+                            float sign) {
+  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= total) return;
+  const int q = half / 4;
+  const long long th = idx / q;
+  const int c = static_cast<int>(idx - th * q) * 4;
+  const long long t = th / heads;
+  const int h = static_cast<int>(th - t * heads);
+  const __nv_bfloat16* src = x + t * x_t + h * x_h + c;
+  const uint2 u1 = *reinterpret_cast<const uint2*>(src), u2 = *reinterpret_cast<const uint2*>(src + half);
+  const float4 co = __ldg(reinterpret_cast<const float4*>(cos_t + t * half + c));
+  float4 si = __ldg(reinterpret_cast<const float4*>(sin_t + t * half + c));
+  si.x *= sign; si.y *= sign; si.z *= sign; si.w *= sign;
+  const float2 a0 = unpack_bf16(u1.x), a1 = unpack_bf16(u1.y), b0 = unpack_bf16(u2.x), b1 = unpack_bf16(u2.y);
+  __nv_bfloat16* dst = y + th * 2 * half + c;
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(a0.x * co.x - b0.x * si.x, a0.y * co.y - b0.y * si.y),
+                                              pack_bf16(a1.x * co.z - b1.x * si.z, a1.y * co.w - b1.y * si.w));
+  *reinterpret_cast<uint2*>(dst + half) = make_uint2(pack_bf16(b0.x * co.x + a0.x * si.x, b0.y * co.y + a0.y * si.y),
+                                                     pack_bf16(b1.x * co.z + a1.x * si.z, b1.y * co.w + a1.y * si.w));
+}
+
+// ============================================================================
 // SwiGLU (standalone).  x: [R, 2F] = [gate | up]; y: [R, F]; optional row_scale [R].
 // ============================================================================
 // `nrows` (optional, device): rows at or beyond *nrows are skipped (padded buffers whose fill is only known on the device)
@@ -1149,6 +1178,17 @@ TTB_EXPORT int ttb_gated_rmsnorm_bwd(const void* dy, const void* x, const void* 
   else if (H == 256) gated_rmsnorm_bwd_kernel<32><<<grid, 256, 0, STREAM(stream)>>>(D, X, G, W, rstd, DX, DG, dw_partial, R, silu);
   else return 901;
   colsum(dw_partial, dw_out, 1, grid, H, STREAM(stream));
+  LAUNCH_RET();
+}
+
+// x, y on 8-byte boundaries, strides multiples of 4 elements; cos / sin fp32 [T, half] on 16-byte boundaries
+TTB_EXPORT int ttb_rope(const void* x, long long x_t, long long x_h, const float* cos_t, const float* sin_t, void* y, long long T,
+                        int heads, int half, float sign, void* stream) {
+  if (half % 4 || x_t % 4 || x_h % 4) return 901;
+  const long long total = T * heads * (half / 4);
+  if (total == 0) return 0;
+  rope_kernel<<<(unsigned)((total + 255) / 256), 256, 0, STREAM(stream)>>>((const __nv_bfloat16*)x, x_t, x_h, cos_t, sin_t,
+                                                                          (__nv_bfloat16*)y, total, heads, half, sign);
   LAUNCH_RET();
 }
 

@@ -434,6 +434,15 @@ def qknorm_rope_bwd(dq, dk, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dq
     return dwq, dwk
 
 
+def rope(x, cos, sin, sign: float = 1.0):
+    """Half-rotation RoPE of bf16 [T, heads, D] (channels contiguous); cos, sin fp32 [T, D / 2].  ``sign=-1`` rotates back."""
+    T, heads, D = x.shape
+    y = torch.empty(T, heads, D, dtype=x.dtype, device=x.device)
+    _check(lib().ttb_rope(_p(x), C.c_longlong(x.stride(0)), C.c_longlong(x.stride(1)), _p(cos), _p(sin), _p(y), C.c_longlong(T),
+                          C.c_int(heads), C.c_int(D // 2), C.c_float(sign), _stream()), "ttb_rope")
+    return y
+
+
 # --------------------------------------------------------------------------------------
 # SwiGLU
 # --------------------------------------------------------------------------------------

@@ -380,6 +380,38 @@ class B200QKNormRope(_B200Op):
                                   sin.float().contiguous(), eps)
 
 
+def _rope_rows(x: torch.Tensor) -> torch.Tensor:
+    """The kernel reads four channels at a time: copied only where they would not start on an 8-byte boundary."""
+    if x.stride(2) != 1 or x.stride(0) % 4 or x.stride(1) % 4 or x.data_ptr() % 8:
+        x = x.clone(memory_format=torch.contiguous_format)
+    return x
+
+
+class RopeFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, cos, sin):
+        ctx.save_for_backward(cos, sin)
+        return K.rope(_rope_rows(x), cos, sin)
+
+    @staticmethod
+    def backward(ctx, dy):
+        cos, sin = ctx.saved_tensors
+        return K.rope(_rope_rows(dy), cos, sin, -1.0), None, None
+
+
+@_custom("rotary_position_embedding", "b200_rope")
+class B200RoPE(_B200Op):
+    """One pass each way over strided heads (a slice of a fused projection needs no copy); the torch formulation takes
+    about ten launches forward and more backward, with fp32 intermediates."""
+
+    def __call__(self, x, cos, sin):
+        D = x.shape[-1]
+        if not _ok(x) or x.dim() != 3 or D % 8 or cos.shape != (x.shape[0], D // 2) or sin.shape != cos.shape \
+                or not (cos.is_cuda and sin.is_cuda) or cos.requires_grad or sin.requires_grad:
+            return N.rope_ref(x, cos, sin)
+        return RopeFn.apply(x, _aligned(cos.float()), _aligned(sin.float()))
+
+
 # ------------------------------------------------------------------------------------------------
 # MoE: router, permutation, experts
 # ------------------------------------------------------------------------------------------------
