@@ -453,20 +453,29 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
-// delta[h, t] = sum_d dO[t,h,d] * O[t,h,d]; also converts nothing else.  One warp per (t, h).
-__global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                                      float* __restrict__ delta, long long T, int Hq) {
-  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= T * Hq) return;
-  const long long t = gw / Hq;
-  const int h = static_cast<int>(gw - t * Hq);
-  const uint2 a = *reinterpret_cast<const uint2*>(dout + gw * BW_D + lane * 4);
-  const uint2 b = *reinterpret_cast<const uint2*>(out + gw * BW_D + lane * 4);
-  const float2 a0 = unpack_bf16(a.x), a1 = unpack_bf16(a.y), b0 = unpack_bf16(b.x), b1 = unpack_bf16(b.y);
-  float s = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
-  s = warp_sum(s);
-  if (lane == 0) delta[static_cast<long long>(h) * T + t] = s;
+// delta[h, t] = sum_d dO[t,h,d] * O[t,h,d].  Sixteen lanes and 16-byte loads per (t, h): 22 -> 16 us for 4096 x 32 rows.
+__global__ void __launch_bounds__(256)
+attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
+                      float* __restrict__ delta, long long T, int Hq) {
+  long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
+  const int l = threadIdx.x & 15;
+  const bool ok = row < T * Hq;
+  if (!ok) row = T * Hq - 1;                 // both halves of a warp take part in the shuffles
+  const uint4 a = *reinterpret_cast<const uint4*>(dout + row * BW_D + l * 8);
+  const uint4 b = *reinterpret_cast<const uint4*>(out + row * BW_D + l * 8);
+  const uint32_t as[4] = {a.x, a.y, a.z, a.w}, bs[4] = {b.x, b.y, b.z, b.w};
+  float s = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 x = unpack_bf16(as[j]), y = unpack_bf16(bs[j]);
+    s += x.x * y.x + x.y * y.y;
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (ok && l == 0) {
+    const long long t = row / Hq;
+    delta[(row - t * Hq) * T + t] = s;
+  }
 }
 
 // dq (bf16) = dq_acc (fp32)
@@ -520,8 +529,8 @@ TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const v
   if ((ldk % 8) || (ldv % 8)) return 902;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   if (T == 0 || n_tiles == 0) return 0;
-  const long long warps = T * Hq;
-  attn_bwd_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>((const __nv_bfloat16*)dout,
+  if ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15) return 906;
+  attn_bwd_delta_kernel<<<(unsigned)((T * Hq + 15) / 16), 256, 0, stream>>>((const __nv_bfloat16*)dout,
                                                                         (const __nv_bfloat16*)out, delta, T, Hq);
   CUtensorMap tq, tdo, tk, tv;
   if (bw_map(&tq, q, T, (long long)Hq * D, Hq * D, 64)) return 101;
@@ -542,14 +551,17 @@ TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const v
                          : (D == 128 ? launch_attn_bwd<128, false>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
                                      : launch_attn_bwd<192, false>(tq, tdo, tk, tv, tdq, p, n_tiles, stream));
   if (rc) return rc;
-  if (with_dq) {
-    const long long n = T * Hq * D;
-    attn_bwd_cast_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, stream>>>(dq_acc, (__nv_bfloat16*)dq, n);
-  }
-  if (Hq != Hk && !group_loop) {
-    const long long nk = T * Hk * D, nv = T * Hk * BW_D;
-    attn_bwd_cast_kernel<<<(unsigned)((nk / 8 + 255) / 256), 256, 0, stream>>>(dk_acc, (__nv_bfloat16*)dk, nk);
-    attn_bwd_cast_kernel<<<(unsigned)((nv / 8 + 255) / 256), 256, 0, stream>>>(dv_acc, (__nv_bfloat16*)dv, nv);
+  // fp32 accumulators -> bf16; the ones that lie back to back on both sides go in one launch
+  const bool grouped = Hq != Hk && !group_loop;
+  const long long n[3] = {with_dq ? T * Hq * D : 0, grouped ? T * Hk * D : 0, grouped ? T * Hk * BW_D : 0};
+  const float* src[3] = {dq_acc, dk_acc, dv_acc};
+  __nv_bfloat16* dst[3] = {(__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv};
+  for (int i = 0; i < 3;) {
+    long long run = n[i];
+    int j = i + 1;
+    while (j < 3 && run > 0 && src[j] == src[i] + run && dst[j] == dst[i] + run) run += n[j++];
+    if (run > 0) attn_bwd_cast_kernel<<<(unsigned)((run / 8 + 255) / 256), 256, 0, stream>>>(src[i], dst[i], run);
+    i = j;
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;

@@ -692,16 +692,29 @@ def build_q_tiles(cu_seqlens, block: int = 128) -> torch.Tensor:
     return torch.tensor(rows, dtype=torch.int32).reshape(-1, 3)
 
 
+def _zero_outside(t: torch.Tensor, rows) -> torch.Tensor:
+    """Rows of `t` that no sequence covers read as zero; `rows` = (first, one past the last) covered row, None = unknown."""
+    if rows is None:
+        return t.zero_()
+    lo, hi = rows
+    if lo > 0:
+        t[:lo].zero_()
+    if hi < t.shape[0]:
+        t[hi:].zero_()
+    return t
+
+
 def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_lse: bool = True,
-             want_max_logit: bool = False):
+             want_max_logit: bool = False, rows=None):
     """q: [T, Hq, D]; k: [T, Hk, D] with D = 128 or 192 (multi-head latent attention); v: [T, Hk, 128] (may be a
-    row-strided view).  Returns (out [T, Hq, 128], lse [Hq, T], max_logit [Hq])."""
+    row-strided view).  `rows` (optional): (first, one past the last) row that the tile table covers; the kernel writes
+    every one of them.  Returns (out [T, Hq, 128], lse [Hq, T], max_logit [Hq])."""
     T, Hq, D = q.shape
     Hk = k.shape[1]
     assert D in (128, 192) and k.shape[2] == D and v.shape[2] == 128
     assert q.stride(2) == 1 and q.stride(1) == D and k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == 128 and v.stride(2) == 1
     # rows past the last sequence boundary are never written by the kernel and must read as zero
-    out = torch.zeros(T, Hq, 128, dtype=q.dtype, device=q.device)
+    out = _zero_outside(torch.empty(T, Hq, 128, dtype=q.dtype, device=q.device), rows)
     lse = torch.full((Hq, T), float("-inf"), dtype=torch.float32, device=q.device) if want_lse else None
     ml = torch.full((Hq,), float("-inf"), dtype=torch.float32, device=q.device) if want_max_logit else None
     _check(lib().ttb_attn_fwd(_p(q), C.c_longlong(q.stride(0)), _p(k), C.c_longlong(k.stride(0)), _p(v),
@@ -1032,8 +1045,8 @@ def ep_gather_vals(peer_ptrs, off_vals, expert, dest_row, El, world, cap_rows, s
 
 
 def attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, *, scale: float, causal: bool = True, q_tiles_dev=None,
-             deterministic: bool = False):
-    """Gradients of `attn_fwd`.  Returns (dq [T,Hq,D], dk [T,Hk,D], dv [T,Hk,128]) in bf16.
+             deterministic: bool = False, rows=None):
+    """Gradients of `attn_fwd`.  Returns (dq [T,Hq,D], dk [T,Hk,D], dv [T,Hk,128]) in bf16; `rows` as in `attn_fwd`.
 
     128-wide heads by default: one kernel; dQ tiles are added into an fp32 scratch buffer by TMA reductions and, with
     grouped-query attention, the dK / dV of a group's query heads are summed with atomics (the order of the adds is not
@@ -1048,18 +1061,32 @@ def attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, *, scale: float, causal: boo
     split = deterministic or D != 128
     if split and q_tiles_dev is None:
         raise ValueError("the query-major dQ pass needs the query tile table")
+    if kv_tiles_dev.shape[0] == 0:                       # no sequence covers a row
+        return torch.zeros_like(q), torch.zeros(T, Hk, D, dtype=q.dtype, device=q.device), \
+            torch.zeros(T, Hk, 128, dtype=q.dtype, device=q.device)
     delta = torch.empty(Hq * T, dtype=torch.float32, device=q.device)
-    dq_acc = None if split else torch.zeros(T, Hq, D, dtype=torch.float32, device=q.device)
-    dq = torch.zeros_like(q) if split else torch.empty_like(q)
-    if Hq != Hk and not deterministic:   # query heads of a group add into fp32 accumulators, converted at the end
-        dk_acc = torch.zeros(T, Hk, D, dtype=torch.float32, device=q.device)
-        dv_acc = torch.zeros(T, Hk, 128, dtype=torch.float32, device=q.device)
-        dk = torch.empty(T, Hk, D, dtype=q.dtype, device=q.device)
-        dv = torch.empty(T, Hk, 128, dtype=q.dtype, device=q.device)
+    dq_acc = dk_acc = dv_acc = None
+    if Hq != Hk and not deterministic:
+        # query heads of a group add into fp32 accumulators, converted at the end; accumulators and results lie back to
+        # back, so that they are cleared and converted by one launch each
+        shapes = ([] if split else [(T, Hq, D)]) + [(T, Hk, D), (T, Hk, 128)]
+        sizes = [a * b * c for a, b, c in shapes]
+        acc = torch.zeros(sum(sizes), dtype=torch.float32, device=q.device).split(sizes)
+        res = torch.empty(sum(sizes), dtype=q.dtype, device=q.device).split(sizes)
+        acc, res = ([t.view(s) for t, s in zip(x, shapes)] for x in (acc, res))
+        (dk_acc, dv_acc), (dk, dv) = acc[-2:], res[-2:]
+        if split:
+            dq = _zero_outside(torch.empty_like(q), rows)
+        else:
+            dq_acc, dq = acc[0], res[0]
     else:
-        dk_acc = dv_acc = None
-        dk = torch.zeros(T, Hk, D, dtype=q.dtype, device=q.device)
-        dv = torch.zeros(T, Hk, 128, dtype=q.dtype, device=q.device)
+        if not split:
+            dq_acc = torch.zeros(T, Hq, D, dtype=torch.float32, device=q.device)
+        dq = torch.empty_like(q)
+        if split:
+            _zero_outside(dq, rows)
+        dk = _zero_outside(torch.empty(T, Hk, D, dtype=q.dtype, device=q.device), rows)
+        dv = _zero_outside(torch.empty(T, Hk, 128, dtype=q.dtype, device=q.device), rows)
     global LAUNCH_COUNT
     _check(lib().ttb_attn_bwd(_p(q), _p(k), C.c_longlong(k.stride(0)), _p(v), C.c_longlong(v.stride(0)), _p(out),
                               _p(dout), _p(lse), _p(delta), _p(dq_acc), _p(dk_acc), _p(dv_acc), _p(dq), _p(dk), _p(dv),
@@ -1067,7 +1094,7 @@ def attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, *, scale: float, causal: boo
                               C.c_int(kv_tiles_dev.shape[0]), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D),
                               C.c_float(scale), C.c_int(int(causal)), C.c_int((2 if deterministic else 0) if split else 1), _stream()),
            "ttb_attn_bwd")
-    LAUNCH_COUNT += (1 if split else 2) + (0 if (Hq == Hk or deterministic) else 2)
+    LAUNCH_COUNT += 2 if (not split or (Hq != Hk and not deterministic)) else 1
     if split:
         _check(lib().ttb_attn_bwd_dq(_p(q), _p(k), C.c_longlong(k.stride(0)), _p(v), C.c_longlong(v.stride(0)), _p(dout),
                                      _p(lse), _p(delta), _p(dq), _p(q_tiles_dev), C.c_int(q_tiles_dev.shape[0]),

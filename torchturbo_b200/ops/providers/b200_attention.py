@@ -17,20 +17,23 @@ from .b200 import BF16, _B200Op, _ok
 
 @cache
 def _tiles_for(cu_seqlens, device):
-    """(query-tile table on the device, number of valid tokens, boundaries on the device) for one batch; built
-    once and shared by every layer (pinned staging keeps the copies asynchronous)."""
+    """(query-tile table on the device, number of valid tokens, boundaries on the device, key-tile table, covered rows)
+    for one batch; built once and shared by every layer (pinned staging keeps the copies asynchronous)."""
     t = K.build_q_tiles(cu_seqlens).pin_memory()
     tk = K.build_kv_tiles(cu_seqlens).pin_memory()
     cu = cu_seqlens.to(torch.int32).pin_memory()
-    return (t.to(device, non_blocking=True), int(cu_seqlens[-1]), cu.to(device, non_blocking=True),
-            tk.to(device, non_blocking=True))
+    offs = cu_seqlens.tolist()
+    # the tables cover [first, last) without holes when the boundaries do not decrease
+    rows = (offs[0], offs[-1]) if all(a <= b for a, b in zip(offs[:-1], offs[1:])) else None
+    return (t.to(device, non_blocking=True), offs[-1], cu.to(device, non_blocking=True),
+            tk.to(device, non_blocking=True), rows)
 
 
 class FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens, max_seqlen, causal, scale, want_ml):
-        tiles, n_valid = _tiles_for(cu_seqlens, q.device)[:2]
-        out, lse, ml = K.attn_fwd(q, k, v, tiles, scale=scale, causal=causal, want_max_logit=want_ml)
+        tiles, n_valid, _, _, rows = _tiles_for(cu_seqlens, q.device)
+        out, lse, ml = K.attn_fwd(q, k, v, tiles, scale=scale, causal=causal, want_max_logit=want_ml, rows=rows)
         ctx.save_for_backward(q, k, v, out, lse)
         ctx.meta = (cu_seqlens, max_seqlen, causal, scale, n_valid)
         if want_ml:
@@ -45,7 +48,8 @@ class FlashAttnFn(torch.autograd.Function):
         if os.environ.get("TORCHTURBO_ATTN_BWD", "tcgen05") == "tcgen05":
             cached = _tiles_for(cu_seqlens, q.device)
             dq, dk, dv = K.attn_bwd(dout.contiguous(), q, k, v, out, lse, cached[3], scale=scale, causal=causal,
-                                    q_tiles_dev=cached[0], deterministic=torch.are_deterministic_algorithms_enabled())
+                                    q_tiles_dev=cached[0], deterministic=torch.are_deterministic_algorithms_enabled(),
+                                    rows=cached[4])
             return dq, dk, dv, None, None, None, None, None
         # library backward on this kernel's out / lse (selected with TORCHTURBO_ATTN_BWD=flash_attn2; used as a baseline)
         from flash_attn.flash_attn_interface import _flash_attn_varlen_backward
