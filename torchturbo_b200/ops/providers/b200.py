@@ -376,8 +376,11 @@ class B200QKNormRope(_B200Op):
     def __call__(self, qkv, n_q, n_kv, head_dim, q_weight, k_weight, cos, sin, eps=1e-6):
         if not _ok(qkv, q_weight, k_weight) or head_dim != 128 or qkv.dim() != 2 or qkv.stride(1) != 1:
             return N.TorchQKNormRope()(qkv, n_q, n_kv, head_dim, q_weight, k_weight, cos, sin, eps)
-        return QKNormRopeFn.apply(qkv, n_q, n_kv, head_dim, q_weight, k_weight, cos.float().contiguous(),
-                                  sin.float().contiguous(), eps)
+        if qkv.data_ptr() % 8 or qkv.stride(0) % 4:        # the kernel reads four channels at a time
+            qkv = qkv.clone(memory_format=torch.contiguous_format)
+        if q_weight is not None:
+            q_weight, k_weight = _aligned(q_weight), _aligned(k_weight)
+        return QKNormRopeFn.apply(qkv, n_q, n_kv, head_dim, q_weight, k_weight, _aligned(cos.float()), _aligned(sin.float()), eps)
 
 
 def _rope_rows(x: torch.Tensor) -> torch.Tensor:
