@@ -494,7 +494,7 @@ def cross_entropy(logits, labels, *, grad_out=None, grad_scale=None, grad_scale_
 # --------------------------------------------------------------------------------------
 # Multi-tensor AdamW / grad norm
 # --------------------------------------------------------------------------------------
-ADAM_CHUNK = 65536
+ADAM_CHUNK = 16384
 
 
 class MultiTensorPlan:
@@ -509,7 +509,7 @@ class MultiTensorPlan:
         self.device = self.params[0].device
         n = len(self.params)
         self.host_meta = torch.zeros(n, 7, dtype=torch.int64).pin_memory()
-        chunks = []
+        counts = []
         for i, p in enumerate(self.params):
             assert p.dtype == torch.float32 and p.is_contiguous()
             self.host_meta[i, 0] = p.data_ptr()
@@ -517,10 +517,12 @@ class MultiTensorPlan:
             self.host_meta[i, 3] = exp_avg_sq[i].data_ptr()
             self.host_meta[i, 4] = shadows[i].data_ptr() if shadows is not None and shadows[i] is not None else 0
             self.host_meta[i, 5] = p.numel()
-            for c in range((p.numel() + ADAM_CHUNK - 1) // ADAM_CHUNK):
-                chunks.append((i, c))
-        self.n_chunks = len(chunks)
-        self.chunks = torch.tensor(chunks, dtype=torch.int32, device=self.device).reshape(-1, 2)
+            counts.append((p.numel() + ADAM_CHUNK - 1) // ADAM_CHUNK)
+        counts = torch.tensor(counts)
+        self.n_chunks = int(counts.sum())
+        tensor = torch.repeat_interleave(torch.arange(n), counts)
+        chunk = torch.arange(self.n_chunks) - torch.repeat_interleave(counts.cumsum(0) - counts, counts)
+        self.chunks = torch.stack((tensor, chunk), 1).to(torch.int32).contiguous().to(self.device)
         self.meta = torch.empty(n, 7, dtype=torch.int64, device=self.device)
         self.partial = torch.empty(max(self.n_chunks, 1), dtype=torch.float32, device=self.device)
 
