@@ -86,6 +86,7 @@ struct GemmParams {
   __nv_bfloat16* preact;  // optional [M, ld_preact] receives gate|up
   long long ld_preact;
   const float* alpha;     // optional device scalar multiplied into the product (plain stores)
+  int k_splits, kb_per_split;  // > 1: "group" g covers k-blocks [g, g + 1) * kb_per_split of one product, stored at C[g]
 };
 
 template <int BN, bool A_MN, bool B_MN>
@@ -166,7 +167,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int groups = p.groups_k > 0 ? p.groups_k : 1;
+  const int groups = p.groups_k > 0 ? p.groups_k : p.k_splits;
   const long long tiles_per_group = static_cast<long long>(p.m_tiles) * p.n_tiles;
   const long long total_tiles = s_dead ? 0 : tiles_per_group * groups;
 
@@ -186,12 +187,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     nt = static_cast<int>(w / band_rows);
     mt = m_base + static_cast<int>(w - static_cast<long long>(nt) * band_rows);
   };
-  // k-range of a tile: dense -> [0, K); grouped-K -> rows of group g.
+  // k-range of a tile: dense -> [0, K); split -> its share of [0, K); grouped-K -> rows of group g.
   auto krange = [&](int g, int& k0, int& nkb) {
     if (p.groups_k > 0) {
       int r0 = p.group_rows[g], r1 = p.group_rows[g + 1];
       k0 = r0;
       nkb = (r1 - r0) / BK;
+    } else if (p.k_splits > 1) {
+      const int kb0 = g * p.kb_per_split;
+      k0 = kb0 * BK;
+      nkb = min(p.kb_per_split, (p.K + BK - 1) / BK - kb0);
     } else {
       k0 = 0;
       nkb = (p.K + BK - 1) / BK;
@@ -749,6 +754,8 @@ struct GemmArgs {
   int num_sms;
   const struct EpFuseArgs* ep;   // optional expert-parallel fusion (grouped-M launches only)
   const float* alpha;            // optional device scalar multiplied into the product (plain stores only)
+  float* split_ws;               // optional fp32 [k_splits, M, N]: the product is formed in k_splits pieces, then added up
+  int k_splits;
 };
 
 // Host description of the expert-parallel fusion of one launch (C ABI; see `EpFuse` for the meaning of the fields).
@@ -779,6 +786,44 @@ struct EpFuseArgs {
   unsigned int* done_counter;
   int ret_rows;
 };
+
+// C (+)= alpha * sum_s ws[s] (+ residual): the second half of a split product, in a fixed order.  Four columns per thread.
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ ws, int splits, int M, int N, void* C, long long ldc, int c_fp32, int accumulate,
+                 const __nv_bfloat16* __restrict__ residual, long long ldr, const float* __restrict__ alpha) {
+  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int nv = N / 4;
+  if (idx >= static_cast<long long>(M) * nv) return;
+  const long long r = idx / nv;
+  const int c = static_cast<int>(idx - r * nv) * 4;
+  const long long plane = static_cast<long long>(M) * N;
+  const float* src = ws + r * N + c;
+  float4 v = *reinterpret_cast<const float4*>(src);
+#pragma unroll 4
+  for (int s = 1; s < splits; ++s) {
+    const float4 u = *reinterpret_cast<const float4*>(src + s * plane);
+    v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+  }
+  if (alpha) { const float a = __ldg(alpha); v.x *= a; v.y *= a; v.z *= a; v.w *= a; }
+  if (c_fp32) {
+    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(C) + r * ldc + c);
+    if (accumulate) { const float4 o = *dst; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+    *dst = v;
+  } else {
+    uint2* dst = reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(C) + r * ldc + c);
+    if (residual) {
+      const uint2 u = *reinterpret_cast<const uint2*>(residual + r * ldr + c);
+      const float2 x = unpack_bf16(u.x), y = unpack_bf16(u.y);
+      v.x += x.x; v.y += x.y; v.z += y.x; v.w += y.y;
+    }
+    if (accumulate) {
+      const uint2 u = *dst;
+      const float2 x = unpack_bf16(u.x), y = unpack_bf16(u.y);
+      v.x += x.x; v.y += x.y; v.z += y.x; v.w += y.y;
+    }
+    *dst = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  }
+}
 
 template <int BN, bool A_MN, bool B_MN, int EPI>
 static int launch(const GemmArgs& a, cudaStream_t stream) {
@@ -863,6 +908,15 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
   p.tile_group = a.tile_group; p.group_rows = a.group_rows;
   p.F = a.F; p.row_scale = a.row_scale; p.alpha = a.alpha;
   p.preact = reinterpret_cast<__nv_bfloat16*>(a.preact); p.ld_preact = a.ld_preact;
+  p.k_splits = 1; p.kb_per_split = 0;
+  const bool split = a.split_ws != nullptr && a.k_splits > 1;
+  if (split) {
+    const int nkb = (a.K + BK - 1) / BK;
+    p.kb_per_split = (nkb + a.k_splits - 1) / a.k_splits;
+    p.k_splits = (nkb + p.kb_per_split - 1) / p.kb_per_split;     // every piece has at least one k-block
+    p.C = a.split_ws; p.ldc = a.N; p.c_group_stride = static_cast<long long>(a.M) * a.N;
+    p.c_fp32 = 1; p.accumulate = 0; p.residual = nullptr; p.alpha = nullptr;
+  }
 
   auto kfn = gemm_kernel<BN, A_MN, B_MN, EPI>;
   static bool smem_done[16] = {};
@@ -870,10 +924,16 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
     const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), L::TOTAL, smem_done);
     if (e != cudaSuccess) return 300 + static_cast<int>(e);
   }
-  long long total = static_cast<long long>(p.m_tiles) * p.n_tiles * (p.groups_k > 0 ? p.groups_k : 1);
+  long long total = static_cast<long long>(p.m_tiles) * p.n_tiles * (p.groups_k > 0 ? p.groups_k : p.k_splits);
   if (total <= 0) return 0;
   int grid = static_cast<int>(total < a.num_sms ? total : a.num_sms);
   kfn<<<grid, p.ep.push_on ? GEMM_THREADS_PUSH : GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, p);
+  if (split) {
+    const long long n = static_cast<long long>(a.M) * (a.N / 4);
+    split_sum_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
+        a.split_ws, p.k_splits, a.M, a.N, a.C, a.ldc, a.c_fp32, a.accumulate, reinterpret_cast<const __nv_bfloat16*>(a.residual), a.ldr,
+        a.alpha);
+  }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + static_cast<int>(e);
 }
@@ -894,6 +954,8 @@ TTB_EXPORT int ttb_gemm_bf16(const ttb::GemmArgs* args, void* stream_ptr) {
   if (a.residual && ((a.ldr % 8) || (reinterpret_cast<uintptr_t>(a.residual) & 15))) return 904;
   if (a.epi == EPI_SWIGLU && ((a.F % 8) || a.c_fp32 || (a.preact && (a.ld_preact % 8)))) return 905;
   if (a.alpha && a.epi != EPI_STORE) return 905;
+  if (a.split_ws && (a.epi != EPI_STORE || a.tile_group || a.groups_k > 0 || a.ep || (a.N % 8) || (reinterpret_cast<uintptr_t>(a.split_ws) & 15)))
+    return 909;
   if (a.ep) {
     const EpFuseArgs& e = *a.ep;
     if (!a.tile_group || a.groups_k > 0 || e.W < 1 || e.W > MAX_RANKS || e.El < 1 || e.El * e.W > 1024 || !e.status) return 906;
