@@ -33,6 +33,7 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
   dc_load_rows<256>(sK, p.k + row0 * p.k_t + h * p.k_h, p.k_t, n);
   dc_load_rows<256>(sV, p.v + row0 * p.v_t + h * p.v_h, p.v_t, n);
   dc_load_gates(p, row0, n, h, sG, sB);
+  dc_wait();
   __syncthreads();
   dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
   dc_row_norms<256>(sK, sRk, p.l2, 1.f);
@@ -154,6 +155,7 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
   dc_load_f32<256, DC_C, 64>(sX, DO_LD, X + hc * DC_C * DC_D + v0, DC_D);
   dc_load_f32<256, DC_C, 64>(sA, DP_LT, Ag + hc * DC_C * DC_C, DC_C);
   if (threadIdx.x < DC_C) sG[threadIdx.x] = threadIdx.x < n ? __ldg(p.g + static_cast<long long>(row0 + threadIdx.x) * p.H + h) : 0.f;
+  dc_wait();
   __syncthreads();
   dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
   if (warp == 0) dc_cumsum(sG, lane);
@@ -235,6 +237,7 @@ delta_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO,
   dc_load_rows<256>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
   dc_load_f32<256, DC_C, 64>(sA, DO_LD, Ag + hc * DC_C * DC_C, DC_C);
   if (threadIdx.x < DC_C) sG[threadIdx.x] = threadIdx.x < n ? __ldg(p.g + static_cast<long long>(row0 + threadIdx.x) * p.H + h) : 0.f;
+  dc_wait();
   __syncthreads();
   dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
   if (warp == 0) dc_cumsum(sG, lane);
@@ -356,6 +359,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   dc_load_rows<NT>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
   dc_load_f32<NT, DC_C, DC_D>(sX, DQ_LD, X + hc * DC_C * DC_D, DC_D);
   dc_load_gates(p, row0, n, h, sG, sB);
+  dc_wait();
   __syncthreads();
   dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
   dc_row_norms<NT>(sK, sRk, p.l2, 1.f);
@@ -445,6 +449,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
       }
     }
   }
+  dc_wait();
   __syncthreads();                               // S, P and R are complete
   // ---- d(q^ e^G) = do S^T, d(beta k^ e^G) = -db S^T, then the score terms R k^, P k^ on the same accumulators
   float dq[4][4] = {}, dk[4][4] = {};

@@ -16,7 +16,8 @@
 // two terms and three products where both sides are fp32.  Norms, decays and masks are applied to fp32 accumulators or
 // fp32 operands, never to the bf16 inputs.
 //
-// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.17 ms, out 0.16, bwd_pre 0.12, bwd_post 0.53; a
+// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.14 ms, out 0.11, bwd_pre 0.09, bwd_post 0.45 (0.17, 0.16,
+// 0.12 and 0.53 while the tiles came in one after the other through registers); with the first form of these kernels a
 // gated-delta-net layer forward + backward went from 10.43 to 3.96 ms.  Before, the chunk-parallel part was about 250
 // launches of fp32 products, element-wise passes and gathers over materialised [chunk, 64, 64 .. 128] tensors.
 //
@@ -149,25 +150,29 @@ __device__ __forceinline__ void dc_mma22(float (&c)[4], const uint32_t (&ah)[4],
   dc_mma(c, ah, bh[0], bh[1]);
 }
 
-// 64 x 128 bf16 rows of one head -> shared tile; rows past `n` are zero
+// Tiles come in by asynchronous copies, so that all tiles of a kernel are on their way together; `dc_wait` before the barrier
+// that publishes them.  64 x 128 bf16 rows of one head -> shared tile; rows past `n` are zero (nothing is read for them).
+__device__ __forceinline__ void dc_copy16(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void dc_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template <int NT>
 __device__ __forceinline__ void dc_load_rows(__nv_bfloat16* s, const __nv_bfloat16* base, long long row_stride, int n) {
 #pragma unroll
   for (int i = threadIdx.x; i < DC_C * 16; i += NT) {
     const int r = i >> 4, c = (i & 15) * 8;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r < n) v = __ldg(reinterpret_cast<const uint4*>(base + r * row_stride + c));
-    *reinterpret_cast<uint4*>(s + r * DC_QS + c) = v;
+    dc_copy16(s + r * DC_QS + c, base + (r < n ? r * row_stride + c : 0), r < n ? 16 : 0);
   }
 }
 // fp32 [rows][cols] tile with row stride `src_ld` -> shared with row stride `ld`
 template <int NT, int ROWS, int COLS>
 __device__ __forceinline__ void dc_load_f32(float* s, int ld, const float* src, int src_ld) {
   constexpr int V = COLS / 4;
-#pragma unroll 4
+#pragma unroll
   for (int i = threadIdx.x; i < ROWS * V; i += NT) {
     const int r = i / V, c = (i - r * V) * 4;
-    *reinterpret_cast<float4*>(s + r * ld + c) = __ldg(reinterpret_cast<const float4*>(src + static_cast<long long>(r) * src_ld + c));
+    dc_copy16(s + r * ld + c, src + static_cast<long long>(r) * src_ld + c, 16);
   }
 }
 // 1 / |row| of a tile (or 1 without normalisation), times `mul`

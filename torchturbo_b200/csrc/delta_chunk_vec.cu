@@ -21,7 +21,8 @@ namespace ttb {
 constexpr int DV_G = 132;    // row stride of G and of tiles read down their columns
 constexpr int DV_A = 136;    // row stride of fp32 tiles read in pairs along a row
 
-// G (units of log2) of a chunk: cumulative sums down 64 rows for 128 channels.  Starts without, ends with a barrier.
+// G (units of log2) of a chunk: cumulative sums down 64 rows for 128 channels.  Starts without, ends with a barrier, which also
+// publishes the tiles that this thread block has asked for before.
 template <int NT>
 __device__ __forceinline__ void dv_cumsum(const DeltaChunkIn& p, float* sG, int ld, int row0, int n, int h) {
   constexpr int PARTS = NT / 128, ROWS = 64 / PARTS;
@@ -31,6 +32,7 @@ __device__ __forceinline__ void dv_cumsum(const DeltaChunkIn& p, float* sG, int 
   float v[ROWS];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) v[r] = part * ROWS + r < n ? __ldg(src + (part * ROWS + r) * step) : 0.f;
+  dc_wait();
   float run = 0.f;
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
@@ -175,6 +177,7 @@ delta_vec_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __res
     }
     *reinterpret_cast<uint4*>(Ko + (hc * DC_C + i) * DC_D + j) = u;
   }
+  dc_wait();                                     // v; published by the barriers of the inversion
   dc_invert(sL, sT);
   {
     float* Tout = Tg + hc * DC_C * DC_C;
