@@ -180,7 +180,8 @@ class GatedDeltaNet(nn.Module):
             qkv, w = torch.cat((q.reshape(Tg, -1), k.reshape(Tg, -1), v.reshape(Tg, -1)), -1), torch.cat((wq, wk, wv), 0)
         cu = ctx.cu_seqlens
         mixed, _ = ops.causal_conv1d(qkv.unsqueeze(0), w, None, activation="silu", cu_seqlens=cu)
-        q, k, v = mixed[0].split([hk * self.dk, hk * self.dk, hv * self.dv], dim=-1)
+        # views of the one row (an index into the batch dimension would cost a cleared buffer and a copy in the backward)
+        q, k, v = mixed.squeeze(0).split([hk * self.dk, hk * self.dk, hv * self.dv], dim=-1)
         q, k, v = q.reshape(1, Tg, hk, self.dk), k.reshape(1, Tg, hk, self.dk), v.reshape(1, Tg, hv, self.dv)
         beta = torch.sigmoid(b.float()).unsqueeze(0)
         g = (-A_log.float().exp() * F.softplus(a.float() + dt_bias.float())).unsqueeze(0)
@@ -188,7 +189,7 @@ class GatedDeltaNet(nn.Module):
             # every key head serves hv / hk value heads; as a broadcast its gradient is a plain sum over them
             q, k = (t.unsqueeze(3).expand(1, Tg, hk, hv // hk, self.dk).reshape(1, Tg, hv, self.dk) for t in (q, k))
         o, _ = ops.gated_delta_rule(q, k, v, g, beta, use_qk_l2norm_in_kernel=True, cu_seqlens=cu)
-        o = o[0]                                                            # [Tg, hv, dv]
+        o = o.squeeze(0)                                                    # [Tg, hv, dv]
         if sp > 1:
             o = gather_heads_scatter_seq(o.contiguous(), ctx.sp_group, sp)  # [T_local, n_v, dv]
         o = self.norm(o.reshape(-1, self.dv), z.reshape(-1, self.dv)).reshape(T, self.value_dim)
@@ -344,7 +345,7 @@ class KimiDeltaAttention(nn.Module):
         o, _ = ops.kda(q, k, v, g.unsqueeze(0), beta.unsqueeze(0), A_log=A_log, dt_bias=dt_bias,
                        use_qk_l2norm_in_kernel=True, use_beta_sigmoid_in_kernel=True, use_gate_in_kernel=True,
                        safe_gate=self.gate_lower_bound is not None, lower_bound=self.gate_lower_bound, cu_seqlens=cu)
-        o = o[0]
+        o = o.squeeze(0)
         if sp > 1:
             o = gather_heads_scatter_seq(o.contiguous(), ctx.sp_group, sp)
         gate = ops.linear(ops.linear(x, self.g_a_proj.weight), self.g_b_proj.weight) if self.low_rank \

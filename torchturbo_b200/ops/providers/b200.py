@@ -319,7 +319,7 @@ class B200CausalConv1d(_B200Op):
                                        output_final_state=output_final_state, cu_seqlens=cu_seqlens, packed_params=packed_params)
         T = x.shape[1]
         start, end = _seq_bounds(cu_seqlens, T, x.device)
-        y = CausalConv1dFn.apply(x[0].contiguous(), weight.contiguous(), bias, start, end, activation is not None)
+        y = CausalConv1dFn.apply(x.squeeze(0).contiguous(), weight.contiguous(), bias, start, end, activation is not None)
         return y.unsqueeze(0), None
 
 
