@@ -163,11 +163,12 @@ class FusedAdamW(torch.optim.Optimizer):
             if not ps:
                 continue
             states = [self._init_state(p) for p in ps]
-            for st in states:
-                st["step"] += 1
+            torch._foreach_add_([st["step"] for st in states], 1)
             step = int(states[0]["step"].item())
             lp0 = _local(ps[0])
             if lp0.is_cuda and K.available():
+                # before the update is launched: the next step's host waits for this copy, not for the update behind it
+                self._note_clip(clip, states)
                 side = [(p, st) for p, st in zip(ps, states) if self._overlappable(p)] if self._buckets else []
                 if side:
                     taken = {id(p) for p, _ in side}
@@ -177,7 +178,6 @@ class FusedAdamW(torch.optim.Optimizer):
                     self._step_side(gi, group, side, step, clip, prescale)
                 else:
                     self._step_cuda(gi, group, ps, states, step, clip, prescale)
-                self._note_clip(clip, states)
             else:
                 self._step_torch(group, ps, states, step, clip, prescale)
         return loss

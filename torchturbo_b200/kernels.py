@@ -532,16 +532,14 @@ class MultiTensorPlan:
         self.device = self.params[0].device
         n = len(self.params)
         self.host_meta = torch.zeros(n, 7, dtype=torch.int64).pin_memory()
-        counts = []
-        for i, p in enumerate(self.params):
-            assert p.dtype == torch.float32 and p.is_contiguous()
-            self.host_meta[i, 0] = p.data_ptr()
-            self.host_meta[i, 2] = exp_avg[i].data_ptr()
-            self.host_meta[i, 3] = exp_avg_sq[i].data_ptr()
-            self.host_meta[i, 4] = shadows[i].data_ptr() if shadows is not None and shadows[i] is not None else 0
-            self.host_meta[i, 5] = p.numel()
-            counts.append((p.numel() + ADAM_CHUNK - 1) // ADAM_CHUNK)
-        counts = torch.tensor(counts)
+        assert all(p.dtype == torch.float32 and p.is_contiguous() for p in self.params)
+        rows = self.host_meta.numpy()
+        rows[:, 0] = [p.data_ptr() for p in self.params]
+        rows[:, 2] = [t.data_ptr() for t in exp_avg[:n]]
+        rows[:, 3] = [t.data_ptr() for t in exp_avg_sq[:n]]
+        rows[:, 4] = [t.data_ptr() if t is not None else 0 for t in (shadows[:n] if shadows is not None else [None] * n)]
+        rows[:, 5] = [p.numel() for p in self.params]
+        counts = (self.host_meta[:, 5] + ADAM_CHUNK - 1) // ADAM_CHUNK
         self.n_chunks = int(counts.sum())
         tensor = torch.repeat_interleave(torch.arange(n), counts)
         chunk = torch.arange(self.n_chunks) - torch.repeat_interleave(counts.cumsum(0) - counts, counts)
@@ -555,10 +553,11 @@ class MultiTensorPlan:
         ev = getattr(self, "_copy_event", None)
         if ev is not None:
             ev.synchronize()
-        for i, g in enumerate(grads):
-            assert g.is_contiguous() and g.numel() == self.host_meta[i, 5]
-            self.host_meta[i, 1] = g.data_ptr()
-            self.host_meta[i, 6] = int(g.dtype == torch.bfloat16)
+        # the table through a numpy view: an element assignment to a tensor costs microseconds, and there are two per gradient
+        rows = self.host_meta.numpy()
+        assert rows[:, 5].tolist() == [g.numel() for g in grads] and all(g.is_contiguous() for g in grads)
+        rows[:, 1] = [g.data_ptr() for g in grads]
+        rows[:, 6] = [g.dtype == torch.bfloat16 for g in grads]
         self.meta.copy_(self.host_meta, non_blocking=True)
         if self.device.type == "cuda":
             self._copy_event = torch.cuda.Event()
