@@ -338,12 +338,21 @@ __global__ void router_bwd_kernel(const RouterBwdParams p) {
   }
 }
 
-__global__ void colsum_f32_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows, int cols) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+// 32 columns and 32 row groups per block, fixed order (296 x 128 partial sums: 11 us with one thread per column)
+__global__ void __launch_bounds__(1024)
+colsum_f32_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows, int cols) {
+  __shared__ float part[32][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + x;
   float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += partial[static_cast<long long>(r) * cols + c];
-  out[c] = s;
+  if (c < cols) {
+#pragma unroll 4
+    for (int r = y; r < rows; r += 32) s += partial[static_cast<long long>(r) * cols + c];
+  }
+  part[y][x] = s;
+  __syncthreads();
+  s = warp_sum(part[x][y]);
+  if (x == 0 && blockIdx.x * 32 + y < cols) out[blockIdx.x * 32 + y] = s;
 }
 
 // ============================================================================
@@ -595,7 +604,7 @@ TTB_EXPORT int ttb_router_fwd(const float* logits, const float* expert_bias, con
   if (grid > need) grid = (int)need;
   router_fwd_kernel<<<grid, 256, E * sizeof(float), STREAM(stream)>>>(p);
   if (score_partial && score_sum)
-    colsum_f32_kernel<<<(E + 127) / 128, 128, 0, STREAM(stream)>>>(score_partial, score_sum, grid, E);
+    colsum_f32_kernel<<<(E + 31) / 32, 1024, 0, STREAM(stream)>>>(score_partial, score_sum, grid, E);
   LAUNCH_RET();
 }
 

@@ -152,6 +152,7 @@ class RMSNormFn(torch.autograd.Function):
         ctx.save_for_backward(xsum, w, rstd)
         ctx.one_plus_w = one_plus_w
         ctx.has_res = residual is not None
+        ctx.set_materialize_grads(False)       # the last norm of a decoder returns a sum that nothing reads
         if residual is not None:
             return y, xsum
         return y
@@ -159,6 +160,8 @@ class RMSNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dsum=None):
         xsum, w, rstd = ctx.saved_tensors
+        if dy is None:
+            dy = torch.zeros_like(xsum)
         dx, dw = K.rmsnorm_bwd(dy.contiguous(), xsum, w, rstd, dres=dsum.contiguous() if dsum is not None else None,
                                one_plus_w=ctx.one_plus_w, dw_dtype=w.dtype)
         return dx, dw, None, (dx if ctx.has_res else None), None
@@ -426,6 +429,7 @@ class RouterFn(torch.autograd.Function):
         ctx.save_for_backward(logits, out["topk_idx"], out["topk_prob"], valid_mask)
         ctx.cfg = (k, score_fn, scaling)
         ctx.mark_non_differentiable(out["topk_idx"], out["aux_counts"], out["counts"])
+        ctx.set_materialize_grads(False)       # no cleared buffers for the index outputs and for statistics nobody used
         return out["topk_idx"], out["topk_prob"], out["score_sum"], out["lse"], out["aux_counts"], out["counts"]
 
     @staticmethod
@@ -463,8 +467,9 @@ class PermuteFn(torch.autograd.Function):
                                       seg_start=pm["seg_start"], val=probs.reshape(-1).contiguous() if probs is not None else None)
         ctx.save_for_backward(pm["row_of"])
         ctx.dims = (T, k, probs is not None)
-        for t in (pm["row_of"], pm["counts"], pm["seg_start"], pm["tile_group"]):
-            ctx.mark_non_differentiable(t)
+        ctx.token_like = (tokens.shape, tokens.dtype, tokens.device)
+        ctx.mark_non_differentiable(pm["row_of"], pm["counts"], pm["seg_start"], pm["tile_group"])
+        ctx.set_materialize_grads(False)
         if row_prob is None:
             row_prob = tokens.new_empty(0, dtype=torch.float32)
         return xp, row_prob, pm["row_of"], pm["counts"], pm["seg_start"], pm["tile_group"]
@@ -473,8 +478,12 @@ class PermuteFn(torch.autograd.Function):
     def backward(ctx, dxp, drow_prob, *_):
         (row_of,) = ctx.saved_tensors
         T, k, has_p = ctx.dims
-        dtok = K.perm_combine(dxp.contiguous(), row_of, T, k)
-        dprobs = drow_prob.index_select(0, row_of.long()).view(T, k) if has_p and drow_prob is not None else None
+        shape, dtype, dev = ctx.token_like
+        dtok = K.perm_combine(dxp.contiguous(), row_of, T, k) if dxp is not None else torch.zeros(shape, dtype=dtype, device=dev)
+        dprobs = None
+        if has_p:
+            dprobs = drow_prob.index_select(0, row_of.long()).view(T, k) if drow_prob is not None else \
+                torch.zeros(T, k, dtype=torch.float32, device=dev)
         return dtok, dprobs, None, None
 
 
