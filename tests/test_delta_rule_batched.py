@@ -203,3 +203,34 @@ def test_fused_chunk_kernels_on_bf16_rows_match_the_fp32_formulation(vec, cu, T,
         assert a.shape == b.shape
         assert (a - b).abs().max() <= 2e-2 * max(1.0, b.abs().max()), (name, (a - b).abs().max(), b.abs().max())
         assert (a - b).norm() <= 2e-2 * b.norm() + 1e-6, (name, (a - b).norm() / b.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H, lens", [(1, [3]), (18, [1, 0, 4]), (19, [2, 1, 1, 2]), (40, [1, 2])])
+@pytest.mark.parametrize("vec", [False, True])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_recurrence_over_both_column_splits(H, lens, vec, reverse):
+    """Few (sequence, head) pairs spread their columns over four CTAs, many over two; both against the torch loop on the
+    operands rounded as the kernel rounds them (bf16 A, B, S and X inside the products: 2^-8 of the largest entry a step)."""
+    from torchturbo_b200 import kernels as K
+
+    gen = torch.Generator().manual_seed(H)
+    NC, nseq = sum(lens), len(lens)
+    seq, c = [], 0
+    for n in lens:
+        seq.append((c, n))
+        c += n
+    a, b = (torch.randn(H, NC, 64, 128, generator=gen).to(torch.bfloat16) * 0.05 for _ in range(2))
+    u = torch.randn(H, NC, 64, 128, generator=gen)
+    decay = torch.rand(H, NC, *([128] if vec else []), generator=gen)
+    init = None if reverse else torch.randn(H, nseq, 128, 128, generator=gen)
+    add = torch.randn(H, NC + nseq, 128, 128, generator=gen) if reverse else None
+    dev = lambda t: t.cuda() if t is not None else None                                            # noqa: E731
+    x, st = K.delta_state_scan(a.cuda(), b.cuda(), u.cuda(), decay.cuda(), dev(init), dev(add),
+                               torch.tensor(seq, dtype=torch.int32).cuda(), reverse=reverse, s1=-1.0, s2=1.0)
+    torch.cuda.synchronize()
+    assert K.status() == (0, 0)
+    wx, ws = _scan_torch(u, a.float(), b.float(), decay, init, seq, reverse=reverse, add=add)
+    for got, want in ((x, wx), (st, ws)):
+        err = (got.cpu() - want).abs().max()
+        assert err <= 2 ** -8 * len(lens) * want.abs().max(), (err, want.abs().max())
