@@ -102,7 +102,7 @@ def lib():
 
 # kernels launched per C entry point (used to report how many of this library's kernels ran in a region)
 _LAUNCHES_PER_CALL = {"ttb_rmsnorm_bwd": 2, "ttb_gated_rmsnorm_bwd": 2, "ttb_layernorm_bwd": 2, "ttb_bias_act_bwd": 2, "ttb_causal_conv1d_bwd": 2,
-                      "ttb_causal_conv1d_row_blocks": 0, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
+                      "ttb_causal_conv1d_row_blocks": 0, "ttb_kda_gate_bwd": 2, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
                       "ttb_ep_combine_all": 3, "ttb_delta_vec_bwd_post": 2, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
                       "ttb_gemm_status": 0}
 LAUNCH_COUNT = 0
@@ -467,6 +467,35 @@ def rope(x, cos, sin, sign: float = 1.0):
     _check(lib().ttb_rope(_p(x), C.c_longlong(x.stride(0)), C.c_longlong(x.stride(1)), _p(cos), _p(sin), _p(y), C.c_longlong(T),
                           C.c_int(heads), C.c_int(D // 2), C.c_float(sign), _stream()), "ttb_rope")
     return y
+
+
+# --------------------------------------------------------------------------------------
+# Kimi delta attention gate
+# --------------------------------------------------------------------------------------
+def _gate_args(g, A_log, dt_bias, lower_bound):
+    half = torch.bfloat16
+    return (_p(g), _p(A_log), C.c_int(int(A_log.dtype == half)), _p(dt_bias), C.c_int(int(dt_bias is not None and dt_bias.dtype == half))), \
+        (C.c_longlong(g.shape[0]), C.c_int(g.shape[1]), C.c_int(int(lower_bound is not None)), C.c_float(lower_bound or 0.0), _stream())
+
+
+def kda_gate_fwd(g, A_log, dt_bias, lower_bound):
+    """Log decay fp32 [rows, H, 128] from the bf16 projection `g`; A_log [H] and dt_bias [H * 128] (or None) in bf16 or fp32."""
+    out = torch.empty(g.shape, dtype=torch.float32, device=g.device)
+    head, tail = _gate_args(g, A_log, dt_bias, lower_bound)
+    _check(lib().ttb_kda_gate_fwd(*head, _p(out), *tail), "ttb_kda_gate_fwd")
+    return out
+
+
+def kda_gate_bwd(dd, g, A_log, dt_bias, lower_bound):
+    """(dg bf16, d(dt) fp32 [H * 128], channel sums of d(A_log) fp32 [H, 128])."""
+    R, H, D = g.shape
+    dg = torch.empty_like(g)
+    blocks = int(lib().ttb_kda_gate_row_blocks(C.c_longlong(R), C.c_int(H)))
+    part = torch.empty(max(blocks, 1), 2, H * D, dtype=torch.float32, device=g.device)
+    sums = (torch.empty if R else torch.zeros)(2, H * D, dtype=torch.float32, device=g.device)
+    head, tail = _gate_args(g, A_log, dt_bias, lower_bound)
+    _check(lib().ttb_kda_gate_bwd(_p(dd), *head, _p(dg), _p(part), _p(sums), *tail), "ttb_kda_gate_bwd")
+    return dg, sums[0], sums[1].view(H, D)
 
 
 # --------------------------------------------------------------------------------------

@@ -319,6 +319,33 @@ def chunk_delta_rule_batched(q, k, v, g, beta, scale=None, initial_state=None, o
     return o.to(dt), final
 
 
+class KDAGate(torch.autograd.Function):
+    """`kda_gate` on bf16 rows of 128-wide heads: one kernel forward, one and a column sum backward."""
+
+    @staticmethod
+    def forward(ctx, g, A_log, dt_bias, lower_bound):
+        ctx.save_for_backward(g, A_log, dt_bias)
+        ctx.lower_bound = lower_bound
+        return K.kda_gate_fwd(g, A_log, dt_bias, lower_bound)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dd):
+        g, A_log, dt_bias = ctx.saved_tensors
+        dg, ddt, da = K.kda_gate_bwd(dd.contiguous(), g, A_log, dt_bias, ctx.lower_bound)
+        return dg, da.sum(-1).to(A_log.dtype), (ddt.to(dt_bias.dtype) if dt_bias is not None else None), None
+
+
+def _gate(g, A_log, dt_bias, lower_bound):
+    H, Kd = g.shape[-2:]
+    plain = (torch.bfloat16, torch.float32)
+    if (_kernel_ok(g, Kd, 128) and g.dtype == torch.bfloat16 and A_log.is_cuda and A_log.shape == (H,) and A_log.dtype in plain
+            and (dt_bias is None or (dt_bias.is_cuda and dt_bias.numel() == H * Kd and dt_bias.dtype in plain))):
+        dt = dt_bias.reshape(H * Kd).contiguous() if dt_bias is not None else None
+        return KDAGate.apply(g.reshape(-1, H, Kd).contiguous(), A_log.contiguous(), dt, lower_bound).view(g.shape)
+    return kda_gate(g, A_log, dt_bias, lower_bound)
+
+
 def _register(op_name: str, impl_name: str):
     return register_op(op_name=op_name, impl_name=impl_name, kind=OpImplKind.CUSTOM, priority=100, devices=(TurboDevice.CUDA,))
 
@@ -357,7 +384,7 @@ class B200KDA(OpImpl):
         if use_gate_in_kernel:
             if A_log is None:
                 raise ValueError("use_gate_in_kernel needs A_log")
-            g = kda_gate(g, A_log, dt_bias, lower_bound if safe_gate else None)
+            g = _gate(g, A_log, dt_bias, lower_bound if safe_gate else None)
         if use_beta_sigmoid_in_kernel:
             beta = torch.sigmoid(beta.float())
         return chunk_delta_rule_batched(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens,
