@@ -56,8 +56,8 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
         if (np > mi) continue;
         uint32_t b[4];
         dc_b(b, sK, np * 16, kk * 16, lane);
-        dc_mma(acc[2 * np], a, b[0], b[1]);
-        dc_mma(acc[2 * np + 1], a, b[2], b[3]);
+        dc_mma11(acc[2 * np], a, b[0], b[1]);
+        dc_mma11(acc[2 * np + 1], a, b[2], b[3]);
       }
     }
     float* Aout = Ag + hc * DC_C * DC_C;
@@ -96,11 +96,8 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
       for (int np = 0; np < 4; ++np) {
         uint32_t b[4];
         dc_b_t(b, which ? sK : sV, n0 + np * 16, kk * 16, lane);
-#pragma unroll
-        for (int i = 2; i >= 0; --i) {
-          dc_mma(acc[2 * np], a[i], b[0], b[1]);
-          dc_mma(acc[2 * np + 1], a[i], b[2], b[3]);
-        }
+        dc_mma31(acc[2 * np], a, b[0], b[1]);
+        dc_mma31(acc[2 * np + 1], a, b[2], b[3]);
       }
     }
 #pragma unroll
@@ -170,8 +167,7 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
     for (int mi = 0; mi < 4; ++mi) {
       uint32_t a[4];
       dc_a(a, sQ, mi * 16, kk * 16, lane);
-#pragma unroll
-      for (int i = 2; i >= 0; --i) dc_mma(acc[mi], a, b[i][0], b[i][1]);
+      dc_mma13(acc[mi], a, b);
     }
   }
 #pragma unroll
@@ -186,13 +182,13 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
   }
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk) {
-    uint32_t b[2][2];
-    dc_bf_t<2>(b, sX, DO_LD, n0, kk * 16, lane);
+    uint32_t b[3][2];
+    dc_bf_t<3>(b, sX, DO_LD, n0, kk * 16, lane);
 #pragma unroll
     for (int mi = kk; mi < 4; ++mi) {
-      uint32_t a[2][4];
-      dc_af<2>(a, sA, DP_LT, mi * 16, kk * 16, lane);
-      dc_mma22(acc[mi], a[0], a[1], b[0], b[1]);
+      uint32_t a[3][4];
+      dc_af<3>(a, sA, DP_LT, mi * 16, kk * 16, lane);
+      dc_mma33(acc[mi], a, b);
     }
   }
   __syncthreads();
@@ -255,11 +251,8 @@ delta_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO,
       for (int mi = 0; mi <= kk; ++mi) {           // rows j of A^T meet rows i >= j only
         uint32_t a[3][4];
         dc_af_t<3>(a, sA, DO_LD, mi * 16, kk * 16, lane);
-#pragma unroll
-        for (int i = 2; i >= 0; --i) {
-          dc_mma(acc[mi][0], a[i], b[0], b[1]);
-          dc_mma(acc[mi][1], a[i], b[2], b[3]);
-        }
+        dc_mma31(acc[mi][0], a, b[0], b[1]);
+        dc_mma31(acc[mi][1], a, b[2], b[3]);
       }
     }
 #pragma unroll
@@ -291,11 +284,8 @@ delta_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO,
       for (int mi = 0; mi < 8; ++mi) {
         uint32_t a[4];
         dc_a_t(a, sQ, mi * 16, kk * 16, lane);
-#pragma unroll
-        for (int i = 2; i >= 0; --i) {
-          dc_mma(acc[mi][0], a, bs[i][0], bs[i][1]);
-          dc_mma(acc[mi][1], a, bs[i][2], bs[i][3]);
-        }
+        dc_mma13(acc[mi][0], a, bs, 0);
+        dc_mma13(acc[mi][1], a, bs, 2);
       }
     }
     float* out = GS + ((static_cast<long long>(h) * (p.NC + nseq) + slot) * DC_D) * DC_D;
@@ -381,13 +371,13 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   {
     float acc[4][4] = {};
     for (int kk = mi; kk < 4; ++kk) {
-      uint32_t a[2][4];
-      dc_af_t<2>(a, sP, DQ_P, m0, kk * 16, lane);
+      uint32_t a[3][4];
+      dc_af_t<3>(a, sP, DQ_P, m0, kk * 16, lane);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        uint32_t b[2][2];
-        dc_bf_t<2>(b, sS, DQ_DX, n0 + nt * 8, kk * 16, lane);
-        dc_mma22(acc[nt], a[0], a[1], b[0], b[1]);
+        uint32_t b[3][2];
+        dc_bf_t<3>(b, sS, DQ_DX, n0 + nt * 8, kk * 16, lane);
+        dc_mma33(acc[nt], a, b);
       }
     }
     const float be0 = sB[i0], be1 = sB[i1];
@@ -415,16 +405,15 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     if (cq <= mi) {
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
-        uint32_t ad[4], ab[2][4];
+        uint32_t ad[4], ab[3][4];
         dc_a(ad, sDO, m0, kk * 16, lane);
-        dc_af<2>(ab, sDB, DQ_LD, m0, kk * 16, lane);
+        dc_af<3>(ab, sDB, DQ_LD, m0, kk * 16, lane);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           uint32_t b[3][2];
           dc_bf<3>(b, sX, DQ_LD, cq * 16 + nt * 8, kk * 16, lane);
-#pragma unroll
-          for (int i = 2; i >= 0; --i) dc_mma(accR[nt], ad, b[i][0], b[i][1]);
-          dc_mma22(accP[nt], ab[0], ab[1], b[0], b[1]);
+          dc_mma13(accR[nt], ad, b);
+          dc_mma33(accP[nt], ab, b);
         }
       }
     }
@@ -455,16 +444,15 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   float dq[4][4] = {}, dk[4][4] = {};
 #pragma unroll 2
   for (int kk = 0; kk < 8; ++kk) {
-    uint32_t ad[4], ab[2][4];
+    uint32_t ad[4], ab[3][4];
     dc_a(ad, sDO, m0, kk * 16, lane);
-    dc_af<2>(ab, sDB, DQ_LD, m0, kk * 16, lane);
+    dc_af<3>(ab, sDB, DQ_LD, m0, kk * 16, lane);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       uint32_t b[3][2];
       dc_bf<3>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
-#pragma unroll
-      for (int i = 2; i >= 0; --i) dc_mma(dq[nt], ad, b[i][0], b[i][1]);
-      dc_mma22(dk[nt], ab[0], ab[1], b[0], b[1]);
+      dc_mma13(dq[nt], ad, b);
+      dc_mma33(dk[nt], ab, b);
     }
   }
   // the gradient of the chunk's end state is fetched while the score terms run
@@ -488,13 +476,10 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     for (int np = 0; np < 2; ++np) {
       uint32_t b[4];
       dc_b_t(b, sK, n0 + np * 16, kk * 16, lane);
-#pragma unroll
-      for (int i = 2; i >= 0; --i) {
-        dc_mma(dq[2 * np], ar[i], b[0], b[1]);
-        dc_mma(dq[2 * np + 1], ar[i], b[2], b[3]);
-        dc_mma(dk[2 * np], ap[i], b[0], b[1]);
-        dc_mma(dk[2 * np + 1], ap[i], b[2], b[3]);
-      }
+      dc_mma31(dq[2 * np], ar, b[0], b[1]);
+      dc_mma31(dq[2 * np + 1], ar, b[2], b[3]);
+      dc_mma31(dk[2 * np], ap, b[0], b[1]);
+      dc_mma31(dk[2 * np + 1], ap, b[2], b[3]);
     }
   }
   uint32_t kv[4][2];                             // this thread's k values (bf16 pairs)
@@ -524,13 +509,10 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
         uint32_t bk[4], bq[4];
         dc_b_t(bk, sK, n0 + np * 16, kk * 16, lane);
         dc_b_t(bq, sQ, n0 + np * 16, kk * 16, lane);
-#pragma unroll
-        for (int i = 2; i >= 0; --i) {
-          dc_mma(acc[2 * np], ap[i], bk[0], bk[1]);
-          dc_mma(acc[2 * np + 1], ap[i], bk[2], bk[3]);
-          dc_mma(acc[2 * np], ar[i], bq[0], bq[1]);
-          dc_mma(acc[2 * np + 1], ar[i], bq[2], bq[3]);
-        }
+        dc_mma31(acc[2 * np], ap, bk[0], bk[1]);
+        dc_mma31(acc[2 * np + 1], ap, bk[2], bk[3]);
+        dc_mma31(acc[2 * np], ar, bq[0], bq[1]);
+        dc_mma31(acc[2 * np + 1], ar, bq[2], bq[3]);
       }
     }
 #pragma unroll
@@ -561,13 +543,13 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     float acc[4][4] = {};
 #pragma unroll 2
     for (int kk = 0; kk < 8; ++kk) {
-      uint32_t a[2][4];
-      dc_af<2>(a, sX, DQ_LD, m0, kk * 16, lane);
+      uint32_t a[3][4];
+      dc_af<3>(a, sX, DQ_LD, m0, kk * 16, lane);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        uint32_t b[2][2];
-        dc_bf<2>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
-        dc_mma22(acc[nt], a[0], a[1], b[0], b[1]);
+        uint32_t b[3][2];
+        dc_bf<3>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
+        dc_mma33(acc[nt], a, b);
       }
     }
 #pragma unroll

@@ -12,14 +12,15 @@
 //             and d(beta k^ e^G) = -db S^T.)
 //
 // Arithmetic.  q, k, v and do are bf16 in memory, so they enter the tensor cores exactly; every fp32 operand (T, A,
-// S, x and the gradients) is split into bf16 terms on the fly: three terms (24 mantissa bits) against an exact operand,
-// two terms and three products where both sides are fp32.  Norms, decays and masks are applied to fp32 accumulators or
-// fp32 operands, never to the bf16 inputs.
+// S, x and the gradients) is split on the fly into three bf16 terms (24 mantissa bits), with three products against an exact
+// operand and six where both sides are fp32.  Norms, decays and masks are applied to fp32 accumulators or fp32 operands,
+// never to the bf16 inputs.  Two terms and three products on both-fp32 products left dg 4 to 14 and dbeta 13 to 16 times as
+// far from 64 bits as fp32 products; now dbeta, gx and gS are closer than those and dg within 1.5 times of them.
 //
-// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.14 ms, out 0.11, bwd_pre 0.09, bwd_post 0.45 (0.17, 0.16,
-// 0.12 and 0.53 while the tiles came in one after the other through registers); with the first form of these kernels a
-// gated-delta-net layer forward + backward went from 10.43 to 3.96 ms.  Before, the chunk-parallel part was about 250
-// launches of fp32 products, element-wise passes and gathers over materialised [chunk, 64, 64 .. 128] tensors.
+// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.15 ms, out 0.13, bwd_pre 0.09, bwd_post 0.60; with two-term
+// operands and sums kept in the tensor cores' accumulators 0.14, 0.11, 0.09 and 0.45.  A gated-delta-net layer forward + backward
+// takes 2.66 ms, against 10.4 when the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and
+// gathers over materialised [chunk, 64, 64 .. 128] tensors.
 //
 // Why mma.sync and not tcgen05: the products are 64 x 64 x 128 at most, each feeds the next through registers and
 // shared memory, and their operands are built element by element (splits, decays); the kernels are bound by moving
@@ -53,6 +54,53 @@ __device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], co
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the same with a zero accumulator
+__device__ __forceinline__ void dc_mul(float (&c)[4], const uint32_t (&a)[4], const uint32_t b0, const uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// Products of operands in bf16 terms, 16 steps of the contraction at a time.  A tensor-core product adds to its accumulator by
+// truncation, which over a whole contraction costs more than the roundings of fp32 products do.  So the terms of one step
+// start from zero, smallest first, and their sum is added with a rounded fp32 addition.
+__device__ __forceinline__ void dc_add(float (&c)[4], const float (&d)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] += d[i];
+}
+// exact x exact
+__device__ __forceinline__ void dc_mma11(float (&c)[4], const uint32_t (&a)[4], const uint32_t b0, const uint32_t b1) {
+  float d[4];
+  dc_mul(d, a, b0, b1);
+  dc_add(c, d);
+}
+// fp32 x exact and exact x fp32 (columns o, o + 1 of the terms): three terms, 24 mantissa bits
+__device__ __forceinline__ void dc_mma31(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t b0, const uint32_t b1) {
+  float d[4];
+  dc_mul(d, a[2], b0, b1);
+  dc_mma(d, a[1], b0, b1);
+  dc_mma(d, a[0], b0, b1);
+  dc_add(c, d);
+}
+template <int W>
+__device__ __forceinline__ void dc_mma13(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[3][W], const int o = 0) {
+  float d[4];
+  dc_mul(d, a, b[2][o], b[2][o + 1]);
+  dc_mma(d, a, b[1][o], b[1][o + 1]);
+  dc_mma(d, a, b[0][o], b[0][o + 1]);
+  dc_add(c, d);
+}
+// fp32 x fp32: the six products down to 2^-16 of the leading one; what is left out (mid lo, lo mid, lo lo) lies below the last
+// bit of an fp32 product
+__device__ __forceinline__ void dc_mma33(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+  float d[4];
+  dc_mul(d, a[2], b[0][0], b[0][1]);
+  dc_mma(d, a[1], b[1][0], b[1][1]);
+  dc_mma(d, a[0], b[2][0], b[2][1]);
+  dc_mma(d, a[1], b[0][0], b[0][1]);
+  dc_mma(d, a[0], b[1][0], b[1][1]);
+  dc_mma(d, a[0], b[0][0], b[0][1]);
+  dc_add(c, d);
 }
 __device__ __forceinline__ void dc_ldm(uint32_t (&r)[4], const __nv_bfloat16* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -143,13 +191,6 @@ __device__ __forceinline__ void dc_bf_t(uint32_t (&b)[N][2], const float* s, int
     for (int i = 0; i < N; ++i) b[i][r] = w[i];
   }
 }
-// fp32 x fp32 with two terms each: hi hi + hi lo + lo hi
-__device__ __forceinline__ void dc_mma22(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[2], const uint32_t (&bl)[2]) {
-  dc_mma(c, al, bh[0], bh[1]);
-  dc_mma(c, ah, bl[0], bl[1]);
-  dc_mma(c, ah, bh[0], bh[1]);
-}
-
 // Tiles come in by asynchronous copies, so that all tiles of a kernel are on their way together; `dc_wait` before the barrier
 // that publishes them.  64 x 128 bf16 rows of one head -> shared tile; rows past `n` are zero (nothing is read for them).
 __device__ __forceinline__ void dc_copy16(void* dst, const void* src, int bytes) {

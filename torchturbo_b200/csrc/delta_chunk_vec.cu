@@ -12,8 +12,8 @@
 // The backward is split in two so that each half fits one SM's shared memory: `score` (T^T dx, dL, dA and the pairwise
 // sums) and `state` (products with S and dS, and the final gradients); 128 KB per chunk and head pass between them.
 //
-// Measured (2047 tokens, 8 heads, three documents): prep 55 us, out 36, bwd_pre 23, score 93, state 67; the operator with its
-// gates, forward + backward, went from 6.9 to 0.99 ms (467 launches before, 35 now).
+// Measured (2047 tokens, 8 heads, three documents): prep 55 us, out 43, bwd_pre 22, score 95, state 72; the operator with its
+// gates, forward + backward, takes 0.86 ms (6.9 ms and 467 launches as batched torch products, 21 launches now).
 #include "delta_chunk.cuh"
 
 namespace ttb {
@@ -198,11 +198,8 @@ delta_vec_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __res
       for (int np = 0; np < 4; ++np) {
         uint32_t b[4];
         dc_b_t(b, sQ, n0 + np * 16, kk * 16, lane);
-#pragma unroll
-        for (int i = 2; i >= 0; --i) {
-          dc_mma(acc[2 * np], a[i], b[0], b[1]);
-          dc_mma(acc[2 * np + 1], a[i], b[2], b[3]);
-        }
+        dc_mma31(acc[2 * np], a, b[0], b[1]);
+        dc_mma31(acc[2 * np + 1], a, b[2], b[3]);
       }
     }
 #pragma unroll
@@ -214,13 +211,13 @@ delta_vec_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __res
   {
     float acc[8][4] = {};
     for (int kk = 0; kk <= mi; ++kk) {
-      uint32_t a[2][4];
-      dc_af<2>(a, sT, DP_LT, m0, kk * 16, lane);
+      uint32_t a[3][4];
+      dc_af<3>(a, sT, DP_LT, m0, kk * 16, lane);
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
-        uint32_t b[2][2];
-        dc_bf_t<2>(b, sG, DV_G, n0 + nt * 8, kk * 16, lane);
-        dc_mma22(acc[nt], a[0], a[1], b[0], b[1]);
+        uint32_t b[3][2];
+        dc_bf_t<3>(b, sG, DV_G, n0 + nt * 8, kk * 16, lane);
+        dc_mma33(acc[nt], a, b);
       }
     }
 #pragma unroll
@@ -279,24 +276,24 @@ delta_vec_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const f
   float acc[4][4] = {};
 #pragma unroll 2
   for (int kk = 0; kk < 8; ++kk) {
-    uint32_t b[2][2];
-    dc_bf_t<2>(b, sS, DO_LD, n0, kk * 16, lane);
+    uint32_t b[3][2];
+    dc_bf_t<3>(b, sS, DO_LD, n0, kk * 16, lane);
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi) {
-      uint32_t a[2][4];
-      dc_af<2>(a, sQ, DV_A, mi * 16, kk * 16, lane);
-      dc_mma22(acc[mi], a[0], a[1], b[0], b[1]);
+      uint32_t a[3][4];
+      dc_af<3>(a, sQ, DV_A, mi * 16, kk * 16, lane);
+      dc_mma33(acc[mi], a, b);
     }
   }
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk) {
-    uint32_t b[2][2];
-    dc_bf_t<2>(b, sX, DO_LD, n0, kk * 16, lane);
+    uint32_t b[3][2];
+    dc_bf_t<3>(b, sX, DO_LD, n0, kk * 16, lane);
 #pragma unroll
     for (int mi = kk; mi < 4; ++mi) {
-      uint32_t a[2][4];
-      dc_af<2>(a, sA, DP_LT, mi * 16, kk * 16, lane);
-      dc_mma22(acc[mi], a[0], a[1], b[0], b[1]);
+      uint32_t a[3][4];
+      dc_af<3>(a, sA, DP_LT, mi * 16, kk * 16, lane);
+      dc_mma33(acc[mi], a, b);
     }
   }
   __syncthreads();
@@ -348,11 +345,8 @@ delta_vec_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__
     for (int kk = mi; kk < 4; ++kk) {
       uint32_t a[3][4];
       dc_af_t<3>(a, sA, DO_LD, mi * 16, kk * 16, lane);
-#pragma unroll
-      for (int i = 2; i >= 0; --i) {
-        dc_mma(acc[0], a[i], b[kk][0], b[kk][1]);
-        dc_mma(acc[1], a[i], b[kk][2], b[kk][3]);
-      }
+      dc_mma31(acc[0], a, b[kk][0], b[kk][1]);
+      dc_mma31(acc[1], a, b[kk][2], b[kk][3]);
     }
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
@@ -368,11 +362,8 @@ delta_vec_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__
     for (int kk = 0; kk < 4; ++kk) {
       uint32_t a[3][4];
       dc_af_t<3>(a, sQ, DV_G, mi * 16, kk * 16, lane);
-#pragma unroll
-      for (int i = 2; i >= 0; --i) {
-        dc_mma(acc[0], a[i], b[kk][0], b[kk][1]);
-        dc_mma(acc[1], a[i], b[kk][2], b[kk][3]);
-      }
+      dc_mma31(acc[0], a, b[kk][0], b[kk][1]);
+      dc_mma31(acc[1], a, b[kk][2], b[kk][3]);
     }
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
@@ -433,13 +424,13 @@ delta_vec_score_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
   {
     float acc[4][4] = {}, part[2] = {0.f, 0.f};
     for (int kk = mi; kk < 4; ++kk) {
-      uint32_t a[2][4];
-      dc_af_t<2>(a, sT, DO_LD, m0, kk * 16, lane);
+      uint32_t a[3][4];
+      dc_af_t<3>(a, sT, DO_LD, m0, kk * 16, lane);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        uint32_t b[2][2];
-        dc_bf_t<2>(b, sDX, DV_G, n0 + nt * 8, kk * 16, lane);
-        dc_mma22(acc[nt], a[0], a[1], b[0], b[1]);
+        uint32_t b[3][2];
+        dc_bf_t<3>(b, sDX, DV_G, n0 + nt * 8, kk * 16, lane);
+        dc_mma33(acc[nt], a, b);
       }
     }
 #pragma unroll
@@ -474,16 +465,15 @@ delta_vec_score_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
     if (cq <= mi) {
 #pragma unroll 2
       for (int kk = 0; kk < 8; ++kk) {
-        uint32_t ad[4], ab[2][4];
+        uint32_t ad[4], ab[3][4];
         dc_a(ad, sDO, m0, kk * 16, lane);
-        dc_af<2>(ab, sDB, DV_A, m0, kk * 16, lane);
+        dc_af<3>(ab, sDB, DV_A, m0, kk * 16, lane);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           uint32_t b[3][2];
           dc_bf<3>(b, sX, DV_A, cq * 16 + nt * 8, kk * 16, lane);
-#pragma unroll
-          for (int i = 2; i >= 0; --i) dc_mma(accR[nt], ad, b[i][0], b[i][1]);
-          dc_mma22(accP[nt], ab[0], ab[1], b[0], b[1]);
+          dc_mma13(accR[nt], ad, b);
+          dc_mma33(accP[nt], ab, b);
         }
       }
     }
@@ -609,16 +599,15 @@ delta_vec_state_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
   float dq[4][4] = {}, dk[4][4] = {};
 #pragma unroll 2
   for (int kk = 0; kk < 8; ++kk) {
-    uint32_t ad[4], ab[2][4];
+    uint32_t ad[4], ab[3][4];
     dc_a(ad, sDO, m0, kk * 16, lane);
-    dc_af<2>(ab, sDB, DV_A, m0, kk * 16, lane);
+    dc_af<3>(ab, sDB, DV_A, m0, kk * 16, lane);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       uint32_t b[3][2];
       dc_bf<3>(b, sS, DV_A, n0 + nt * 8, kk * 16, lane);
-#pragma unroll
-      for (int i = 2; i >= 0; --i) dc_mma(dq[nt], ad, b[i][0], b[i][1]);
-      dc_mma22(dk[nt], ab[0], ab[1], b[0], b[1]);
+      dc_mma13(dq[nt], ad, b);
+      dc_mma33(dk[nt], ab, b);
     }
   }
   float gate[4][4];
@@ -661,13 +650,13 @@ delta_vec_state_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
   float out[4][4] = {};
 #pragma unroll 2
   for (int kk = 0; kk < 8; ++kk) {
-    uint32_t a[2][4];
-    dc_af<2>(a, sX, DV_A, m0, kk * 16, lane);
+    uint32_t a[3][4];
+    dc_af<3>(a, sX, DV_A, m0, kk * 16, lane);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      uint32_t b[2][2];
-      dc_bf<2>(b, sS, DV_A, n0 + nt * 8, kk * 16, lane);
-      dc_mma22(out[nt], a[0], a[1], b[0], b[1]);
+      uint32_t b[3][2];
+      dc_bf<3>(b, sS, DV_A, n0 + nt * 8, kk * 16, lane);
+      dc_mma33(out[nt], a, b);
     }
   }
   __syncthreads();                               // x, db and dS are no longer read: their space takes the sums below
