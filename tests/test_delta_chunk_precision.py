@@ -168,3 +168,23 @@ def test_keys_that_cancel_keep_fp32_operands(vec):
     w = K.delta_prep(q, k, v, g, torch.ones_like(beta), rows, l2=False, scale=1.0)[3]
     assert (w[0, 0, 0].float() - k[0, 0].float() * g[0].exp().reshape(-1)).abs().max() <= 2 ** -8 * 0.125
     assert w[0, 0, 1:].float().norm() <= 2 ** -21 * 0.125 * (63 * 64) ** 0.5, w[0, 0, 1:].float().norm() / (0.125 * (63 * 64) ** 0.5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vec", [False, True])
+def test_decays_are_exponentials_over_their_whole_range(vec):
+    """One row per head, so the chunk's decay is exp(g) of a single number, -inf (a reset) included.  expf and exp2f are good to
+    2^-22; per channel g is first rounded in units of log2, half a unit of 2^-23 of it."""
+    from torchturbo_b200 import kernels as K
+
+    x = torch.cat((torch.linspace(-110, 20, 4093), torch.tensor([0.0, -1e30, -float("inf")]))).cuda()
+    H = x.numel()
+    q, k, v = (torch.ones(1, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    g = x.view(1, H, 1).expand(1, H, D).contiguous() if vec else x.view(1, H)
+    rows = torch.tensor([[0, 1, 0]], dtype=torch.int32, device="cuda")
+    got = K.delta_prep(q, k, v, g, torch.ones(1, H, device="cuda"), rows, l2=True, scale=1.0)[5].reshape(H, -1).double()
+    want = x.double().exp()[:, None]
+    tol = 2 ** -22 + (x.abs().double()[:, None] * 2 ** -23 if vec else 0.0)
+    normal = want >= 2 ** -126
+    assert (((got - want).abs() <= tol * want) | ~normal).all()
+    assert (got[(~normal).expand_as(got)] <= 2 ** -126).all() and (got[-1] == 0).all() and (got[-2] == 0).all()

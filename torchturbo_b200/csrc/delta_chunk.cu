@@ -39,8 +39,8 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
   dc_row_norms<256>(sK, sRk, p.l2, 1.f);
   if (warp == 0) dc_cumsum(sG, lane);
   __syncthreads();
-  if (tid < DC_C) sW[tid] = sB[tid] * sRk[tid] * dc_exp(sG[tid]);
-  if (tid == 0) decay[hc] = dc_exp(sG[DC_C - 1]);
+  if (tid < DC_C) sW[tid] = sB[tid] * sRk[tid] * expf(sG[tid]);
+  if (tid == 0) decay[hc] = expf(sG[DC_C - 1]);
 
   const int mi = warp & 3, m0 = mi * 16, g = lane >> 2, t2 = (lane & 3) * 2;
   {
@@ -68,8 +68,8 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
         const int i = m0 + g + rr * 8, j = nt * 8 + t2;
         float2 o = make_float2(0.f, 0.f);
         const float ri = is_q ? sRq[i] : sRk[i] * sB[i];
-        if (is_q ? (j <= i) : (j < i)) o.x = acc[nt][2 * rr] * (ri * sRk[j]) * dc_exp(sG[i] - sG[j]);
-        if (is_q ? (j + 1 <= i) : (j + 1 < i)) o.y = acc[nt][2 * rr + 1] * (ri * sRk[j + 1]) * dc_exp(sG[i] - sG[j + 1]);
+        if (is_q ? (j <= i) : (j < i)) o.x = acc[nt][2 * rr] * (ri * sRk[j]) * expf(sG[i] - sG[j]);
+        if (is_q ? (j + 1 <= i) : (j + 1 < i)) o.y = acc[nt][2 * rr + 1] * (ri * sRk[j + 1]) * expf(sG[i] - sG[j + 1]);
         *reinterpret_cast<float2*>(is_q ? Aout + i * DC_C + j : sL + i * DP_LT + j) = o;
       }
     }
@@ -113,7 +113,7 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
 #pragma unroll
   for (int e = tid; e < DC_C * 16; e += 256) {
     const int i = e >> 4, j = (e & 15) * 8;
-    const float f = dc_exp(sG[DC_C - 1] - sG[i]) * sRk[i];
+    const float f = expf(sG[DC_C - 1] - sG[i]) * sRk[i];
     uint4 u = *reinterpret_cast<const uint4*>(sK + i * DC_QS + j);
     uint32_t* w = reinterpret_cast<uint32_t*>(&u);
 #pragma unroll
@@ -175,7 +175,7 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       const int i = mi * 16 + g + rr * 8;
-      const float f = sRq[i] * dc_exp(sG[i]);
+      const float f = sRq[i] * expf(sG[i]);
       acc[mi][2 * rr] *= f;
       acc[mi][2 * rr + 1] *= f;
     }
@@ -238,7 +238,7 @@ delta_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO,
   dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
   if (warp == 0) dc_cumsum(sG, lane);
   __syncthreads();
-  if (threadIdx.x < DC_C) sF[threadIdx.x] = sRq[threadIdx.x] * dc_exp(sG[threadIdx.x]);
+  if (threadIdx.x < DC_C) sF[threadIdx.x] = sRq[threadIdx.x] * expf(sG[threadIdx.x]);
   __syncthreads();
   const int g = lane >> 2, t2 = (lane & 3) * 2, n0 = warp * 16;
   {
@@ -356,8 +356,8 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   if (warp == 0) dc_cumsum(sG, lane);
   __syncthreads();
   if (tid < DC_C) {
-    sE[tid] = dc_exp(sG[tid]);
-    sL[tid] = dc_exp(sG[DC_C - 1] - sG[tid]);
+    sE[tid] = expf(sG[tid]);
+    sL[tid] = expf(sG[DC_C - 1] - sG[tid]);
     sBk[tid] = sB[tid] * sRk[tid];
   }
   // warp tile: 16 rows x 32 columns
@@ -424,12 +424,12 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
         const int i = rr ? i1 : i0, j = cq * 16 + nt * 8 + t2;
         float2 pv = make_float2(0.f, 0.f), rv = make_float2(0.f, 0.f);
         if (j <= i) {
-          const float d = dc_exp(sG[i] - sG[j]);
+          const float d = expf(sG[i] - sG[j]);
           rv.x = accR[nt][2 * rr] * d;
           if (j < i) pv.x = -accP[nt][2 * rr] * d;
         }
         if (j + 1 <= i) {
-          const float d = dc_exp(sG[i] - sG[j + 1]);
+          const float d = expf(sG[i] - sG[j + 1]);
           rv.y = accR[nt][2 * rr + 1] * d;
           if (j + 1 < i) pv.y = -accP[nt][2 * rr + 1] * d;
         }

@@ -43,13 +43,6 @@ struct DeltaChunkIn {
   float scale;
 };
 
-__device__ __forceinline__ float dc_exp(float x) {
-  // e^x with the rounding error of x * log2(e) carried along: the plain product loses |x| 2^-24 relative to the result
-  const float h = x * 1.44269502f;
-  const float l = fmaf(x, 1.44269502f, -h) + x * 1.92596303e-8f;
-  return exp2f(h) * fmaf(l, 0.693147182f, 1.f);
-}
-
 __device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t b0, const uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])

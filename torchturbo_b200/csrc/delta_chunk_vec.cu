@@ -492,6 +492,7 @@ delta_vec_score_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
   // ---- pairwise sums: a thread owns one channel and, of every 16 rows, the four of its row group; ek of all 64 rows
   //      accumulates in registers and is added up over the four groups at the end
   const int ch = tid & 127, rg = tid >> 7;
+  if (tid < DC_C) sPart[tid] = 1.f / sRk[tid];   // takes |k_j| out of ek again; read behind the barriers of the last loop
   float ek[DC_C];
 #pragma unroll
   for (int j = 0; j < DC_C; ++j) ek[j] = 0.f;
@@ -538,7 +539,7 @@ delta_vec_score_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
         float v = ek[j];
         if (grp > 0) v += sDX[j * DV_G + ch];
         if (grp < 3) sDX[j * DV_G + ch] = v;
-        else EK[(hc * DC_C + j) * DC_D + ch] = v / sRk[j];
+        else EK[(hc * DC_C + j) * DC_D + ch] = v * sPart[j];
       }
     }
     __syncthreads();
