@@ -41,3 +41,32 @@ def test_other_widths_take_the_formula():
     g = torch.randn(1, 5, 2, 64, device="cuda").to(torch.bfloat16)
     out = _gate(g, torch.zeros(2, device="cuda"), None, None)
     assert torch.equal(out, kda_gate(g, torch.zeros(2, device="cuda"), None, None)) and KDAGate is not None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bound", [None, -5.0])
+def test_gate_values_are_as_accurate_as_fp32_torch(bound):
+    """Every value and every bias gradient (one row: nothing is summed) against 64 bits: the largest relative error is at most
+    twice that of the same formula in fp32 torch.  Approximate exponentials are off by |x| 2^-24, thirty times as much at -60."""
+    H = 64
+    gen = torch.Generator().manual_seed(0)
+    g = (torch.rand(1, 1, H, 128, generator=gen) * 90 - 60).to(torch.bfloat16)
+    A = (torch.rand(H, generator=gen) * 2 - 2).bfloat16().float()
+    bias = torch.zeros(H * 128)
+    if bound is not None:                                   # sigmoid(a x) with a x exact: only the exponential rounds
+        A = torch.zeros(H)
+    res = []
+    for fn, dev, dt in ((_gate, "cuda", None), (kda_gate, "cuda", None), (None, "cpu", torch.float64)):
+        leaves = [t.to(dev, dt) if dt else t.to(dev) for t in (g, A, bias)]
+        leaves[2].requires_grad_(True)
+        if fn is not None:
+            out = fn(*leaves, bound)
+        else:
+            x, a = leaves[0] + leaves[2].view(H, 128), leaves[1].exp().view(H, 1)
+            out = bound * torch.sigmoid(a * x) if bound is not None else -a * torch.nn.functional.softplus(x)
+        out.sum().backward()
+        res.append([out.detach().double().cpu().reshape(-1), leaves[2].grad.double().cpu()])
+    for mine, fp32, want in zip(*res):
+        big = want.abs() > 2 ** -120
+        err, ref = (((t - want).abs() / want.abs())[big].max().item() for t in (mine, fp32))
+        assert err <= 2 * ref + 2 ** -23, (err, ref)

@@ -27,7 +27,7 @@ NVCC_FLAGS = [
 # Approximate exponentials, divisions and roots wherever a result leaves in bf16 anyway.  Sources whose fp32 results stand in
 # for fp32 torch operations are compiled without; -ftz alone keeps an exp2f at one instruction.
 FAST_MATH = ["--use_fast_math"]
-PRECISE = {"delta_chunk.cu": [], "delta_chunk_vec.cu": ["-ftz=true"]}
+PRECISE = {"delta_chunk.cu": [], "delta_chunk_vec.cu": ["-ftz=true"], "gates.cu": []}
 
 
 def _nvcc() -> str:

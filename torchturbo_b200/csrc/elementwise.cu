@@ -11,6 +11,7 @@
 //   CE        : fp32, reduction=sum, ignore_index=-100                (ops/providers/native/cross_entropy_loss.py:17-33)
 //   AdamW     : torch fused AdamW math on fp32 shards                  (engine/backends/fsdp2/optimizers/adamw.py:226-251)
 #include "common.cuh"
+#include "rowops.cuh"
 
 namespace ttb {
 
@@ -162,32 +163,6 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
 #pragma unroll
     for (int j = 0; j < 8; ++j) dst[j] = dwacc[it][j];
   }
-}
-
-// Column sum of partial[rows][H] -> out[H] (fp32 or bf16); deterministic order.  32 columns and 32 row groups per block:
-// the sums are a few hundred rows long at most, so what counts is how many loads are in flight (2048 columns: 4.9 us with one
-// thread per column, 2.3 now; the six sums of a ViT block 76 and 19 us).
-__device__ __forceinline__ void store_scalar(float* p, float v) { *p = v; }
-__device__ __forceinline__ void store_scalar(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
-
-template <typename Out>
-__global__ void __launch_bounds__(1024) colsum_kernel(const float* __restrict__ partial, Out* __restrict__ out, int rows, int H) {
-  __shared__ float part[32][33];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + x;
-  float s = 0.f;
-  if (c < H) {
-#pragma unroll 4
-    for (int r = y; r < rows; r += 32) s += partial[static_cast<long long>(r) * H + c];
-  }
-  part[y][x] = s;
-  __syncthreads();
-  s = warp_sum(part[x][y]);
-  if (x == 0 && blockIdx.x * 32 + y < H) store_scalar(out + blockIdx.x * 32 + y, s);
-}
-static void colsum(const float* partial, void* out, int out_bf16, int rows, int H, cudaStream_t st) {
-  if (out_bf16) colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(partial, static_cast<__nv_bfloat16*>(out), rows, H);
-  else colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(partial, static_cast<float*>(out), rows, H);
 }
 
 // ============================================================================
@@ -965,63 +940,6 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, long long x_t, 
 }
 
 // ============================================================================
-// Kimi delta attention gate: per-channel log decay of [rows, H, 128] from the raw projection,
-//   d = -exp(A_h) softplus(x)   or, with a lower bound,   d = bound * sigmoid(exp(A_h) x),      x = g + dt
-// One block row of 128 channels per head; the backward returns dg and, per block of rows, the channel sums behind d(dt) and
-// d(A), which colsum adds up in a fixed order.  fp32 arithmetic; softplus is the identity above 20, as in torch.
-// In torch this is about seven launches forward and fifteen backward over fp32 tensors;
-// 2047 x 8 heads: 6 and 10 us, the operator 907 -> 819 us (35 -> 21 launches).
-// ============================================================================
-__device__ __forceinline__ float load_scalar(const void* p, long long i, int bf16) {
-  return bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
-}
-
-__global__ void __launch_bounds__(128)
-kda_gate_fwd_kernel(const __nv_bfloat16* __restrict__ g, const void* __restrict__ A, int a_bf16, const void* __restrict__ dt,
-                    int dt_bf16, float* __restrict__ out, long long rows, int H, int bounded, float bound, int rows_per_block) {
-  const int h = blockIdx.x;
-  const long long col = static_cast<long long>(h) * 128 + threadIdx.x, step = static_cast<long long>(H) * 128;
-  const float a = expf(load_scalar(A, h, a_bf16)), b = dt ? load_scalar(dt, col, dt_bf16) : 0.f;
-  const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_block, r1 = min(r0 + rows_per_block, rows);
-#pragma unroll 4
-  for (long long r = r0; r < r1; ++r) {
-    const float x = __bfloat162float(g[r * step + col]) + b;
-    out[r * step + col] = bounded ? bound / (1.f + expf(-a * x)) : -a * (x > 20.f ? x : log1pf(expf(x)));
-  }
-}
-
-__global__ void __launch_bounds__(128)
-kda_gate_bwd_kernel(const float* __restrict__ dd, const __nv_bfloat16* __restrict__ g, const void* __restrict__ A, int a_bf16,
-                    const void* __restrict__ dt, int dt_bf16, __nv_bfloat16* __restrict__ dg, float* __restrict__ part,
-                    long long rows, int H, int bounded, float bound, int rows_per_block) {
-  const int h = blockIdx.x;
-  const long long col = static_cast<long long>(h) * 128 + threadIdx.x, step = static_cast<long long>(H) * 128;
-  const float a = expf(load_scalar(A, h, a_bf16)), b = dt ? load_scalar(dt, col, dt_bf16) : 0.f;
-  const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_block, r1 = min(r0 + rows_per_block, rows);
-  float sum_dt = 0.f, sum_a = 0.f;
-#pragma unroll 4
-  for (long long r = r0; r < r1; ++r) {
-    const float x = __bfloat162float(g[r * step + col]) + b, d = dd[r * step + col];
-    float dx, da;
-    if (bounded) {
-      const float sg = 1.f / (1.f + expf(-a * x)), slope = d * bound * sg * (1.f - sg);
-      dx = slope * a;
-      da = slope * a * x;
-    } else {
-      const bool linear = x > 20.f;
-      const float e = expf(x);
-      dx = -d * a * (linear ? 1.f : e / (1.f + e));
-      da = -d * a * (linear ? x : log1pf(e));
-    }
-    dg[r * step + col] = __float2bfloat16(dx);
-    sum_dt += dx;
-    sum_a += da;
-  }
-  part[blockIdx.y * 2 * step + col] = sum_dt;
-  part[(blockIdx.y * 2 + 1) * step + col] = sum_a;
-}
-
-// ============================================================================
 // SwiGLU (standalone).  x: [R, 2F] = [gate | up]; y: [R, F]; optional row_scale [R].
 // ============================================================================
 // `nrows` (optional, device): rows at or beyond *nrows are skipped (padded buffers whose fill is only known on the device)
@@ -1425,43 +1343,6 @@ TTB_EXPORT int ttb_rope(const void* x, long long x_t, long long x_h, const float
   if (total == 0) return 0;
   rope_kernel<<<(unsigned)((total + 255) / 256), 256, 0, STREAM(stream)>>>((const __nv_bfloat16*)x, x_t, x_h, cos_t, sin_t,
                                                                           (__nv_bfloat16*)y, total, heads, half, sign);
-  LAUNCH_RET();
-}
-
-static int kda_gate_rows(long long rows, int H, int& blocks) {
-  long long want = (148LL * 8 + H - 1) / H;                 // about eight blocks per SM
-  if (want > rows) want = rows;
-  if (want < 1) want = 1;
-  const int per = static_cast<int>((rows + want - 1) / want);
-  blocks = static_cast<int>((rows + per - 1) / per);
-  return per;
-}
-
-TTB_EXPORT int ttb_kda_gate_row_blocks(long long rows, int H) {
-  int blocks = 0;
-  kda_gate_rows(rows, H, blocks);
-  return blocks;
-}
-
-TTB_EXPORT int ttb_kda_gate_fwd(const void* g, const void* A, int a_bf16, const void* dt, int dt_bf16, float* out, long long rows,
-                                int H, int bounded, float bound, void* stream) {
-  if (rows == 0 || H == 0) return 0;
-  int blocks;
-  const int per = kda_gate_rows(rows, H, blocks);
-  kda_gate_fwd_kernel<<<dim3(H, blocks), 128, 0, STREAM(stream)>>>((const __nv_bfloat16*)g, A, a_bf16, dt, dt_bf16, out, rows, H,
-                                                                  bounded, bound, per);
-  LAUNCH_RET();
-}
-
-// part: fp32 [row_blocks, 2, H * 128]; sums: fp32 [2, H * 128] (d(dt), then the channel sums of d(A))
-TTB_EXPORT int ttb_kda_gate_bwd(const float* dd, const void* g, const void* A, int a_bf16, const void* dt, int dt_bf16, void* dg,
-                                float* part, float* sums, long long rows, int H, int bounded, float bound, void* stream) {
-  if (rows == 0 || H == 0) return 0;
-  int blocks;
-  const int per = kda_gate_rows(rows, H, blocks);
-  kda_gate_bwd_kernel<<<dim3(H, blocks), 128, 0, STREAM(stream)>>>(dd, (const __nv_bfloat16*)g, A, a_bf16, dt, dt_bf16,
-                                                                  (__nv_bfloat16*)dg, part, rows, H, bounded, bound, per);
-  colsum(part, sums, 0, blocks, 2 * H * 128, STREAM(stream));
   LAUNCH_RET();
 }
 
