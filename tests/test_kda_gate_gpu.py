@@ -6,14 +6,27 @@ from torchturbo_b200.ops.providers.b200_linear_attention import KDAGate, _gate
 from torchturbo_b200.ops.providers.native_linear_attention import kda_gate
 
 
+def test_row_blocks_cover_every_row_and_none_of_no_rows():
+    import ctypes as C
+
+    from torchturbo_b200 import kernels as K
+
+    if not K.is_built():
+        pytest.skip("library not built")
+    blocks = lambda rows, H: K.lib().ttb_kda_gate_row_blocks(C.c_longlong(rows), C.c_int(H))                     # noqa: E731
+    assert blocks(0, 3) == 0 and blocks(5, 0) == 0
+    assert blocks(1, 1) == 1 and blocks(2047, 8) == 147 and blocks(33, 200) == 6
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("T, H", [(1, 1), (7, 3), (1200, 2), (33, 200)])
+@pytest.mark.parametrize("T, H", [(0, 2), (1, 1), (7, 3), (1200, 2), (33, 200)])
 @pytest.mark.parametrize("bias, bound, dtype", [(True, None, torch.bfloat16), (False, None, torch.float32), (True, -5.0, torch.float32)])
 def test_gate_and_its_gradients(T, H, bias, bound, dtype):
     """fp32 on one side, fp64 on the other; dg and bf16 parameter gradients add their rounding (2^-9)."""
     gen = torch.Generator().manual_seed(T)
     g0 = (torch.randn(1, T, H, 128, generator=gen) * 4).to(torch.bfloat16)
-    g0[0, 0, 0, :3] = torch.tensor([30.0, -60.0, 20.5])              # linear branch, underflow, just behind the threshold
+    if T:
+        g0[0, 0, 0, :3] = torch.tensor([30.0, -60.0, 20.5])              # linear branch, underflow, just behind the threshold
     A0 = torch.rand(H, generator=gen).mul(15).add(1).log().to(dtype)
     b0 = torch.randn(H * 128, generator=gen).to(dtype) if bias else None
     w = torch.randn(1, T, H, 128, generator=gen)
@@ -26,9 +39,10 @@ def test_gate_and_its_gradients(T, H, bias, bound, dtype):
     a = ref[1].exp().view(H, 1)
     want = bound * torch.sigmoid(a * x) if bound is not None else -a * torch.nn.functional.softplus(x)
     (want * w.double()).sum().backward()
-    assert (out.cpu().double() - want).abs().max() <= 4e-6 * want.abs().max()
-    mine = kda_gate(g0.cuda(), A0.cuda(), b0.cuda() if bias else None, bound)
-    assert (out - mine).abs().max() <= 4e-6 * mine.abs().max()
+    if T:
+        assert (out.cpu().double() - want).abs().max() <= 4e-6 * want.abs().max()
+        mine = kda_gate(g0.cuda(), A0.cuda(), b0.cuda() if bias else None, bound)
+        assert (out - mine).abs().max() <= 4e-6 * mine.abs().max()
     for got, r, d in zip(leaves, ref, (torch.bfloat16, dtype, dtype)):
         if got is not None:
             tol = 2 ** -8 if d == torch.bfloat16 else 1e-5

@@ -70,9 +70,12 @@ using namespace ttb;
 #define LAUNCH_RET() do { cudaError_t e__ = cudaGetLastError(); return e__ == cudaSuccess ? 0 : 400 + (int)e__; } while (0)
 
 static int kda_gate_rows(long long rows, int H, int& blocks) {
+  if (rows <= 0 || H <= 0) {
+    blocks = 0;
+    return 1;
+  }
   long long want = (148LL * 8 + H - 1) / H;                 // about eight blocks per SM
   if (want > rows) want = rows;
-  if (want < 1) want = 1;
   const int per = static_cast<int>((rows + want - 1) / want);
   blocks = static_cast<int>((rows + per - 1) / per);
   return per;
