@@ -1,4 +1,5 @@
-"""The rotary kernel against the torch formulation, forward and backward, over strides and odd sizes."""
+"""The rotary kernel against the torch formulation: forward and backward over strides and odd sizes, higher derivatives, and
+the transforms and tracers under which the operator stays made of torch operations."""
 import pytest
 import torch
 
@@ -33,3 +34,68 @@ def test_rope_kernel_matches_the_torch_formulation(T, heads, D, layout):
         assert a.shape == b.shape and a.dtype == b.dtype
         assert (a.float() - b.float()).abs().max() <= 2 ** -8 * b.float().abs().max()
         assert (a.float() - b.float()).norm() <= 2 ** -9 * b.float().norm()
+
+
+def _second(fn, x, probe):
+    """d/dx of <grad of sum(fn(x)^2 + x^3), probe>."""
+    x = x.detach().requires_grad_(True)
+    y = fn(x)
+    (g,) = torch.autograd.grad((y.float() ** 2).sum() + (x.float() ** 3).sum(), x, create_graph=True)
+    (h,) = torch.autograd.grad((g.float() * probe).sum(), x)
+    return g.detach().float(), h.float()
+
+
+def test_gradient_of_the_gradient_goes_through_the_rotation(monkeypatch):
+    """The autograd function around a stand-in for the kernel, which autograd cannot see through either."""
+    from torchturbo_b200.ops.providers import b200
+
+    def kernel(x, cos, sin, sign=1.0):
+        with torch.no_grad():
+            return rope_ref(x, cos, sign * sin)
+
+    monkeypatch.setattr(b200.K, "rope", kernel)
+    torch.manual_seed(0)
+    x, ang, probe = torch.randn(5, 2, 16), torch.randn(5, 8), torch.randn(5, 2, 16)
+    got = _second(lambda t: b200.RopeFn.apply(t, ang.cos(), ang.sin(), 1.0), x, probe)
+    want = _second(lambda t: rope_ref(t, ang.cos(), ang.sin()), x, probe)
+    for a, b in zip(got, want):
+        assert torch.allclose(a, b, atol=1e-5, rtol=1e-5)
+
+
+def test_only_ordinary_tensors_outside_transforms_are_eager():
+    from torch.autograd import forward_ad
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from torchturbo_b200.ops.providers.b200 import _eager
+
+    x, seen = torch.randn(3, 4), []
+    note = lambda t: seen.append(_eager(t)) or t.sin()                                                    # noqa: E731
+    note(x)
+    note(torch.nn.Parameter(x))
+    torch.func.vmap(note)(x)
+    torch.func.jvp(note, (x,), (x,))
+    torch.func.grad(lambda t: note(t).sum())(x)
+    make_fx(note)(x)
+    torch.jit.trace(note, (x,), check_trace=False)
+    with forward_ad.dual_level():
+        note(forward_ad.make_dual(x, x))
+        note(x)
+    note(torch.Tensor._make_subclass(type("Sub", (torch.Tensor,), {}), x))
+    assert seen == [True, True, False, False, False, False, False, False, True, False]
+
+
+@pytest.mark.gpu
+def test_second_derivative_and_transforms_match_the_torch_formulation():
+    """bf16 gradients on both sides: 2^-7 of the largest entry (two roundings on the way to the second derivative)."""
+    torch.manual_seed(1)
+    x = torch.randn(33, 4, 64, device="cuda").to(torch.bfloat16)
+    ang, probe = torch.randn(33, 32, device="cuda"), torch.randn(33, 4, 64, device="cuda")
+    cos, sin = ang.cos(), ang.sin()
+    op = lambda t: ops.rotary_position_embedding(t, cos, sin)                                             # noqa: E731
+    ref = lambda t: rope_ref(t, cos, sin)                                                                 # noqa: E731
+    for a, b in zip(_second(op, x, probe), _second(ref, x, probe)):
+        assert (a - b).abs().max() <= 2 ** -7 * b.abs().max()
+    batch = torch.stack((x, 2 * x))
+    assert torch.equal(torch.func.vmap(op)(batch), torch.func.vmap(ref)(batch))
+    for a, b in zip(torch.func.jvp(op, (x,), (x,)), torch.func.jvp(ref, (x,), (x,))):
+        assert torch.equal(a, b)

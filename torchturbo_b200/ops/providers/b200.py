@@ -11,6 +11,7 @@ import math
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from ... import kernels as K
 from ...runtime import TurboDevice
@@ -393,16 +394,30 @@ def _rope_rows(x: torch.Tensor) -> torch.Tensor:
     return x
 
 
+def _eager(*tensors) -> bool:
+    """Ordinary tensors outside tracers, function transforms and forward-mode differentiation.  An operator that has always
+    been made of torch operations stays so for everything else."""
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active()
+                or torch._C._get_dispatch_mode(torch._C._TorchDispatchModeKey.PROXY) is not None) and all(
+        type(t) in (torch.Tensor, torch.nn.Parameter) and forward_ad.unpack_dual(t).tangent is None for t in tensors)
+
+
 class RopeFn(torch.autograd.Function):
+    """A rotation by `sign` times the angles.  Its gradient is the rotation back, again a `RopeFn`, so that it can be
+    differentiated as often as the torch formulation."""
+
     @staticmethod
-    def forward(ctx, x, cos, sin):
+    def forward(ctx, x, cos, sin, sign):
         ctx.save_for_backward(cos, sin)
-        return K.rope(_rope_rows(x), cos, sin)
+        ctx.sign = sign
+        return K.rope(_rope_rows(x), cos, sin, sign)
 
     @staticmethod
     def backward(ctx, dy):
         cos, sin = ctx.saved_tensors
-        return K.rope(_rope_rows(dy), cos, sin, -1.0), None, None
+        if torch.is_grad_enabled():
+            return RopeFn.apply(dy, cos, sin, -ctx.sign), None, None, None
+        return K.rope(_rope_rows(dy), cos, sin, -ctx.sign), None, None, None
 
 
 @_custom("rotary_position_embedding", "b200_rope")
@@ -413,9 +428,9 @@ class B200RoPE(_B200Op):
     def __call__(self, x, cos, sin):
         D = x.shape[-1]
         if not _ok(x) or x.dim() != 3 or D % 8 or cos.shape != (x.shape[0], D // 2) or sin.shape != cos.shape \
-                or not (cos.is_cuda and sin.is_cuda) or cos.requires_grad or sin.requires_grad:
+                or not (cos.is_cuda and sin.is_cuda) or cos.requires_grad or sin.requires_grad or not _eager(x, cos, sin):
             return N.rope_ref(x, cos, sin)
-        return RopeFn.apply(x, _aligned(cos.float()), _aligned(sin.float()))
+        return RopeFn.apply(x, _aligned(cos.float()), _aligned(sin.float()), 1.0)
 
 
 # ------------------------------------------------------------------------------------------------
