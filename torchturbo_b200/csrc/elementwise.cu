@@ -582,18 +582,17 @@ causal_conv1d_w4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
       float xs[WM][4], pre[4];
       unpack4(cx[u], xs[0]);
 #pragma unroll
+      for (int j = 0; j < 4; ++j) pre[j] = bs[j] + wt[0][j] * xs[0][j];
+#pragma unroll
       for (int s = 1; s < WM; ++s) {
         unpack4(hist[s - 1], xs[s]);
-        if (s > reach || s >= W) {
+        if (s <= reach && s < W) {                 // (not a product with zero: rows and taps may be infinite)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) pre[j] += wt[s][j] * xs[s][j];
+        } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j) xs[s][j] = 0.f;
         }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        pre[j] = bs[j];
-#pragma unroll
-        for (int s = 0; s < WM; ++s) pre[j] += wt[s][j] * xs[s][j];
       }
       if (!BWD) {
         float o[4];
@@ -619,7 +618,7 @@ causal_conv1d_w4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
           // this row reaches the dx of the rows up to W - 1 behind it in its sequence
           acc[0][j] = wt[0][j] * d;
 #pragma unroll
-          for (int s = 1; s < WM; ++s) acc[s][j] += (s <= reach) ? wt[s][j] * d : 0.f;
+          for (int s = 1; s < WM; ++s) acc[s][j] += (s <= reach && s < W) ? wt[s][j] * d : 0.f;
         }
         const long long done = t - (WM - 1);        // no later row reaches it
         if (done >= r0 && done < r1) store4(out + done * D + c, acc[WM - 1]);
