@@ -873,9 +873,11 @@ def delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, 
     a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
     dq, dk, dv = (torch.empty(q.shape, dtype=torch.bfloat16, device=q.device) for _ in range(3))
     dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
-    scratch = [_p(torch.empty(4, *x.shape, dtype=torch.float32, device=q.device))] if g.dim() == 3 else []
+    # held until the launches are queued: a pointer alone would let another thread of this stream be given the block first
+    scratch = torch.empty(4, *x.shape, dtype=torch.float32, device=q.device) if g.dim() == 3 else None
     _delta_call("bwd_post", g, C.byref(a), _p(do), _p(T), _p(x), _p(dx), _p(states), _p(dstates), C.c_int(states.shape[1] - a.NC),
-                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta), *scratch, _stream())
+                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta),
+                *([_p(scratch)] if scratch is not None else []), _stream())
     return dq, dk, dv, dg, dbeta
 
 
