@@ -1307,10 +1307,11 @@ TTB_EXPORT int ttb_layernorm_bwd(const void* dy, const void* x, const void* w, c
   LAUNCH_RET();
 }
 
-// H: 64, 128 or 256
+// H: 64, 128 or 256; all bf16 pointers on 16-byte boundaries
 TTB_EXPORT int ttb_gated_rmsnorm_fwd(const void* x, const void* gate, const void* w, void* y, float* rstd, long long R, int H, float eps,
                                      int silu, int grid, void* stream) {
   if (R == 0) return 0;
+  if (((uintptr_t)x | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)y) & 15) return 902;
   auto X = (const __nv_bfloat16*)x; auto G = (const __nv_bfloat16*)gate; auto W = (const __nv_bfloat16*)w;
   auto Y = (__nv_bfloat16*)y;
   if (H == 64) gated_rmsnorm_fwd_kernel<8><<<grid, 256, 0, STREAM(stream)>>>(X, G, W, Y, rstd, R, eps, silu);
@@ -1324,6 +1325,7 @@ TTB_EXPORT int ttb_gated_rmsnorm_fwd(const void* x, const void* gate, const void
 TTB_EXPORT int ttb_gated_rmsnorm_bwd(const void* dy, const void* x, const void* gate, const void* w, const float* rstd, void* dx,
                                      void* dgate, float* dw_partial, void* dw_out, long long R, int H, int silu, int grid, void* stream) {
   if (R == 0) return 0;
+  if (((uintptr_t)dy | (uintptr_t)x | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)dx | (uintptr_t)dgate) & 15) return 902;
   auto D = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto G = (const __nv_bfloat16*)gate;
   auto W = (const __nv_bfloat16*)w; auto DX = (__nv_bfloat16*)dx; auto DG = (__nv_bfloat16*)dgate;
   if (H == 64) gated_rmsnorm_bwd_kernel<8><<<grid, 256, 0, STREAM(stream)>>>(D, X, G, W, rstd, DX, DG, dw_partial, R, silu);
@@ -1338,6 +1340,7 @@ TTB_EXPORT int ttb_gated_rmsnorm_bwd(const void* dy, const void* x, const void* 
 TTB_EXPORT int ttb_rope(const void* x, long long x_t, long long x_h, const float* cos_t, const float* sin_t, void* y, long long T,
                         int heads, int half, float sign, void* stream) {
   if (half % 4 || x_t % 4 || x_h % 4) return 901;
+  if (((uintptr_t)x | (uintptr_t)y) & 7 || ((uintptr_t)cos_t | (uintptr_t)sin_t) & 15) return 902;
   const long long total = T * heads * (half / 4);
   if (total == 0) return 0;
   rope_kernel<<<(unsigned)((total + 255) / 256), 256, 0, STREAM(stream)>>>((const __nv_bfloat16*)x, x_t, x_h, cos_t, sin_t,

@@ -32,6 +32,12 @@ def _ok(*tensors) -> bool:
     return all(t is None or (t.is_cuda and t.dtype == BF16) for t in tensors)
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on a 16-byte boundary (the kernels read and write eight bf16 values at a time)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _B200Op(OpImpl):
     def available(self) -> bool:
         return K.available()
@@ -191,13 +197,7 @@ class GatedRMSNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, gate, w, rstd = ctx.saved_tensors
-        return (*K.gated_rmsnorm_bwd(dy.contiguous(), x, gate, w, rstd, ctx.silu), None, None)
-
-
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    """Contiguous and on a 16-byte boundary (the kernels read and write eight bf16 values at a time)."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
+        return (*K.gated_rmsnorm_bwd(_aligned(dy), x, gate, w, rstd, ctx.silu), None, None)
 
 
 @_custom("gated_rms_norm", "b200_gated_rms_norm")

@@ -29,6 +29,7 @@ from ... import kernels as K
 from ...runtime import TurboDevice
 from ..base import OpImpl, OpImplKind
 from ..registry import register_op
+from .b200 import _aligned
 from .native_linear_attention import _bounds, kda_gate, l2norm
 
 CHUNK = 64
@@ -126,7 +127,7 @@ class ChunkDelta(torch.autograd.Function):
     def backward(ctx, do, dfinal):
         q, k, v, g, beta, T, A, w, k_out, decay, x, states, seq, chunk_rows, last, first = ctx.saved_tensors
         kw, has_init = ctx.meta
-        do = do.contiguous() if do is not None else torch.zeros(q.shape, dtype=q.dtype, device=q.device)
+        do = _aligned(do) if do is not None else torch.zeros(q.shape, dtype=q.dtype, device=q.device)
         gx, gs = K.delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, seq.shape[0], **kw)
         if dfinal is None:
             gs.index_fill_(1, last, 0.0)
