@@ -40,6 +40,28 @@ def test_gated_norm_kernel_matches_the_separate_operations(rows, width, activati
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("activation", ["silu", "sigmoid"])
+@pytest.mark.parametrize("lo, hi", [(-80, -60), (-60, -30), (-30, 10)])
+def test_gate_is_the_fp32_activation(activation, lo, hi):
+    """Rows of +-1 normalise exactly, so values and gate gradients are those of the separate operations bit by bit unless the
+    activation differs: approximate exponentials turn one bf16 value in a thousand at gates of -40."""
+    gen = torch.Generator("cuda").manual_seed(0)
+    rows, width = 8192, 128
+    x = torch.where(torch.rand(rows, width, generator=gen, device="cuda") < 0.5, -1.0, 1.0).to(torch.bfloat16)
+    gate = (torch.rand(rows, width, generator=gen, device="cuda") * (hi - lo) + lo).to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(width, generator=gen, device="cuda")).to(torch.bfloat16)
+    res = []
+    for impl in ("b200_gated_rms_norm", "torch_gated_rms_norm"):
+        g = gate.clone().requires_grad_(True)
+        y = ops.gated_rms_norm(x, g, w, 1e-6, activation=activation, impl=impl)
+        y.backward(torch.full_like(y, 0.37))
+        res.append((y.detach(), g.grad))
+    (y, dg), (want_y, want_dg) = res
+    assert torch.equal(y, want_y)
+    assert (dg != want_dg).float().mean().item() <= 2 ** -20
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("rows, width", [(1, 8), (31, 40), (300, 2048), (297, 1000), (5, 8192)])
 def test_norm_weight_gradients_sum_every_row_once(rows, width):
     """Exact oracle: with dy = 1 and x of one value per row the weight gradient is the sum of the row signs."""

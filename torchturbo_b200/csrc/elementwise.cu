@@ -166,113 +166,6 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
 }
 
 // ============================================================================
-// Gated RMSNorm of short rows (head widths of the linear-attention layers): y = bf16(n * act(gate)) with
-// n = bf16(bf16(x * rstd) * w), H = 8 L channels held by L lanes, so a warp normalises 32 / L rows with shuffles only.
-//   dn = bf16(dy * act(gate)), dgate = dy * n * act'(gate), dx and dw as in the plain norm with dn in the place of dy
-// Every rounding of the separate kernels (norm, fp32 product, cast) is kept.  Bound by memory: 131072 rows of 128 take 24 us
-// forward and 37 us backward (100 and 168 MB); the plain norm's block per row alone took 380 us backward on them.
-// ============================================================================
-template <int L>
-__device__ __forceinline__ float lane_group_sum(float v) {
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
-  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
-__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
-  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
-}
-__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
-
-template <int L>
-__global__ void __launch_bounds__(256) gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate,
-                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                               float* __restrict__ rstd_out, long long R, float eps, int silu) {
-  constexpr int H = 8 * L, ROWS = 256 / L;
-  const int l = threadIdx.x % L, c = l * 8;
-  float wf[8];
-  load8(w + c, wf);
-  // all lanes of a warp stay in the loop (the shuffles name the whole warp); rows past the end are computed and dropped
-  const long long last = (R + ROWS - 1) / ROWS * ROWS;
-  for (long long row = static_cast<long long>(blockIdx.x) * ROWS + threadIdx.x / L; row < last; row += static_cast<long long>(gridDim.x) * ROWS) {
-    const bool ok = row < R;
-    float f[8] = {}, g[8] = {};
-    if (ok) { load8(x + row * H + c, f); load8(gate + row * H + c, g); }
-    float ss = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
-    const float rstd = rsqrtf(lane_group_sum<L>(ss) / static_cast<float>(H) + eps);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sg = 1.f / (1.f + __expf(-g[j]));
-      f[j] = round_bf16(round_bf16(f[j] * rstd) * wf[j]) * (silu ? g[j] * sg : sg);
-    }
-    if (ok) {
-      store8(y + row * H + c, f);
-      if (l == 0) rstd_out[row] = rstd;
-    }
-  }
-}
-
-template <int L>
-__global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                               const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ w,
-                                                               const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                                                               __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_partial,
-                                                               long long R, int silu) {
-  constexpr int H = 8 * L, ROWS = 256 / L;
-  __shared__ float red[ROWS][H];
-  const int l = threadIdx.x % L, c = l * 8, r0 = threadIdx.x / L;
-  float wf[8], dw[8] = {};
-  load8(w + c, wf);
-  const long long last = (R + ROWS - 1) / ROWS * ROWS;
-  for (long long row = static_cast<long long>(blockIdx.x) * ROWS + r0; row < last; row += static_cast<long long>(gridDim.x) * ROWS) {
-    const bool ok = row < R;
-    float f[8] = {}, g[8] = {}, d[8] = {};
-    float rstd = 0.f;
-    if (ok) {
-      load8(x + row * H + c, f);
-      load8(gate + row * H + c, g);
-      load8(dy + row * H + c, d);
-      rstd = rstd_in[row];
-    }
-    float dot = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sg = 1.f / (1.f + __expf(-g[j])), act = silu ? g[j] * sg : sg;
-      const float n = round_bf16(round_bf16(f[j] * rstd) * wf[j]);
-      const float slope = silu ? sg * (1.f + g[j] * (1.f - sg)) : sg * (1.f - sg);
-      g[j] = d[j] * n * slope;
-      f[j] *= rstd;
-      const float dn = round_bf16(d[j] * act);
-      dw[j] += dn * f[j];
-      d[j] = dn * wf[j];
-      dot += d[j] * f[j];
-    }
-    dot = lane_group_sum<L>(dot) / static_cast<float>(H);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) d[j] = rstd * (d[j] - f[j] * dot);
-    if (ok) {
-      store8(dx + row * H + c, d);
-      store8(dgate + row * H + c, g);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) red[r0][c + j] = dw[j];
-  __syncthreads();
-  for (int e = threadIdx.x; e < H; e += 256) {
-    float s = 0.f;
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) s += red[r][e];
-    dw_partial[static_cast<long long>(blockIdx.x) * H + e] = s;
-  }
-}
-
-// ============================================================================
 // LayerNorm (weight + bias) for the vision tower: fp32 statistics, bf16 in / out.
 //   y = (x - mean) * rstd * w + b
 //   dx = rstd * (g - mean(g) - xhat * mean(g * xhat)),  g = dy * w ; dw = sum dy * xhat ; db = sum dy
@@ -1304,35 +1197,6 @@ TTB_EXPORT int ttb_layernorm_bwd(const void* dy, const void* x, const void* w, c
   else if (iters <= 4) layernorm_bwd_kernel<4><<<grid, threads, 0, STREAM(stream)>>>(DY, X, W, mean, rstd, (__nv_bfloat16*)dx, part, T, H);
   else return 902;
   colsum(part, dwdb_out, out_bf16, grid, 2 * H, STREAM(stream));
-  LAUNCH_RET();
-}
-
-// H: 64, 128 or 256; all bf16 pointers on 16-byte boundaries
-TTB_EXPORT int ttb_gated_rmsnorm_fwd(const void* x, const void* gate, const void* w, void* y, float* rstd, long long R, int H, float eps,
-                                     int silu, int grid, void* stream) {
-  if (R == 0) return 0;
-  if (((uintptr_t)x | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)y) & 15) return 902;
-  auto X = (const __nv_bfloat16*)x; auto G = (const __nv_bfloat16*)gate; auto W = (const __nv_bfloat16*)w;
-  auto Y = (__nv_bfloat16*)y;
-  if (H == 64) gated_rmsnorm_fwd_kernel<8><<<grid, 256, 0, STREAM(stream)>>>(X, G, W, Y, rstd, R, eps, silu);
-  else if (H == 128) gated_rmsnorm_fwd_kernel<16><<<grid, 256, 0, STREAM(stream)>>>(X, G, W, Y, rstd, R, eps, silu);
-  else if (H == 256) gated_rmsnorm_fwd_kernel<32><<<grid, 256, 0, STREAM(stream)>>>(X, G, W, Y, rstd, R, eps, silu);
-  else return 901;
-  LAUNCH_RET();
-}
-
-// dw_partial must hold grid * H floats
-TTB_EXPORT int ttb_gated_rmsnorm_bwd(const void* dy, const void* x, const void* gate, const void* w, const float* rstd, void* dx,
-                                     void* dgate, float* dw_partial, void* dw_out, long long R, int H, int silu, int grid, void* stream) {
-  if (R == 0) return 0;
-  if (((uintptr_t)dy | (uintptr_t)x | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)dx | (uintptr_t)dgate) & 15) return 902;
-  auto D = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto G = (const __nv_bfloat16*)gate;
-  auto W = (const __nv_bfloat16*)w; auto DX = (__nv_bfloat16*)dx; auto DG = (__nv_bfloat16*)dgate;
-  if (H == 64) gated_rmsnorm_bwd_kernel<8><<<grid, 256, 0, STREAM(stream)>>>(D, X, G, W, rstd, DX, DG, dw_partial, R, silu);
-  else if (H == 128) gated_rmsnorm_bwd_kernel<16><<<grid, 256, 0, STREAM(stream)>>>(D, X, G, W, rstd, DX, DG, dw_partial, R, silu);
-  else if (H == 256) gated_rmsnorm_bwd_kernel<32><<<grid, 256, 0, STREAM(stream)>>>(D, X, G, W, rstd, DX, DG, dw_partial, R, silu);
-  else return 901;
-  colsum(dw_partial, dw_out, 1, grid, H, STREAM(stream));
   LAUNCH_RET();
 }
 

@@ -1,8 +1,17 @@
-// Column sums shared by the kernels that reduce over rows.
+// Loads of eight values and column sums, shared by the kernels that walk rows.
 #pragma once
 #include "common.cuh"
 
 namespace ttb {
+
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
 
 // Column sum of partial[rows][H] -> out[H] (fp32 or bf16); deterministic order.  32 columns and 32 row groups per block:
 // the sums are a few hundred rows long at most, so what counts is how many loads are in flight (2048 columns: 4.9 us with one
