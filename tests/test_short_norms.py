@@ -15,6 +15,37 @@ def test_gated_norm_is_the_norm_times_the_activation_on_cpu(activation):
     assert torch.allclose(got, want, atol=1e-6, rtol=1e-5)
 
 
+@pytest.mark.parametrize("activation", ["silu", "sigmoid"])
+def test_second_derivatives_go_through_the_separate_operations(activation, monkeypatch):
+    """The autograd function around stand-ins for the kernels, with a loss whose gradient is not linear in the gate."""
+    from torchturbo_b200.ops.providers import b200, native
+
+    silu = activation == "silu"
+
+    def kernel(x, gate, w, eps, is_silu):
+        with torch.no_grad():
+            return native.TorchGatedRMSNorm()(x, gate, w, eps, activation=activation), torch.ones(x.shape[0])
+
+    def kernel_bwd(dy, x, gate, w, rstd, is_silu):
+        with torch.enable_grad():
+            leaves = [t.detach().requires_grad_(True) for t in (x, gate, w)]
+            y = native.TorchGatedRMSNorm()(*leaves, 1e-6, activation=activation)
+        return torch.autograd.grad(y, leaves, dy.detach())
+
+    monkeypatch.setattr(b200.K, "gated_rmsnorm_fwd", kernel)
+    monkeypatch.setattr(b200.K, "gated_rmsnorm_bwd", kernel_bwd)
+    torch.manual_seed(0)
+    start = [torch.randn(6, 64), torch.randn(6, 64), torch.rand(64)]
+    probe = torch.randn(6, 64)
+    res = []
+    for fn in (lambda *t: b200.GatedRMSNormFn.apply(*t, 1e-6, silu), lambda *t: native.TorchGatedRMSNorm()(*t, 1e-6, activation=activation)):
+        x, gate, w = (t.clone().requires_grad_(True) for t in start)
+        (g,) = torch.autograd.grad(fn(x, gate, w).square().sum(), gate, create_graph=True)
+        res.append([g.detach(), *torch.autograd.grad((g * probe).sum(), (x, gate, w))])
+    for a, b in zip(*res):
+        assert torch.allclose(a, b, atol=1e-5, rtol=1e-5)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows, width, activation, strided", [
     (1, 128, "silu", False), (15, 128, "sigmoid", True), (33, 64, "silu", False), (9, 256, "sigmoid", False),

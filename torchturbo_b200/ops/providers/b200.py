@@ -191,12 +191,18 @@ class GatedRMSNormFn(torch.autograd.Function):
     def forward(ctx, x, gate, w, eps, silu):
         y, rstd = K.gated_rmsnorm_fwd(x, gate, w, eps, silu)
         ctx.save_for_backward(x, gate, w, rstd)
-        ctx.silu = silu
+        ctx.eps, ctx.silu = eps, silu
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, gate, w, rstd = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            # a graph of the gradient is wanted, which a kernel does not leave: by way of the separate operations
+            needs = ctx.needs_input_grad[:3]
+            y = N.TorchGatedRMSNorm()(x, gate, w, ctx.eps, activation="silu" if ctx.silu else "sigmoid")
+            grads = iter(torch.autograd.grad(y, [t for t, n in zip((x, gate, w), needs) if n], dy, create_graph=True))
+            return (*(next(grads) if n else None for n in needs), None, None)
         return (*K.gated_rmsnorm_bwd(_aligned(dy), x, gate, w, rstd, ctx.silu), None, None)
 
 
