@@ -5,11 +5,56 @@ import torch
 from torchturbo_b200.ops import ops
 
 
+def _on_cpu(monkeypatch):
+    """Torch products in the place of the kernels."""
+    from torchturbo_b200.ops.providers import b200
+
+    def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, accumulate=False, alpha=None):
+        c = (a.t() if a_mn else a).float() @ (b if b_mn else b.t()).float() * (alpha if alpha is not None else 1.0)
+        if out is None:
+            return c.to(out_dtype)
+        return out.copy_(c + out if accumulate else c)
+
+    def cross_entropy(logits, labels, grad_out=None):
+        x = logits.float().requires_grad_(True)
+        with torch.enable_grad():
+            loss = torch.nn.functional.cross_entropy(x, labels, ignore_index=-100, reduction="none")
+            (g,) = torch.autograd.grad(loss.sum(), x)
+        if grad_out is not None:
+            grad_out.copy_(g)
+        return loss.detach()
+
+    monkeypatch.setattr(b200.K, "gemm", gemm)
+    monkeypatch.setattr(b200.K, "cross_entropy", cross_entropy)
+    return b200.LinearCrossEntropyFn
+
+
+@pytest.mark.parametrize("T, chunk, held", [
+    (16, 4, "logits"), (16, 64, "logits"), (17, 64, "direct"), (17, 17, "direct"), (17, 16, "accumulator"), (17, 4, "accumulator")])
+def test_what_is_held_for_the_backward_follows_from_the_rows(T, chunk, held, monkeypatch):
+    """H = 8: up to 16 rows d(logits); beyond that d(W), in the weight's dtype from one chunk and in fp32 from several."""
+    fn = _on_cpu(monkeypatch)
+    torch.manual_seed(T)
+    H, V = 8, 24
+    h, w = torch.randn(T, H).to(torch.bfloat16).requires_grad_(True), torch.randn(V, H).to(torch.bfloat16).requires_grad_(True)
+    lab = torch.randint(0, V, (T,))
+    loss = fn.apply(h, w, lab, chunk) * 0.5
+    kept = {(tuple(t.shape), t.dtype) for t in loss.grad_fn.next_functions[0][0].saved_tensors if t is not None}
+    want = {"logits": {((T, V), torch.bfloat16), ((T, H), torch.bfloat16)}, "direct": {((V, H), torch.bfloat16), ((T, H), torch.bfloat16)},
+            "accumulator": {((V, H), torch.float32), ((T, H), torch.bfloat16)}}[held]
+    assert kept == want
+    loss.backward()
+    hd, wd = h.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    torch.nn.functional.cross_entropy(hd @ wd.t(), lab, reduction="sum").mul(0.5).backward()
+    for a, b in ((h.grad, hd.grad), (w.grad, wd.grad)):
+        assert (a.double() - b).norm() <= 2 ** -6 * b.norm()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("T, H, V, chunk", [(1, 64, 128, 4), (130, 128, 1000, 64), (257, 128, 1000, 64), (200, 64, 520, 512), (256, 128, 1032, 100)])
 @pytest.mark.parametrize("scale", [1.0, 0.37])
 def test_whole_and_chunked_forms_agree_with_fp64(T, H, V, chunk, scale):
-    """T <= 2 H or one chunk takes the single piece, (257, 128) the chunked form.  d(logits) are rounded to bf16 (2^-9) and
+    """T <= 2 H takes the single piece, (200, 64) one chunk, (257, 128) several.  d(logits) are rounded to bf16 (2^-9) and
     gradients once more, so 2^-7 of the norm bounds both."""
     gen = torch.Generator().manual_seed(T)
     h0, w0 = torch.randn(T, H, generator=gen).to(torch.bfloat16), (torch.randn(V, H, generator=gen) * H ** -0.5).to(torch.bfloat16)

@@ -654,10 +654,13 @@ class LinearCrossEntropyFn(torch.autograd.Function):
     produce d(hidden) and d(W).
 
     Rows in one piece (`whole`): d(logits) of all rows are kept and the backward makes d(W) with a single GEMM over all
-    tokens, the incoming gradient folded into its epilogue.  Otherwise rows go chunk by chunk, d(W) accumulates in fp32 and
-    the backward scales it.  An fp32 accumulator costs a read and a write of `4 V H` bytes per chunk and another pass to
-    scale and round it; d(logits) of T rows take `2 T V` bytes, so up to T = 2 H rows (or one chunk) the single piece needs no more memory
-    than the accumulator it replaces.  4096 x 2048 x 151936, forward + backward: 13.1 ms in four chunks,
+    tokens, the incoming gradient folded into its epilogue.  Otherwise rows go chunk by chunk: one chunk writes d(W) directly,
+    several accumulate it in fp32, and the backward scales it.
+
+    An fp32 accumulator costs a read and a write of `4 V H` bytes per chunk and another pass to scale and round it.
+    d(logits) of T rows take `2 T V` bytes from the forward to the backward, so up to T = 2 H rows the single piece holds no more
+    than the accumulator (a d(W) of one chunk holds `2 V H`, but both forms peak at `2 T V + 2 V H`).  More rows than that keep
+    the chunks, whatever their size.  4096 x 2048 x 151936, forward + backward: 13.1 ms in four chunks,
     6.9 ms in one piece (the input-gradient GEMM also gets 256 tiles instead of 64 at a time)."""
 
     @staticmethod
@@ -667,7 +670,7 @@ class LinearCrossEntropyFn(torch.autograd.Function):
         T, V = h2.shape[0], weight.shape[0]
         need_h, need_w = hidden.requires_grad, weight.requires_grad
         mg = getattr(weight, "main_grad", None)
-        ctx.whole = need_w and mg is None and 0 < T <= max(chunk_size, 2 * h2.shape[1])
+        ctx.whole = need_w and mg is None and 0 < T <= 2 * h2.shape[1]
         ctx.meta = (hidden.shape, weight.dtype, mg is not None)
         if ctx.whole:
             logits = K.gemm(h2, weight)
@@ -678,7 +681,8 @@ class LinearCrossEntropyFn(torch.autograd.Function):
             return total
         dh = torch.empty_like(h2) if need_h else None
         dw = None
-        if need_w:
+        direct = need_w and mg is None and 0 < T <= chunk_size
+        if need_w and not direct:
             dw = mg if mg is not None else torch.zeros(V, h2.shape[1], dtype=torch.float32, device=h2.device)
         total = torch.zeros((), dtype=torch.float32, device=h2.device)
         for s in range(0, T, chunk_size):
@@ -688,7 +692,9 @@ class LinearCrossEntropyFn(torch.autograd.Function):
             total += loss.sum()
             if need_h:
                 K.gemm(logits, weight, b_mn=True, out=dh[s:s + chunk_size])
-            if need_w:
+            if direct:
+                dw = K.gemm(logits, hc, a_mn=True, b_mn=True, out_dtype=weight.dtype)
+            elif need_w:
                 K.gemm(logits, hc, a_mn=True, b_mn=True, out=dw, accumulate=True)
         ctx.save_for_backward(dh, dw if (need_w and mg is None) else None)
         return total
