@@ -6,9 +6,10 @@ from torchturbo_b200.ops import ops
 
 
 def _on_cpu(monkeypatch):
-    """Torch products in the place of the kernels."""
+    """Torch products in the place of the kernels, unseen by autograd as those are."""
     from torchturbo_b200.ops.providers import b200
 
+    @torch.no_grad()
     def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, accumulate=False, alpha=None):
         c = (a.t() if a_mn else a).float() @ (b if b_mn else b.t()).float() * (alpha if alpha is not None else 1.0)
         if out is None:
@@ -48,6 +49,19 @@ def test_what_is_held_for_the_backward_follows_from_the_rows(T, chunk, held, mon
     torch.nn.functional.cross_entropy(hd @ wd.t(), lab, reduction="sum").mul(0.5).backward()
     for a, b in ((h.grad, hd.grad), (w.grad, wd.grad)):
         assert (a.double() - b).norm() <= 2 ** -6 * b.norm()
+
+
+@pytest.mark.parametrize("T", [16, 17])
+def test_incoming_gradient_stays_in_a_graph_of_the_gradients(T, monkeypatch):
+    """d(grad)/d(scale) for a loss that a trainable scale multiplies, in the single piece (16 rows) as in the other forms."""
+    fn = _on_cpu(monkeypatch)
+    torch.manual_seed(0)
+    h, w = torch.randn(T, 8).to(torch.bfloat16).requires_grad_(True), torch.randn(24, 8).to(torch.bfloat16).requires_grad_(True)
+    scale, lab = torch.tensor(0.5, requires_grad=True), torch.randint(0, 24, (T,))
+    gh, gw = torch.autograd.grad(fn.apply(h, w, lab, 64) * scale, (h, w), create_graph=True)
+    for g in (gh, gw):
+        (d,) = torch.autograd.grad(g.float().square().sum(), scale, retain_graph=True)
+        assert abs(d.item() - 4 * g.float().square().sum().item()) <= 2 ** -5 * abs(d.item())      # grad = scale * x
 
 
 @pytest.mark.gpu

@@ -704,7 +704,10 @@ class LinearCrossEntropyFn(torch.autograd.Function):
         shape, wdtype, fused = ctx.meta
         if ctx.whole:
             dh, dlogits, h2 = ctx.saved_tensors
-            gw = K.gemm(dlogits, h2, a_mn=True, b_mn=True, out_dtype=wdtype, alpha=g.float().reshape(1))
+            if torch.is_grad_enabled():            # the factor stays where a graph of the gradient can see it
+                gw = (K.gemm(dlogits, h2, a_mn=True, b_mn=True, out_dtype=torch.float32) * g).to(wdtype)
+            else:
+                gw = K.gemm(dlogits, h2, a_mn=True, b_mn=True, out_dtype=wdtype, alpha=g.float().reshape(1))
         else:
             dh, dw = ctx.saved_tensors
             gw = (dw * g).to(wdtype) if dw is not None else None
