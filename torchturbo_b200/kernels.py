@@ -159,9 +159,10 @@ def status(reset: bool = False) -> tuple[int, int]:
 def gemm_splits(M: int, N: int, K: int, sms: int) -> int:
     """Into how many pieces along K a dense product is cut.  A product with few output tiles keeps few SMs busy for
     ``K / 64`` steps each; cut in ``S`` pieces it keeps ``S`` times as many busy for ``1 / S`` of the steps, plus a pass over
-    ``S`` fp32 partial results.  Worth it while at most half of the SMs have a tile and every piece keeps 32 k-blocks, so
-    that the loop outweighs the second launch (6 tiles of 500 steps, the input gradient of a 32000-row loss head: 150 us less
-    for a sum of 4 us); short K stays whole."""
+    ``S`` fp32 partial results.  Worth it while at most half of the SMs have a tile and a piece keeps 32 k-blocks (the pieces
+    are equal but for the last, which takes what is left: 97 blocks go 33, 33, 31), so that the loop outweighs the second
+    launch (6 tiles of 500 steps, the input gradient of a 32000-row loss head: 150 us less for a sum of 4 us); short K stays
+    whole."""
     tiles = ((M + 127) // 128) * ((N + 255) // 256 if N > 128 else 1)
     if N % 8 or tiles == 0:
         return 1
