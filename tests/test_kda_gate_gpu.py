@@ -84,3 +84,9 @@ def test_gate_values_are_as_accurate_as_fp32_torch(bound):
         big = want.abs() > 2 ** -120
         err, ref = (((t - want).abs() / want.abs())[big].max().item() for t in (mine, fp32))
         assert err <= 2 * ref + 2 ** -23, (err, ref)
+
+
+@pytest.mark.gpu
+def test_bound_given_as_a_tensor_takes_the_formula():
+    g, A, bound = torch.randn(1, 5, 2, 128, device="cuda").to(torch.bfloat16), torch.zeros(2, device="cuda"), torch.tensor(-5.0, device="cuda")
+    assert torch.equal(_gate(g, A, None, bound), kda_gate(g, A, None, bound))

@@ -340,7 +340,8 @@ class KDAGate(torch.autograd.Function):
 def _gate(g, A_log, dt_bias, lower_bound):
     H, Kd = g.shape[-2:]
     plain = (torch.bfloat16, torch.float32)
-    if (_kernel_ok(g, Kd, 128) and g.dtype == torch.bfloat16 and A_log.is_cuda and A_log.shape == (H,) and A_log.dtype in plain
+    if (_kernel_ok(g, Kd, 128) and (lower_bound is None or isinstance(lower_bound, (int, float)))
+            and g.dtype == torch.bfloat16 and A_log.is_cuda and A_log.shape == (H,) and A_log.dtype in plain
             and (dt_bias is None or (dt_bias.is_cuda and dt_bias.numel() == H * Kd and dt_bias.dtype in plain))):
         dt = dt_bias.reshape(H * Kd).contiguous() if dt_bias is not None else None
         return KDAGate.apply(g.reshape(-1, H, Kd).contiguous(), A_log.contiguous(), dt, lower_bound).view(g.shape)
