@@ -22,9 +22,13 @@
 // takes 2.66 ms, against 10.4 when the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and
 // gathers over materialised [chunk, 64, 64 .. 128] tensors.
 //
-// Why mma.sync and not tcgen05: the products are 64 x 64 x 128 at most, each feeds the next through registers and
-// shared memory, and their operands are built element by element (splits, decays); the kernels are bound by moving
-// states and by these small dependent steps, not by the tensor pipe.
+// Why mma.sync and not tcgen05: the products are 64 x 64 x 128 at most, each feeds the next through registers and shared
+// memory, and their operands are built element by element (splits, decays).  What bounds them, from the counters of the same
+// case: bwd_post moves 0.69 GB (0.11 ms at the copy rate) and keeps the tensor pipe 33 % active with 12,000 mma.sync per chunk
+// and head; one CTA of 16 warps fills 43 % of the issue slots, and its warps wait for the tensor pipe, for results of their own
+// instructions, at barriers between the phases and for loads in similar shares.  out and prep: tensor pipe 30 and 14 %, issue
+// slots 49 and 44 %, traffic a third and a quarter of their time.  So neither memory nor the tensor pipe is full: it is the chain
+// of phases, in which every warp splits again the fp32 tiles that it shares with three others.
 #pragma once
 #include "common.cuh"
 

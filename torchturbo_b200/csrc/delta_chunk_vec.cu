@@ -12,7 +12,7 @@
 // The backward is split in two so that each half fits one SM's shared memory: `score` (T^T dx, dL, dA and the pairwise
 // sums) and `state` (products with S and dS, and the final gradients); 128 KB per chunk and head pass between them.
 //
-// Measured (2047 tokens, 8 heads, three documents): prep 55 us, out 43, bwd_pre 22, score 95, state 72; the operator with its
+// Measured (2047 tokens, 8 heads, three documents): prep 54 us, out 42, bwd_pre 22, score 92, state 73; the operator with its
 // gates, forward + backward, takes 0.86 ms (6.9 ms and 467 launches as batched torch products, 21 launches now).
 #include "delta_chunk.cuh"
 
