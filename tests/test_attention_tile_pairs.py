@@ -1,0 +1,81 @@
+"""Forward attention with two query tiles per thread block, and the choice between one and two."""
+import math
+
+import pytest
+import torch
+
+from torchturbo_b200 import kernels as K
+
+
+@pytest.mark.parametrize("lens,heads,causal,rows", [
+    ([16001], 40, True, 256), ([1100, 900, 1300, 796], 32, True, 256), ([784, 816], 16, False, 256),
+    ([2048], 16, True, 128), ([8192], 4, True, 128), ([100, 100, 100], 8, True, 128), ([784], 16, False, 128),
+    ([0, 5, 0], 1, True, 128), ([], 1, True, 128),
+])
+def test_query_rows_per_block(lens, heads, causal, rows):
+    """Many blocks take two tiles each; where the longest block would decide, each takes one."""
+    assert K.attn_tile_rows(lens, heads, causal, 148) == rows
+
+
+def test_pair_table_covers_the_same_rows():
+    cu = torch.tensor([3, 3, 4, 260, 516, 773, 1000], dtype=torch.int32)
+    one, two = (K.build_q_tiles(cu, b).tolist() for b in (128, 256))
+    covered = sorted((q, s, e) for q0, s, e in two for q in (q0, q0 + 128) if q < e)
+    assert covered == sorted(map(tuple, one))
+
+
+def _reference(q, k, v, cu, causal, scale):
+    """fp32 result, sum of |p v| and logsumexp."""
+    rep = q.shape[1] // k.shape[1]
+    out, mag = torch.zeros(2, q.shape[0], q.shape[1], 128, device=q.device)
+    lse = torch.full((q.shape[1], q.shape[0]), -math.inf, device=q.device)
+    for a, b in zip(cu[:-1], cu[1:]):
+        qq = q[a:b].float().transpose(0, 1)
+        kk, vv = (t[a:b].float().repeat_interleave(rep, 1).transpose(0, 1) for t in (k, v))
+        s = qq @ kk.transpose(1, 2) * scale
+        if causal:
+            s = s.masked_fill(torch.ones(b - a, b - a, dtype=torch.bool, device=q.device).triu(1), -math.inf)
+        p = s.softmax(-1)
+        out[a:b], mag[a:b] = (p @ vv).transpose(0, 1), (p @ vv.abs()).transpose(0, 1)
+        lse[:, a:b] = s.logsumexp(-1)
+    return out, mag, lse
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [128, 256])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("D,Hq,Hk", [(128, 4, 2), (192, 2, 2)])
+@pytest.mark.parametrize("rising", [False, True])
+def test_both_tile_counts(rows, causal, D, Hq, Hk, rising):
+    """Documents around the tile edges.  `rising`: the keys grow along a document, so that later blocks raise a row's maximum
+    and the accumulator is rescaled."""
+    lens = [1, 127, 128, 129, 255, 256, 257, 384, 385, 640, 900]
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    T = cu[-1] + 5                                      # rows behind the last boundary read as zero
+    g = torch.Generator("cuda").manual_seed(D + rows)
+    q, k, v = (torch.randn(T, h, d, generator=g, device="cuda") for h, d in ((Hq, D), (Hk, D), (Hk, 128)))
+    if rising:
+        pos = torch.cat([torch.arange(n) for n in lens + [5]]).cuda().float()
+        k = k + q[:, :Hk].sign() * (pos / 20)[:, None, None]
+        q = q.abs() * 0.5 + q.sign() * 0.1
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    bounds = torch.tensor(cu, dtype=torch.int32)
+    scale = D ** -0.5
+    out, lse, ml = K.attn_fwd(q, k, v, K.build_q_tiles(bounds, rows).cuda(), scale=scale, causal=causal, want_max_logit=True,
+                              rows=(cu[0], cu[-1]), tile_rows=rows)
+    torch.cuda.synchronize()
+    assert K.attn_status()[0] == 0
+    ref, mag, ref_lse = _reference(q, k, v, cu, causal, scale)
+    assert torch.equal(out[cu[-1]:], torch.zeros_like(out[cu[-1]:]))
+    # probabilities are rounded to bf16 and so is the result: 8 significant bits, half a unit in the last place is 2^-8 relative;
+    # scores up to about 2^7 in fp32, sums of up to 900 terms and the fp32 reference itself account for another 1e-4 of the
+    # magnitudes
+    bound = 2.0 ** -8 * (mag + ref.abs()) + 1e-4 * mag + 1e-6
+    assert ((out.float() - ref).abs() <= bound)[: cu[-1]].all()
+    assert (lse[:, : cu[-1]] - ref_lse[:, : cu[-1]]).abs().max() < 1e-4 * max(1.0, float(ref_lse[:, : cu[-1]].abs().max()))
+    top = max(float((q[a:b].float().transpose(0, 1) @ k[a:b].float().repeat_interleave(Hq // Hk, 1).permute(1, 2, 0) * scale)
+                    .masked_fill(torch.ones(b - a, b - a, dtype=torch.bool, device="cuda").triu(1) & causal, -math.inf).max())
+              for a, b in zip(cu[:-1], cu[1:]))
+    assert abs(float(ml.max()) - top) <= 1e-4 * max(1.0, abs(top))

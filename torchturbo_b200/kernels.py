@@ -729,15 +729,23 @@ def attn_status(reset: bool = False) -> tuple[int, int]:
 def build_kv_tiles(cu_seqlens, block: int = 128) -> torch.Tensor:
     """Table of 128-row KV tiles for the backward pass, earliest tile of a document first (under a causal mask the
     earliest KV tiles are seen by the most query tiles, so they carry the most work)."""
+    return torch.tensor(kv_tile_rows(cu_seqlens, block), dtype=torch.int32).reshape(-1, 3)
+
+
+def kv_tile_rows(cu_seqlens, block: int = 128) -> list:
     offs = cu_seqlens.tolist() if isinstance(cu_seqlens, torch.Tensor) else list(cu_seqlens)
     rows = [(k0, a, b) for a, b in zip(offs[:-1], offs[1:]) for k0 in range(a, b, block)]
-    rows.sort(key=lambda r: -(r[2] - r[0]))
-    return torch.tensor(rows, dtype=torch.int32).reshape(-1, 3)
+    rows.sort(key=lambda r: r[0] - r[2])
+    return rows
 
 
 def build_q_tiles(cu_seqlens, block: int = 128) -> torch.Tensor:
     """Host-side table of 128-row query tiles `[n, 3] = (first row, document start, document end)` from packed
     boundaries (a CPU tensor or list); no device synchronisation is involved."""
+    return torch.tensor(q_tile_rows(cu_seqlens, block), dtype=torch.int32).reshape(-1, 3)
+
+
+def q_tile_rows(cu_seqlens, block: int = 128) -> list:
     offs = cu_seqlens.tolist() if isinstance(cu_seqlens, torch.Tensor) else list(cu_seqlens)
     rows = []
     for a, b in zip(offs[:-1], offs[1:]):
@@ -745,8 +753,32 @@ def build_q_tiles(cu_seqlens, block: int = 128) -> torch.Tensor:
         # emit them first to shorten the tail of the launch
         for q0 in range(a + ((b - a - 1) // block) * block, a - 1, -block) if b > a else ():
             rows.append((q0, a, b))
-    rows.sort(key=lambda r: -(r[0] - r[1]))          # across documents too: the tiles with the most KV blocks first
-    return torch.tensor(rows, dtype=torch.int32).reshape(-1, 3)
+    rows.sort(key=lambda r: r[1] - r[0])             # across documents too: the tiles with the most KV blocks first
+    return rows
+
+
+def attn_tile_rows(lens, heads: int, causal: bool, sms: int) -> int:
+    """Query rows that a thread block of the forward kernel takes (the `block` of `build_q_tiles`): two tiles of 128 rows where
+    that fills the GPU, one where the longest block of the launch would then be what everything waits for.
+
+    Compared are the estimates of both launches in thousands of clocks: the longest block against the sum of all blocks over
+    the SMs.  A kv block costs 2.05 with one query tile and 3.35 with two (16001 tokens, 40 heads: 2442 us and 2110 us), and
+    every block 8 more to start and end.  Measured, one tile / two: 8192 tokens x 4 heads 76 / 121 us, 2048 x 16 31 / 39,
+    2048 x 24 46 / 39, 2048 x 32 54 / 46, 4 documents of 4096 x 32 82 / 68; full attention, 784 tokens x 16 heads 17 / 23,
+    two such documents 29 / 25."""
+
+    def launch(step: int, per_block: float) -> float:
+        longest = total = 0.0
+        for n in lens:
+            tiles = (n + 127) // 128
+            entries = (tiles + step - 1) // step
+            # entry i of a causal document sees min(step (i + 1), tiles) blocks, each entry of a full one all of them
+            blocks = step * entries * (entries - 1) // 2 + tiles if causal and tiles else entries * tiles
+            total += blocks * per_block + 8.0 * entries
+            longest = max(longest, tiles * per_block + 8.0)
+        return max(longest, total * heads / sms)
+
+    return 256 if launch(2, 3.35) < launch(1, 2.05) else 128
 
 
 def _zero_outside(t: torch.Tensor, rows) -> torch.Tensor:
@@ -762,9 +794,10 @@ def _zero_outside(t: torch.Tensor, rows) -> torch.Tensor:
 
 
 def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_lse: bool = True,
-             want_max_logit: bool = False, rows=None):
+             want_max_logit: bool = False, rows=None, tile_rows: int = 128):
     """q: [T, Hq, D]; k: [T, Hk, D] with D = 128 or 192 (multi-head latent attention); v: [T, Hk, 128] (may be a
-    row-strided view).  `rows` (optional): (first, one past the last) row that the tile table covers; the kernel writes
+    row-strided view).  `q_tiles_dev`: `build_q_tiles(cu, tile_rows)`, one thread block per entry and query head, with
+    `tile_rows` 128 or 256.  `rows` (optional): (first, one past the last) row that the tile table covers; the kernel writes
     every one of them.  Returns (out [T, Hq, 128], lse [Hq, T], max_logit [Hq])."""
     T, Hq, D = q.shape
     Hk = k.shape[1]
@@ -776,7 +809,7 @@ def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_ls
     ml = torch.full((Hq,), float("-inf"), dtype=torch.float32, device=q.device) if want_max_logit else None
     _check(lib().ttb_attn_fwd(_p(q), C.c_longlong(q.stride(0)), _p(k), C.c_longlong(k.stride(0)), _p(v),
                               C.c_longlong(v.stride(0)), _p(out), _p(lse), _p(ml), _p(q_tiles_dev),
-                              C.c_int(q_tiles_dev.shape[0]), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D),
+                              C.c_int(q_tiles_dev.shape[0]), C.c_int(tile_rows), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D),
                               C.c_float(scale), C.c_int(int(causal)), _stream()), "ttb_attn_fwd")
     return out, lse, ml
 

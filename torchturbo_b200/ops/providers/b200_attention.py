@@ -15,27 +15,45 @@ from . import native as N
 from .b200 import BF16, _B200Op, _ok
 
 
+class _Tiles:
+    """Tile tables of one batch on the device: query tiles of 128 rows and pairs of them, key tiles and the boundaries, in one
+    copy from pinned memory (asynchronous), with what the host knows of the boundaries."""
+
+    def __init__(self, cu_seqlens, device):
+        offs = cu_seqlens.tolist()
+        tables = K.q_tile_rows(offs), K.q_tile_rows(offs, 256), K.kv_tile_rows(offs)
+        flat = torch.tensor([x for table in tables for row in table for x in row] + offs, dtype=torch.int32)
+        *views, self.cu = flat.pin_memory().to(device, non_blocking=True).split([3 * len(t) for t in tables] + [len(offs)])
+        q1, q2, self.kv = (v.view(-1, 3) for v in views)
+        self.q = {128: q1, 256: q2}
+        self.n_valid = offs[-1]
+        # the tables cover [first, last) without holes when the boundaries do not decrease
+        self.rows = (offs[0], offs[-1]) if all(a <= b for a, b in zip(offs[:-1], offs[1:])) else None
+        self.lens = [max(b - a, 0) for a, b in zip(offs[:-1], offs[1:])]
+        self._tile_rows: dict = {}
+
+    def tile_rows(self, heads: int, causal: bool) -> int:
+        key = (heads, causal)
+        if key not in self._tile_rows:
+            self._tile_rows[key] = K.attn_tile_rows(self.lens, heads, causal, K.num_sms(self.cu.device.index))
+        return self._tile_rows[key]
+
+
 @cache
-def _tiles_for(cu_seqlens, device):
-    """(query-tile table on the device, number of valid tokens, boundaries on the device, key-tile table, covered rows)
-    for one batch; built once and shared by every layer (pinned staging keeps the copies asynchronous)."""
-    t = K.build_q_tiles(cu_seqlens).pin_memory()
-    tk = K.build_kv_tiles(cu_seqlens).pin_memory()
-    cu = cu_seqlens.to(torch.int32).pin_memory()
-    offs = cu_seqlens.tolist()
-    # the tables cover [first, last) without holes when the boundaries do not decrease
-    rows = (offs[0], offs[-1]) if all(a <= b for a, b in zip(offs[:-1], offs[1:])) else None
-    return (t.to(device, non_blocking=True), offs[-1], cu.to(device, non_blocking=True),
-            tk.to(device, non_blocking=True), rows)
+def _tiles_for(cu_seqlens, device) -> _Tiles:
+    """Built once for a batch and shared by every layer."""
+    return _Tiles(cu_seqlens, device)
 
 
 class FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens, max_seqlen, causal, scale, want_ml):
-        tiles, n_valid, _, _, rows = _tiles_for(cu_seqlens, q.device)
-        out, lse, ml = K.attn_fwd(q, k, v, tiles, scale=scale, causal=causal, want_max_logit=want_ml, rows=rows)
+        tiles = _tiles_for(cu_seqlens, q.device)
+        block = tiles.tile_rows(q.shape[1], causal)
+        out, lse, ml = K.attn_fwd(q, k, v, tiles.q[block], scale=scale, causal=causal, want_max_logit=want_ml, rows=tiles.rows,
+                                  tile_rows=block)
         ctx.save_for_backward(q, k, v, out, lse)
-        ctx.meta = (cu_seqlens, max_seqlen, causal, scale, n_valid)
+        ctx.meta = (cu_seqlens, max_seqlen, causal, scale, tiles.n_valid)
         if want_ml:
             ctx.mark_non_differentiable(ml)
             return out, ml
@@ -46,15 +64,15 @@ class FlashAttnFn(torch.autograd.Function):
         q, k, v, out, lse = ctx.saved_tensors
         cu_seqlens, max_seqlen, causal, scale, n = ctx.meta
         if os.environ.get("TORCHTURBO_ATTN_BWD", "tcgen05") == "tcgen05":
-            cached = _tiles_for(cu_seqlens, q.device)
-            dq, dk, dv = K.attn_bwd(dout.contiguous(), q, k, v, out, lse, cached[3], scale=scale, causal=causal,
-                                    q_tiles_dev=cached[0], deterministic=torch.are_deterministic_algorithms_enabled(),
-                                    rows=cached[4])
+            tiles = _tiles_for(cu_seqlens, q.device)
+            dq, dk, dv = K.attn_bwd(dout.contiguous(), q, k, v, out, lse, tiles.kv, scale=scale, causal=causal,
+                                    q_tiles_dev=tiles.q[128], deterministic=torch.are_deterministic_algorithms_enabled(),
+                                    rows=tiles.rows)
             return dq, dk, dv, None, None, None, None, None
         # library backward on this kernel's out / lse (selected with TORCHTURBO_ATTN_BWD=flash_attn2; used as a baseline)
         from flash_attn.flash_attn_interface import _flash_attn_varlen_backward
 
-        cu = _tiles_for(cu_seqlens, q.device)[2]
+        cu = _tiles_for(cu_seqlens, q.device).cu
         if max_seqlen is None:
             max_seqlen = int((cu_seqlens[1:] - cu_seqlens[:-1]).max())
         dq, dk, dv = torch.zeros_like(q), torch.zeros_like(k), torch.zeros(k.shape, dtype=k.dtype, device=k.device)
