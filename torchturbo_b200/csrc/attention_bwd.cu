@@ -200,14 +200,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
+    // ---------------------------------------------------------------- MMA issuer (the whole warp, see umma_ss_w)
+    // One diverged lane took long enough over the descriptors to hold up the tensor cores: 4096 tokens, 32 / 8 heads, four
+    // documents 268 -> 260 us; 192-wide heads 207 -> 199; 8192 tokens, 32 heads 1772 -> 1700.
+    {
       constexpr uint32_t id_s = make_idesc_bf16(128, 64, false, false);
       constexpr uint32_t id_acc = make_idesc_bf16(128, 128, false, true);
       constexpr uint32_t id_dk = make_idesc_bf16(128, DQK, false, true);
       constexpr uint32_t id_dq = make_idesc_bf16(128, 64, true, true);
-      const uint32_t sK = smem_u32(smem + BwdSmem::K), sV = smem_u32(smem + BwdSmem::V);
-      const uint32_t sPT = smem_u32(smem + BwdSmem::PT), sDST = smem_u32(smem + BwdSmem::DST);
+      const uint32_t leader = elect_one() ? 1u : 0u;
+      // operands read along their rows (K-major) and, where a product reduces over rows, across them (MN-major)
+      const SmemDesc dK = make_smem_desc2(smem_u32(smem + BwdSmem::K), 16, 1024), dV = make_smem_desc2(smem_u32(smem + BwdSmem::V), 16, 1024);
+      const SmemDesc dQ = make_smem_desc2(smem_u32(smem + BwdSmem::Q0), 16, 1024), dDO = make_smem_desc2(smem_u32(smem + BwdSmem::DO0), 16, 1024);
+      const SmemDesc dPT = make_smem_desc2(smem_u32(smem + BwdSmem::PT), 16, 1024), dDST = make_smem_desc2(smem_u32(smem + BwdSmem::DST), 16, 1024);
+      const SmemDesc dKt = make_smem_desc2(smem_u32(smem + BwdSmem::K), 16384, 1024), dDSt = make_smem_desc2(smem_u32(smem + BwdSmem::DST), 8192, 1024);
+      const SmemDesc dQt = make_smem_desc2(smem_u32(smem + BwdSmem::Q0), 8192, 1024), dDOt = make_smem_desc2(smem_u32(smem + BwdSmem::DO0), 8192, 1024);
       bool ok = mbar_wait(kv_full, 0, KID_ATTN_BWD, 2);
       auto issue_scores = [&](int it) -> bool {
         const int st = it & 1;
@@ -215,21 +222,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (!mbar_wait(&qdo_full[st], ph, KID_ATTN_BWD, 3)) return false;
         if (!mbar_wait(st_empty, (it & 1) ^ 1, KID_ATTN_BWD, 4)) return false;
         tc_fence_after();
-        const uint32_t sQ = smem_u32(smem + BwdSmem::Q0 + st * Q_BYTES);
-        const uint32_t sDO = smem_u32(smem + BwdSmem::DO0 + st * 16384);
+        const SmemDesc q = desc_at(dQ, st * Q_BYTES), d_o = desc_at(dDO, st * 16384);
 #pragma unroll
         for (int kk = 0; kk < DQK / 16; ++kk) {  // reduction over the query / key head width
           const uint32_t offa = (kk >> 2) * 16384 + (kk & 3) * 32;   // K / V tiles: [128 rows][64 d] panels
           const uint32_t offb = (kk >> 2) * 8192 + (kk & 3) * 32;    // Q / dO tiles: [64 rows][64 d] panels
-          umma_ss(tm_ST, make_smem_desc(sK + offa, 16, 1024), make_smem_desc(sQ + offb, 16, 1024), id_s, kk != 0);
+          umma_ss_w(leader, tm_ST, desc_at(dK, offa), desc_at(q, offb), id_s, kk != 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t offa = (kk >> 2) * 16384 + (kk & 3) * 32;
           const uint32_t offb = (kk >> 2) * 8192 + (kk & 3) * 32;
-          umma_ss(tm_DPT, make_smem_desc(sV + offa, 16, 1024), make_smem_desc(sDO + offb, 16, 1024), id_s, kk != 0);
+          umma_ss_w(leader, tm_DPT, desc_at(dV, offa), desc_at(d_o, offb), id_s, kk != 0);
         }
-        umma_commit(st_full);
+        umma_commit_w(leader, st_full);
         return true;
       };
       if (ok && n_it > 0) ok = issue_scores(0);
@@ -244,33 +250,29 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (!mbar_wait(&dq_empty[st], ph2 ^ 1, KID_ATTN_BWD, 6)) { ok = false; break; }
         }
         tc_fence_after();
-        const uint32_t sPTb = sPT + st * 16384, sDSTb = sDST + st * 16384;
-        const uint32_t sQ = smem_u32(smem + BwdSmem::Q0 + st * Q_BYTES);
-        const uint32_t sDO = smem_u32(smem + BwdSmem::DO0 + st * 16384);
+        const SmemDesc pt = desc_at(dPT, st * 16384), dst = desc_at(dDST, st * 16384), dst_t = desc_at(dDSt, st * 16384);
+        const SmemDesc q_t = desc_at(dQt, st * Q_BYTES), do_t = desc_at(dDOt, st * 16384);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {  // reduction over q = 64
           // A: P^T / dS^T K-major single panel; B: dO / Q as [q rows][d] MN-major, d panels 8 KB apart
-          umma_ss(tm_DV, make_smem_desc(sPTb + kk * 32, 16, 1024), make_smem_desc(sDO + kk * 2048, 8192, 1024), id_acc,
-                  (it | kk) != 0);
+          umma_ss_w(leader, tm_DV, desc_at(pt, kk * 32), desc_at(do_t, kk * 2048), id_acc, (it | kk) != 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-          umma_ss(tm_DK, make_smem_desc(sDSTb + kk * 32, 16, 1024), make_smem_desc(sQ + kk * 2048, 8192, 1024), id_dk,
-                  (it | kk) != 0);
+          umma_ss_w(leader, tm_DK, desc_at(dst, kk * 32), desc_at(q_t, kk * 2048), id_dk, (it | kk) != 0);
         }
-        umma_commit(&qdo_empty[st]);
+        umma_commit_w(leader, &qdo_empty[st]);
         if (WITH_DQ) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {  // reduction over kv = 128
             // A: K^T from the K tile ([kv rows][d], MN-major, d panels 16 KB apart); B: dS^T ([kv rows][q]) MN-major
-            umma_ss(tm_DQT + st * 64, make_smem_desc(sK + kk * 2048, 16384, 1024),
-                    make_smem_desc(sDSTb + kk * 2048, 8192, 1024), id_dq, kk != 0);
+            umma_ss_w(leader, tm_DQT + st * 64, desc_at(dKt, kk * 2048), desc_at(dst_t, kk * 2048), id_dq, kk != 0);
           }
-          umma_commit(&dq_full[st]);
+          umma_commit_w(leader, &dq_full[st]);
         }
-        umma_commit(&pds_empty[st]);
+        umma_commit_w(leader, &pds_empty[st]);
       }
-      if (ok) umma_commit(acc_full);
+      if (ok) umma_commit_w(leader, acc_full);
     }
   } else if (warp < 10) {
     // ---------------------------------------------------------------- softmax / dS (thread = kv row, 32 query columns)

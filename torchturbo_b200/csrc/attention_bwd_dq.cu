@@ -130,11 +130,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
+    // ---------------------------------------------------------------- MMA issuer (the whole warp, see umma_ss_w)
+    {
       constexpr uint32_t id_s = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t id_dq = make_idesc_bf16(128, DQK, false, true);
-      const uint32_t sQ = smem_u32(smem + Smem::Q), sDO = smem_u32(smem + Smem::DO);
+      const uint32_t leader = elect_one() ? 1u : 0u;
+      const SmemDesc dQ = make_smem_desc2(smem_u32(smem + Smem::Q), 16, 1024), dDO = make_smem_desc2(smem_u32(smem + Smem::DO), 16, 1024);
+      const SmemDesc dK = make_smem_desc2(smem_u32(smem + Smem::K0), 16, 1024), dV = make_smem_desc2(smem_u32(smem + Smem::V0), 16, 1024);
+      const SmemDesc dKt = make_smem_desc2(smem_u32(smem + Smem::K0), 16384, 1024);
       bool ok = mbar_wait(q_full, 0, KID_ATTN_DQ, 3);
       auto issue_scores = [&](int j) -> bool {
         const int st = j & 1, vs = j % VS;
@@ -142,20 +145,19 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!mbar_wait(&v_full[vs], (j / VS) & 1, KID_ATTN_DQ, 5)) return false;
         if (!mbar_wait(s_empty, (j & 1) ^ 1, KID_ATTN_DQ, 6)) return false;
         tc_fence_after();
-        const uint32_t sK = smem_u32(smem + Smem::K0 + st * QK_BYTES);
-        const uint32_t sV = smem_u32(smem + Smem::V0 + vs * DQ_TILE);
+        const SmemDesc k = desc_at(dK, st * QK_BYTES), v = desc_at(dV, vs * DQ_TILE);
 #pragma unroll
         for (int kk = 0; kk < DQK / 16; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_ss(tm_S, make_smem_desc(sQ + off, 16, 1024), make_smem_desc(sK + off, 16, 1024), id_s, kk != 0);
+          umma_ss_w(leader, tm_S, desc_at(dQ, off), desc_at(k, off), id_s, kk != 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_ss(tm_DP, make_smem_desc(sDO + off, 16, 1024), make_smem_desc(sV + off, 16, 1024), id_s, kk != 0);
+          umma_ss_w(leader, tm_DP, desc_at(dDO, off), desc_at(v, off), id_s, kk != 0);
         }
-        umma_commit(s_full);
-        umma_commit(&v_empty[vs]);
+        umma_commit_w(leader, s_full);
+        umma_commit_w(leader, &v_empty[vs]);
         return true;
       };
       if (ok && nblk > 0) ok = issue_scores(0);
@@ -163,17 +165,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (j + 1 < nblk && !issue_scores(j + 1)) { ok = false; break; }
         if (!mbar_wait(ds_full, j & 1, KID_ATTN_DQ, 7)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t sK = smem_u32(smem + Smem::K0 + (j & 1) * QK_BYTES);
+        const SmemDesc k_t = desc_at(dKt, (j & 1) * QK_BYTES);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           // A = dS from TMEM (a k-step of 16 kv columns is 8 packed columns); B = K: MN-major [kv rows][d], a k-step of
           // 16 kv rows = 2048 bytes, d panels 16 KB apart
-          umma_ts(tm_DQ, tm_DS + kk * 8, make_smem_desc(sK + kk * 2048, 16384, 1024), id_dq, (j | kk) != 0);
+          umma_ts_w(leader, tm_DQ, tm_DS + kk * 8, desc_at(k_t, kk * 2048), id_dq, (j | kk) != 0);
         }
-        umma_commit(&k_empty[j & 1]);
-        umma_commit(ds_empty);
+        umma_commit_w(leader, &k_empty[j & 1]);
+        umma_commit_w(leader, ds_empty);
       }
-      if (ok) umma_commit(dq_done);
+      if (ok) umma_commit_w(leader, dq_done);
     }
   } else {
     // ---------------------------------------------------------------- softmax / dS (thread = query row, 64 kv columns)

@@ -296,9 +296,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
+    // ------------------------------------------------------------ MMA issuer (the whole warp, see umma_ss_w)
+    {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+      const uint32_t leader = elect_one() ? 1u : 0u;
+      const SmemDesc dA = make_smem_desc2(smem_u32(smem), A_MN ? 8192 : 16, 1024);
+      const SmemDesc dB = make_smem_desc2(smem_u32(smem) + L::A_BYTES, B_MN ? 8192 : 16, 1024);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -314,26 +317,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(&full[stage], phase, KID_GEMM, 3, consumer_budget)) {
-            if (p.ep.status) atomicCAS(p.ep.status, 0, 0x10000 | (11 << 8));
+            if (p.ep.status && leader) atomicCAS(p.ep.status, 0, 0x10000 | (11 << 8));
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * L::STAGE_BYTES);
-          const uint32_t sb = sa + L::A_BYTES;
+          const SmemDesc a = desc_at(dA, stage * L::STAGE_BYTES), b = desc_at(dB, stage * L::STAGE_BYTES);
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc(sa + kk * 2048, 8192, 1024)
-                                     : make_smem_desc(sa + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc(sb + kk * 2048, 8192, 1024)
-                                     : make_smem_desc(sb + kk * 32, 16, 1024);
-            umma_ss(d_tmem, da, db, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_ss_w(leader, d_tmem, desc_at(a, kk * (A_MN ? 2048 : 32)), desc_at(b, kk * (B_MN ? 2048 : 32)), idesc, (kb | kk) != 0);
           }
-          umma_commit(&empty[stage]);
+          umma_commit_w(leader, &empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);
+        umma_commit_w(leader, &tfull[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
