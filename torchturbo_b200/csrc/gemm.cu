@@ -1,5 +1,5 @@
 // Persistent, warp-specialised bf16 GEMM for sm_100a: TMA -> shared (128B swizzle)
-// -> tcgen05.mma (cta_group::1, M=128) -> TMEM (double-buffered accumulator)
+// -> tcgen05.mma (M=128, or M=256 by a pair of CTAs, see `pays_in_pairs`) -> TMEM (double-buffered accumulator)
 // -> tcgen05.ld epilogue.  One kernel body covers
 //   * dense  C[M,N] = A . B          with A / B each K-major or MN-major in memory,
 //   * grouped-M (MoE forward / dX): rows are grouped by expert in 128-row aligned
@@ -89,12 +89,12 @@ struct GemmParams {
   int k_splits, kb_per_split;  // > 1: "group" g covers k-blocks [g, g + 1) * kb_per_split of one product, stored at C[g]
 };
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool PAIR>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = BN * BK * 2;
+  static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;   // a CTA of a pair holds half of the tile's columns
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;
+  static constexpr int STAGES = (BN == 256 && !PAIR) ? 4 : 6;
   static constexpr int EPI_STAGE_BYTES = 32 * 32 * 4;   // one 32-row x 32-column fp32 chunk per epilogue warp
   static constexpr int EPI_BYTES = 8 * EPI_STAGE_BYTES;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/;
@@ -119,10 +119,10 @@ __device__ __forceinline__ uint32_t epi_piece_addr64(uint32_t base, int row, int
   return base + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4);
 }
 
-template <int BN, bool A_MN, bool B_MN, int EPI>
+template <int BN, bool A_MN, bool B_MN, int EPI, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS_PUSH, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-  using L = SmemLayout<BN, A_MN, B_MN>;
+  using L = SmemLayout<BN, PAIR>;
   constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -140,6 +140,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const int rank = PAIR ? static_cast<int>(cluster_ctarank()) : 0;   // CTA of the pair
+  // tiles are walked by CTAs, or by pairs of them
+  const int walker = PAIR ? blockIdx.x >> 1 : blockIdx.x, walkers = PAIR ? gridDim.x >> 1 : gridDim.x;
   // With the push prologue the producer may spend up to the exchange budget waiting for a peer's rows; the warps
   // downstream of it (MMA issuer, epilogue) must outwait it, or they give up on tiles whose rows arrive later.
   const uint64_t consumer_budget = p.ep.push_on ? p.ep.budget_ns + kWaitBudgetNs : kWaitBudgetNs;
@@ -154,38 +157,45 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], EPI_WARPS);
+      mbar_init(&tempty[a], PAIR ? 2 * EPI_WARPS : EPI_WARPS);
     }
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 2 * BN);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(tmem_slot, 2 * BN);
+    } else {
+      tmem_alloc(tmem_slot, 2 * BN);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();     // the barriers of both CTAs are set up
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
   const int groups = p.groups_k > 0 ? p.groups_k : p.k_splits;
-  const long long tiles_per_group = static_cast<long long>(p.m_tiles) * p.n_tiles;
-  const long long total_tiles = s_dead ? 0 : tiles_per_group * groups;
+  const int tiles_per_group = p.m_tiles * p.n_tiles;      // the launch checks that all tiles can be counted in 31 bits
+  const int total_tiles = s_dead ? 0 : tiles_per_group * groups;
 
   // Decode tile -> (g, m_tile, n_tile).  Tiles are walked in bands of RASTER_M m-tiles: inside a band m runs
   // fastest, then n, so the ~148 tiles in flight cover a near-square RASTER_M x (148 / RASTER_M) block of C.  Per wave
   // that needs RASTER_M A panels and ~9 B panels instead of every A panel, and a band's A panels stay in L2 while
   // its n-tiles are walked (an m-fastest walk over all m-tiles re-read A from DRAM once per n-tile column).
-  constexpr int RASTER_M = 16;
-  auto decode = [&](long long t, int& g, int& mt, int& nt) {
-    g = static_cast<int>(t / tiles_per_group);
-    const long long r = t - static_cast<long long>(g) * tiles_per_group;
-    const long long per_band = static_cast<long long>(RASTER_M) * p.n_tiles;
-    const int band = static_cast<int>(r / per_band);
+  // A pair's tile has 256 rows, so its bands have half as many; `mt` is the 128-row tile of this CTA.
+  constexpr int RASTER_M = PAIR ? 8 : 16;
+  auto decode = [&](int t, int& g, int& mt, int& nt) {
+    g = t / tiles_per_group;
+    const int r = t - g * tiles_per_group;
+    const int per_band = RASTER_M * p.n_tiles;
+    const int band = r / per_band;
     const int m_base = band * RASTER_M;
     const int band_rows = (p.m_tiles - m_base) < RASTER_M ? (p.m_tiles - m_base) : RASTER_M;
-    const long long w = r - static_cast<long long>(band) * per_band;
-    nt = static_cast<int>(w / band_rows);
-    mt = m_base + static_cast<int>(w - static_cast<long long>(nt) * band_rows);
+    const int w = r - band * per_band;
+    nt = w / band_rows;
+    mt = m_base + w - nt * band_rows;
+    if (PAIR) mt = 2 * mt + rank;
   };
   // k-range of a tile: dense -> [0, K); split -> its share of [0, K); grouped-K -> rows of group g.
   auto krange = [&](int g, int& k0, int& nkb) {
@@ -217,32 +227,46 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (!mbar_wait(&empty[stage], phase ^ 1, KID_GEMM, 1)) return false;
         uint8_t* sa = smem + stage * L::STAGE_BYTES;
         uint8_t* sb = sa + L::A_BYTES;
-        mbar_expect_tx(&full[stage], L::STAGE_BYTES);
+        // a pair's loads all complete on the leading CTA's barrier, which expects both shares
+        const uint32_t bar = PAIR ? leader_addr(&full[stage]) : 0u;
+        if (rank == 0) mbar_expect_tx(&full[stage], (PAIR ? 2 : 1) * L::STAGE_BYTES);
+        auto load_a = [&](void* dst, int x, int y) {
+          if (PAIR) tma_load_2d_pair(dst, &tmA, bar, x, y);
+          else tma_load_2d(dst, &tmA, &full[stage], x, y);
+        };
+        auto load_b = [&](void* dst, int x, int y) {
+          if (PAIR) tma_load_3d_pair(dst, &tmB, bar, x, y, bgroup);
+          else tma_load_3d(dst, &tmB, &full[stage], x, y, bgroup);
+        };
         const int kc = k0 + kb * BK;
         if (!A_MN) {
-          tma_load_2d(sa, &tmA, &full[stage], kc, m0);
+          load_a(sa, kc, m0);
         } else {
-          tma_load_2d(sa, &tmA, &full[stage], m0, kc);
-          tma_load_2d(sa + 8192, &tmA, &full[stage], m0 + 64, kc);
+          load_a(sa, m0, kc);
+          load_a(sa + 8192, m0 + 64, kc);
         }
         if (!B_MN) {
-          if (EPI == EPI_SWIGLU) {
-            tma_load_3d(sb, &tmB, &full[stage], kc, n0, bgroup);
-            tma_load_3d(sb + (BN / 2) * 128, &tmB, &full[stage], kc, p.F + n0, bgroup);
+          if (PAIR) {
+            load_b(sb, kc, EPI == EPI_SWIGLU ? rank * p.F + n0 : n0 + rank * (BN / 2));
+          } else if (EPI == EPI_SWIGLU) {
+            load_b(sb, kc, n0);
+            load_b(sb + (BN / 2) * 128, kc, p.F + n0);
           } else {
-            tma_load_3d(sb, &tmB, &full[stage], kc, n0, bgroup);
+            load_b(sb, kc, n0);
           }
         } else {
-          constexpr int PANELS = BN / 64;
+          constexpr int PANELS = BN / 64;                       // of the tile
+          constexpr int MINE = PAIR ? PANELS / 2 : PANELS;      // of this CTA
 #pragma unroll
-          for (int q = 0; q < PANELS; ++q) {
+          for (int i = 0; i < MINE; ++i) {
+            const int q = PAIR ? rank * MINE + i : i;
             int nc;
             if (EPI == EPI_SWIGLU) {
               nc = (q < PANELS / 2) ? (n0 + q * 64) : (p.F + n0 + (q - PANELS / 2) * 64);
             } else {
               nc = n0 + q * 64;
             }
-            tma_load_3d(sb + q * 8192, &tmB, &full[stage], nc, kc, bgroup);
+            load_b(sb + i * 8192, nc, kc);
           }
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -253,7 +277,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       if (elect_one()) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        for (long long t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+        for (int t = walker; t < total_tiles; t += walkers) {
           int g, mt, nt;
           decode(t, g, mt, nt);
           int bgroup = 0;
@@ -274,7 +298,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
       const int* my_flags = reinterpret_cast<const int*>(p.ep.peers.base[p.ep.rank] + p.ep.off_flags);
       bool ok = true;
-      for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      for (int t = walker; t < total_tiles && ok; t += walkers) {
         int g, mt, nt;
         decode(t, g, mt, nt);
         const int bgroup = p.tile_group[mt];
@@ -297,8 +321,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the whole warp, see umma_ss_w)
-    {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+    if (rank == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(PAIR ? 2 * BM : BM, BN, A_MN, B_MN);
       const uint32_t leader = elect_one() ? 1u : 0u;
       const SmemDesc dA = make_smem_desc2(smem_u32(smem), A_MN ? 8192 : 16, 1024);
       const SmemDesc dB = make_smem_desc2(smem_u32(smem) + L::A_BYTES, B_MN ? 8192 : 16, 1024);
@@ -307,7 +331,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      for (int t = walker; t < total_tiles && ok; t += walkers) {
         int g, mt, nt, k0, nkb;
         decode(t, g, mt, nt);
         if (p.tile_group && p.tile_group[mt] < 0) continue;
@@ -325,13 +349,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           const SmemDesc a = desc_at(dA, stage * L::STAGE_BYTES), b = desc_at(dB, stage * L::STAGE_BYTES);
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            umma_ss_w(leader, d_tmem, desc_at(a, kk * (A_MN ? 2048 : 32)), desc_at(b, kk * (B_MN ? 2048 : 32)), idesc, (kb | kk) != 0);
+            const SmemDesc ak = desc_at(a, kk * (A_MN ? 2048 : 32)), bk = desc_at(b, kk * (B_MN ? 2048 : 32));
+            if (PAIR) umma_ss_pair_w(leader, d_tmem, ak, bk, idesc, (kb | kk) != 0);
+            else umma_ss_w(leader, d_tmem, ak, bk, idesc, (kb | kk) != 0);
           }
-          umma_commit_w(leader, &empty[stage]);
+          if (PAIR) umma_commit_pair_w(leader, &empty[stage]);
+          else umma_commit_w(leader, &empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_w(leader, &tfull[acc]);
+        if (PAIR) umma_commit_pair_w(leader, &tfull[acc]);
+        else umma_commit_w(leader, &tfull[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
@@ -342,7 +370,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+    for (int t = walker; t < total_tiles && ok; t += walkers) {
       int g, mt, nt, k0, nkb;
       decode(t, g, mt, nt);
       if (p.tile_group && p.tile_group[mt] < 0) continue;
@@ -410,6 +438,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             // warp-uniform branch: every lane takes part in the transposition, rows past M are skipped on the way out
             const uint32_t st = smem_u32(epi_stage + (warp - 2) * L::EPI_STAGE_BYTES);
             __syncwarp();  // the previous chunk's readers are done with the staging area
+            if (!p.c_fp32 && !p.residual && !p.accumulate) {
+              // nothing is added in fp32: the chunk is parked as bf16, half the shared-memory traffic (grouped weight gradients,
+              // whose tiles are mostly epilogue, 342 -> 287 and 185 -> 150 us for 128 experts of 256 rows, 2048 x 1536 and 768 x 2048)
+              const int q = lane & 3;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) w[e] = pack_bf16(__uint_as_float(v[8 * i + 2 * e]), __uint_as_float(v[8 * i + 2 * e + 1]));
+                st_shared_v4(epi_piece_addr64(st, lane, i), w[0], w[1], w[2], w[3]);
+              }
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (rowptr[j] == nullptr) continue;
+                uint4 w;
+                ld_shared_v4(epi_piece_addr64(st, (lane >> 2) + 8 * j, q), w.x, w.y, w.z, w.w);
+                *reinterpret_cast<uint4*>(rowptr[j] + col0 + 8 * q) = w;
+              }
+              continue;
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               st_shared_v4(epi_piece_addr(st, lane, i), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
@@ -618,7 +667,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[acc]);
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(leader_addr(&tempty[acc]));
+        else mbar_arrive(&tempty[acc]);
+      }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
     if (p.ep.scat_on) __threadfence_system();   // this thread's peer stores are ordered before the "returned" flag
@@ -700,9 +752,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();     // the other CTA's products no longer read this shared memory, nor arrive on these barriers
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * BN);
+    if (PAIR) tmem_dealloc_pair(tmem_base, 2 * BN);
+    else tmem_dealloc(tmem_base, 2 * BN);
   }
   if (p.ep.scat_on) {
     // the last CTA to get here tells every peer that this rank has returned all of its rows
@@ -823,9 +877,9 @@ split_sum_kernel(const float* __restrict__ ws, int splits, int M, int N, void* C
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, int EPI>
+template <int BN, bool A_MN, bool B_MN, int EPI, bool PAIR>
 static int launch(const GemmArgs& a, cudaStream_t stream) {
-  using L = SmemLayout<BN, A_MN, B_MN>;
+  using L = SmemLayout<BN, PAIR>;
   CUtensorMap tmA, tmB;
   // ---- A map (2D)
   {
@@ -864,7 +918,7 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
       dims[0] = static_cast<uint64_t>(a.K);
       dims[1] = rows_b;
       box[0] = BK;
-      box[1] = (EPI == EPI_SWIGLU) ? BN / 2 : BN;
+      box[1] = (EPI == EPI_SWIGLU || PAIR) ? BN / 2 : BN;
     } else {
       // memory [K rows][N contiguous]
       dims[0] = static_cast<uint64_t>(n_mem);
@@ -897,7 +951,8 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
   }
   p.M = a.M; p.N = a.N; p.K = a.K;
   constexpr int TN = (EPI == EPI_SWIGLU) ? BN / 2 : BN;
-  p.m_tiles = a.tile_group ? a.m_tiles_cap : (a.M + BM - 1) / BM;
+  constexpr int TM = PAIR ? 2 * BM : BM;
+  p.m_tiles = a.tile_group ? a.m_tiles_cap : (a.M + TM - 1) / TM;
   p.n_tiles = (a.N + TN - 1) / TN;
   p.groups_k = a.groups_k;
   p.C = a.C; p.ldc = a.ldc; p.c_group_stride = a.c_group_stride;
@@ -916,7 +971,7 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
     p.c_fp32 = 1; p.accumulate = 0; p.residual = nullptr; p.alpha = nullptr;
   }
 
-  auto kfn = gemm_kernel<BN, A_MN, B_MN, EPI>;
+  auto kfn = gemm_kernel<BN, A_MN, B_MN, EPI, PAIR>;
   static bool smem_done[16] = {};
   {
     const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), L::TOTAL, smem_done);
@@ -924,8 +979,25 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
   }
   long long total = static_cast<long long>(p.m_tiles) * p.n_tiles * (p.groups_k > 0 ? p.groups_k : p.k_splits);
   if (total <= 0) return 0;
-  int grid = static_cast<int>(total < a.num_sms ? total : a.num_sms);
-  kfn<<<grid, p.ep.push_on ? GEMM_THREADS_PUSH : GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, p);
+  if (total >= (1ll << 31) - 65536) return 910;
+  if (PAIR) {
+    const int pairs = static_cast<int>(total < a.num_sms / 2 ? total : a.num_sms / 2);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = L::TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tmA, tmB, p);
+    if (e != cudaSuccess) return 400 + static_cast<int>(e);
+  } else {
+    const int grid = static_cast<int>(total < a.num_sms ? total : a.num_sms);
+    kfn<<<grid, p.ep.push_on ? GEMM_THREADS_PUSH : GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, p);
+  }
   if (split) {
     const long long n = static_cast<long long>(a.M) * (a.N / 4);
     split_sum_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
@@ -934,6 +1006,27 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + static_cast<int>(e);
+}
+
+// Whether two CTAs share a 256-row tile (wide products whose tiles are all of one problem).  Each then loads half of B for twice
+// the rows: a third less traffic into shared memory and out of L2, and less power for it, which under the power cap is clock.
+// Measured, one CTA per 128-row tile -> pairs: 8192^3 748 -> 712 us; 8192 x 24576 x 4096 with SwiGLU 1130 -> 1072;
+// 4096 x 151936 x 2048 1762 -> 1594; 24576 x 4096 x 8192 (both operands across rows) 1097 -> 1036; 4096 x 5120 x 2048 68 -> 64.
+// Where the line lies:
+//  * a tile of 256 rows can waste half of itself at M's end: the waves decide, one of pairs costing at most 0.95 of a single one
+//    (300 x 32000 x 512, four waves of pairs against three: 21 -> 27 us);
+//  * short runs do not make up for the handshakes between the two at the first loads and the last stores: 32 k-blocks per CTA
+//    (2048^3) 21 -> 23 us, 47 (3456 x 1152 x 3000) the same, 68 (3000 x 1152 x 4304) 39 -> 35;
+//  * grouped weight gradients have few k-blocks per tile (four at 256 rows per expert), so a tile is mostly its epilogue, and the
+//    epilogue of one half waits for the other's: 128 x 2048 x 1536 and 128 x 768 x 2048 of 256 rows 287 -> 350 and 150 -> 186.
+static bool pays_in_pairs(const GemmArgs& a) {
+  if (a.tile_group || a.ep || a.groups_k > 0 || a.M <= BM || a.num_sms < 2) return false;
+  const long long nt = a.epi == EPI_SWIGLU ? (a.N + 127) / 128 : (a.N + 255) / 256;
+  const int splits = a.split_ws && a.k_splits > 1 ? a.k_splits : 1, pairs = a.num_sms / 2;
+  const long long one = ((a.M + BM - 1) / BM * nt * splits + a.num_sms - 1) / a.num_sms;                // waves
+  const long long two = ((a.M + 2 * BM - 1) / (2 * BM) * nt * splits + pairs - 1) / pairs;
+  const long long kb = (static_cast<long long>(a.K) + BK - 1) / BK / splits;
+  return 19 * two <= 20 * one && one * kb >= 48;
 }
 
 }  // namespace ttb
@@ -966,10 +1059,12 @@ TTB_EXPORT int ttb_gemm_bf16(const ttb::GemmArgs* args, void* stream_ptr) {
       return 908;
   }
   const bool wide = (a.epi == EPI_SWIGLU) ? true : (a.N > 128);
-#define TTB_DISPATCH(AMN, BMN)                                                             \
-  if (a.epi == EPI_SWIGLU) return launch<256, AMN, BMN, EPI_SWIGLU>(a, stream);            \
-  if (wide) return launch<256, AMN, BMN, EPI_STORE>(a, stream);                            \
-  return launch<128, AMN, BMN, EPI_STORE>(a, stream);
+  const bool pair = wide && pays_in_pairs(a);
+#define TTB_DISPATCH(AMN, BMN)                                                                                            \
+  if (a.epi == EPI_SWIGLU)                                                                                                \
+    return pair ? launch<256, AMN, BMN, EPI_SWIGLU, true>(a, stream) : launch<256, AMN, BMN, EPI_SWIGLU, false>(a, stream); \
+  if (wide) return pair ? launch<256, AMN, BMN, EPI_STORE, true>(a, stream) : launch<256, AMN, BMN, EPI_STORE, false>(a, stream); \
+  return launch<128, AMN, BMN, EPI_STORE, false>(a, stream);
   if (!a.a_mn && !a.b_mn) { TTB_DISPATCH(false, false) }
   if (!a.a_mn && a.b_mn) { TTB_DISPATCH(false, true) }
   if (a.a_mn && a.b_mn) { TTB_DISPATCH(true, true) }
