@@ -130,7 +130,7 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
 // ------------------------------------------------------------------------------------------------
 struct DoSmem {
   static constexpr int Q = 0, S = Q + DC_C * DC_QS * 2, X = S + DC_D * DO_LD * 4, A = X + DC_C * DO_LD * 4;
-  static constexpr int ROWS = A + DC_C * DP_LT * 4;
+  static constexpr int ROWS = A + 3 * DC_C * DP_LT * 2;             // A in planes: all eight warps read all of it
   static constexpr int TOTAL = ROWS + 2 * DC_C * 4;
 };
 
@@ -141,7 +141,7 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sm + DoSmem::Q);
   float* sS = reinterpret_cast<float*>(sm + DoSmem::S);
   float* sX = reinterpret_cast<float*>(sm + DoSmem::X);
-  float* sA = reinterpret_cast<float*>(sm + DoSmem::A);
+  __nv_bfloat16* sA = reinterpret_cast<__nv_bfloat16*>(sm + DoSmem::A);
   float* sG = reinterpret_cast<float*>(sm + DoSmem::ROWS);
   float* sRq = sG + DC_C;
   const int c = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * 64, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -150,8 +150,17 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
   dc_load_rows<256>(sQ, p.q + row0 * p.q_t + h * p.q_h, p.q_t, n);
   dc_load_f32<256, DC_D, 64>(sS, DO_LD, St + ((static_cast<long long>(h) * (p.NC + nseq) + slot) * DC_D) * DC_D + v0, DC_D);
   dc_load_f32<256, DC_C, 64>(sX, DO_LD, X + hc * DC_C * DC_D + v0, DC_D);
-  dc_load_f32<256, DC_C, 64>(sA, DP_LT, Ag + hc * DC_C * DC_C, DC_C);
   if (threadIdx.x < DC_C) sG[threadIdx.x] = threadIdx.x < n ? __ldg(p.g + static_cast<long long>(row0 + threadIdx.x) * p.H + h) : 0.f;
+  {
+    float4 va[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) va[e] = __ldg(reinterpret_cast<const float4*>(Ag + hc * DC_C * DC_C) + threadIdx.x + e * 256);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int f = threadIdx.x + e * 256;
+      dc_put(sA + (f >> 4) * DP_LT + (f & 15) * 4, DC_C * DP_LT, va[e]);
+    }
+  }
   dc_wait();
   __syncthreads();
   dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
@@ -187,7 +196,7 @@ delta_out_kernel(const DeltaChunkIn p, const float* __restrict__ Ag, const float
 #pragma unroll
     for (int mi = kk; mi < 4; ++mi) {
       uint32_t a[3][4];
-      dc_af<3>(a, sA, DP_LT, mi * 16, kk * 16, lane);
+      dc_pa<DP_LT>(a, sA, DC_C * DP_LT, mi * 16, kk * 16, lane);
       dc_mma33(acc[mi], a, b);
     }
   }
@@ -303,20 +312,20 @@ delta_bwd_pre_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO,
 // ------------------------------------------------------------------------------------------------
 // bwd_post: dq, dk, dv, dg, dbeta of one chunk and head
 // ------------------------------------------------------------------------------------------------
-constexpr int DQ_LD = 136;   // row stride of fp32 tiles read in pairs along a row
-constexpr int DQ_DX = 132;   // row stride of dx, read down its columns
-constexpr int DQ_P = 68;     // row stride of T / P and R
+constexpr int DQ_T = 72;                 // row stride of 64-column planes: rows of ldmatrix fall on distinct banks
+constexpr int DQ_PT = DC_C * DQ_T;       // elements of one
+constexpr int DQ_PL = DC_C * DC_QS;      // elements of a 128-column plane
 struct DqSmem {
-  static constexpr int Q = 0, K = Q + DC_C * DC_QS * 2, DO = K + DC_C * DC_QS * 2;
-  static constexpr int S = DO + DC_C * DC_QS * 2;                    // dx, then S, then dS
-  static constexpr int X = S + DC_D * DQ_LD * 4, DB = X + DC_C * DQ_LD * 4;
-  static constexpr int P = DB + DC_C * DQ_LD * 4, R = P + DC_C * DQ_P * 4;
-  static constexpr int ROWS = R + DC_C * DQ_P * 4;                   // G, beta, 1/|k|, scale/|q|, e^G, e^(Gl-G), beta/|k|
-  static constexpr int PART = P;                                     // [6][4][64] row sums per column quarter (after P, R)
-  static constexpr int RED = ROWS + 7 * DC_C * 4;
+  static constexpr int Q = 0, K = Q + DQ_PL * 2, DO = K + DQ_PL * 2;
+  static constexpr int X = DO + DQ_PL * 2;               // planes of x
+  static constexpr int W = X + 3 * DQ_PL * 2;            // planes of dx, then of S and of dS, 64 of the 128 rows at a time
+  static constexpr int DB = W + 3 * DQ_PL * 2;           // planes of T, then of db, then of R and P
+  static constexpr int ROWS = DB + 6 * DQ_PT * 2;        // G, beta, 1/|k|, scale/|q|, e^G, e^(Gl-G), beta/|k|
+  static constexpr int PART = ROWS + 7 * DC_C * 4;       // [6][4][64] row sums per column quarter, [2][64]
+  static constexpr int RED = PART + 26 * DC_C * 4;
   static constexpr int TOTAL = RED + 32 * 4;
 };
-static_assert(DqSmem::TOTAL <= 232448, "one CTA per SM");
+static_assert(2 * DQ_PT >= DQ_PL && DqSmem::TOTAL <= 232448, "one CTA per SM");
 
 __global__ void __launch_bounds__(512, 1)
 delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO, const float* __restrict__ Tg,
@@ -328,11 +337,10 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::Q);
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::K);
   __nv_bfloat16* sDO = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::DO);
-  float* sS = reinterpret_cast<float*>(sm + DqSmem::S);
-  float* sX = reinterpret_cast<float*>(sm + DqSmem::X);
-  float* sDB = reinterpret_cast<float*>(sm + DqSmem::DB);
-  float* sP = reinterpret_cast<float*>(sm + DqSmem::P);
-  float* sR = reinterpret_cast<float*>(sm + DqSmem::R);
+  __nv_bfloat16* sX = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::X);
+  __nv_bfloat16* sW = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::W);
+  __nv_bfloat16* sDB = reinterpret_cast<__nv_bfloat16*>(sm + DqSmem::DB);
+  __nv_bfloat16 *sR = sDB, *sP = sDB + 3 * DQ_PT;
   float* sPart = reinterpret_cast<float*>(sm + DqSmem::PART);
   float* sG = reinterpret_cast<float*>(sm + DqSmem::ROWS);
   float *sB = sG + DC_C, *sRk = sB + DC_C, *sRq = sRk + DC_C, *sE = sRq + DC_C, *sL = sE + DC_C, *sBk = sL + DC_C;
@@ -341,14 +349,39 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   const int row0 = p.chunk_rows[3 * c], n = p.chunk_rows[3 * c + 1], slot = c + p.chunk_rows[3 * c + 2];
   const long long hc = static_cast<long long>(h) * p.NC + c;
   const long long st_at = ((static_cast<long long>(h) * (p.NC + nseq) + slot) * DC_D) * DC_D;
+  // 64 rows of 128 columns, four vectors a thread: to registers, and from there to planes
+  auto fetch = [&](float4 (&v)[4], const float* src) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = __ldg(reinterpret_cast<const float4*>(src) + tid + e * NT);
+  };
+  auto store = [&](__nv_bfloat16* dst, const float4 (&v)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int f = tid + e * NT;
+      dc_put(dst + (f >> 5) * DC_QS + (f & 31) * 4, DQ_PL, v[e]);
+    }
+  };
 
-  dc_load_f32<NT, DC_C, DC_D>(sS, DQ_DX, dX + hc * DC_C * DC_D, DC_D);
-  dc_load_f32<NT, DC_C, 64>(sP, DQ_P, Tg + hc * DC_C * DC_C, DC_C);
   dc_load_rows<NT>(sQ, p.q + row0 * p.q_t + h * p.q_h, p.q_t, n);
   dc_load_rows<NT>(sK, p.k + row0 * p.k_t + h * p.k_h, p.k_t, n);
   dc_load_rows<NT>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
-  dc_load_f32<NT, DC_C, DC_D>(sX, DQ_LD, X + hc * DC_C * DC_D, DC_D);
   dc_load_gates(p, row0, n, h, sG, sB);
+  float4 va[4], vb[4];
+  {
+    float4 vt[2];
+    fetch(va, dX + hc * DC_C * DC_D);
+    fetch(vb, X + hc * DC_C * DC_D);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) vt[e] = __ldg(reinterpret_cast<const float4*>(Tg + hc * DC_C * DC_C) + tid + e * NT);
+    store(sW, va);
+    store(sX, vb);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int f = tid + e * NT;
+      dc_put(sDB + (f >> 4) * DQ_T + (f & 15) * 4, DQ_PT, vt[e]);
+    }
+  }
+  fetch(va, St + st_at);                         // the first half of S is on its way while db is formed
   dc_wait();
   __syncthreads();
   dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
@@ -360,9 +393,10 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     sL[tid] = expf(sG[DC_C - 1] - sG[tid]);
     sBk[tid] = sB[tid] * sRk[tid];
   }
-  // warp tile: 16 rows x 32 columns
-  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
+  // warp tile: 16 rows x 32 columns, 16 of each half of the 128
+  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 16, g = lane >> 2, t2 = (lane & 3) * 2;
   const int i0 = m0 + g, i1 = i0 + 8;
+  auto col_of = [&](int nt) { return (nt >> 1) * 64 + n0 + (nt & 1) * 8 + t2; };
   // sums over a row's 128 channels: four lanes, then four warps (added in a fixed order at the end)
   float part[6][2];
 #pragma unroll
@@ -372,23 +406,27 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     float acc[4][4] = {};
     for (int kk = mi; kk < 4; ++kk) {
       uint32_t a[3][4];
-      dc_af_t<3>(a, sP, DQ_P, m0, kk * 16, lane);
+      dc_pa_t<DQ_T>(a, sDB, DQ_PT, m0, kk * 16, lane);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        uint32_t b[3][2];
-        dc_bf_t<3>(b, sS, DQ_DX, n0 + nt * 8, kk * 16, lane);
-        dc_mma33(acc[nt], a, b);
+      for (int np = 0; np < 2; ++np) {
+        uint32_t b[3][4];
+        dc_pb_t<DC_QS>(b, sW, DQ_PL, np * 64 + n0, kk * 16, lane);
+        dc_mma33(acc[2 * np], a, b, 0);
+        dc_mma33(acc[2 * np + 1], a, b, 2);
       }
     }
+    __syncthreads();                             // dx and T are no longer read: S and db take their places
+    store(sW, va);
+    fetch(va, St + st_at + 64 * DC_D);
     const float be0 = sB[i0], be1 = sB[i1];
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      const int col = n0 + nt * 8 + t2;
+      const int col = col_of(nt);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int i = rr ? i1 : i0;
         const float x = acc[nt][2 * rr], y = acc[nt][2 * rr + 1], be = rr ? be1 : be0;
-        *reinterpret_cast<float2*>(sDB + i * DQ_LD + col) = make_float2(x, y);
+        dc_put(sDB + i * DC_QS + col, DQ_PL, x, y);
         if (i < n) {
           const float2 v = unpack_bf16(__ldg(reinterpret_cast<const uint32_t*>(p.v + (row0 + i) * p.v_t + h * p.v_h + col)));
           part[0][rr] += x * v.x + y * v.y;
@@ -397,68 +435,71 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
       }
     }
   }
-  __syncthreads();                               // db is complete, dx and T are no longer read
-  dc_load_f32<NT, DC_D, DC_D>(sS, DQ_LD, St + st_at, DC_D);
-  // ---- P = dL . D with dL = -strict_lower(db x^T), R = dA . D with dA = lower(do x^T); 16 x 16 per warp
-  {
-    float accP[2][4] = {}, accR[2][4] = {};
-    if (cq <= mi) {
+  __syncthreads();
+  // ---- P = dL . D with dL = -strict_lower(db x^T), R = dA . D with dA = lower(do x^T); 16 x 16 per warp, kept in registers
+  // until db has made room for their planes
+  float accP[2][4] = {}, accR[2][4] = {};
+  if (cq <= mi) {
+#pragma unroll 2
+    for (int kk = 0; kk < 8; ++kk) {
+      uint32_t ad[4], ab[3][4], b[3][4];
+      dc_a(ad, sDO, m0, kk * 16, lane);
+      dc_pa<DC_QS>(ab, sDB, DQ_PL, m0, kk * 16, lane);
+      dc_pb<DC_QS>(b, sX, DQ_PL, n0, kk * 16, lane);
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
-        uint32_t ad[4], ab[3][4];
-        dc_a(ad, sDO, m0, kk * 16, lane);
-        dc_af<3>(ab, sDB, DQ_LD, m0, kk * 16, lane);
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          uint32_t b[3][2];
-          dc_bf<3>(b, sX, DQ_LD, cq * 16 + nt * 8, kk * 16, lane);
-          dc_mma13(accR[nt], ad, b);
-          dc_mma33(accP[nt], ab, b);
-        }
+      for (int nt = 0; nt < 2; ++nt) {
+        dc_mma13(accR[nt], ad, b, 2 * nt);
+        dc_mma33(accP[nt], ab, b, 2 * nt);
       }
     }
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
-      for (int rr = 0; rr < 2; ++rr) {
-        const int i = rr ? i1 : i0, j = cq * 16 + nt * 8 + t2;
-        float2 pv = make_float2(0.f, 0.f), rv = make_float2(0.f, 0.f);
-        if (j <= i) {
-          const float d = expf(sG[i] - sG[j]);
-          rv.x = accR[nt][2 * rr] * d;
-          if (j < i) pv.x = -accP[nt][2 * rr] * d;
-        }
-        if (j + 1 <= i) {
-          const float d = expf(sG[i] - sG[j + 1]);
-          rv.y = accR[nt][2 * rr + 1] * d;
-          if (j + 1 < i) pv.y = -accP[nt][2 * rr + 1] * d;
-        }
-        *reinterpret_cast<float2*>(sP + i * DQ_P + j) = pv;
-        *reinterpret_cast<float2*>(sR + i * DQ_P + j) = rv;
+      for (int x = 0; x < 4; ++x) {
+        const int i = x < 2 ? i0 : i1, j = n0 + nt * 8 + t2 + (x & 1);
+        const float d = j <= i ? expf(sG[i] - sG[j]) : 0.f;
+        accR[nt][x] = j <= i ? accR[nt][x] * d : 0.f;
+        accP[nt][x] = j < i ? -accP[nt][x] * d : 0.f;
       }
     }
   }
-  dc_wait();
-  __syncthreads();                               // S, P and R are complete
+  // R and P with column (row) factors, as planes: those of the blocks on and below the diagonal, nothing reads the others
+  auto put_scores = [&](bool rows) {
+    if (cq > mi) return;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int i = rr ? i1 : i0, j = n0 + nt * 8 + t2;
+        const float r0 = rows ? sRq[i] : sRk[j], r1 = rows ? sRq[i] : sRk[j + 1];
+        const float p0 = rows ? sBk[i] : sRk[j], p1 = rows ? sBk[i] : sRk[j + 1];
+        dc_put(sR + i * DQ_T + j, DQ_PT, accR[nt][2 * rr] * r0, accR[nt][2 * rr + 1] * r1);
+        dc_put(sP + i * DQ_T + j, DQ_PT, accP[nt][2 * rr] * p0, accP[nt][2 * rr + 1] * p1);
+      }
+    }
+  };
   // ---- d(q^ e^G) = do S^T, d(beta k^ e^G) = -db S^T, then the score terms R k^, P k^ on the same accumulators
   float dq[4][4] = {}, dk[4][4] = {};
-#pragma unroll 2
-  for (int kk = 0; kk < 8; ++kk) {
-    uint32_t ad[4], ab[3][4];
-    dc_a(ad, sDO, m0, kk * 16, lane);
-    dc_af<3>(ab, sDB, DQ_LD, m0, kk * 16, lane);
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      uint32_t b[3][2];
-      dc_bf<3>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
-      dc_mma13(dq[nt], ad, b);
-      dc_mma33(dk[nt], ab, b);
+  for (int half = 0; half < 2; ++half) {
+    if (half == 1) {
+      __syncthreads();
+      store(sW, va);
+      __syncthreads();
+    }
+#pragma unroll 2
+    for (int kk = 0; kk < 8; ++kk) {
+      uint32_t ad[4], ab[3][4], b[3][4];
+      dc_a(ad, sDO, m0, kk * 16, lane);
+      dc_pa<DC_QS>(ab, sDB, DQ_PL, m0, kk * 16, lane);
+      dc_pb<DC_QS>(b, sW, DQ_PL, n0, kk * 16, lane);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        dc_mma13(dq[2 * half + nt], ad, b, 2 * nt);
+        dc_mma33(dk[2 * half + nt], ab, b, 2 * nt);
+      }
     }
   }
-  // the gradient of the chunk's end state is fetched while the score terms run
-  float4 ds[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) ds[e] = __ldg(reinterpret_cast<const float4*>(dSt + st_at + DC_D * DC_D) + tid + e * NT);
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
@@ -468,26 +509,34 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
       dk[nt][x] *= -e;
     }
   }
+  __syncthreads();                               // db and S are no longer read
+  put_scores(false);
+  // the gradient of the chunk's end state, and S once more for <dS, S>, are fetched while the score terms run
+  fetch(va, dSt + st_at + DC_D * DC_D);
+  fetch(vb, St + st_at);
+  __syncthreads();
   for (int kk = 0; kk <= mi; ++kk) {
     uint32_t ar[3][4], ap[3][4];
-    dc_af<3>(ar, sR, DQ_P, m0, kk * 16, lane, sRk);
-    dc_af<3>(ap, sP, DQ_P, m0, kk * 16, lane, sRk);
+    dc_pa<DQ_T>(ar, sR, DQ_PT, m0, kk * 16, lane);
+    dc_pa<DQ_T>(ap, sP, DQ_PT, m0, kk * 16, lane);
 #pragma unroll
     for (int np = 0; np < 2; ++np) {
       uint32_t b[4];
-      dc_b_t(b, sK, n0 + np * 16, kk * 16, lane);
+      dc_b_t(b, sK, np * 64 + n0, kk * 16, lane);
       dc_mma31(dq[2 * np], ar, b[0], b[1]);
       dc_mma31(dq[2 * np + 1], ar, b[2], b[3]);
       dc_mma31(dk[2 * np], ap, b[0], b[1]);
       dc_mma31(dk[2 * np + 1], ap, b[2], b[3]);
     }
   }
+  __syncthreads();
+  put_scores(true);
   uint32_t kv[4][2];                             // this thread's k values (bf16 pairs)
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
-      const int at = (rr ? i1 : i0) * DC_QS + n0 + nt * 8 + t2;
+      const int at = (rr ? i1 : i0) * DC_QS + col_of(nt);
       kv[nt][rr] = *reinterpret_cast<const uint32_t*>(sK + at);
       const float2 kf = unpack_bf16(kv[nt][rr]), qf = unpack_bf16(*reinterpret_cast<const uint32_t*>(sQ + at));
       part[1][rr] += qf.x * dq[nt][2 * rr] + qf.y * dq[nt][2 * rr + 1];
@@ -497,18 +546,26 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
       dk[nt][2 * rr + 1] *= be;
     }
   }
+  float dot = 0.f;
+  auto take_ds = [&]() {                         // <dS, S> on the way in
+    store(sW, va);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dot += vb[e].x * va[e].x + vb[e].y * va[e].y + vb[e].z * va[e].z + vb[e].w * va[e].w;
+  };
+  take_ds();
+  __syncthreads();
   // ---- k in the role of the earlier row: P^T (beta k^) + R^T q^
   {
     float acc[4][4] = {};
     for (int kk = mi; kk < 4; ++kk) {
       uint32_t ar[3][4], ap[3][4];
-      dc_af_t<3>(ar, sR, DQ_P, m0, kk * 16, lane, sRq);
-      dc_af_t<3>(ap, sP, DQ_P, m0, kk * 16, lane, sBk);
+      dc_pa_t<DQ_T>(ar, sR, DQ_PT, m0, kk * 16, lane);
+      dc_pa_t<DQ_T>(ap, sP, DQ_PT, m0, kk * 16, lane);
 #pragma unroll
       for (int np = 0; np < 2; ++np) {
         uint32_t bk[4], bq[4];
-        dc_b_t(bk, sK, n0 + np * 16, kk * 16, lane);
-        dc_b_t(bq, sQ, n0 + np * 16, kk * 16, lane);
+        dc_b_t(bk, sK, np * 64 + n0, kk * 16, lane);
+        dc_b_t(bq, sQ, np * 64 + n0, kk * 16, lane);
         dc_mma31(acc[2 * np], ap, bk[0], bk[1]);
         dc_mma31(acc[2 * np + 1], ap, bk[2], bk[3]);
         dc_mma31(acc[2 * np], ar, bq[0], bq[1]);
@@ -525,31 +582,26 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
         dk[nt][2 * rr + 1] += acc[nt][2 * rr + 1];
       }
   }
-  __syncthreads();                               // S is no longer read
-  float dot = 0.f;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {                  // <dS, S> on the way in
-    const int f = tid + e * NT, r = f >> 5, col = (f & 31) * 4;
-    float4* at = reinterpret_cast<float4*>(sS + r * DQ_LD + col);
-    const float4 s = *at;
-    dot += s.x * ds[e].x + s.y * ds[e].y + s.z * ds[e].z + s.w * ds[e].w;
-    *at = ds[e];
-  }
-  dot = warp_sum(dot);
-  if (lane == 0) sRed[warp] = dot;
-  __syncthreads();
   // ---- d(k_out) = x dS^T
   {
     float acc[4][4] = {};
-#pragma unroll 2
-    for (int kk = 0; kk < 8; ++kk) {
-      uint32_t a[3][4];
-      dc_af<3>(a, sX, DQ_LD, m0, kk * 16, lane);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        uint32_t b[3][2];
-        dc_bf<3>(b, sS, DQ_LD, n0 + nt * 8, kk * 16, lane);
-        dc_mma33(acc[nt], a, b);
+    for (int half = 0; half < 2; ++half) {
+      if (half == 0) {
+        fetch(va, dSt + st_at + DC_D * DC_D + 64 * DC_D);
+        fetch(vb, St + st_at + 64 * DC_D);
+      } else {
+        __syncthreads();
+        take_ds();
+        __syncthreads();
+      }
+#pragma unroll 2
+      for (int kk = 0; kk < 8; ++kk) {
+        uint32_t a[3][4], b[3][4];
+        dc_pa<DC_QS>(a, sX, DQ_PL, m0, kk * 16, lane);
+        dc_pb<DC_QS>(b, sW, DQ_PL, n0, kk * 16, lane);
+        dc_mma33(acc[2 * half], a, b, 0);
+        dc_mma33(acc[2 * half + 1], a, b, 2);
       }
     }
 #pragma unroll
@@ -564,7 +616,8 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
         part[5][rr] += kf.x * dk[nt][2 * rr] + kf.y * dk[nt][2 * rr + 1];
       }
   }
-  // (P and R were last read before the two barriers above: their space takes the row sums)
+  dot = warp_sum(dot);
+  if (lane == 0) sRed[warp] = dot;
 #pragma unroll
   for (int x = 0; x < 6; ++x)
 #pragma unroll
@@ -587,7 +640,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     const float tq = p.l2 ? r0 * r0 * row_sum(1, i) : 0.f, tk = p.l2 ? rk * rk * row_sum(5, i) : 0.f;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      const int col = n0 + nt * 8 + t2;
+      const int col = col_of(nt);
       const long long at = (static_cast<long long>(row0 + i) * p.H + h) * DC_D + col;
       const float2 kf = unpack_bf16(kv[nt][rr]), qf = unpack_bf16(*reinterpret_cast<const uint32_t*>(sQ + i * DC_QS + col));
       *reinterpret_cast<uint32_t*>(dQ + at) = pack_bf16(rq * (dq[nt][2 * rr] - qf.x * tq), rq * (dq[nt][2 * rr + 1] - qf.y * tq));

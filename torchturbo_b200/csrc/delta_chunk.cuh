@@ -12,23 +12,23 @@
 //             and d(beta k^ e^G) = -db S^T.)
 //
 // Arithmetic.  q, k, v and do are bf16 in memory, so they enter the tensor cores exactly; every fp32 operand (T, A,
-// S, x and the gradients) is split on the fly into three bf16 terms (24 mantissa bits), with three products against an exact
-// operand and six where both sides are fp32.  Norms, decays and masks are applied to fp32 accumulators or fp32 operands,
+// S, x and the gradients) is split into three bf16 terms (24 mantissa bits; bwd_post keeps them as planes in shared memory, the
+// others split as they load), with three products against an exact operand and six where both sides are fp32.  Norms, decays and masks are applied to fp32 accumulators or fp32 operands,
 // never to the bf16 inputs.  Two terms and three products on both-fp32 products left dg 4 to 14 and dbeta 13 to 16 times as
 // far from 64 bits as fp32 products; now dbeta, gx and gS are closer than those and dg within 1.5 times of them.
 //
-// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.15 ms, out 0.13, bwd_pre 0.09, bwd_post 0.60; with two-term
-// operands and sums kept in the tensor cores' accumulators 0.14, 0.11, 0.09 and 0.45.  A gated-delta-net layer forward + backward
-// takes 2.66 ms, against 10.4 when the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and
+// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.15 ms, out 0.13, bwd_pre 0.09, bwd_post 0.57 (0.60
+// when every warp split again the fp32 tiles that it shares with three others); with two-term operands and sums kept in the tensor
+// cores' accumulators 0.14, 0.11, 0.09 and 0.45.  A gated-delta-net layer forward + backward takes 2.5 ms, against 10.4 when the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and
 // gathers over materialised [chunk, 64, 64 .. 128] tensors.
 //
 // Why mma.sync and not tcgen05: the products are 64 x 64 x 128 at most, each feeds the next through registers and shared
 // memory, and their operands are built element by element (splits, decays).  What bounds them, from the counters of the same
-// case: bwd_post moves 0.69 GB (0.11 ms at the copy rate) and keeps the tensor pipe 33 % active with 12,000 mma.sync per chunk
-// and head; one CTA of 16 warps fills 43 % of the issue slots, and its warps wait for the tensor pipe, for results of their own
+// case: bwd_post moves 0.69 GB (0.11 ms at the copy rate) and kept the tensor pipe 33 % active with 12,000 mma.sync per chunk
+// and head before its planes; one CTA of 16 warps filled 43 % of the issue slots, and its warps waited for the tensor pipe, for results of their own
 // instructions, at barriers between the phases and for loads in similar shares.  out and prep: tensor pipe 30 and 14 %, issue
 // slots 49 and 44 %, traffic a third and a quarter of their time.  So neither memory nor the tensor pipe is full: it is the chain
-// of phases, in which every warp splits again the fp32 tiles that it shares with three others.
+// of phases on one CTA per SM.  That splitting once took only 4 % off bwd_post says the same.
 #pragma once
 #include "common.cuh"
 
@@ -89,14 +89,15 @@ __device__ __forceinline__ void dc_mma13(float (&c)[4], const uint32_t (&a)[4], 
 }
 // fp32 x fp32: the six products down to 2^-16 of the leading one; what is left out (mid lo, lo mid, lo lo) lies below the last
 // bit of an fp32 product
-__device__ __forceinline__ void dc_mma33(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+template <int W>
+__device__ __forceinline__ void dc_mma33(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][W], const int o = 0) {
   float d[4];
-  dc_mul(d, a[2], b[0][0], b[0][1]);
-  dc_mma(d, a[1], b[1][0], b[1][1]);
-  dc_mma(d, a[0], b[2][0], b[2][1]);
-  dc_mma(d, a[1], b[0][0], b[0][1]);
-  dc_mma(d, a[0], b[1][0], b[1][1]);
-  dc_mma(d, a[0], b[0][0], b[0][1]);
+  dc_mul(d, a[2], b[0][o], b[0][o + 1]);
+  dc_mma(d, a[1], b[1][o], b[1][o + 1]);
+  dc_mma(d, a[0], b[2][o], b[2][o + 1]);
+  dc_mma(d, a[1], b[0][o], b[0][o + 1]);
+  dc_mma(d, a[0], b[1][o], b[1][o + 1]);
+  dc_mma(d, a[0], b[0][o], b[0][o + 1]);
   dc_add(c, d);
 }
 __device__ __forceinline__ void dc_ldm(uint32_t (&r)[4], const __nv_bfloat16* p) {
@@ -187,6 +188,44 @@ __device__ __forceinline__ void dc_bf_t(uint32_t (&b)[N][2], const float* s, int
 #pragma unroll
     for (int i = 0; i < N; ++i) b[i][r] = w[i];
   }
+}
+// Planes: the three bf16 terms of an fp32 tile, each a bf16 tile of its own (`plane` elements apart, row stride LD), split once
+// where the tile is written.  Their fragments come by ldmatrix like those of exact tiles; a fragment of an fp32 tile costs its
+// warp about twelve instructions per register, and a tile's fragments are needed by four warps.
+__device__ __forceinline__ void dc_put(__nv_bfloat16* s, int plane, float x, float y) {
+  uint32_t w[3];
+  dc_split<3>(x, y, w);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(s + i * plane) = w[i];
+}
+__device__ __forceinline__ void dc_put(__nv_bfloat16* s, int plane, float4 v) {
+  uint32_t a[3], b[3];
+  dc_split<3>(v.x, v.y, a);
+  dc_split<3>(v.z, v.w, b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(s + i * plane) = make_uint2(a[i], b[i]);
+}
+// A fragment (16 rows x 16 k) of a tile stored [m][k] / of the transpose of one stored [k][m]
+template <int LD>
+__device__ __forceinline__ void dc_pa(uint32_t (&r)[3][4], const __nv_bfloat16* s, int plane, int m0, int k0, int lane) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) dc_ldm(r[i], s + i * plane + (m0 + (lane & 15)) * LD + k0 + (lane >> 4) * 8);
+}
+template <int LD>
+__device__ __forceinline__ void dc_pa_t(uint32_t (&r)[3][4], const __nv_bfloat16* s, int plane, int m0, int k0, int lane) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) dc_ldm_t(r[i], s + i * plane + (k0 + (lane & 7) + ((lane >> 4) << 3)) * LD + m0 + ((lane >> 3) & 1) * 8);
+}
+// B fragments of two n-tiles (columns 0-1 and 2-3 of r) of a tile stored [n][k] / stored [k][n]
+template <int LD>
+__device__ __forceinline__ void dc_pb(uint32_t (&r)[3][4], const __nv_bfloat16* s, int plane, int n0, int k0, int lane) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) dc_ldm(r[i], s + i * plane + (n0 + (lane & 7) + ((lane >> 4) << 3)) * LD + k0 + ((lane >> 3) & 1) * 8);
+}
+template <int LD>
+__device__ __forceinline__ void dc_pb_t(uint32_t (&r)[3][4], const __nv_bfloat16* s, int plane, int n0, int k0, int lane) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) dc_ldm_t(r[i], s + i * plane + (k0 + (lane & 15)) * LD + n0 + (lane >> 4) * 8);
 }
 // Tiles come in by asynchronous copies, so that all tiles of a kernel are on their way together; `dc_wait` before the barrier
 // that publishes them.  64 x 128 bf16 rows of one head -> shared tile; rows past `n` are zero (nothing is read for them).
