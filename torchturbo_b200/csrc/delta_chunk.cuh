@@ -45,6 +45,7 @@ struct DeltaChunkIn {
   const int* chunk_rows;                               // [NC, 3]: first row, rows (1 .. 64), sequence
   int H, NC, l2;
   float scale;
+  int rep;                                             // value heads per key head: head h reads q and k of head h / rep
 };
 
 __device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t b0, const uint32_t b1) {
@@ -356,7 +357,7 @@ inline int dc_launched() {
 }
 inline bool dc_bad(const DeltaChunkIn& a) {
   const uintptr_t p = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v);
-  return (p & 15) || ((a.q_t | a.q_h | a.k_t | a.k_h | a.v_t | a.v_h) & 7) || a.H <= 0 || a.H > 65535 || a.NC <= 0;
+  return (p & 15) || ((a.q_t | a.q_h | a.k_t | a.k_h | a.v_t | a.v_h) & 7) || a.H <= 0 || a.H > 65535 || a.NC <= 0 || a.rep <= 0 || a.H % a.rep;
 }
 
 }  // namespace ttb

@@ -741,7 +741,7 @@ using namespace ttb;
 
 // Arguments as in delta_chunk.cu with g fp32 [rows, H, 128] and decay fp32 [H, NC, 128]
 TTB_EXPORT int ttb_delta_vec_prep(const DeltaChunkIn* in, float* T, float* A, float* U, void* W, void* Ko, float* decay, void* stream) {
-  if (dc_bad(*in)) return 921;
+  if (in->rep != 1 || dc_bad(*in)) return 921;
   static bool done[16] = {};
   if (int e = dc_ready(delta_vec_prep_kernel, VpSmem::TOTAL, done)) return e;
   delta_vec_prep_kernel<<<dim3(in->NC, in->H), 256, VpSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
@@ -750,7 +750,7 @@ TTB_EXPORT int ttb_delta_vec_prep(const DeltaChunkIn* in, float* T, float* A, fl
 }
 
 TTB_EXPORT int ttb_delta_vec_out(const DeltaChunkIn* in, const float* A, const float* X, const float* states, int nseq, void* O, void* stream) {
-  if (dc_bad(*in)) return 921;
+  if (in->rep != 1 || dc_bad(*in)) return 921;
   static bool done[16] = {};
   if (int e = dc_ready(delta_vec_out_kernel, VoSmem::TOTAL, done)) return e;
   delta_vec_out_kernel<<<dim3(in->NC, in->H, 2), 256, VoSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
@@ -759,7 +759,7 @@ TTB_EXPORT int ttb_delta_vec_out(const DeltaChunkIn* in, const float* A, const f
 }
 
 TTB_EXPORT int ttb_delta_vec_bwd_pre(const DeltaChunkIn* in, const void* dO, const float* A, int nseq, float* GX, float* GS, void* stream) {
-  if (dc_bad(*in) || (reinterpret_cast<uintptr_t>(dO) & 15)) return 921;
+  if (in->rep != 1 || dc_bad(*in) || (reinterpret_cast<uintptr_t>(dO) & 15)) return 921;
   static bool done[16] = {};
   if (int e = dc_ready(delta_vec_bwd_pre_kernel, VbSmem::TOTAL, done)) return e;
   delta_vec_bwd_pre_kernel<<<dim3(in->NC, in->H), 256, VbSmem::TOTAL, reinterpret_cast<cudaStream_t>(stream)>>>(
@@ -771,7 +771,7 @@ TTB_EXPORT int ttb_delta_vec_bwd_pre(const DeltaChunkIn* in, const void* dO, con
 TTB_EXPORT int ttb_delta_vec_bwd_post(const DeltaChunkIn* in, const void* dO, const float* T, const float* X, const float* dX,
                                       const float* states, const float* dstates, int nseq, void* dQ, void* dK, void* dV, float* dG,
                                       float* dBeta, float* scratch, void* stream) {
-  if (dc_bad(*in) || (reinterpret_cast<uintptr_t>(dO) & 15)) return 921;
+  if (in->rep != 1 || dc_bad(*in) || (reinterpret_cast<uintptr_t>(dO) & 15)) return 921;
   static bool done_s[16] = {}, done_t[16] = {};
   if (int e = dc_ready(delta_vec_score_kernel, VsSmem::TOTAL, done_s)) return e;
   if (int e = dc_ready(delta_vec_state_kernel, VtSmem::TOTAL, done_t)) return e;

@@ -847,22 +847,25 @@ class _DeltaChunkIn(C.Structure):
                 ("q_t", C.c_longlong), ("q_h", C.c_longlong), ("k_t", C.c_longlong), ("k_h", C.c_longlong),
                 ("v_t", C.c_longlong), ("v_h", C.c_longlong),
                 ("g", C.c_void_p), ("beta", C.c_void_p), ("chunk_rows", C.c_void_p),
-                ("H", C.c_int), ("NC", C.c_int), ("l2", C.c_int), ("scale", C.c_float)]
+                ("H", C.c_int), ("NC", C.c_int), ("l2", C.c_int), ("scale", C.c_float), ("rep", C.c_int)]
 
 
 def _delta_in(q, k, v, g, beta, chunk_rows, l2: bool, scale: float) -> _DeltaChunkIn:
-    """q, k, v: bf16 [rows, H, 128] (any row / head stride that keeps 16-byte alignment); g: fp32 [rows, H]
+    """v: bf16 [rows, H, 128]; q, k: the same or, with one decay per head, of H / rep heads that serve rep value heads each (any
+    row / head stride that keeps 16-byte alignment); g: fp32 [rows, H]
     or [rows, H, 128] (one decay per head, or per head and channel); beta: fp32 [rows, H]; chunk_rows: int32 [NC, 3] on the device (first row, number of rows, sequence of every chunk)."""
-    R, H, D = q.shape
+    R, H, _ = v.shape
+    Hk = q.shape[1]
     check_device(q)
-    for t in (q, k, v):
-        assert t.dtype == torch.bfloat16 and t.shape == (R, H, 128) and t.stride(2) == 1
+    for t, heads in ((q, Hk), (k, Hk), (v, H)):
+        assert t.dtype == torch.bfloat16 and t.shape == (R, heads, 128) and t.stride(2) == 1
+    assert H % Hk == 0 and (Hk == H or g.dim() == 2)
     assert g.dtype == torch.float32 and g.shape in ((R, H), (R, H, 128)) and g.is_contiguous()
     assert beta.dtype == torch.float32 and beta.shape == (R, H) and beta.is_contiguous()
     assert chunk_rows.dtype == torch.int32 and chunk_rows.is_contiguous() and chunk_rows.shape[1] == 3
     return _DeltaChunkIn(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0), k.stride(1),
                          v.stride(0), v.stride(1), g.data_ptr(), beta.data_ptr(), chunk_rows.data_ptr(), H,
-                         chunk_rows.shape[0], int(l2), scale)
+                         chunk_rows.shape[0], int(l2), scale, H // Hk)
 
 
 def _delta_call(step: str, g, *args) -> None:
@@ -886,7 +889,7 @@ def delta_prep(q, k, v, g, beta, chunk_rows, *, l2: bool, scale: float):
 def delta_out(q, k, v, g, beta, chunk_rows, A, x, states, *, l2: bool, scale: float):
     """o bf16 [rows, H, 128] from the new values `x` and the chunk-start states of the recurrence."""
     a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    o = torch.empty(q.shape, dtype=torch.bfloat16, device=q.device)
+    o = torch.empty(v.shape, dtype=torch.bfloat16, device=q.device)
     _delta_call("out", g, C.byref(a), _p(A), _p(x), _p(states), C.c_int(states.shape[1] - a.NC), _p(o), _stream())
     return o
 
@@ -895,7 +898,7 @@ def delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq: int, *, l2: bool, s
     """Gradients that reach the recurrence directly: (gx like x, gS [H, NC + nseq, 128, 128]; the slots behind the last
     chunk of a sequence are left to the caller)."""
     a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    assert do.is_contiguous() and do.dtype == torch.bfloat16 and do.shape == q.shape
+    assert do.is_contiguous() and do.dtype == torch.bfloat16 and do.shape == v.shape
     gx = torch.empty(a.H, a.NC, 64, 128, dtype=torch.float32, device=q.device)
     gs = torch.empty(a.H, a.NC + nseq, 128, 128, dtype=torch.float32, device=q.device)
     _delta_call("bwd_pre", g, C.byref(a), _p(do), _p(A), C.c_int(nseq), _p(gx), _p(gs), _stream())
@@ -903,15 +906,19 @@ def delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq: int, *, l2: bool, s
 
 
 def delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, *, l2: bool, scale: float):
-    """(dq, dk, dv bf16 [rows, H, 128], dg like g, dbeta fp32 [rows, H])."""
+    """(dq, dk bf16 like q, dv bf16 [rows, H, 128], dg like g, dbeta fp32 [rows, H])."""
     a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    dq, dk, dv = (torch.empty(q.shape, dtype=torch.bfloat16, device=q.device) for _ in range(3))
+    dq, dk, dv = (torch.empty(v.shape, dtype=torch.bfloat16, device=q.device) for _ in range(3))   # of every value head
     dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
     # held until the launches are queued: a pointer alone would let another thread of this stream be given the block first
     scratch = torch.empty(4, *x.shape, dtype=torch.float32, device=q.device) if g.dim() == 3 else None
     _delta_call("bwd_post", g, C.byref(a), _p(do), _p(T), _p(x), _p(dx), _p(states), _p(dstates), C.c_int(states.shape[1] - a.NC),
                 _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta),
                 *([_p(scratch)] if scratch is not None else []), _stream())
+    if a.rep > 1:
+        per_head, (dq, dk) = (dq, dk), (torch.empty(q.shape, dtype=torch.bfloat16, device=q.device) for _ in range(2))
+        _check(lib().ttb_delta_head_sum(_p(per_head[0]), _p(per_head[1]), _p(dq), _p(dk), C.c_longlong(q.shape[0] * q.shape[1]),
+                                        C.c_int(a.rep), _stream()), "ttb_delta_head_sum")
     return dq, dk, dv, dg, dbeta
 
 

@@ -185,10 +185,8 @@ class GatedDeltaNet(nn.Module):
         q, k, v = q.reshape(1, Tg, hk, self.dk), k.reshape(1, Tg, hk, self.dk), v.reshape(1, Tg, hv, self.dv)
         beta = torch.sigmoid(b.float()).unsqueeze(0)
         g = (-A_log.float().exp() * F.softplus(a.float() + dt_bias.float())).unsqueeze(0)
-        if hv // hk > 1:
-            # every key head serves hv / hk value heads; as a broadcast its gradient is a plain sum over them
-            q, k = (t.unsqueeze(3).expand(1, Tg, hk, hv // hk, self.dk).reshape(1, Tg, hv, self.dk) for t in (q, k))
-        o, _ = ops.gated_delta_rule(q, k, v, g, beta, use_qk_l2norm_in_kernel=True, cu_seqlens=cu)
+        shared = dict(heads_per_key=hv // hk) if hv // hk > 1 else {}        # every key head serves hv / hk value heads
+        o, _ = ops.gated_delta_rule(q, k, v, g, beta, use_qk_l2norm_in_kernel=True, cu_seqlens=cu, **shared)
         o = o.squeeze(0)                                                    # [Tg, hv, dv]
         if sp > 1:
             o = gather_heads_scatter_seq(o.contiguous(), ctx.sp_group, sp)  # [T_local, n_v, dv]

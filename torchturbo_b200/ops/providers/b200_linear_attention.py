@@ -31,7 +31,7 @@ from ...runtime import TurboDevice
 from ..base import OpImpl, OpImplKind
 from ..registry import register_op
 from .b200 import _aligned
-from .native_linear_attention import _bounds, kda_gate, l2norm
+from .native_linear_attention import _bounds, kda_gate, l2norm, repeat_key_heads
 
 CHUNK = 64
 
@@ -108,7 +108,7 @@ class StateScan(torch.autograd.Function):
 
 class ChunkDelta(torch.autograd.Function):
     """(Gated) delta rule on bf16 rows: a few kernels around the recurrence instead of batched fp32
-    products over materialised chunk tensors.  q, k, v [rows, H, 128]; g fp32 [rows, H] or [rows, H, 128]; beta fp32 [rows, H]; init [H, nseq, 128, 128]
+    products over materialised chunk tensors.  v [rows, H, 128]; q, k the same or of H / rep heads; g fp32 [rows, H] or [rows, H, 128]; beta fp32 [rows, H]; init [H, nseq, 128, 128]
     or None; `tables` = (seq_chunks, chunk_rows, last slots, first slots) on the device."""
 
     @staticmethod
@@ -128,7 +128,7 @@ class ChunkDelta(torch.autograd.Function):
     def backward(ctx, do, dfinal):
         q, k, v, g, beta, T, A, w, k_out, decay, x, states, seq, chunk_rows, last, first = ctx.saved_tensors
         kw, has_init = ctx.meta
-        do = _aligned(do) if do is not None else torch.zeros(q.shape, dtype=q.dtype, device=q.device)
+        do = _aligned(do) if do is not None else torch.zeros(v.shape, dtype=v.dtype, device=v.device)
         gx, gs = K.delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, seq.shape[0], **kw)
         if dfinal is None:
             gs.index_fill_(1, last, 0.0)
@@ -167,14 +167,15 @@ def _chunk_tables(segs, C: int, device):
     return seq_d.view(nseq, 2), rows_d.view(c, 3), last_d, first_d
 
 
-def _fused_usable(q, k, v, g, beta, segs, scale) -> bool:
+def _fused_usable(q, k, v, g, beta, segs, scale, rep: int = 1) -> bool:
     """The fused kernels take bf16 q / k / v of 128-wide heads and sequences that cover every row (fp32 rows would lose
     mantissa bits as tensor-core operands; they keep the batched fp32 products)."""
     R = q.shape[0] * q.shape[1]
     return (_kernel_ok(q, q.shape[-1], v.shape[-1]) and all(t.dtype == torch.bfloat16 and t.is_cuda for t in (q, k, v))
-            and k.shape == q.shape and v.shape == q.shape and g.shape in (q.shape, q.shape[:3])
-            and beta.shape == q.shape[:3] and scale != 0
-            and 0 < q.shape[2] <= 65535 and R > 0 and sum(b - a for _, a, b in segs) == R
+            and k.shape == q.shape and v.shape == (*q.shape[:2], q.shape[2] * rep, q.shape[3])
+            and (g.shape == v.shape[:3] or (rep == 1 and g.shape == v.shape))
+            and beta.shape == v.shape[:3] and scale != 0
+            and 0 < v.shape[2] <= 65535 and R > 0 and sum(b - a for _, a, b in segs) == R
             and all(0 <= a <= b <= q.shape[1] for _, a, b in segs))
 
 
@@ -231,10 +232,11 @@ def _channel_decay_products(kb, qc, kc, G, head_slab: int = 8, sub: int = 16):
 
 
 def chunk_delta_rule_batched(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, cu_seqlens=None,
-                             use_qk_l2norm=False, head_slab: int = 8):
-    """q, k: [B, T, H, K]; v: [B, T, H, V]; g: [B, T, H] (scalar log decay) or [B, T, H, K]; beta: [B, T, H].
+                             use_qk_l2norm=False, head_slab: int = 8, heads_per_key: int = 1):
+    """q, k: [B, T, H / heads_per_key, K]; v: [B, T, H, V]; g: [B, T, H] (scalar log decay) or [B, T, H, K]; beta: [B, T, H].
     Returns (o [B, T, H, V] in v's dtype, final state [N, H, K, V] fp32 or None)."""
     B, T, H, Kd = q.shape
+    H *= heads_per_key
     V = v.shape[-1]
     dt = v.dtype
     dev = q.device
@@ -243,13 +245,14 @@ def chunk_delta_rule_batched(q, k, v, g, beta, scale=None, initial_state=None, o
     if cu_seqlens is not None and B != 1:
         raise ValueError("packed delta rule expects a single row")
     segs = [(0, a, b) for a, b in _bounds(cu_seqlens, T)] if cu_seqlens is not None else [(r * T, 0, T) for r in range(B)]
-    if _fused_usable(q, k, v, g, beta, segs, scale):
+    if _fused_usable(q, k, v, g, beta, segs, scale, heads_per_key):
         R = B * T
         tables = _chunk_tables(segs, C, dev)
         init = initial_state.float().transpose(0, 1).contiguous() if initial_state is not None else None
         o, final = ChunkDelta.apply(*(_rows_for_kernel(t, R) for t in (q, k, v)), g.float().reshape(R, *g.shape[2:]).contiguous(),
                                     beta.float().reshape(R, H).contiguous(), init, tables, float(scale), bool(use_qk_l2norm))
         return o.view(B, T, H, V), (final.transpose(0, 1).contiguous() if output_final_state else None)
+    q, k = (repeat_key_heads(t, heads_per_key) for t in (q, k))
     qf, kf, vf, gf, bf = (t.float() for t in (q, k, v, g, beta))
     if use_qk_l2norm:
         qf, kf = l2norm(qf), l2norm(kf)
@@ -359,13 +362,13 @@ class B200GatedDeltaRule(OpImpl):
         return K.available()
 
     def __call__(self, q, k, v, g, beta, *, scale=None, initial_state=None, output_final_state=False,
-                 use_qk_l2norm_in_kernel=False, cu_seqlens=None, packed_params=None, chunk_size=64, **_):
+                 use_qk_l2norm_in_kernel=False, cu_seqlens=None, packed_params=None, chunk_size=64, heads_per_key=1, **_):
         if packed_params is not None:
             if cu_seqlens is not None:
                 raise ValueError("pass either cu_seqlens or packed_params, not both")
             cu_seqlens = packed_params.cu_seqlens
         return chunk_delta_rule_batched(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens,
-                                        use_qk_l2norm_in_kernel)
+                                        use_qk_l2norm_in_kernel, heads_per_key=heads_per_key)
 
 
 @_register("kda", "b200_chunk_kda")

@@ -223,10 +223,21 @@ def chunk_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, output_fi
     return o, (torch.stack(finals, 0) if output_final_state else None)
 
 
+def repeat_key_heads(t, heads_per_key: int):
+    """[B, T, H, K] -> [B, T, H * heads_per_key, K], every head in a row; as a broadcast its gradient is a plain sum."""
+    if heads_per_key == 1:
+        return t
+    B, T, H, Kd = t.shape
+    return t.unsqueeze(3).expand(B, T, H, heads_per_key, Kd).reshape(B, T, H * heads_per_key, Kd)
+
+
 @_native("gated_delta_rule", "torch_chunk_gated_delta_rule")
 class TorchGatedDeltaRule(OpImpl):
+    """q, k: [B, T, H / heads_per_key, K], each head serving `heads_per_key` value heads in a row; v: [B, T, H, V]."""
+
     def __call__(self, q, k, v, g, beta, *, scale=None, initial_state=None, output_final_state=False,
-                 use_qk_l2norm_in_kernel=False, cu_seqlens=None, packed_params=None, chunk_size=64, **_):
+                 use_qk_l2norm_in_kernel=False, cu_seqlens=None, packed_params=None, chunk_size=64, heads_per_key=1, **_):
+        q, k = repeat_key_heads(q, heads_per_key), repeat_key_heads(k, heads_per_key)
         if packed_params is not None:
             if cu_seqlens is not None:
                 raise ValueError("pass either cu_seqlens or packed_params, not both")
