@@ -10,6 +10,7 @@
 //                                                                       models/modules/moe/experts.py:181-186)
 //   CE        : fp32, reduction=sum, ignore_index=-100                (ops/providers/native/cross_entropy_loss.py:17-33)
 //   AdamW     : torch fused AdamW math on fp32 shards                  (engine/backends/fsdp2/optimizers/adamw.py:226-251)
+#include <type_traits>
 #include "common.cuh"
 #include "rowops.cuh"
 
@@ -396,11 +397,13 @@ __global__ void bias_act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const 
 // ============================================================================
 constexpr int CONV_MAX_W = 8;   // widest supported filter
 
-// Filters of up to four taps (every linear-attention layer): a thread owns 4 channels (8 would spill the window), walks its rows four at a time with the
-// next four rows' loads already issued, and keeps the taps' window in registers, so that x (and dy) are read once.  One pass
-// each way: the backward adds every dpre row into the W rows of dx that it reaches while they are still in registers (the
-// W - 1 rows behind a block are recomputed by it), which saves writing and re-reading dpre.  4096 x 8192, W = 4: forward 59 -> 45 us,
-// backward 180 (two kernels) -> 136 us; what is left is arithmetic (two exponentials and 48 products per element pair).
+// Filters of up to four taps (every linear-attention layer): a thread owns 4 channels (8 would spill the window), walks its rows four
+// at a time with the next four rows' loads already issued, and keeps the taps' window in registers, so that x (and dy) are read
+// once.  One pass each way: the backward adds every dpre row into the W rows of dx that it reaches while they are still in registers
+// (the W - 1 rows behind a block are recomputed by it), which saves writing and re-reading dpre.  What bounds it is the issue of its
+// arithmetic (two exponentials and 48 products per element pair), so steps in which every tap of every row counts run without the
+// checks, and products go two channels at a time.  4096 x 8192, W = 4: forward 59 -> 45 -> 41 us, backward 180 (two kernels) -> 136
+// -> 102 us; 31 us of it would be memory.
 constexpr int CONV_ROWS = 4;    // rows per step
 
 __device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
@@ -409,6 +412,18 @@ __device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
 }
 __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&f)[4]) {
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+}
+
+// c += a * b for two neighbouring channels (one instruction; each half rounds as an fma of its own)
+__device__ __forceinline__ void fma2(float& c0, float& c1, float a0, float a1, float b0, float b1) {
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%0, %1};\n\t"
+      "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "+f"(c0), "+f"(c1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ void fma4(float (&c)[4], const float (&a)[4], const float (&b)[4]) {
+  fma2(c[0], c[1], a[0], a[1], b[0], b[1]);
+  fma2(c[2], c[3], a[2], a[3], b[2], b[3]);
 }
 
 template <bool BWD>
@@ -467,21 +482,22 @@ causal_conv1d_w4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
       cf[u] = nf[u];
     }
     if (t0 + CONV_ROWS < re) fetch(t0 + CONV_ROWS);
-#pragma unroll
-    for (int u = 0; u < CONV_ROWS; ++u) {
+    // INNER: all four taps of all four rows lie in their sequences, the rows are this block's and so are the rows they complete
+    auto row = [&](auto inner, int u) {
+      constexpr bool INNER = decltype(inner)::value;
       const long long t = t0 + u;
-      if (t >= re) break;
+      if (!INNER && t >= re) return;
       const int reach = static_cast<int>(t - cf[u] < WM ? t - cf[u] : WM);   // how far back the sequence goes, at most WM
       float xs[WM][4], pre[4];
       unpack4(cx[u], xs[0]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) pre[j] = bs[j] + wt[0][j] * xs[0][j];
+      for (int j = 0; j < 4; ++j) pre[j] = bs[j];
+      fma4(pre, wt[0], xs[0]);
 #pragma unroll
       for (int s = 1; s < WM; ++s) {
         unpack4(hist[s - 1], xs[s]);
-        if (s <= reach && s < W) {                 // (not a product with zero: rows and taps may be infinite)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) pre[j] += wt[s][j] * xs[s][j];
+        if (INNER || (s <= reach && s < W)) {      // (not a product with zero: rows and taps may be infinite)
+          fma4(pre, wt[s], xs[s]);
         } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j) xs[s][j] = 0.f;
@@ -493,28 +509,32 @@ causal_conv1d_w4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
         for (int j = 0; j < 4; ++j) o[j] = silu ? pre[j] / (1.f + __expf(-pre[j])) : pre[j];
         store4(out + t * D + c, o);
       } else {
-        float g[4];
-        unpack4(cg[u], g);
+        float d[4];
+        unpack4(cg[u], d);
+        if (silu) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float sg = 1.f / (1.f + __expf(-pre[j]));
+            d[j] *= sg * (1.f + pre[j] * (1.f - sg));
+          }
+        }
+        if (INNER || t < r1) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dbacc[j] += d[j];
+#pragma unroll
+          for (int s = 0; s < WM; ++s) fma4(dwacc[s], d, xs[s]);
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float d = g[j];
-          if (silu) {
-            const float sg = 1.f / (1.f + __expf(-pre[j]));
-            d *= sg * (1.f + pre[j] * (1.f - sg));
-          }
-          if (t < r1) {
-            dbacc[j] += d;
-#pragma unroll
-            for (int s = 0; s < WM; ++s) dwacc[s][j] += d * xs[s][j];
-          }
-          d = __bfloat162float(__float2bfloat16(d));
-          // this row reaches the dx of the rows up to W - 1 behind it in its sequence
-          acc[0][j] = wt[0][j] * d;
-#pragma unroll
-          for (int s = 1; s < WM; ++s) acc[s][j] += (s <= reach && s < W) ? wt[s][j] * d : 0.f;
+          d[j] = __bfloat162float(__float2bfloat16(d[j]));
+          acc[0][j] = wt[0][j] * d[j];
         }
+        // this row reaches the dx of the rows up to W - 1 behind it in its sequence
+#pragma unroll
+        for (int s = 1; s < WM; ++s)
+          if (INNER || (s <= reach && s < W)) fma4(acc[s], wt[s], d);
         const long long done = t - (WM - 1);        // no later row reaches it
-        if (done >= r0 && done < r1) store4(out + done * D + c, acc[WM - 1]);
+        if (INNER || (done >= r0 && done < r1)) store4(out + done * D + c, acc[WM - 1]);
 #pragma unroll
         for (int s = WM - 1; s > 0; --s)
 #pragma unroll
@@ -523,6 +543,16 @@ causal_conv1d_w4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 #pragma unroll
       for (int s = WM - 2; s > 0; --s) hist[s] = hist[s - 1];
       hist[0] = cx[u];
+    };
+    bool inner = W == WM && t0 + CONV_ROWS <= r1 && (!BWD || t0 >= r0 + WM - 1);
+#pragma unroll
+    for (int u = 0; u < CONV_ROWS; ++u) inner = inner && t0 + u - cf[u] >= WM - 1;
+    if (inner) {
+#pragma unroll
+      for (int u = 0; u < CONV_ROWS; ++u) row(std::true_type{}, u);
+    } else {
+#pragma unroll
+      for (int u = 0; u < CONV_ROWS; ++u) row(std::false_type{}, u);
     }
   }
   if (BWD) {
