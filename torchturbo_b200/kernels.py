@@ -448,17 +448,21 @@ def qknorm_rope_fwd(qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, eps, use_norm=Tr
     return q, k, rstd
 
 
-def qknorm_rope_bwd(dq, dk, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dqkv, use_norm=True):
-    """Writes the q and k column blocks of ``dqkv`` ([T, ld]) and returns (dwq, dwk) in fp32."""
+def qknorm_rope_bwd(dq, dk, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dqkv, use_norm=True, dv=None, dw_dtype=torch.float32):
+    """Writes the q and k column blocks of ``dqkv`` ([T, ld]), with ``dv`` ([T, n_kv, D]) the v block too, and returns (dwq, dwk)
+    in ``dw_dtype`` (fp32 or bf16)."""
     T = qkv.shape[0]
-    dwq = torch.zeros(head_dim, dtype=torch.float32, device=qkv.device)
-    dwk = torch.zeros(head_dim, dtype=torch.float32, device=qkv.device)
-    grid = max(1, min((T * (n_q + n_kv) + 7) // 8, 4 * num_sms(qkv.device.index)))
-    _check(lib().ttb_qknorm_rope_bwd(_p(dq), _p(dk), _p(qkv), C.c_longlong(qkv.stride(0)), C.c_int(n_q), C.c_int(n_kv),
+    groups = (n_q + n_kv * (1 if dv is None else 2) + 3) // 4          # a warp takes four heads of a token
+    grid = max(1, min((T * groups + 7) // 8, 4 * num_sms(qkv.device.index)))
+    dw = (torch.empty if use_norm and T else torch.zeros)(2, head_dim, dtype=dw_dtype, device=qkv.device)
+    part = torch.empty(grid, 2 * head_dim, dtype=torch.float32, device=qkv.device) if use_norm else None
+    _check(lib().ttb_qknorm_rope_bwd(_p(dq), _p(dk), _p(dv), _p(qkv), C.c_longlong(qkv.stride(0)), C.c_int(n_q), C.c_int(n_kv),
                                      C.c_int(head_dim), _p(wq), _p(wk), _p(cos), _p(sin), _p(rstd), _p(dqkv),
-                                     C.c_longlong(dqkv.stride(0)), _p(dwq), _p(dwk), C.c_longlong(T),
-                                     C.c_int(int(use_norm)), C.c_int(grid), _stream()), "ttb_qknorm_rope_bwd")
-    return dwq, dwk
+                                     C.c_longlong(dqkv.stride(0)), _p(part), _p(dw), C.c_int(int(dw_dtype == torch.bfloat16)),
+                                     C.c_longlong(T), C.c_int(int(use_norm)), C.c_int(grid), _stream()), "ttb_qknorm_rope_bwd")
+    global LAUNCH_COUNT
+    LAUNCH_COUNT += 1 if use_norm else 0
+    return dw[0], dw[1]
 
 
 def rope(x, cos, sin, sign: float = 1.0):

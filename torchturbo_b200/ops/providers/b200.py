@@ -372,11 +372,9 @@ class QKNormRopeFn(torch.autograd.Function):
         qkv, wq, wk, cos, sin, rstd = ctx.saved_tensors
         n_q, n_kv, D, use_norm = ctx.dims
         dqkv = torch.empty_like(qkv)
-        dqkv[:, (n_q + n_kv) * D:] = dv.reshape(qkv.shape[0], n_kv * D)
-        dwq, dwk = K.qknorm_rope_bwd(dq.contiguous(), dk.contiguous(), qkv, n_q, n_kv, D, wq, wk, cos, sin, rstd, dqkv,
-                                     use_norm)
-        return (dqkv, None, None, None, dwq.to(wq.dtype) if use_norm else None, dwk.to(wk.dtype) if use_norm else None,
-                None, None, None)
+        dwq, dwk = K.qknorm_rope_bwd(_aligned(dq), _aligned(dk), qkv, n_q, n_kv, D, wq, wk, cos, sin, rstd, dqkv, use_norm,
+                                     dv=_aligned(dv), dw_dtype=BF16)
+        return (dqkv, None, None, None, dwq if use_norm else None, dwk if use_norm else None, None, None, None)
 
 
 @_custom("qk_norm_rope", "b200_qk_norm_rope")
