@@ -1,5 +1,5 @@
-// Variable-length flash attention backward for sm_100a (GQA, causal or full; value heads 128 wide, query / key heads
-// 128 wide, or 192 for multi-head latent attention).  The kernel is built in two forms: with the dQ^T product and its
+// Variable-length flash attention backward for sm_100a (GQA, causal or full; heads up to 128 wide in multiples of 8, or value
+// heads 128 wide with query / key heads 192 for multi-head latent attention).  The kernel is built in two forms: with the dQ^T product and its
 // reduction (128-wide heads, the default), and without it, where dQ comes from the query-major pass in
 // attention_bwd_dq.cu (192-wide heads, whose accumulators do not fit tensor memory together, and the bit-reproducible
 // mode of 128-wide heads).
@@ -27,6 +27,7 @@
 // Replaces flash-attn 2's backward used through the reference attention interface
 // (models/modules/attention/interface.py:114-158).
 #include "common.cuh"
+#include <type_traits>
 
 namespace ttb {
 
@@ -45,6 +46,7 @@ struct AttnBwdParams {
   float* dk_acc;         // [T, Hk, D] fp32, zero-initialised (used when Hq > Hk)
   float* dv_acc;
   int Hq, Hk;
+  int D, Dv;             // width of query / key heads and of value heads
   long long T;
   float scale;
   int causal;
@@ -99,13 +101,20 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&out)[64]) {
   }
 }
 
-template <int DQK, bool WITH_DQ>
+// FULL: heads as wide as the tiles (widths known at compile time, two-dimensional maps).  With the widths as variables and
+// three-dimensional maps the 128-wide case (4096 tokens, 32 / 8 heads) took 269 us instead of 257.
+template <int DQK, bool WITH_DQ, bool FULL>
 __global__ void __launch_bounds__(448, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                 const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                 const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
   static_assert(DQK == 128 || !WITH_DQ, "the fused dQ path exists for 128-wide heads only");
   using BwdSmem = ttb::BwdSmem<DQK, WITH_DQ>;
+  const int D = FULL ? DQK : p.D, Dv = FULL ? BW_D : p.Dv;
+  auto load_head = [](void* dst, const CUtensorMap* map, uint64_t* bar, int col, int head, int width, int row) {
+    if (FULL) tma_load_2d(dst, map, bar, head * width + col, row);
+    else tma_load_3d(dst, map, bar, col, head, row);
+  };
   constexpr int NP = DQK / 64, Q_BYTES = BwdSmem::Q_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -182,9 +191,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmDO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
       mbar_expect_tx(kv_full, BwdSmem::K_BYTES + 32768);
 #pragma unroll
-      for (int pn = 0; pn < NP; ++pn) tma_load_2d(smem + BwdSmem::K + pn * 16384, &tmK, kv_full, hk * DQK + pn * 64, kv0);
-      tma_load_2d(smem + BwdSmem::V, &tmV, kv_full, hk * BW_D, kv0);
-      tma_load_2d(smem + BwdSmem::V + 16384, &tmV, kv_full, hk * BW_D + 64, kv0);
+      for (int pn = 0; pn < NP; ++pn) load_head(smem + BwdSmem::K + pn * 16384, &tmK, kv_full, pn * 64, hk, DQK, kv0);
+      load_head(smem + BwdSmem::V, &tmV, kv_full, 0, hk, 128, kv0);
+      load_head(smem + BwdSmem::V + 16384, &tmV, kv_full, 64, hk, 128, kv0);
       for (int it = 0; it < n_it; ++it) {
         const int st = it & 1;
         const uint32_t ph = (it >> 1) & 1;
@@ -194,9 +203,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         uint8_t* sq = smem + BwdSmem::Q0 + st * Q_BYTES;
         uint8_t* sd = smem + BwdSmem::DO0 + st * 16384;
 #pragma unroll
-        for (int pn = 0; pn < NP; ++pn) tma_load_2d(sq + pn * 8192, &tmQ, &qdo_full[st], h * DQK + pn * 64, q0);
-        tma_load_2d(sd, &tmDO, &qdo_full[st], h * BW_D, q0);
-        tma_load_2d(sd + 8192, &tmDO, &qdo_full[st], h * BW_D + 64, q0);
+        for (int pn = 0; pn < NP; ++pn) load_head(sq + pn * 8192, &tmQ, &qdo_full[st], pn * 64, h, DQK, q0);
+        load_head(sd, &tmDO, &qdo_full[st], 0, h, 128, q0);
+        load_head(sd + 8192, &tmDO, &qdo_full[st], 64, h, 128, q0);
       }
     }
   } else if (warp == 1) {
@@ -205,8 +214,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // documents 268 -> 260 us; 192-wide heads 207 -> 199; 8192 tokens, 32 heads 1772 -> 1700.
     {
       constexpr uint32_t id_s = make_idesc_bf16(128, 64, false, false);
-      constexpr uint32_t id_acc = make_idesc_bf16(128, 128, false, true);
-      constexpr uint32_t id_dk = make_idesc_bf16(128, DQK, false, true);
+      const uint32_t id_acc = make_idesc_bf16(128, (Dv + 15) / 16 * 16, false, true);
+      const uint32_t id_dk = make_idesc_bf16(128, (D + 15) / 16 * 16, false, true);
       constexpr uint32_t id_dq = make_idesc_bf16(128, 64, true, true);
       const uint32_t leader = elect_one() ? 1u : 0u;
       // operands read along their rows (K-major) and, where a product reduces over rows, across them (MN-major)
@@ -227,13 +236,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int kk = 0; kk < DQK / 16; ++kk) {  // reduction over the query / key head width
           const uint32_t offa = (kk >> 2) * 16384 + (kk & 3) * 32;   // K / V tiles: [128 rows][64 d] panels
           const uint32_t offb = (kk >> 2) * 8192 + (kk & 3) * 32;    // Q / dO tiles: [64 rows][64 d] panels
-          umma_ss_w(leader, tm_ST, desc_at(dK, offa), desc_at(q, offb), id_s, kk != 0);
+          umma_ss_w(kk * 16 < D ? leader : 0u, tm_ST, desc_at(dK, offa), desc_at(q, offb), id_s, kk != 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t offa = (kk >> 2) * 16384 + (kk & 3) * 32;
           const uint32_t offb = (kk >> 2) * 8192 + (kk & 3) * 32;
-          umma_ss_w(leader, tm_DPT, desc_at(dV, offa), desc_at(d_o, offb), id_s, kk != 0);
+          umma_ss_w(kk * 16 < Dv ? leader : 0u, tm_DPT, desc_at(dV, offa), desc_at(d_o, offb), id_s, kk != 0);
         }
         umma_commit_w(leader, st_full);
         return true;
@@ -371,13 +380,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t lane_off = static_cast<uint32_t>(lg * 32) << 16;
       {
         const int which = half;                  // columns 0-31 group: dV, the other group: dK
-        const int width = which == 0 ? BW_D : DQK;
+        const int width = which == 0 ? Dv : D;
         const long long off = (static_cast<long long>(kv) * p.Hk + hk) * width;
         __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + off;
         float* acc = (which == 0 ? p.dv_acc : p.dk_acc) + off;
         const uint32_t tm = (which == 0 ? tm_DV : tm_DK) + lane_off;
 #pragma unroll 1
-        for (int cb = 0; cb < width / 32; ++cb) {
+        for (int cb = 0; cb * 32 < width; ++cb) {
           uint32_t v[32];
           if (n_it > 0) {
             tmem_ld_32x32b_x32(tm + cb * 32, v);
@@ -390,6 +399,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (G == 1 || p.group_loop) {
 #pragma unroll
               for (int i = 0; i < 32; i += 8) {
+                if (cb * 32 + i >= width) continue;
                 uint4 w;
                 w.x = pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
                 w.y = pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
@@ -400,6 +410,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             } else {
 #pragma unroll
               for (int i = 0; i < 32; i += 4) {
+                if (cb * 32 + i >= width) continue;
                 atomicAdd(reinterpret_cast<float4*>(acc + cb * 32 + i),
                           make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
                                       __uint_as_float(v[i + 3])));
@@ -434,13 +445,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (*s_dead_dq) break;
       // transpose: this thread's d column of the [64 q][128 d] tile (a warp writes 128 contiguous bytes per row).
       // Query rows past the end of the document carry exact zeros (their P and dS were masked), so the full tile
-      // is added; rows past the end of the tensor are clipped by the copy engine.
+      // is added; rows past the end of the tensor and columns past the head are clipped by the copy engine.
 #pragma unroll
       for (int col = 0; col < BW_Q; ++col) sdq[col * BW_D + d] = v[col];
       fence_proxy_async_smem();
       asm volatile("bar.sync 2, 128;" ::: "memory");
       if (tid_dq == 0) {
-        tma_reduce_add_2d(&tmDQ, sdq, hq * BW_D, q0);
+        if (FULL) tma_reduce_add_2d(&tmDQ, sdq, hq * BW_D, q0);
+        else tma_reduce_add_3d(&tmDQ, sdq, 0, hq, q0);
         bulk_commit_group();
       }
     }
@@ -458,13 +470,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // delta[h, t] = sum_d dO[t,h,d] * O[t,h,d].  Sixteen lanes and 16-byte loads per (t, h): 22 -> 16 us for 4096 x 32 rows.
 __global__ void __launch_bounds__(256)
 attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                      float* __restrict__ delta, long long T, int Hq) {
+                      float* __restrict__ delta, long long T, int Hq, int Dv) {
   long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
   const int l = threadIdx.x & 15;
   const bool ok = row < T * Hq;
   if (!ok) row = T * Hq - 1;                 // both halves of a warp take part in the shuffles
-  const uint4 a = *reinterpret_cast<const uint4*>(dout + row * BW_D + l * 8);
-  const uint4 b = *reinterpret_cast<const uint4*>(out + row * BW_D + l * 8);
+  const bool in = l * 8 < Dv;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const uint4 a = in ? *reinterpret_cast<const uint4*>(dout + row * Dv + l * 8) : zero;
+  const uint4 b = in ? *reinterpret_cast<const uint4*>(out + row * Dv + l * 8) : zero;
   const uint32_t as[4] = {a.x, a.y, a.z, a.w}, bs[4] = {b.x, b.y, b.z, b.w};
   float s = 0.f;
 #pragma unroll
@@ -490,72 +504,73 @@ __global__ void attn_bwd_cast_kernel(const float* __restrict__ acc, __nv_bfloat1
   *reinterpret_cast<uint4*>(dq + i) = w;
 }
 
-static int bw_map(CUtensorMap* m, const void* base, long long rows, long long row_stride, int cols, int box_rows) {
-  uint64_t dims[2] = {static_cast<uint64_t>(cols), static_cast<uint64_t>(rows)};
-  uint64_t str[1] = {static_cast<uint64_t>(row_stride) * 2};
-  uint32_t box[2] = {64, static_cast<uint32_t>(box_rows)};
-  return make_tmap_bf16(m, base, 2, dims, str, box);
-}
-
 }  // namespace ttb
 
 using namespace ttb;
 
-template <int DQK, bool WITH_DQ>
+template <int DQK, bool WITH_DQ, bool FULL>
 static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv,
                            const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, cudaStream_t stream) {
   static bool smem_done[16] = {};
   using Smem = ttb::BwdSmem<DQK, WITH_DQ>;
-  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_bwd_kernel<DQK, WITH_DQ>), Smem::TOTAL, smem_done);
+  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_bwd_kernel<DQK, WITH_DQ, FULL>), Smem::TOTAL, smem_done);
   if (e != cudaSuccess) return 300 + static_cast<int>(e);
   const int heads = p.group_loop ? p.Hk : p.Hq;
   dim3 grid(WITH_DQ ? n_tiles : heads, WITH_DQ ? heads : n_tiles);
-  attn_bwd_kernel<DQK, WITH_DQ><<<grid, WITH_DQ ? 448 : 320, Smem::TOTAL, stream>>>(tq, tdo, tk, tv, tdq, p);
+  attn_bwd_kernel<DQK, WITH_DQ, FULL><<<grid, WITH_DQ ? 448 : 320, Smem::TOTAL, stream>>>(tq, tdo, tk, tv, tdq, p);
   return 0;
 }
 
-// q: [T, Hq*D] contiguous rows; dout, out: [T, Hq*128] contiguous rows; k: [T, Hk*D] (ldk); v: [T, Hk*128] (ldv, may be
-// strided); D = 128 or 192.  delta fp32 [Hq*T] scratch (left filled with rowsum(dO * O) for the query-major dQ pass).
-// with_dq != 0 (D = 128 only): dQ too, reduced into dq_acc (fp32 [T*Hq*128], zero-initialised) and cast to dq;
+// q: [T, Hq, D] contiguous; dout, out: [T, Hq, Dv] contiguous; k: [T, Hk, D] (ldk); v: [T, Hk, Dv] (ldv, may be strided); D and
+// Dv up to 128 in multiples of 8, or D = 192 with Dv = 128.  delta fp32 [Hq*T] scratch (left filled with rowsum(dO * O) for the query-major dQ pass).
+// with_dq != 0 (D <= 128 only): dQ too, reduced into dq_acc (fp32 [T*Hq*D], zero-initialised) and cast to dq;
 // with_dq == 0: dK and dV only (dq_acc and dq unused); with_dq == 2: the same with one CTA per kv head looping over the
-// query heads of its group, so that dK / dV are written once and without atomics (no accumulators needed).  dk: [T, Hk, D], dv: [T, Hk, 128]; with Hq > Hk the fp32
+// query heads of its group, so that dK / dV are written once and without atomics (no accumulators needed).  dk: [T, Hk, D], dv: [T, Hk, Dv]; with Hq > Hk the fp32
 // accumulators dk_acc / dv_acc (zero-initialised, same shapes) are required.
 TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const void* v, long long ldv, const void* out,
                             const void* dout, const float* lse, float* delta, float* dq_acc, float* dk_acc,
-                            float* dv_acc, void* dq, void* dk, void* dv, const int* kv_tiles, int n_tiles, long long T, int Hq, int Hk, int D, float scale,
+                            float* dv_acc, void* dq, void* dk, void* dv, const int* kv_tiles, int n_tiles, long long T, int Hq, int Hk, int D, int Dv, float scale,
                             int causal, int with_dq, void* stream_ptr) {
-  if ((D != 128 && D != 192) || Hq % Hk) return 901;
+  if (D < 8 || Dv < 8 || D % 8 || Dv % 8 || Dv > BW_D || (D > 128 && !(D == 192 && Dv == BW_D)) || Hq % Hk) return 901;
   const int group_loop = with_dq == 2;
   if (group_loop) with_dq = 0;
-  if (with_dq && D != 128) return 904;
+  if (with_dq && D > 128) return 904;
   if ((ldk % 8) || (ldv % 8)) return 902;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   if (T == 0 || n_tiles == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15) return 906;
   attn_bwd_delta_kernel<<<(unsigned)((T * Hq + 15) / 16), 256, 0, stream>>>((const __nv_bfloat16*)dout,
-                                                                        (const __nv_bfloat16*)out, delta, T, Hq);
+                                                                        (const __nv_bfloat16*)out, delta, T, Hq, Dv);
+  const bool full = D >= 128 && Dv == BW_D;
+  const auto map = full ? make_rows_map : make_heads_map;
   CUtensorMap tq, tdo, tk, tv;
-  if (bw_map(&tq, q, T, (long long)Hq * D, Hq * D, 64)) return 101;
-  if (bw_map(&tdo, dout, T, (long long)Hq * BW_D, Hq * BW_D, 64)) return 102;
-  if (bw_map(&tk, k, T, ldk, Hk * D, 128)) return 103;
-  if (bw_map(&tv, v, T, ldv, Hk * BW_D, 128)) return 104;
+  if (map(&tq, q, T, (long long)Hq * D, Hq, D, 64)) return 101;
+  if (map(&tdo, dout, T, (long long)Hq * Dv, Hq, Dv, 64)) return 102;
+  if (map(&tk, k, T, ldk, Hk, D, 128)) return 103;
+  if (map(&tv, v, T, ldv, Hk, Dv, 128)) return 104;
   CUtensorMap tdq = tq;   // placeholder in the form without dQ
   if (with_dq) {
     if (dq_acc == nullptr || dq == nullptr) return 905;
-    uint64_t dims[2] = {static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T)};
-    uint64_t str[1] = {static_cast<uint64_t>(Hq) * D * 4};
-    uint32_t box[2] = {static_cast<uint32_t>(D), 64};
-    if (make_tmap_f32_linear(&tdq, dq_acc, 2, dims, str, box)) return 105;
+    // the staging tile's rows, clipped to the head where it is narrower
+    const uint64_t dims2[2] = {static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T)};
+    const uint64_t dims3[3] = {static_cast<uint64_t>(D), static_cast<uint64_t>(Hq), static_cast<uint64_t>(T)};
+    const uint64_t str[2] = {static_cast<uint64_t>(D) * 4, static_cast<uint64_t>(Hq) * D * 4};
+    const uint32_t box2[2] = {static_cast<uint32_t>(BW_D), 64}, box3[3] = {static_cast<uint32_t>(BW_D), 1, 64};
+    if (full ? make_tmap_f32_linear(&tdq, dq_acc, 2, dims2, str + 1, box2) : make_tmap_f32_linear(&tdq, dq_acc, 3, dims3, str, box3)) return 105;
   }
   if (Hq != Hk && !group_loop && (dk_acc == nullptr || dv_acc == nullptr)) return 903;
-  AttnBwdParams p{kv_tiles, lse, delta, dq_acc, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_acc, dv_acc, Hq, Hk, T, scale, causal, group_loop};
-  const int rc = with_dq ? launch_attn_bwd<128, true>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
-                         : (D == 128 ? launch_attn_bwd<128, false>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
-                                     : launch_attn_bwd<192, false>(tq, tdo, tk, tv, tdq, p, n_tiles, stream));
+  AttnBwdParams p{kv_tiles, lse, delta, dq_acc, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_acc, dv_acc, Hq, Hk, D, Dv, T, scale, causal, group_loop};
+  auto run = [&](auto is_full) {
+    constexpr bool FULL = decltype(is_full)::value;
+    return with_dq ? launch_attn_bwd<128, true, FULL>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
+                   : launch_attn_bwd<128, false, FULL>(tq, tdo, tk, tv, tdq, p, n_tiles, stream);
+  };
+  const int rc = D == 192 ? launch_attn_bwd<192, false, true>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
+                          : (full ? run(std::true_type{}) : run(std::false_type{}));
   if (rc) return rc;
   // fp32 accumulators -> bf16; the ones that lie back to back on both sides go in one launch
   const bool grouped = Hq != Hk && !group_loop;
-  const long long n[3] = {with_dq ? T * Hq * D : 0, grouped ? T * Hk * D : 0, grouped ? T * Hk * BW_D : 0};
+  const long long n[3] = {with_dq ? T * Hq * D : 0, grouped ? T * Hk * D : 0, grouped ? T * Hk * Dv : 0};
   const float* src[3] = {dq_acc, dk_acc, dv_acc};
   __nv_bfloat16* dst[3] = {(__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv};
   for (int i = 0; i < 3;) {

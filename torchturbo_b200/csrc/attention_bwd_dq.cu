@@ -27,8 +27,9 @@ struct AttnDqParams {
   const int* q_tiles;   // [n_tiles, 3]: first query row, document start, document end
   const float* lse;     // [Hq, T]
   const float* delta;   // [Hq, T]
-  __nv_bfloat16* dq;    // [T, Hq, DQK]
+  __nv_bfloat16* dq;    // [T, Hq, D]
   int Hq, Hk;
+  int D, Dv;            // width of query / key heads and of value heads
   long long T;
   float scale;
   int causal;
@@ -52,11 +53,17 @@ __device__ __forceinline__ float dq_exp2(float x) {
   return y;
 }
 
-template <int DQK>
+// FULL: heads as wide as the tiles (see attn_bwd_kernel)
+template <int DQK, bool FULL>
 __global__ void __launch_bounds__(320, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnDqParams p) {
   using Smem = DqSmem<DQK>;
+  const int D = FULL ? DQK : p.D, Dv = FULL ? 128 : p.Dv;
+  auto load_head = [](void* dst, const CUtensorMap* map, uint64_t* bar, int col, int head, int width, int row) {
+    if (FULL) tma_load_2d(dst, map, bar, head * width + col, row);
+    else tma_load_3d(dst, map, bar, col, head, row);
+  };
   constexpr int QK_BYTES = Smem::QK_BYTES, VS = Smem::VS, NP = DQK / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -112,9 +119,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmDO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
       mbar_expect_tx(q_full, QK_BYTES + DQ_TILE);
 #pragma unroll
-      for (int pn = 0; pn < NP; ++pn) tma_load_2d(smem + Smem::Q + pn * 16384, &tmQ, q_full, h * DQK + pn * 64, q0);
-      tma_load_2d(smem + Smem::DO, &tmDO, q_full, h * 128, q0);
-      tma_load_2d(smem + Smem::DO + 16384, &tmDO, q_full, h * 128 + 64, q0);
+      for (int pn = 0; pn < NP; ++pn) load_head(smem + Smem::Q + pn * 16384, &tmQ, q_full, pn * 64, h, DQK, q0);
+      load_head(smem + Smem::DO, &tmDO, q_full, 0, h, 128, q0);
+      load_head(smem + Smem::DO + 16384, &tmDO, q_full, 64, h, 128, q0);
       for (int j = 0; j < nblk; ++j) {
         const int st = j & 1, vs = j % VS;
         const int kv0 = ds + j * 128;
@@ -122,18 +129,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_expect_tx(&k_full[st], QK_BYTES);
 #pragma unroll
         for (int pn = 0; pn < NP; ++pn)
-          tma_load_2d(smem + Smem::K0 + st * QK_BYTES + pn * 16384, &tmK, &k_full[st], hk * DQK + pn * 64, kv0);
+          load_head(smem + Smem::K0 + st * QK_BYTES + pn * 16384, &tmK, &k_full[st], pn * 64, hk, DQK, kv0);
         if (!mbar_wait(&v_empty[vs], ((j / VS) & 1) ^ 1, KID_ATTN_DQ, 2)) break;
         mbar_expect_tx(&v_full[vs], DQ_TILE);
-        tma_load_2d(smem + Smem::V0 + vs * DQ_TILE, &tmV, &v_full[vs], hk * 128, kv0);
-        tma_load_2d(smem + Smem::V0 + vs * DQ_TILE + 16384, &tmV, &v_full[vs], hk * 128 + 64, kv0);
+        load_head(smem + Smem::V0 + vs * DQ_TILE, &tmV, &v_full[vs], 0, hk, 128, kv0);
+        load_head(smem + Smem::V0 + vs * DQ_TILE + 16384, &tmV, &v_full[vs], 64, hk, 128, kv0);
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer (the whole warp, see umma_ss_w)
     {
       constexpr uint32_t id_s = make_idesc_bf16(128, 128, false, false);
-      constexpr uint32_t id_dq = make_idesc_bf16(128, DQK, false, true);
+      const uint32_t id_dq = make_idesc_bf16(128, (D + 15) / 16 * 16, false, true);
       const uint32_t leader = elect_one() ? 1u : 0u;
       const SmemDesc dQ = make_smem_desc2(smem_u32(smem + Smem::Q), 16, 1024), dDO = make_smem_desc2(smem_u32(smem + Smem::DO), 16, 1024);
       const SmemDesc dK = make_smem_desc2(smem_u32(smem + Smem::K0), 16, 1024), dV = make_smem_desc2(smem_u32(smem + Smem::V0), 16, 1024);
@@ -149,12 +156,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int kk = 0; kk < DQK / 16; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_ss_w(leader, tm_S, desc_at(dQ, off), desc_at(k, off), id_s, kk != 0);
+          umma_ss_w(kk * 16 < D ? leader : 0u, tm_S, desc_at(dQ, off), desc_at(k, off), id_s, kk != 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_ss_w(leader, tm_DP, desc_at(dDO, off), desc_at(v, off), id_s, kk != 0);
+          umma_ss_w(kk * 16 < Dv ? leader : 0u, tm_DP, desc_at(dDO, off), desc_at(v, off), id_s, kk != 0);
         }
         umma_commit_w(leader, s_full);
         umma_commit_w(leader, &v_empty[vs]);
@@ -244,7 +251,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (ok) {
       tc_fence_after();
       constexpr int COLS = DQK / 2;               // 64 or 96 columns per half
-      __nv_bfloat16* dst = p.dq + (static_cast<long long>(qrow) * p.Hq + h) * DQK + half * COLS;
+      __nv_bfloat16* dst = p.dq + (static_cast<long long>(qrow) * p.Hq + h) * D + half * COLS;
 #pragma unroll
       for (int cb = 0; cb < COLS / 32; ++cb) {
         uint32_t v[32];
@@ -258,6 +265,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (row_ok) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
+            if (half * COLS + cb * 32 + i >= D) continue;
             uint4 o;
             o.x = pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
             o.y = pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
@@ -278,21 +286,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 }
 
-static int dq_rows_map(CUtensorMap* m, const void* base, long long rows, long long row_stride_elems, int cols) {
-  uint64_t dims[2] = {static_cast<uint64_t>(cols), static_cast<uint64_t>(rows)};
-  uint64_t str[1] = {static_cast<uint64_t>(row_stride_elems) * 2};
-  uint32_t box[2] = {64, 128};
-  return make_tmap_bf16(m, base, 2, dims, str, box);
-}
-
-template <int DQK>
+template <int DQK, bool FULL>
 static int launch_attn_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv,
                           const AttnDqParams& p, int n_tiles, cudaStream_t stream) {
   static bool smem_done[16] = {};
-  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_bwd_dq_kernel<DQK>), DqSmem<DQK>::TOTAL, smem_done);
+  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_bwd_dq_kernel<DQK, FULL>), DqSmem<DQK>::TOTAL, smem_done);
   if (e != cudaSuccess) return 300 + static_cast<int>(e);
   dim3 grid(p.Hq, n_tiles);
-  attn_bwd_dq_kernel<DQK><<<grid, 320, DqSmem<DQK>::TOTAL, stream>>>(tq, tdo, tk, tv, p);
+  attn_bwd_dq_kernel<DQK, FULL><<<grid, 320, DqSmem<DQK>::TOTAL, stream>>>(tq, tdo, tk, tv, p);
   return 0;
 }
 
@@ -300,24 +301,27 @@ static int launch_attn_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const C
 
 using namespace ttb;
 
-// q: [T, Hq*D] contiguous rows; dout: [T, Hq*128] contiguous; k: [T, Hk*D] (ldk); v: [T, Hk*128] (ldv); lse, delta:
+// q: [T, Hq, D] contiguous; dout: [T, Hq, Dv] contiguous; k: [T, Hk, D] (ldk); v: [T, Hk, Dv] (ldv); lse, delta:
 // fp32 [Hq, T] (delta = rowsum(dO * O), from the backward's row-dot kernel); dq: bf16 [T, Hq, D], rows outside every
-// document are not written.  D = 128 or 192.
+// document are not written.  D and Dv as for ttb_attn_bwd.
 TTB_EXPORT int ttb_attn_bwd_dq(const void* q, const void* k, long long ldk, const void* v, long long ldv, const void* dout,
                                const float* lse, const float* delta, void* dq, const int* q_tiles, int n_tiles, long long T,
-                               int Hq, int Hk, int D, float scale, int causal, void* stream_ptr) {
-  if ((D != 128 && D != 192) || Hq % Hk) return 901;
+                               int Hq, int Hk, int D, int Dv, float scale, int causal, void* stream_ptr) {
+  if (D < 8 || Dv < 8 || D % 8 || Dv % 8 || Dv > 128 || (D > 128 && !(D == 192 && Dv == 128)) || Hq % Hk) return 901;
   if ((ldk % 8) || (ldv % 8)) return 902;
   if (T == 0 || n_tiles == 0) return 0;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+  const bool full = D >= 128 && Dv == 128;
+  const auto map = full ? make_rows_map : make_heads_map;
   CUtensorMap tq, tdo, tk, tv;
-  if (dq_rows_map(&tq, q, T, (long long)Hq * D, Hq * D)) return 101;
-  if (dq_rows_map(&tdo, dout, T, (long long)Hq * 128, Hq * 128)) return 102;
-  if (dq_rows_map(&tk, k, T, ldk, Hk * D)) return 103;
-  if (dq_rows_map(&tv, v, T, ldv, Hk * 128)) return 104;
-  AttnDqParams p{q_tiles, lse, delta, (__nv_bfloat16*)dq, Hq, Hk, T, scale, causal};
-  const int rc = D == 128 ? launch_attn_dq<128>(tq, tdo, tk, tv, p, n_tiles, stream)
-                          : launch_attn_dq<192>(tq, tdo, tk, tv, p, n_tiles, stream);
+  if (map(&tq, q, T, (long long)Hq * D, Hq, D, 128)) return 101;
+  if (map(&tdo, dout, T, (long long)Hq * Dv, Hq, Dv, 128)) return 102;
+  if (map(&tk, k, T, ldk, Hk, D, 128)) return 103;
+  if (map(&tv, v, T, ldv, Hk, Dv, 128)) return 104;
+  AttnDqParams p{q_tiles, lse, delta, (__nv_bfloat16*)dq, Hq, Hk, D, Dv, T, scale, causal};
+  const int rc = D == 192 ? launch_attn_dq<192, true>(tq, tdo, tk, tv, p, n_tiles, stream)
+                          : (full ? launch_attn_dq<128, true>(tq, tdo, tk, tv, p, n_tiles, stream)
+                                  : launch_attn_dq<128, false>(tq, tdo, tk, tv, p, n_tiles, stream));
   if (rc) return rc;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;

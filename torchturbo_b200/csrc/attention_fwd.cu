@@ -1,5 +1,8 @@
-// Variable-length (packed) flash attention forward for sm_100a, GQA, causal or full; value heads 128 wide, query / key
-// heads 128 wide or 192 (multi-head latent attention: 128 without position + 64 rotary).
+// Variable-length (packed) flash attention forward for sm_100a, GQA, causal or full; heads up to 128 wide (narrow ones, 72 in a
+// ViT, in multiples of 8: the tiles' missing columns read as zero and take no part in the products beyond the next multiple of
+// 16), or value heads 128 wide with query / key heads 192 (multi-head latent attention: 128 without position + 64 rotary).
+// Padding the heads first cost a ViT block (16 heads of 72, 3000 rows, forward + backward) 12 launches and 120 of 1063 us on the
+// device; the kernels themselves take the same time.
 //
 // One CTA handles two neighbouring 128-row query tiles of one document for one query head, or one.  Warp roles:
 //   warp 0      TMA producer   : Q once, then K_j / V_j tiles, shared by both query tiles
@@ -49,10 +52,11 @@ constexpr float AT_LAZY = 8.f;             // raise the running maximum only bey
 struct AttnFwdParams {
   const int* q_tiles;   // [n_tiles, 3]: first query row, document start, document end (token indices)
   int tile_rows;        // query rows per table entry: 128 (one tile per CTA) or 256 (two)
-  __nv_bfloat16* out;   // [T, Hq, D]
+  __nv_bfloat16* out;   // [T, Hq, Dv]
   float* lse;           // [Hq, T] natural-log logsumexp of the scaled logits (or null)
   float* max_logit;     // [Hq] per-head maximum scaled logit (atomic max; or null)
   int Hq, Hk;
+  int D, Dv;            // width of query / key heads and of value heads
   long long T;
   float scale;          // softmax scale (1/sqrt(D))
   int causal;
@@ -156,7 +160,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           mbar_expect_tx(&q_full[t], QK_BYTES);
 #pragma unroll
           for (int pn = 0; pn < NP; ++pn)
-            tma_load_2d(smem + AttnSmem::Q + t * QK_BYTES + pn * 16384, &tmQ, &q_full[t], h * DQK + pn * 64, q0 + t * AT_BM);
+            tma_load_3d(smem + AttnSmem::Q + t * QK_BYTES + pn * 16384, &tmQ, &q_full[t], pn * 64, h, q0 + t * AT_BM);
         };
         auto load_k = [&](int j) -> bool {
           const int ks = j % KS;
@@ -165,7 +169,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           mbar_expect_tx(&k_full[ks], QK_BYTES);
 #pragma unroll
           for (int pn = 0; pn < NP; ++pn)
-            tma_load_2d(smem + AttnSmem::K0 + ks * QK_BYTES + pn * 16384, &tmK, &k_full[ks], hk * DQK + pn * 64, kv0);
+            tma_load_3d(smem + AttnSmem::K0 + ks * QK_BYTES + pn * 16384, &tmK, &k_full[ks], pn * 64, hk, kv0);
           return true;
         };
         if (nblk > 0) load_q(0);
@@ -181,8 +185,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (two && j + ahead < nblk && !load_k(j + ahead)) break;
           if (!mbar_wait(&v_empty[vs], vph, KID_ATTN_FWD, 2)) break;
           mbar_expect_tx(&v_full[vs], TILE_BYTES);
-          tma_load_2d(smem + AttnSmem::v_at(vs), &tmV, &v_full[vs], hk * AT_D, kv0);
-          tma_load_2d(smem + AttnSmem::v_at(vs) + 16384, &tmV, &v_full[vs], hk * AT_D + 64, kv0);
+          tma_load_3d(smem + AttnSmem::v_at(vs), &tmV, &v_full[vs], 0, hk, kv0);
+          tma_load_3d(smem + AttnSmem::v_at(vs) + 16384, &tmV, &v_full[vs], 64, hk, kv0);
           if (++vs == n_vs) { vs = 0; vph ^= 1; }
           if (!two && j + ahead < nblk) ok = load_k(j + ahead);
         }
@@ -190,7 +194,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     } else if (warp == 1) {
       // ---------------------------------------------------------------- MMA issuer (the whole warp, see umma_ss_w)
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);  // Q (K-major) x K (K-major)
-      constexpr uint32_t idesc_o = make_idesc_bf16(128, 128, false, true);   // P (K-major) x V (MN-major)
+      const uint32_t idesc_o = make_idesc_bf16(128, (p.Dv + 15) / 16 * 16, false, true);   // P (K-major) x V (MN-major)
       const uint32_t leader = elect_one() ? 1u : 0u;
       const SmemDesc dQ = make_smem_desc2(smem_u32(smem + AttnSmem::Q), 16, 1024);
       const SmemDesc dK = make_smem_desc2(smem_u32(smem + AttnSmem::K0), 16, 1024);
@@ -202,7 +206,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int kk = 0; kk < DQK / 16; ++kk) {
           const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_ss_w(leader, tm_S + slot * 128, desc_at(a, off), desc_at(b, off), idesc_s, kk != 0);
+          umma_ss_w(kk * 16 < p.D ? leader : 0u, tm_S + slot * 128, desc_at(a, off), desc_at(b, off), idesc_s, kk != 0);
         }
         umma_commit_w(leader, &s_full[slot]);
       };
@@ -377,7 +381,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (ok) {
         tc_fence_after();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        __nv_bfloat16* dst = p.out + (static_cast<long long>(qrow) * p.Hq + h) * AT_D;
+        __nv_bfloat16* dst = p.out + (static_cast<long long>(qrow) * p.Hq + h) * p.Dv;
 #pragma unroll
         for (int cb = 0; cb < 4; ++cb) {
           uint32_t v[32];
@@ -386,6 +390,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (row_ok) {
 #pragma unroll
             for (int i = 0; i < 32; i += 8) {
+              if (cb * 32 + i >= p.Dv) continue;
               uint4 w;
               w.x = pack_bf16(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv);
               w.y = pack_bf16(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
@@ -418,32 +423,27 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
   return 0;
 }
 
-static int make_rows_map(CUtensorMap* m, const void* base, long long rows, long long row_stride_elems, int cols) {
-  uint64_t dims[2] = {static_cast<uint64_t>(cols), static_cast<uint64_t>(rows)};
-  uint64_t str[1] = {static_cast<uint64_t>(row_stride_elems) * 2};
-  uint32_t box[2] = {64, 128};
-  return make_tmap_bf16(m, base, 2, dims, str, box);
-}
-
 }  // namespace ttb
 
 using namespace ttb;
 
-// q: [T, Hq*D] (row stride ldq), k: [T, Hk*D] (ldk), v: [T, Hk*128] (ldv; may be a strided view); D = 128 or 192
+// q: [T, Hq, D] (row stride ldq), k: [T, Hk, D] (ldk), v: [T, Hk, Dv] (ldv; may be a strided view), out: [T, Hq, Dv]; D and Dv up
+// to 128 in multiples of 8, or D = 192 with Dv = 128
 TTB_EXPORT int ttb_attn_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                             void* out, float* lse, float* max_logit, const int* q_tiles, int n_tiles, int tile_rows, long long T,
-                            int Hq, int Hk, int D, float scale, int causal, void* stream) {
-  if ((D != 128 && D != 192) || Hq % Hk) return 901;
+                            int Hq, int Hk, int D, int Dv, float scale, int causal, void* stream) {
+  if (D < 8 || Dv < 8 || D % 8 || Dv % 8 || Dv > AT_D || (D > 128 && !(D == 192 && Dv == AT_D)) || Hq % Hk) return 901;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8)) return 902;
-  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) return 903;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15)
+    return 903;
   if (tile_rows != 128 && tile_rows != 256) return 904;
   if (n_tiles == 0) return 0;
   CUtensorMap tq, tk, tv;
-  if (make_rows_map(&tq, q, T, ldq, Hq * D)) return 101;
-  if (make_rows_map(&tk, k, T, ldk, Hk * D)) return 102;
-  if (make_rows_map(&tv, v, T, ldv, Hk * AT_D)) return 103;
-  AttnFwdParams p{q_tiles, tile_rows, (__nv_bfloat16*)out, lse, max_logit, Hq, Hk, T, scale, causal};
-  const int rc = D == 128 ? launch_attn_fwd<128>(tq, tk, tv, p, n_tiles, reinterpret_cast<cudaStream_t>(stream))
+  if (make_heads_map(&tq, q, T, ldq, Hq, D, AT_BM)) return 101;
+  if (make_heads_map(&tk, k, T, ldk, Hk, D, AT_BN)) return 102;
+  if (make_heads_map(&tv, v, T, ldv, Hk, Dv, AT_BN)) return 103;
+  AttnFwdParams p{q_tiles, tile_rows, (__nv_bfloat16*)out, lse, max_logit, Hq, Hk, D, Dv, T, scale, causal};
+  const int rc = D <= 128 ? launch_attn_fwd<128>(tq, tk, tv, p, n_tiles, reinterpret_cast<cudaStream_t>(stream))
                           : launch_attn_fwd<192>(tq, tk, tv, p, n_tiles, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
   cudaError_t e = cudaGetLastError();

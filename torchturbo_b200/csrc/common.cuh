@@ -124,12 +124,18 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 // Tile in shared memory added element-wise into a tile of a global tensor (fp32 add done by the L2), tracked by the
-// thread's bulk async-group.  The x coordinate times the element size must be a multiple of 16 B and no coordinate
-// may be negative.
+// thread's bulk async-group; what lies outside the tensor is left out.  The x coordinate times the element size must be a
+// multiple of 16 B and no coordinate may be negative.
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const void* smem_src, int x, int y) {
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
                :
                : "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               :
+               : "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -504,10 +510,26 @@ inline int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const ui
   return make_tmap_typed(out, base, rank, dims, strides_bytes, box, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-// fp32 tiles without swizzle (rows of the box contiguous in shared memory): TMA stores and reductions
+// fp32 tiles without swizzle (rows of the box contiguous in shared memory): TMA reductions
 inline int make_tmap_f32_linear(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                                 const uint64_t* strides_bytes, const uint32_t* box) {
   return make_tmap_typed(out, base, rank, dims, strides_bytes, box, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+// Rows of heads, [rows][heads][width] bf16 with contiguous heads: boxes of 64 columns of one head and `box_rows` rows.  Columns
+// past a head's width read as zero, so that a narrow head fills a wider tile without a padded copy.
+inline int make_heads_map(CUtensorMap* m, const void* base, long long rows, long long row_stride_elems, int heads, int width, int box_rows) {
+  const uint64_t dims[3] = {static_cast<uint64_t>(width), static_cast<uint64_t>(heads), static_cast<uint64_t>(rows)};
+  const uint64_t str[2] = {static_cast<uint64_t>(width) * 2, static_cast<uint64_t>(row_stride_elems) * 2};
+  const uint32_t box[3] = {64, 1, static_cast<uint32_t>(box_rows)};
+  return make_tmap_bf16(m, base, 3, dims, str, box);
+}
+// the same for heads that are whole panels of 64 columns: [rows][heads * width]
+inline int make_rows_map(CUtensorMap* m, const void* base, long long rows, long long row_stride_elems, int heads, int width, int box_rows) {
+  const uint64_t dims[2] = {static_cast<uint64_t>(heads) * width, static_cast<uint64_t>(rows)};
+  const uint64_t str[1] = {static_cast<uint64_t>(row_stride_elems) * 2};
+  const uint32_t box[2] = {64, static_cast<uint32_t>(box_rows)};
+  return make_tmap_bf16(m, base, 2, dims, str, box);
 }
 
 inline int make_tmap_typed(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,

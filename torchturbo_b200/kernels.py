@@ -799,21 +799,22 @@ def _zero_outside(t: torch.Tensor, rows) -> torch.Tensor:
 
 def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_lse: bool = True,
              want_max_logit: bool = False, rows=None, tile_rows: int = 128):
-    """q: [T, Hq, D]; k: [T, Hk, D] with D = 128 or 192 (multi-head latent attention); v: [T, Hk, 128] (may be a
-    row-strided view).  `q_tiles_dev`: `build_q_tiles(cu, tile_rows)`, one thread block per entry and query head, with
+    """q: [T, Hq, D]; k: [T, Hk, D]; v: [T, Hk, Dv] (may be a row-strided view), D and Dv up to 128 in multiples of 8, or D = 192
+    with Dv = 128 (multi-head latent attention).  `q_tiles_dev`: `build_q_tiles(cu, tile_rows)`, one thread block per entry and query head, with
     `tile_rows` 128 or 256.  `rows` (optional): (first, one past the last) row that the tile table covers; the kernel writes
-    every one of them.  Returns (out [T, Hq, 128], lse [Hq, T], max_logit [Hq])."""
+    every one of them.  Returns (out [T, Hq, Dv], lse [Hq, T], max_logit [Hq])."""
     T, Hq, D = q.shape
     Hk = k.shape[1]
-    assert D in (128, 192) and k.shape[2] == D and v.shape[2] == 128
-    assert q.stride(2) == 1 and q.stride(1) == D and k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == 128 and v.stride(2) == 1
+    Dv = v.shape[2]
+    assert k.shape[2] == D and ((D <= 128 and Dv <= 128 and D % 8 == 0 and Dv % 8 == 0) or (D, Dv) == (192, 128))
+    assert q.stride(2) == 1 and q.stride(1) == D and k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == Dv and v.stride(2) == 1
     # rows past the last sequence boundary are never written by the kernel and must read as zero
-    out = _zero_outside(torch.empty(T, Hq, 128, dtype=q.dtype, device=q.device), rows)
+    out = _zero_outside(torch.empty(T, Hq, Dv, dtype=q.dtype, device=q.device), rows)
     lse = torch.full((Hq, T), float("-inf"), dtype=torch.float32, device=q.device) if want_lse else None
     ml = torch.full((Hq,), float("-inf"), dtype=torch.float32, device=q.device) if want_max_logit else None
     _check(lib().ttb_attn_fwd(_p(q), C.c_longlong(q.stride(0)), _p(k), C.c_longlong(k.stride(0)), _p(v),
                               C.c_longlong(v.stride(0)), _p(out), _p(lse), _p(ml), _p(q_tiles_dev),
-                              C.c_int(q_tiles_dev.shape[0]), C.c_int(tile_rows), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D),
+                              C.c_int(q_tiles_dev.shape[0]), C.c_int(tile_rows), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_int(Dv),
                               C.c_float(scale), C.c_int(int(causal)), _stream()), "ttb_attn_fwd")
     return out, lse, ml
 
@@ -1149,30 +1150,30 @@ def ep_gather_vals(peer_ptrs, off_vals, expert, dest_row, El, world, cap_rows, s
 
 def attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, *, scale: float, causal: bool = True, q_tiles_dev=None,
              deterministic: bool = False, rows=None):
-    """Gradients of `attn_fwd`.  Returns (dq [T,Hq,D], dk [T,Hk,D], dv [T,Hk,128]) in bf16; `rows` as in `attn_fwd`.
+    """Gradients of `attn_fwd`.  Returns (dq [T,Hq,D], dk [T,Hk,D], dv [T,Hk,Dv]) in bf16; `rows` as in `attn_fwd`.
 
-    128-wide heads by default: one kernel; dQ tiles are added into an fp32 scratch buffer by TMA reductions and, with
+    Heads up to 128 wide by default: one kernel; dQ tiles are added into an fp32 scratch buffer by TMA reductions and, with
     grouped-query attention, the dK / dV of a group's query heads are summed with atomics (the order of the adds is not
     fixed).  For 192-wide query / key heads that kernel computes dK / dV only and dQ comes from the query-major pass
     (`q_tiles_dev` required), which writes every dQ tile once.  `deterministic=True` uses that split for every width
     and lets one CTA per kv head walk the query heads of its group, so nothing is reduced with atomics and the result
     is bit-reproducible."""
     T, Hq, D = q.shape
-    Hk = k.shape[1]
+    Hk, Dv = k.shape[1], v.shape[2]
     assert dout.is_contiguous() and out.is_contiguous() and q.is_contiguous()
-    assert k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == 128 and v.stride(2) == 1
-    split = deterministic or D != 128
+    assert k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == Dv and v.stride(2) == 1
+    split = deterministic or D > 128
     if split and q_tiles_dev is None:
         raise ValueError("the query-major dQ pass needs the query tile table")
     if kv_tiles_dev.shape[0] == 0:                       # no sequence covers a row
         return torch.zeros_like(q), torch.zeros(T, Hk, D, dtype=q.dtype, device=q.device), \
-            torch.zeros(T, Hk, 128, dtype=q.dtype, device=q.device)
+            torch.zeros(T, Hk, Dv, dtype=q.dtype, device=q.device)
     delta = torch.empty(Hq * T, dtype=torch.float32, device=q.device)
     dq_acc = dk_acc = dv_acc = None
     if Hq != Hk and not deterministic:
         # query heads of a group add into fp32 accumulators, converted at the end; accumulators and results lie back to
         # back, so that they are cleared and converted by one launch each
-        shapes = ([] if split else [(T, Hq, D)]) + [(T, Hk, D), (T, Hk, 128)]
+        shapes = ([] if split else [(T, Hq, D)]) + [(T, Hk, D), (T, Hk, Dv)]
         sizes = [a * b * c for a, b, c in shapes]
         acc = torch.zeros(sum(sizes), dtype=torch.float32, device=q.device).split(sizes)
         res = torch.empty(sum(sizes), dtype=q.dtype, device=q.device).split(sizes)
@@ -1189,19 +1190,19 @@ def attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, *, scale: float, causal: boo
         if split:
             _zero_outside(dq, rows)
         dk = _zero_outside(torch.empty(T, Hk, D, dtype=q.dtype, device=q.device), rows)
-        dv = _zero_outside(torch.empty(T, Hk, 128, dtype=q.dtype, device=q.device), rows)
+        dv = _zero_outside(torch.empty(T, Hk, Dv, dtype=q.dtype, device=q.device), rows)
     global LAUNCH_COUNT
     _check(lib().ttb_attn_bwd(_p(q), _p(k), C.c_longlong(k.stride(0)), _p(v), C.c_longlong(v.stride(0)), _p(out),
                               _p(dout), _p(lse), _p(delta), _p(dq_acc), _p(dk_acc), _p(dv_acc), _p(dq), _p(dk), _p(dv),
                               _p(kv_tiles_dev),
-                              C.c_int(kv_tiles_dev.shape[0]), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D),
+                              C.c_int(kv_tiles_dev.shape[0]), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_int(Dv),
                               C.c_float(scale), C.c_int(int(causal)), C.c_int((2 if deterministic else 0) if split else 1), _stream()),
            "ttb_attn_bwd")
     LAUNCH_COUNT += 2 if (not split or (Hq != Hk and not deterministic)) else 1
     if split:
         _check(lib().ttb_attn_bwd_dq(_p(q), _p(k), C.c_longlong(k.stride(0)), _p(v), C.c_longlong(v.stride(0)), _p(dout),
                                      _p(lse), _p(delta), _p(dq), _p(q_tiles_dev), C.c_int(q_tiles_dev.shape[0]),
-                                     C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_float(scale),
+                                     C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_int(Dv), C.c_float(scale),
                                      C.c_int(int(causal)), _stream()), "ttb_attn_bwd_dq")
     return dq, dk, dv
 

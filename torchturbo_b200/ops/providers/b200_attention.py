@@ -12,7 +12,7 @@ from ...utils.functools import cache
 from ..base import OpImplKind
 from ..registry import register_op
 from . import native as N
-from .b200 import BF16, _B200Op, _ok
+from .b200 import BF16, _aligned, _B200Op, _ok
 
 
 class _Tiles:
@@ -63,9 +63,9 @@ class FlashAttnFn(torch.autograd.Function):
     def backward(ctx, dout, *_):
         q, k, v, out, lse = ctx.saved_tensors
         cu_seqlens, max_seqlen, causal, scale, n = ctx.meta
-        if os.environ.get("TORCHTURBO_ATTN_BWD", "tcgen05") == "tcgen05":
+        if not _library_backward():
             tiles = _tiles_for(cu_seqlens, q.device)
-            dq, dk, dv = K.attn_bwd(dout.contiguous(), q, k, v, out, lse, tiles.kv, scale=scale, causal=causal,
+            dq, dk, dv = K.attn_bwd(_aligned(dout), q, k, v, out, lse, tiles.kv, scale=scale, causal=causal,
                                     q_tiles_dev=tiles.q[128], deterministic=torch.are_deterministic_algorithms_enabled(),
                                     rows=tiles.rows)
             return dq, dk, dv, None, None, None, None, None
@@ -91,6 +91,23 @@ def _LIB_FALLBACK(q, k, v, cu_seqlens, max_seqlen, *, causal, scale):
     return N.attention_ref(q, k, v, cu_seqlens, causal, scale)
 
 
+def _library_backward() -> bool:
+    return os.environ.get("TORCHTURBO_ATTN_BWD", "tcgen05") != "tcgen05"
+
+
+def _narrow(q, k, v):
+    """Head widths below 128 in multiples of 8 (ViT: 72, 80), which the kernels take as they are: the loads fill the tiles' missing
+    columns with zeros."""
+    return _paddable(q, k, v) and q.shape[-1] % 8 == 0 and v.shape[-1] % 8 == 0 and not _library_backward()
+
+
+def _rows_of_heads(t):
+    """[T, H, D] whose heads lie in a row and whose rows start on 16 bytes; copied only where they do not."""
+    if t.stride(2) != 1 or t.stride(1) != t.shape[2] or t.stride(0) % 8 or t.data_ptr() % 16:
+        t = t.clone(memory_format=torch.contiguous_format)
+    return t
+
+
 def _usable(q, k, v):
     """128-wide heads, or multi-head latent attention (query / key 192 wide, value 128 wide)."""
     return _ok(q, k, v) and q.shape[-1] in (128, 192) and k.shape[-1] == q.shape[-1] and v.shape[-1] == 128 and q.dim() == 3 \
@@ -98,17 +115,20 @@ def _usable(q, k, v):
 
 
 def _paddable(q, k, v):
-    """Head widths below 128 (ViT: 72, 80) run on the 128-wide kernel with zero columns: padded query / key columns add
+    """Any head width below 128 can run on the 128-wide kernel with zero columns: padded query / key columns add
     nothing to the logits and padded value columns only produce output columns that are sliced away."""
     return _ok(q, k, v) and q.dim() == 3 and q.shape[1] % k.shape[1] == 0 and q.shape[-1] == k.shape[-1] and \
         q.shape[-1] <= 128 and v.shape[-1] <= 128 and (q.shape[-1] < 128 or v.shape[-1] < 128)
 
 
-def _padded_call(q, k, v, cu, max_seqlen, causal, scale, want_ml):
+def _narrow_call(q, k, v, cu, max_seqlen, causal, scale, want_ml):
     import torch.nn.functional as F
 
     dqk, dv = q.shape[-1], v.shape[-1]
     scale = scale if scale is not None else 1.0 / math.sqrt(dqk)
+    if _narrow(q, k, v):
+        return FlashAttnFn.apply(_aligned(q), _aligned(k), _rows_of_heads(v), cu.cpu() if cu.is_cuda else cu, max_seqlen, causal,
+                                 float(scale), want_ml)
     qp, kp, vp = F.pad(q, (0, 128 - dqk)), F.pad(k, (0, 128 - dqk)), F.pad(v, (0, 128 - dv))
     res = FlashAttnFn.apply(qp, kp, vp, cu.cpu() if cu.is_cuda else cu, max_seqlen, causal, float(scale), want_ml)
     if want_ml:
@@ -123,7 +143,7 @@ class B200Attention(_B200Op):
         cu = cu_seqlens if isinstance(cu_seqlens, torch.Tensor) else torch.tensor(cu_seqlens, dtype=torch.int32)
         if not _usable(q, k, v):
             if _paddable(q, k, v):
-                return _padded_call(q, k, v, cu, max_seqlen, causal, scale, False)
+                return _narrow_call(q, k, v, cu, max_seqlen, causal, scale, False)
             # other head widths: the library kernel
             return _LIB_FALLBACK(q, k, v, cu_seqlens, max_seqlen, causal=causal, scale=scale)
         scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
@@ -138,7 +158,7 @@ class B200AttentionWithMaxLogits(_B200Op):
         cu = cu_seqlens if isinstance(cu_seqlens, torch.Tensor) else torch.tensor(cu_seqlens, dtype=torch.int32)
         if not _usable(q, k, v):
             if _paddable(q, k, v):
-                return _padded_call(q, k, v, cu, max_seqlen, causal, scale, True)
+                return _narrow_call(q, k, v, cu, max_seqlen, causal, scale, True)
             return N.attention_ref(q, k, v, cu_seqlens, causal, scale, want_max_logits=True)
         scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
         return FlashAttnFn.apply(q.contiguous(), k.contiguous(), v, cu.cpu() if cu.is_cuda else cu, max_seqlen, causal,
