@@ -3,7 +3,9 @@
 The kernels expose a C ABI (`extern "C"`), take raw device pointers plus the CUDA
 stream handle, and are loaded with ctypes, so no torch headers are needed and a
 full rebuild takes seconds.  The shared object is written next to the package
-(`torchturbo_b200/_lib/libttb200.so`).
+(`torchturbo_b200/_lib/libttb200.so`).  `host.cpp`, the launch functions of the hot
+operators, is a small extension module against the framework's headers beside it
+(`ttb_host.so`).
 """
 from __future__ import annotations
 
@@ -11,12 +13,16 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
+
+import torch
 
 CSRC = Path(__file__).resolve().parent
 LIB_DIR = CSRC.parent / "_lib"
 LIB_PATH = LIB_DIR / "libttb200.so"
+HOST_SOURCE, HOST_PATH = CSRC / "host.cpp", LIB_DIR / "ttb_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -43,12 +49,22 @@ def sources() -> list[Path]:
 
 def _digest(paths: list[Path]) -> str:
     h = hashlib.sha256()
-    for p in sorted(paths) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")):
+    for p in sorted(paths) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [HOST_SOURCE]:
         h.update(p.name.encode())
         h.update(p.read_bytes())
     h.update(" ".join(NVCC_FLAGS + FAST_MATH).encode())
     h.update(repr(sorted(PRECISE.items())).encode())
+    h.update(f"{torch.__version__} {sys.version}".encode())
     return h.hexdigest()
+
+
+def _host_command() -> list[str]:
+    inc = Path(torch.__file__).resolve().parent
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f"-I{inc}/include", f"-I{inc}/include/torch/csrc/api/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}",
+            str(HOST_SOURCE), "-o", str(HOST_PATH), f"-L{inc}/lib", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch",
+            f"-L{LIB_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> Path:
@@ -57,7 +73,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     srcs = sources()
     stamp = LIB_DIR / "build.stamp"
     digest = _digest(srcs)
-    if not force and LIB_PATH.exists() and stamp.exists() and stamp.read_text() == digest:
+    if not force and LIB_PATH.exists() and HOST_PATH.exists() and stamp.exists() and stamp.read_text() == digest:
         return LIB_PATH
     nvcc = _nvcc()
     obj_dir = LIB_DIR / "obj"
@@ -80,6 +96,9 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    res = subprocess.run(_host_command(), capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{HOST_SOURCE.name} failed:\n{res.stdout}\n{res.stderr}")
     stamp.write_text(digest)
     return LIB_PATH
 

@@ -1,4 +1,5 @@
-"""ctypes bindings for the sm_100a CUDA library (`_lib/libttb200.so`).
+"""Bindings for the sm_100a CUDA library (`_lib/libttb200.so`): ctypes, and for the operators that a training step calls by the
+hundred the extension module `_lib/ttb_host.so` (csrc/host.cpp).
 
 Every function here launches hand-written kernels on the *current* CUDA stream
 and takes/returns torch tensors.  Nothing falls back to PyTorch: if the library
@@ -9,14 +10,17 @@ can never pass for the native one.  CPU-only processes never touch this module
 from __future__ import annotations
 
 import ctypes as C
-import os
+import importlib.machinery
+import importlib.util
 from functools import lru_cache
 from pathlib import Path
 
 import torch
 
 _LIB_PATH = Path(__file__).resolve().parent / "_lib" / "libttb200.so"
+_HOST_PATH = _LIB_PATH.with_name("ttb_host.so")
 _lib = None
+_host = None
 
 SEG_ALIGN = 128  # rows; every expert segment of a permuted buffer is padded to this
 SCORE_FN = {"softmax_pre": 0, "softmax_post": 1, "sigmoid": 2}
@@ -24,29 +28,6 @@ SCORE_FN = {"softmax_pre": 0, "softmax_post": 1, "sigmoid": 2}
 
 class KernelError(RuntimeError):
     pass
-
-
-class _GemmArgs(C.Structure):
-    _fields_ = [
-        ("A", C.c_void_p), ("lda", C.c_longlong),
-        ("B", C.c_void_p), ("ldb", C.c_longlong),
-        ("b_group_stride", C.c_longlong), ("b_groups", C.c_int),
-        ("C", C.c_void_p), ("ldc", C.c_longlong), ("c_group_stride", C.c_longlong),
-        ("M", C.c_int), ("N", C.c_int), ("K", C.c_int),
-        ("a_mn", C.c_int), ("b_mn", C.c_int),
-        ("c_fp32", C.c_int), ("accumulate", C.c_int),
-        ("residual", C.c_void_p), ("ldr", C.c_longlong),
-        ("tile_group", C.c_void_p), ("m_tiles_cap", C.c_int),
-        ("group_rows", C.c_void_p), ("groups_k", C.c_int),
-        ("total_rows", C.c_longlong),
-        ("epi", C.c_int), ("F", C.c_int),
-        ("row_scale", C.c_void_p), ("preact", C.c_void_p), ("ld_preact", C.c_longlong),
-        ("num_sms", C.c_int),
-        ("ep", C.c_void_p),
-        ("alpha", C.c_void_p),
-        ("split_ws", C.c_void_p),
-        ("k_splits", C.c_int),
-    ]
 
 
 class EpFuseArgs(C.Structure):
@@ -95,13 +76,26 @@ def lib():
                 "(or __graft_entry__.build()) before using the CUDA ops"
             )
         _lib = C.CDLL(str(_LIB_PATH))
-        _lib.ttb_gemm_bf16.argtypes = [C.POINTER(_GemmArgs), C.c_void_p]
-        _lib.ttb_gemm_bf16.restype = C.c_int
     return _lib
 
 
+def host():
+    """The launch functions of the hot operators."""
+    global _host
+    if _host is None:
+        lib()
+        if not _HOST_PATH.exists():
+            raise KernelError(f"{_HOST_PATH} is missing: run `python -m torchturbo_b200.csrc.build` (or __graft_entry__.build())")
+        loader = importlib.machinery.ExtensionFileLoader("ttb_host", str(_HOST_PATH))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ttb_host", str(_HOST_PATH), loader=loader))
+        loader.exec_module(module)
+        module.setup(KernelError, torch.OutOfMemoryError, gemm_splits)
+        _host = module
+    return _host
+
+
 # kernels launched per C entry point (used to report how many of this library's kernels ran in a region)
-_LAUNCHES_PER_CALL = {"ttb_rmsnorm_bwd": 2, "ttb_gated_rmsnorm_bwd": 2, "ttb_layernorm_bwd": 2, "ttb_bias_act_bwd": 2, "ttb_causal_conv1d_bwd": 2,
+_LAUNCHES_PER_CALL = {"ttb_gated_rmsnorm_bwd": 2, "ttb_causal_conv1d_bwd": 2,
                       "ttb_causal_conv1d_row_blocks": 0, "ttb_kda_gate_bwd": 2, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
                       "ttb_ep_combine_all": 3, "ttb_delta_vec_bwd_post": 2, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
                       "ttb_gemm_status": 0}
@@ -110,7 +104,7 @@ LAUNCH_COUNT = 0
 
 def launch_count() -> int:
     """Number of CUDA kernels of this library launched so far in this process."""
-    return LAUNCH_COUNT
+    return LAUNCH_COUNT + (_host.launches() if _host is not None else 0)
 
 
 def _check(code: int, what: str) -> None:
@@ -169,6 +163,11 @@ def gemm_splits(M: int, N: int, K: int, sms: int) -> int:
     return max(1, min(sms // tiles, (K + 63) // 64 // 32))
 
 
+def _is_f32(dtype: torch.dtype) -> bool:
+    assert dtype in (torch.bfloat16, torch.float32), dtype
+    return dtype == torch.float32
+
+
 def gemm(
     a: torch.Tensor,
     b: torch.Tensor,
@@ -200,81 +199,8 @@ def gemm(
         ``silu(gate) * up * row_scale`` of width ``F``; ``preact`` (``[M, 2F]``) optionally keeps gate|up.
       * ``alpha`` (one fp32 value on the device) is multiplied into the fp32 product before it is rounded or added.
     """
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    assert a.stride(-1) == 1 and b.stride(-1) == 1
-    check_device(a)
-    args = _GemmArgs()
-    groups_k = 0
-    if group_rows is not None:
-        assert a_mn and b_mn and a.dim() == 2 and b.dim() == 2
-        groups_k = group_rows.numel() - 1
-        M, N, K = a.shape[1], b.shape[1], 0
-        args.total_rows = a.shape[0]
-        assert b.shape[0] == a.shape[0]
-    else:
-        if a_mn:
-            K, M = a.shape
-        else:
-            M, K = a.shape
-        if b_mn:
-            Kb, Nmem = b.shape[-2], b.shape[-1]
-        else:
-            Nmem, Kb = b.shape[-2], b.shape[-1]
-        assert Kb == K, (a.shape, b.shape, a_mn, b_mn)
-        N = Nmem // 2 if swiglu else Nmem
-    args.A, args.lda = a.data_ptr(), a.stride(0)
-    args.B = b.data_ptr()
-    args.ldb = b.stride(-2)
-    if b.dim() == 3:
-        args.b_groups, args.b_group_stride = b.shape[0], b.stride(0)
-        assert tile_group is not None
-    else:
-        args.b_groups, args.b_group_stride = 1, 0
-    if out is None:
-        shape = (groups_k, M, N) if groups_k else (M, N)
-        out = torch.empty(shape, dtype=out_dtype, device=a.device)
-        assert not accumulate
-    assert out.stride(-1) == 1 and out.dtype in (torch.bfloat16, torch.float32)
-    args.C, args.ldc = out.data_ptr(), out.stride(-2)
-    args.c_group_stride = out.stride(0) if groups_k else 0
-    args.M, args.N, args.K = M, N, K
-    args.a_mn, args.b_mn = int(a_mn), int(b_mn)
-    args.c_fp32, args.accumulate = int(out.dtype == torch.float32), int(accumulate)
-    if residual is not None:
-        assert residual.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
-        args.residual, args.ldr = residual.data_ptr(), residual.stride(0)
-    if tile_group is not None:
-        assert tile_group.dtype == torch.int32
-        args.tile_group, args.m_tiles_cap = tile_group.data_ptr(), tile_group.numel()
-        assert M <= tile_group.numel() * 128
-    if group_rows is not None:
-        assert group_rows.dtype == torch.int32
-        args.group_rows, args.groups_k = group_rows.data_ptr(), groups_k
-    args.epi = 1 if swiglu else 0
-    args.F = N if swiglu else 0
-    if row_scale is not None:
-        assert row_scale.dtype == torch.float32
-        args.row_scale = row_scale.data_ptr()
-    if preact is not None:
-        assert preact.dtype == torch.bfloat16
-        args.preact, args.ld_preact = preact.data_ptr(), preact.stride(0)
-    args.num_sms = num_sms(a.device.index)
-    if alpha is not None:
-        assert alpha.dtype == torch.float32 and alpha.numel() == 1 and alpha.device == a.device and not swiglu
-        args.alpha = alpha.data_ptr()
-    if ep is not None:
-        args.ep = C.addressof(ep)
-    splits = 1
-    if K >= 4096 and not swiglu and tile_group is None and ep is None:
-        splits = gemm_splits(M, N, K, args.num_sms)
-        if splits > 1:
-            ws = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)
-            args.split_ws, args.k_splits = ws.data_ptr(), splits
-    _check(lib().ttb_gemm_bf16(C.byref(args), _stream()), "ttb_gemm_bf16")
-    if splits > 1:
-        global LAUNCH_COUNT
-        LAUNCH_COUNT += 1
-    return out
+    return host().gemm(a, b, a_mn, b_mn, out, _is_f32(out_dtype), accumulate, residual, tile_group, group_rows, swiglu, row_scale, preact,
+                       C.addressof(ep) if ep is not None else 0, alpha)
 
 
 # --------------------------------------------------------------------------------------
@@ -282,35 +208,12 @@ def gemm(
 # --------------------------------------------------------------------------------------
 def rmsnorm_fwd(x, weight, eps, residual=None, one_plus_w=False):
     """Returns (y, rstd, x_sum) where x_sum is ``x + residual`` (or ``x`` itself without residual)."""
-    H = x.shape[-1]
-    x2 = x.reshape(-1, H)
-    T = x2.shape[0]
-    y = torch.empty_like(x2)
-    rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-    if residual is not None:
-        r2 = residual.reshape(-1, H)
-        xsum = torch.empty_like(x2)
-    else:
-        r2, xsum = None, None
-    _check(lib().ttb_rmsnorm_fwd(_p(x2), _p(r2), _p(weight), _p(y), _p(xsum), _p(rstd), C.c_longlong(T), C.c_int(H),
-                                 C.c_float(eps), C.c_int(int(one_plus_w)), _stream()), "ttb_rmsnorm_fwd")
-    return y.view(x.shape), rstd, (xsum.view(x.shape) if xsum is not None else x)
+    return host().rmsnorm_fwd(x, weight, eps, residual, one_plus_w)
 
 
 def rmsnorm_bwd(dy, x_sum, weight, rstd, dres=None, one_plus_w=False, dw_dtype=torch.float32):
     """Returns (dx, dw in ``dw_dtype``: fp32 or bf16); ``dres`` (gradient arriving on the residual stream) is added into dx."""
-    H = x_sum.shape[-1]
-    x2, dy2 = x_sum.reshape(-1, H), dy.reshape(-1, H)
-    T = x2.shape[0]
-    grid = max(1, min(T, 2 * num_sms(x_sum.device.index)))
-    dx = torch.empty_like(x2)
-    partial = torch.empty(grid, H, dtype=torch.float32, device=x_sum.device)
-    dw = torch.empty(H, dtype=dw_dtype, device=x_sum.device)
-    d2 = dres.reshape(-1, H) if dres is not None else None
-    _check(lib().ttb_rmsnorm_bwd(_p(dy2), _p(x2), _p(weight), _p(rstd), _p(d2), _p(dx), _p(partial), _p(dw),
-                                 C.c_int(int(dw_dtype == torch.bfloat16)), C.c_longlong(T), C.c_int(H), C.c_int(int(one_plus_w)), C.c_int(grid), _stream()),
-           "ttb_rmsnorm_bwd")
-    return dx.view(x_sum.shape), dw
+    return host().rmsnorm_bwd(dy, x_sum, weight, rstd, dres, one_plus_w, dw_dtype != torch.bfloat16)
 
 
 def _gated_grid(R: int, H: int, device) -> int:
@@ -349,56 +252,22 @@ ACT = {None: 0, "none": 0, "identity": 0, "gelu_tanh": 1, "gelu_pytorch_tanh": 1
 
 def layernorm_fwd(x, weight, bias, eps):
     """Returns (y, mean, rstd); statistics in fp32."""
-    H = x.shape[-1]
-    x2 = x.reshape(-1, H)
-    T = x2.shape[0]
-    y = torch.empty_like(x2)
-    mean = torch.empty(T, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-    _check(lib().ttb_layernorm_fwd(_p(x2), _p(weight), _p(bias), _p(y), _p(mean), _p(rstd), C.c_longlong(T), C.c_int(H),
-                                   C.c_float(eps), _stream()), "ttb_layernorm_fwd")
-    return y.view(x.shape), mean, rstd
+    return host().layernorm_fwd(x, weight, bias, eps)
 
 
 def layernorm_bwd(dy, x, weight, mean, rstd, dw_dtype=torch.float32):
     """Returns (dx, dw, db), the last two in ``dw_dtype`` (fp32 or bf16)."""
-    H = x.shape[-1]
-    x2, dy2 = x.reshape(-1, H), dy.reshape(-1, H)
-    T = x2.shape[0]
-    grid = max(1, min(T, 2 * num_sms(x.device.index)))
-    dx = torch.empty_like(x2)
-    part = torch.empty(grid, 2 * H, dtype=torch.float32, device=x.device)
-    dwdb = torch.empty(2, H, dtype=dw_dtype, device=x.device)
-    _check(lib().ttb_layernorm_bwd(_p(dy2), _p(x2), _p(weight), _p(mean), _p(rstd), _p(dx), _p(part), _p(dwdb),
-                                   C.c_int(int(dw_dtype == torch.bfloat16)), C.c_longlong(T), C.c_int(H), C.c_int(grid), _stream()), "ttb_layernorm_bwd")
-    return dx.view(x.shape), dwdb[0], dwdb[1]
+    return host().layernorm_bwd(dy, x, weight, mean, rstd, dw_dtype != torch.bfloat16)
 
 
 def bias_act_fwd(x, bias, act, residual=None):
     """y = act(x + bias) (+ residual) on bf16 rows."""
-    Cn = x.shape[-1]
-    x2 = x.reshape(-1, Cn)
-    y = torch.empty_like(x2)
-    r2 = residual.reshape(-1, Cn) if residual is not None else None
-    _check(lib().ttb_bias_act_fwd(_p(x2), _p(bias), _p(r2), _p(y), C.c_longlong(x2.shape[0]), C.c_int(Cn), C.c_int(ACT[act]),
-                                  _stream()), "ttb_bias_act_fwd")
-    return y.view(x.shape)
+    return host().bias_act_fwd(x, bias, ACT[act], residual)
 
 
 def bias_act_bwd(dy, x, bias, act, db_dtype=torch.float32):
     """Returns (dx, dbias in ``db_dtype``: fp32 or bf16); with the identity activation dx is dy itself."""
-    Cn = x.shape[-1]
-    x2, dy2 = x.reshape(-1, Cn), dy.reshape(-1, Cn)
-    R = x2.shape[0]
-    code = ACT[act]
-    grid = max(1, min(R, 2 * num_sms(x.device.index)))
-    dx = torch.empty_like(x2) if code else None
-    part = torch.empty(grid, Cn, dtype=torch.float32, device=x.device)
-    db = torch.empty(Cn, dtype=db_dtype, device=x.device)
-    _check(lib().ttb_bias_act_bwd(_p(dy2), _p(x2), _p(bias), _p(dx), _p(part), _p(db),
-                                  C.c_int(int(db_dtype == torch.bfloat16)), C.c_longlong(R), C.c_int(Cn),
-                                  C.c_int(code), C.c_int(grid), _stream()), "ttb_bias_act_bwd")
-    return (dx.view(x.shape) if dx is not None else dy), db
+    return host().bias_act_bwd(dy, x, bias, ACT[act], db_dtype != torch.bfloat16)
 
 
 # --------------------------------------------------------------------------------------
@@ -437,41 +306,18 @@ def causal_conv1d_bwd(dy, x, weight, bias, seq_start, seq_end, silu: bool):
 # --------------------------------------------------------------------------------------
 def qknorm_rope_fwd(qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, eps, use_norm=True):
     """qkv: [T, (n_q + 2 n_kv) * D] -> (q [T, n_q, D], k [T, n_kv, D], rstd [T * (n_q + n_kv)])."""
-    T = qkv.shape[0]
-    q = torch.empty(T, n_q, head_dim, dtype=qkv.dtype, device=qkv.device)
-    k = torch.empty(T, n_kv, head_dim, dtype=qkv.dtype, device=qkv.device)
-    rstd = torch.empty(T * (n_q + n_kv), dtype=torch.float32, device=qkv.device)
-    _check(lib().ttb_qknorm_rope_fwd(_p(qkv), C.c_longlong(qkv.stride(0)), C.c_int(n_q), C.c_int(n_kv),
-                                     C.c_int(head_dim), _p(wq), _p(wk), _p(cos), _p(sin), _p(q), _p(k), _p(rstd),
-                                     C.c_longlong(T), C.c_float(eps), C.c_int(int(use_norm)), _stream()),
-           "ttb_qknorm_rope_fwd")
-    return q, k, rstd
+    return host().qknorm_rope_fwd(qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, eps, use_norm)
 
 
 def qknorm_rope_bwd(dq, dk, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dqkv, use_norm=True, dv=None, dw_dtype=torch.float32):
     """Writes the q and k column blocks of ``dqkv`` ([T, ld]), with ``dv`` ([T, n_kv, D]) the v block too, and returns (dwq, dwk)
     in ``dw_dtype`` (fp32 or bf16)."""
-    T = qkv.shape[0]
-    groups = (n_q + n_kv * (1 if dv is None else 2) + 3) // 4          # a warp takes four heads of a token
-    grid = max(1, min((T * groups + 7) // 8, 4 * num_sms(qkv.device.index)))
-    dw = (torch.empty if use_norm and T else torch.zeros)(2, head_dim, dtype=dw_dtype, device=qkv.device)
-    part = torch.empty(grid, 2 * head_dim, dtype=torch.float32, device=qkv.device) if use_norm else None
-    _check(lib().ttb_qknorm_rope_bwd(_p(dq), _p(dk), _p(dv), _p(qkv), C.c_longlong(qkv.stride(0)), C.c_int(n_q), C.c_int(n_kv),
-                                     C.c_int(head_dim), _p(wq), _p(wk), _p(cos), _p(sin), _p(rstd), _p(dqkv),
-                                     C.c_longlong(dqkv.stride(0)), _p(part), _p(dw), C.c_int(int(dw_dtype == torch.bfloat16)),
-                                     C.c_longlong(T), C.c_int(int(use_norm)), C.c_int(grid), _stream()), "ttb_qknorm_rope_bwd")
-    global LAUNCH_COUNT
-    LAUNCH_COUNT += 1 if use_norm else 0
-    return dw[0], dw[1]
+    return host().qknorm_rope_bwd(dq, dk, dv, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dqkv, use_norm, dw_dtype != torch.bfloat16)
 
 
 def rope(x, cos, sin, sign: float = 1.0):
     """Half-rotation RoPE of bf16 [T, heads, D] (channels contiguous); cos, sin fp32 [T, D / 2].  ``sign=-1`` rotates back."""
-    T, heads, D = x.shape
-    y = torch.empty(T, heads, D, dtype=x.dtype, device=x.device)
-    _check(lib().ttb_rope(_p(x), C.c_longlong(x.stride(0)), C.c_longlong(x.stride(1)), _p(cos), _p(sin), _p(y), C.c_longlong(T),
-                          C.c_int(heads), C.c_int(D // 2), C.c_float(sign), _stream()), "ttb_rope")
-    return y
+    return host().rope(x, cos, sin, sign)
 
 
 # --------------------------------------------------------------------------------------
@@ -508,26 +354,13 @@ def kda_gate_bwd(dd, g, A_log, dt_bias, lower_bound):
 # --------------------------------------------------------------------------------------
 def swiglu_fwd(x, row_scale=None, nrows=None):
     """`nrows` (int32 device scalar, optional): only the first `nrows[0]` rows are computed (padded buffers)."""
-    R, F2 = x.shape
-    F = F2 // 2
-    y = torch.empty(R, F, dtype=x.dtype, device=x.device)
-    _check(lib().ttb_swiglu_fwd(_p(x), C.c_longlong(x.stride(0)), _p(y), C.c_longlong(y.stride(0)), _p(row_scale),
-                                C.c_longlong(R), C.c_int(F), _p(nrows), _stream()), "ttb_swiglu_fwd")
-    return y
+    return host().swiglu_fwd(x, row_scale, nrows)
 
 
 def swiglu_bwd(dy, x, row_scale=None, want_dscale=False, nrows=None, y_out=None):
     """`nrows` (int32 device scalar, optional): rows from `nrows[0]` on are left untouched (padded buffers).  `y_out` (bf16
     [R, F], optional) receives the forward result, as `swiglu_fwd` computes it."""
-    R, F2 = x.shape
-    F = F2 // 2
-    dx = torch.empty_like(x)
-    dscale = torch.empty(R, dtype=torch.float32, device=x.device) if want_dscale else None
-    _check(lib().ttb_swiglu_bwd(_p(dy), C.c_longlong(dy.stride(0)), _p(x), C.c_longlong(x.stride(0)), _p(row_scale),
-                                _p(dx), C.c_longlong(dx.stride(0)), _p(dscale), _p(y_out),
-                                C.c_longlong(y_out.stride(0) if y_out is not None else 0), C.c_longlong(R), C.c_int(F), _p(nrows),
-                                _stream()), "ttb_swiglu_bwd")
-    return dx, dscale
+    return host().swiglu_bwd(dy, x, row_scale, want_dscale, nrows, y_out)
 
 
 # --------------------------------------------------------------------------------------
@@ -785,16 +618,9 @@ def attn_tile_rows(lens, heads: int, causal: bool, sms: int) -> int:
     return 256 if launch(2, 3.35) < launch(1, 2.05) else 128
 
 
-def _zero_outside(t: torch.Tensor, rows) -> torch.Tensor:
-    """Rows of `t` that no sequence covers read as zero; `rows` = (first, one past the last) covered row, None = unknown."""
-    if rows is None:
-        return t.zero_()
-    lo, hi = rows
-    if lo > 0:
-        t[:lo].zero_()
-    if hi < t.shape[0]:
-        t[hi:].zero_()
-    return t
+def _covered(rows) -> tuple[int, int]:
+    """(first, one past the last) covered row, or a negative first for unknown."""
+    return rows if rows is not None else (-1, -1)
 
 
 def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_lse: bool = True,
@@ -803,20 +629,7 @@ def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_ls
     with Dv = 128 (multi-head latent attention).  `q_tiles_dev`: `build_q_tiles(cu, tile_rows)`, one thread block per entry and query head, with
     `tile_rows` 128 or 256.  `rows` (optional): (first, one past the last) row that the tile table covers; the kernel writes
     every one of them.  Returns (out [T, Hq, Dv], lse [Hq, T], max_logit [Hq])."""
-    T, Hq, D = q.shape
-    Hk = k.shape[1]
-    Dv = v.shape[2]
-    assert k.shape[2] == D and ((D <= 128 and Dv <= 128 and D % 8 == 0 and Dv % 8 == 0) or (D, Dv) == (192, 128))
-    assert q.stride(2) == 1 and q.stride(1) == D and k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == Dv and v.stride(2) == 1
-    # rows past the last sequence boundary are never written by the kernel and must read as zero
-    out = _zero_outside(torch.empty(T, Hq, Dv, dtype=q.dtype, device=q.device), rows)
-    lse = torch.full((Hq, T), float("-inf"), dtype=torch.float32, device=q.device) if want_lse else None
-    ml = torch.full((Hq,), float("-inf"), dtype=torch.float32, device=q.device) if want_max_logit else None
-    _check(lib().ttb_attn_fwd(_p(q), C.c_longlong(q.stride(0)), _p(k), C.c_longlong(k.stride(0)), _p(v),
-                              C.c_longlong(v.stride(0)), _p(out), _p(lse), _p(ml), _p(q_tiles_dev),
-                              C.c_int(q_tiles_dev.shape[0]), C.c_int(tile_rows), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_int(Dv),
-                              C.c_float(scale), C.c_int(int(causal)), _stream()), "ttb_attn_fwd")
-    return out, lse, ml
+    return host().attn_fwd(q, k, v, q_tiles_dev, scale, causal, want_lse, want_max_logit, *_covered(rows), tile_rows)
 
 
 def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, reverse: bool, s1: float, s2: float):
@@ -1158,53 +971,7 @@ def attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, *, scale: float, causal: boo
     (`q_tiles_dev` required), which writes every dQ tile once.  `deterministic=True` uses that split for every width
     and lets one CTA per kv head walk the query heads of its group, so nothing is reduced with atomics and the result
     is bit-reproducible."""
-    T, Hq, D = q.shape
-    Hk, Dv = k.shape[1], v.shape[2]
-    assert dout.is_contiguous() and out.is_contiguous() and q.is_contiguous()
-    assert k.stride(1) == D and k.stride(2) == 1 and v.stride(1) == Dv and v.stride(2) == 1
-    split = deterministic or D > 128
-    if split and q_tiles_dev is None:
-        raise ValueError("the query-major dQ pass needs the query tile table")
-    if kv_tiles_dev.shape[0] == 0:                       # no sequence covers a row
-        return torch.zeros_like(q), torch.zeros(T, Hk, D, dtype=q.dtype, device=q.device), \
-            torch.zeros(T, Hk, Dv, dtype=q.dtype, device=q.device)
-    delta = torch.empty(Hq * T, dtype=torch.float32, device=q.device)
-    dq_acc = dk_acc = dv_acc = None
-    if Hq != Hk and not deterministic:
-        # query heads of a group add into fp32 accumulators, converted at the end; accumulators and results lie back to
-        # back, so that they are cleared and converted by one launch each
-        shapes = ([] if split else [(T, Hq, D)]) + [(T, Hk, D), (T, Hk, Dv)]
-        sizes = [a * b * c for a, b, c in shapes]
-        acc = torch.zeros(sum(sizes), dtype=torch.float32, device=q.device).split(sizes)
-        res = torch.empty(sum(sizes), dtype=q.dtype, device=q.device).split(sizes)
-        acc, res = ([t.view(s) for t, s in zip(x, shapes)] for x in (acc, res))
-        (dk_acc, dv_acc), (dk, dv) = acc[-2:], res[-2:]
-        if split:
-            dq = _zero_outside(torch.empty_like(q), rows)
-        else:
-            dq_acc, dq = acc[0], res[0]
-    else:
-        if not split:
-            dq_acc = torch.zeros(T, Hq, D, dtype=torch.float32, device=q.device)
-        dq = torch.empty_like(q)
-        if split:
-            _zero_outside(dq, rows)
-        dk = _zero_outside(torch.empty(T, Hk, D, dtype=q.dtype, device=q.device), rows)
-        dv = _zero_outside(torch.empty(T, Hk, Dv, dtype=q.dtype, device=q.device), rows)
-    global LAUNCH_COUNT
-    _check(lib().ttb_attn_bwd(_p(q), _p(k), C.c_longlong(k.stride(0)), _p(v), C.c_longlong(v.stride(0)), _p(out),
-                              _p(dout), _p(lse), _p(delta), _p(dq_acc), _p(dk_acc), _p(dv_acc), _p(dq), _p(dk), _p(dv),
-                              _p(kv_tiles_dev),
-                              C.c_int(kv_tiles_dev.shape[0]), C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_int(Dv),
-                              C.c_float(scale), C.c_int(int(causal)), C.c_int((2 if deterministic else 0) if split else 1), _stream()),
-           "ttb_attn_bwd")
-    LAUNCH_COUNT += 2 if (not split or (Hq != Hk and not deterministic)) else 1
-    if split:
-        _check(lib().ttb_attn_bwd_dq(_p(q), _p(k), C.c_longlong(k.stride(0)), _p(v), C.c_longlong(v.stride(0)), _p(dout),
-                                     _p(lse), _p(delta), _p(dq), _p(q_tiles_dev), C.c_int(q_tiles_dev.shape[0]),
-                                     C.c_longlong(T), C.c_int(Hq), C.c_int(Hk), C.c_int(D), C.c_int(Dv), C.c_float(scale),
-                                     C.c_int(int(causal)), _stream()), "ttb_attn_bwd_dq")
-    return dq, dk, dv
+    return host().attn_bwd(dout, q, k, v, out, lse, kv_tiles_dev, scale, causal, q_tiles_dev, deterministic, *_covered(rows))
 
 
 # --------------------------------------------------------------------------------------
