@@ -1,0 +1,78 @@
+"""The native launch functions: what they refuse, and operand layouts against contiguous operands (bit for bit)."""
+import threading
+
+import pytest
+import torch
+
+from torchturbo_b200 import kernels as K
+
+
+def test_wrong_arguments_are_refused():
+    x = torch.zeros(8, 64, dtype=torch.bfloat16)
+    with pytest.raises(AssertionError):
+        K.gemm(x.float(), x)
+    with pytest.raises(AssertionError):
+        K.gemm(x, x, out_dtype=torch.float16)
+    with pytest.raises(TypeError):
+        K.host().rope(x)
+    with pytest.raises(TypeError):
+        K.host().rmsnorm_fwd(x, None, 1e-6, None, False)
+    with pytest.raises(TypeError):
+        K.host().rmsnorm_fwd(x, x, "eps", None, False)
+
+
+def _calls(rows, cols):
+    g = torch.Generator("cuda").manual_seed(rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()                                # noqa: E731
+    x, dy, res, w, b = rnd(rows, cols), rnd(rows, cols), rnd(rows, cols), rnd(cols), rnd(cols)
+    _, rstd, _ = K.rmsnorm_fwd(x, w, 1e-6)
+    _, mean, lstd = K.layernorm_fwd(x, w, b, 1e-6)
+    return x, dy, res, {
+        "rmsnorm_fwd": lambda x, dy, res: K.rmsnorm_fwd(x, w, 1e-6, res),
+        "rmsnorm_bwd": lambda x, dy, res: K.rmsnorm_bwd(dy, x, w, rstd, res, dw_dtype=torch.bfloat16),
+        "layernorm_fwd": lambda x, dy, res: K.layernorm_fwd(x, w, b, 1e-6),
+        "layernorm_bwd": lambda x, dy, res: K.layernorm_bwd(dy, x, w, mean, lstd),
+        "bias_act_fwd": lambda x, dy, res: K.bias_act_fwd(x, b, "gelu_tanh", res),
+        "bias_act_bwd": lambda x, dy, res: K.bias_act_bwd(dy, x, b, "gelu_tanh"),
+    }
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 64), (61, 2048), (300, 1152)])
+def test_layouts(rows, cols):
+    """Columns first, rows further apart, one row for all, three dimensions, a side stream and another thread."""
+    x, dy, res, calls = _calls(rows, cols)
+    forms = {
+        "columns": lambda t: t.t().contiguous().t(),
+        "apart": lambda t: torch.cat([t, t], 1)[:, :cols],
+        "leading": lambda t: t[None],
+    }
+    for name, call in calls.items():
+        want = call(x, dy, res)
+        want = want if isinstance(want, tuple) else (want,)
+
+        def same(got, what):
+            got = got if isinstance(got, tuple) else (got,)
+            for a, b in zip(want, got):
+                assert a.dtype == b.dtype and bool((a.reshape(-1) == b.reshape(-1)).all()), (name, what)
+
+        for form, make in forms.items():
+            got = call(make(x), make(dy), make(res))
+            same(got, form)
+            first = got[0] if isinstance(got, tuple) else got
+            assert first.shape == make(x).shape and first.is_contiguous()
+        row = dy[:1].expand(rows, cols)
+        a, b = call(x, row, res), call(x, row.contiguous(), res)
+        for u, v in zip(a if isinstance(a, tuple) else (a,), b if isinstance(b, tuple) else (b,)):
+            assert bool((u == v).all()), (name, "one row for all")
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            got = call(x, dy, res)
+        torch.cuda.current_stream().wait_stream(side)
+        same(got, "side stream")
+        box = []
+        t = threading.Thread(target=lambda: (box.append(call(x, dy, res)), torch.cuda.synchronize()))
+        t.start()
+        t.join()
+        same(box[0], "thread")
