@@ -318,7 +318,7 @@ constexpr int DQ_PL = DC_C * DC_QS;      // elements of a 128-column plane
 struct DqSmem {
   static constexpr int Q = 0, K = Q + DQ_PL * 2, DO = K + DQ_PL * 2;
   static constexpr int X = DO + DQ_PL * 2;               // planes of x
-  static constexpr int W = X + 3 * DQ_PL * 2;            // planes of dx, then of S and of dS, 64 of the 128 rows at a time
+  static constexpr int W = X + 3 * DQ_PL * 2;            // planes of dx, then of S and of dS, 64 of the 128 rows at a time (`fetch_half`)
   static constexpr int DB = W + 3 * DQ_PL * 2;           // planes of T, then of db, then of R and P
   static constexpr int ROWS = DB + 6 * DQ_PT * 2;        // G, beta, 1/|k|, scale/|q|, e^G, e^(Gl-G), beta/|k|
   static constexpr int PART = ROWS + 7 * DC_C * 4;       // [6][4][64] row sums per column quarter, [2][64]
@@ -354,6 +354,11 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = __ldg(reinterpret_cast<const float4*>(src) + tid + e * NT);
   };
+  // 16 of every 32 rows of a 128-row tile, so that each half holds rows of every warp's 32 columns
+  auto fetch_half = [&](float4 (&v)[4], const float* src, int half) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = __ldg(reinterpret_cast<const float4*>(src) + tid + (2 * e + half) * NT);
+  };
   auto store = [&](__nv_bfloat16* dst, const float4 (&v)[4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -381,7 +386,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
       dc_put(sDB + (f >> 4) * DQ_T + (f & 15) * 4, DQ_PT, vt[e]);
     }
   }
-  fetch(va, St + st_at);                         // the first half of S is on its way while db is formed
+  fetch_half(va, St + st_at, 0);                 // the first half of S is on its way while db is formed
   dc_wait();
   __syncthreads();
   dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
@@ -393,10 +398,11 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     sL[tid] = expf(sG[DC_C - 1] - sG[tid]);
     sBk[tid] = sB[tid] * sRk[tid];
   }
-  // warp tile: 16 rows x 32 columns, 16 of each half of the 128
-  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 16, g = lane >> 2, t2 = (lane & 3) * 2;
+  // Warp tile: 16 rows x 32 neighbouring columns, so that a row's sums are four quarters of 32 channels.  (16 columns of each half
+  // of the 128 gave the same products but other roundings of those sums: 3e-4 in the 2-norm of a layer's bf16 gradients.)
+  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 16, c0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
   const int i0 = m0 + g, i1 = i0 + 8;
-  auto col_of = [&](int nt) { return (nt >> 1) * 64 + n0 + (nt & 1) * 8 + t2; };
+  auto col_of = [&](int nt) { return c0 + nt * 8 + t2; };
   // sums over a row's 128 channels: four lanes, then four warps (added in a fixed order at the end)
   float part[6][2];
 #pragma unroll
@@ -410,14 +416,14 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
 #pragma unroll
       for (int np = 0; np < 2; ++np) {
         uint32_t b[3][4];
-        dc_pb_t<DC_QS>(b, sW, DQ_PL, np * 64 + n0, kk * 16, lane);
+        dc_pb_t<DC_QS>(b, sW, DQ_PL, c0 + np * 16, kk * 16, lane);
         dc_mma33(acc[2 * np], a, b, 0);
         dc_mma33(acc[2 * np + 1], a, b, 2);
       }
     }
     __syncthreads();                             // dx and T are no longer read: S and db take their places
     store(sW, va);
-    fetch(va, St + st_at + 64 * DC_D);
+    fetch_half(va, St + st_at, 1);
     const float be0 = sB[i0], be1 = sB[i1];
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
@@ -512,8 +518,8 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   __syncthreads();                               // db and S are no longer read
   put_scores(false);
   // the gradient of the chunk's end state, and S once more for <dS, S>, are fetched while the score terms run
-  fetch(va, dSt + st_at + DC_D * DC_D);
-  fetch(vb, St + st_at);
+  fetch_half(va, dSt + st_at + DC_D * DC_D, 0);
+  fetch_half(vb, St + st_at, 0);
   __syncthreads();
   for (int kk = 0; kk <= mi; ++kk) {
     uint32_t ar[3][4], ap[3][4];
@@ -522,7 +528,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
 #pragma unroll
     for (int np = 0; np < 2; ++np) {
       uint32_t b[4];
-      dc_b_t(b, sK, np * 64 + n0, kk * 16, lane);
+      dc_b_t(b, sK, c0 + np * 16, kk * 16, lane);
       dc_mma31(dq[2 * np], ar, b[0], b[1]);
       dc_mma31(dq[2 * np + 1], ar, b[2], b[3]);
       dc_mma31(dk[2 * np], ap, b[0], b[1]);
@@ -546,13 +552,13 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
       dk[nt][2 * rr + 1] *= be;
     }
   }
-  float dot = 0.f;
-  auto take_ds = [&]() {                         // <dS, S> on the way in
+  float dots[8];                                 // <dS, S> on the way in, added up in the order of the rows
+  auto take_ds = [&](int half) {
     store(sW, va);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) dot += vb[e].x * va[e].x + vb[e].y * va[e].y + vb[e].z * va[e].z + vb[e].w * va[e].w;
+    for (int e = 0; e < 4; ++e) dots[2 * e + half] = vb[e].x * va[e].x + vb[e].y * va[e].y + vb[e].z * va[e].z + vb[e].w * va[e].w;
   };
-  take_ds();
+  take_ds(0);
   __syncthreads();
   // ---- k in the role of the earlier row: P^T (beta k^) + R^T q^
   {
@@ -564,8 +570,8 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
 #pragma unroll
       for (int np = 0; np < 2; ++np) {
         uint32_t bk[4], bq[4];
-        dc_b_t(bk, sK, np * 64 + n0, kk * 16, lane);
-        dc_b_t(bq, sQ, np * 64 + n0, kk * 16, lane);
+        dc_b_t(bk, sK, c0 + np * 16, kk * 16, lane);
+        dc_b_t(bq, sQ, c0 + np * 16, kk * 16, lane);
         dc_mma31(acc[2 * np], ap, bk[0], bk[1]);
         dc_mma31(acc[2 * np + 1], ap, bk[2], bk[3]);
         dc_mma31(acc[2 * np], ar, bq[0], bq[1]);
@@ -588,11 +594,11 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       if (half == 0) {
-        fetch(va, dSt + st_at + DC_D * DC_D + 64 * DC_D);
-        fetch(vb, St + st_at + 64 * DC_D);
+        fetch_half(va, dSt + st_at + DC_D * DC_D, 1);
+        fetch_half(vb, St + st_at, 1);
       } else {
         __syncthreads();
-        take_ds();
+        take_ds(1);
         __syncthreads();
       }
 #pragma unroll 2
@@ -616,6 +622,9 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
         part[5][rr] += kf.x * dk[nt][2 * rr] + kf.y * dk[nt][2 * rr + 1];
       }
   }
+  float dot = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) dot += dots[e];
   dot = warp_sum(dot);
   if (lane == 0) sRed[warp] = dot;
 #pragma unroll
