@@ -98,12 +98,15 @@ def _library_backward() -> bool:
 def _narrow(q, k, v):
     """Head widths below 128 in multiples of 8 (ViT: 72, 80), which the kernels take as they are: the loads fill the tiles' missing
     columns with zeros."""
-    return _paddable(q, k, v) and q.shape[-1] % 8 == 0 and v.shape[-1] % 8 == 0 and not _library_backward()
+    widths = q.shape[-1], v.shape[-1]
+    return _paddable(q, k, v) and min(widths) > 0 and not any(w % 8 for w in widths) and not _library_backward()
 
 
 def _rows_of_heads(t):
-    """[T, H, D] whose heads lie in a row and whose rows start on 16 bytes; copied only where they do not."""
-    if t.stride(2) != 1 or t.stride(1) != t.shape[2] or t.stride(0) % 8 or t.data_ptr() % 16:
+    """[T, H, D] whose heads lie in a row and whose rows start on 16 bytes and do not overlap; copied only where they do not.  Goes
+    by the strides: a tensor with one token or one head counts as contiguous whatever the stride of that dimension."""
+    H, D = t.shape[1:]
+    if t.stride(2) != 1 or t.stride(1) != D or t.stride(0) < H * D or t.stride(0) % 8 or t.data_ptr() % 16:
         t = t.clone(memory_format=torch.contiguous_format)
     return t
 
@@ -127,8 +130,8 @@ def _narrow_call(q, k, v, cu, max_seqlen, causal, scale, want_ml):
     dqk, dv = q.shape[-1], v.shape[-1]
     scale = scale if scale is not None else 1.0 / math.sqrt(dqk)
     if _narrow(q, k, v):
-        return FlashAttnFn.apply(_aligned(q), _aligned(k), _rows_of_heads(v), cu.cpu() if cu.is_cuda else cu, max_seqlen, causal,
-                                 float(scale), want_ml)
+        return FlashAttnFn.apply(_rows_of_heads(_aligned(q)), _rows_of_heads(_aligned(k)), _rows_of_heads(v),
+                                 cu.cpu() if cu.is_cuda else cu, max_seqlen, causal, float(scale), want_ml)
     qp, kp, vp = F.pad(q, (0, 128 - dqk)), F.pad(k, (0, 128 - dqk)), F.pad(v, (0, 128 - dv))
     res = FlashAttnFn.apply(qp, kp, vp, cu.cpu() if cu.is_cuda else cu, max_seqlen, causal, float(scale), want_ml)
     if want_ml:
