@@ -34,6 +34,23 @@ def test_against_torch(T, nq, nkv, norm):
         assert bool(((a.float() - b).abs() <= 2.0 ** -8 * b.abs() + 2.0 ** -9 * b.abs().mean()).all())
 
 
+@pytest.mark.parametrize("norm", [True, False])
+def test_value_gradients_can_be_differentiated_again(norm):
+    """The value columns are passed through, so a gradient with respect to them has a gradient of its own."""
+    T, nq, nkv, D = 9, 2, 1, 128
+    x = torch.randn(T, (nq + 2 * nkv) * D, device="cuda").bfloat16().requires_grad_(True)
+    w = torch.ones(D, device="cuda", dtype=torch.bfloat16) if norm else None
+    ang = torch.randn(T, D // 2, device="cuda")
+    _, _, v = ops.qk_norm_rope(x, nq, nkv, D, w, w, ang.cos(), ang.sin(), 1e-6)
+    first, = torch.autograd.grad(v.float().pow(3).sum(), x, create_graph=True)
+    second, = torch.autograd.grad(first.float().sum(), x)
+    vx = x.detach().float()[:, (nq + nkv) * D:]
+    assert bool((first[:, : (nq + nkv) * D] == 0).all()) and bool((second[:, : (nq + nkv) * D] == 0).all())
+    # 3 v^2 and 6 v, rounded to bf16 once
+    assert bool(((first[:, (nq + nkv) * D:].float() - 3 * vx * vx).abs() <= 2.0 ** -8 * 3 * vx * vx).all())
+    assert bool(((second[:, (nq + nkv) * D:].float() - 6 * vx).abs() <= 2.0 ** -8 * 6 * vx.abs()).all())
+
+
 def test_weight_gradients_in_fp32_repeat_bit_for_bit():
     T, nq, nkv, D = 500, 8, 2, 128
     qkv = torch.randn(T, 12 * D, device="cuda").bfloat16()

@@ -372,8 +372,12 @@ class QKNormRopeFn(torch.autograd.Function):
         qkv, wq, wk, cos, sin, rstd = ctx.saved_tensors
         n_q, n_kv, D, use_norm = ctx.dims
         dqkv = torch.empty_like(qkv)
+        # a gradient that is differentiated again: the copy of the value columns stays visible in its graph
+        graph = torch.is_grad_enabled() and dv.requires_grad
+        if graph:
+            dqkv[:, (n_q + n_kv) * D:] = dv.reshape(qkv.shape[0], n_kv * D)
         dwq, dwk = K.qknorm_rope_bwd(_aligned(dq), _aligned(dk), qkv, n_q, n_kv, D, wq, wk, cos, sin, rstd, dqkv, use_norm,
-                                     dv=_aligned(dv), dw_dtype=BF16)
+                                     dv=None if graph else _aligned(dv), dw_dtype=BF16)
         return (dqkv, None, None, None, dwq if use_norm else None, dwk if use_norm else None, None, None, None)
 
 
