@@ -57,6 +57,21 @@ def test_dense(K, M, N, Kd, a_mn, b_mn):
     assert K.status()[0] == 0
 
 
+def test_one_launch_after_another(K):
+    """Products with fewer k-blocks than stages, as many and more, whose blocks end and start beside each other: the last signals of
+    one may not reach the next."""
+    torch.manual_seed(0)
+    cases = []
+    for M, N, Kd in ((256, 128 * 128, 3072), (512, 74 * 256, 64 * 48), (304, 304, 3080), (9600, 2048, 384)):
+        a, b = _rand(M, Kd), _rand(N, Kd)
+        cases.append((a, b, K.gemm(a, b)))
+    got = [K.gemm(a, b) for _ in range(20) for a, b, _ in cases]
+    torch.cuda.synchronize()
+    assert K.status()[0] == 0
+    for i, o in enumerate(got):
+        assert torch.equal(o, cases[i % len(cases)][2])
+
+
 @pytest.mark.parametrize("M,F,Kd", [(136, 64, 3080), (300, 200, 3072), (520, 328, 3144), (300, 200, 64)])
 def test_swiglu(K, M, F, Kd):
     torch.manual_seed(F)

@@ -287,6 +287,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           if (!load_tile(g, mt, nt, bgroup)) break;
         }
+        // The leading CTA's products release the stages of both CTAs.  The last releases, which no load waits for, have to be here
+        // before this CTA may end: each stage is waited for once more (at once for one that was never used).
+        if (PAIR) {
+          for (int i = 0; i < STAGES && mbar_wait(&empty[stage], phase ^ 1, KID_GEMM, 5); ++i)
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
       }
     } else {
       // Push prologue active: the rows of A arrive from the peers while this kernel runs.  The whole warp walks the
@@ -752,7 +758,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync();     // the other CTA's products no longer read this shared memory, nor arrive on these barriers
+  // The other CTA's products no longer read this shared memory (both tiles' epilogues waited for them), and neither its commits
+  // (drained by the producer) nor its epilogue (which arrives before it gets here) has anything left to signal on these barriers.
+  if (PAIR) cluster_sync();
   if (warp == 1) {
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, 2 * BN);
