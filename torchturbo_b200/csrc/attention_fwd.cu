@@ -261,8 +261,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (!ok) break;
           if (more) issue_s(0, j & 1);
         }
-        // committed behind everything issued above
-        umma_commit_w(leader, &v_empty[vs]);
+        // committed behind everything issued above, where a later block waits for it: behind the last product of the tiles nothing
+        // may be left that signals a barrier, or it could arrive when the CTA has ended
+        if (j + n_vs < nblk) umma_commit_w(leader, &v_empty[vs]);
         if (++vs == n_vs) { vs = 0; vph ^= 1; }
         if (more) free_k();
       }
