@@ -1,5 +1,7 @@
 """The native launch functions: what they refuse, and operand layouts against contiguous operands (bit for bit)."""
+import re
 import threading
+from pathlib import Path
 
 import pytest
 import torch
@@ -19,6 +21,29 @@ def test_wrong_arguments_are_refused():
         K.host().rmsnorm_fwd(x, None, 1e-6, None, False)
     with pytest.raises(TypeError):
         K.host().rmsnorm_fwd(x, x, "eps", None, False)
+
+
+def test_declared_once():
+    """Both sides of the C interface see one declaration, so that a change of one of them alone does not compile."""
+    csrc = Path(K.__file__).parent / "csrc"
+    text = {p.name: p.read_text() for p in [*csrc.glob("*.cu"), *csrc.glob("*.cuh"), *csrc.glob("*.h"), *csrc.glob("*.cpp")]}
+    assert [name for name, t in text.items() if re.search(r"struct GemmArgs\s*\{", t)] == ["entries.h"]
+    assert '#include "entries.h"' in text["common.cuh"] and '#include "entries.h"' in text["host.cpp"]
+    declared = set(re.findall(r"\b(ttb_\w+)\(", text["entries.h"]))
+    called = set(re.findall(r"return (ttb_\w+)\(", text["host.cpp"]))
+    defined = {name for f, t in text.items() if f.endswith(".cu") for name in re.findall(r"^TTB_EXPORT int (ttb_\w+)\(", t, re.M)}
+    assert called == declared and declared <= defined and not re.search(r"\bttb_\w+\([^;{]*\);\s*$", text["host.cpp"].split("namespace {")[0], re.M)
+
+
+@pytest.mark.parametrize("flags", ["NVCC_FLAGS", "FAST_MATH", "HOST_FLAGS", "HOST_LIBS"])
+def test_built_again_when_a_flag_changes(flags, monkeypatch):
+    from torchturbo_b200.csrc import build
+
+    before = build._digest(build.sources())
+    monkeypatch.setattr(build, flags, [*getattr(build, flags), "-DOTHER"])
+    assert build._digest(build.sources()) != before
+    if flags.startswith("HOST"):
+        assert "-DOTHER" in build._host_command()
 
 
 def _calls(rows, cols):

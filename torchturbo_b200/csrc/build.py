@@ -34,6 +34,8 @@ NVCC_FLAGS = [
 # for fp32 torch operations are compiled without; -ftz alone keeps an exp2f at one instruction.
 FAST_MATH = ["--use_fast_math"]
 PRECISE = {"delta_chunk.cu": [], "delta_chunk_vec.cu": ["-ftz=true"], "gates.cu": []}
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+HOST_LIBS = ["-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch"]
 
 
 def _nvcc() -> str:
@@ -52,7 +54,7 @@ def _digest(paths: list[Path]) -> str:
     for p in sorted(paths) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [HOST_SOURCE]:
         h.update(p.name.encode())
         h.update(p.read_bytes())
-    h.update(" ".join(NVCC_FLAGS + FAST_MATH).encode())
+    h.update(" ".join(NVCC_FLAGS + FAST_MATH + HOST_FLAGS + HOST_LIBS).encode())
     h.update(repr(sorted(PRECISE.items())).encode())
     h.update(f"{torch.__version__} {sys.version}".encode())
     return h.hexdigest()
@@ -61,10 +63,9 @@ def _digest(paths: list[Path]) -> str:
 def _host_command() -> list[str]:
     inc = Path(torch.__file__).resolve().parent
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    return [os.environ.get("CXX", "g++"), *HOST_FLAGS,
             f"-I{inc}/include", f"-I{inc}/include/torch/csrc/api/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}",
-            str(HOST_SOURCE), "-o", str(HOST_PATH), f"-L{inc}/lib", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch",
-            f"-L{LIB_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN"]
+            str(HOST_SOURCE), "-o", str(HOST_PATH), f"-L{inc}/lib", *HOST_LIBS, f"-L{LIB_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> Path:

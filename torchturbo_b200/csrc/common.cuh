@@ -13,7 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#define TTB_EXPORT extern "C" __attribute__((visibility("default")))
+#include "entries.h"
 
 namespace ttb {
 

@@ -786,38 +786,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 // ----------------------------------------------------------------------------
 // Host launcher
 // ----------------------------------------------------------------------------
-struct GemmArgs {
-  const void* A;      // bf16
-  long long lda;      // elements: row stride of A's memory matrix
-  const void* B;      // bf16
-  long long ldb;      // elements: row stride of B's memory matrix
-  long long b_group_stride;  // elements between B[g] (grouped-M), 0 otherwise
-  int b_groups;       // number of B groups (>=1)
-  void* C;
-  long long ldc;
-  long long c_group_stride;
-  int M, N, K;        // grouped-K: K ignored, M = rows of A^T ( = columns of A memory ), N = cols of B memory
-  int a_mn, b_mn;     // memory orientation: 0 = K contiguous, 1 = M/N contiguous
-  int c_fp32, accumulate;
-  const void* residual;
-  long long ldr;
-  const int* tile_group;
-  int m_tiles_cap;    // grouped-M: number of m tiles to schedule (capacity)
-  const int* group_rows;
-  int groups_k;
-  long long total_rows;  // grouped-K: total rows of A/B memory matrices
-  int epi;            // 0 store, 1 swiglu
-  int F;
-  const float* row_scale;
-  void* preact;
-  long long ld_preact;
-  int num_sms;
-  const struct EpFuseArgs* ep;   // optional expert-parallel fusion (grouped-M launches only)
-  const float* alpha;            // optional device scalar multiplied into the product (plain stores only)
-  float* split_ws;               // optional fp32 [k_splits, M, N]: the product is formed in k_splits pieces, then added up
-  int k_splits;
-};
-
 // Host description of the expert-parallel fusion of one launch (C ABI; see `EpFuse` for the meaning of the fields).
 struct EpFuseArgs {
   const unsigned long long* peer_ptrs;   // [W] base address of every rank's symmetric buffer

@@ -14,57 +14,14 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include "entries.h"
+
 #include <atomic>
 #include <cmath>
 #include <string>
 
 using at::Tensor;
-
-// ---------------------------------------------------------------------------------------------
-// C entry points of libttb200.so
-// ---------------------------------------------------------------------------------------------
-struct GemmArgs {           // `struct GemmArgs` of gemm.cu
-  const void* A; long long lda;
-  const void* B; long long ldb;
-  long long b_group_stride; int b_groups;
-  void* C; long long ldc, c_group_stride;
-  int M, N, K, a_mn, b_mn, c_fp32, accumulate;
-  const void* residual; long long ldr;
-  const int* tile_group; int m_tiles_cap;
-  const int* group_rows; int groups_k;
-  long long total_rows;
-  int epi, F;
-  const float* row_scale;
-  void* preact; long long ld_preact;
-  int num_sms;
-  const void* ep;
-  const float* alpha;
-  float* split_ws;
-  int k_splits;
-};
-extern "C" {
-int ttb_gemm_bf16(const GemmArgs*, void*);
-int ttb_rmsnorm_fwd(const void*, const void*, const void*, void*, void*, float*, long long, int, float, int, void*);
-int ttb_rmsnorm_bwd(const void*, const void*, const void*, const float*, const void*, void*, float*, void*, int, long long, int, int, int, void*);
-int ttb_layernorm_fwd(const void*, const void*, const void*, void*, float*, float*, long long, int, float, void*);
-int ttb_layernorm_bwd(const void*, const void*, const void*, const float*, const float*, void*, float*, void*, int, long long, int, int, void*);
-int ttb_bias_act_fwd(const void*, const void*, const void*, void*, long long, int, int, void*);
-int ttb_bias_act_bwd(const void*, const void*, const void*, void*, float*, void*, int, long long, int, int, int, void*);
-int ttb_qknorm_rope_fwd(const void*, long long, int, int, int, const void*, const void*, const float*, const float*, void*, void*, float*, long long,
-                        float, int, void*);
-int ttb_qknorm_rope_bwd(const void*, const void*, const void*, const void*, long long, int, int, int, const void*, const void*, const float*,
-                        const float*, const float*, void*, long long, float*, void*, int, long long, int, int, void*);
-int ttb_rope(const void*, long long, long long, const float*, const float*, void*, long long, int, int, float, void*);
-int ttb_swiglu_fwd(const void*, long long, void*, long long, const float*, long long, int, const int*, void*);
-int ttb_swiglu_bwd(const void*, long long, const void*, long long, const float*, void*, long long, float*, void*, long long, long long, int, const int*,
-                   void*);
-int ttb_attn_fwd(const void*, long long, const void*, long long, const void*, long long, void*, float*, float*, const int*, int, int, long long, int, int,
-                 int, int, float, int, void*);
-int ttb_attn_bwd(const void*, const void*, long long, const void*, long long, const void*, const void*, const float*, float*, float*, float*, float*,
-                 void*, void*, void*, const int*, int, long long, int, int, int, int, float, int, int, void*);
-int ttb_attn_bwd_dq(const void*, const void*, long long, const void*, long long, const void*, const float*, const float*, void*, const int*, int,
-                    long long, int, int, int, int, float, int, void*);
-}
+using ttb::GemmArgs;
 
 namespace {
 
@@ -261,7 +218,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
       need(alpha.scalar_type() == at::kFloat && alpha.numel() == 1 && alpha.device() == a.device() && !swiglu, "alpha is one fp32 value on the device");
       g.alpha = f32(alpha);
     }
-    g.ep = reinterpret_cast<const void*>(ep);
+    g.ep = reinterpret_cast<const ttb::EpFuseArgs*>(ep);
     Tensor ws;
     int kernels = 1;
     if (K >= 4096 && !swiglu && !tile_group.defined() && !ep) {
