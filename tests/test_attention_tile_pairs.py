@@ -7,14 +7,16 @@ import torch
 from torchturbo_b200 import kernels as K
 
 
-@pytest.mark.parametrize("lens,heads,causal,rows", [
-    ([16001], 40, True, 256), ([1100, 900, 1300, 796], 32, True, 256), ([784, 816], 16, False, 256),
-    ([2048], 16, True, 128), ([8192], 4, True, 128), ([100, 100, 100], 8, True, 128), ([784], 16, False, 128),
-    ([0, 5, 0], 1, True, 128), ([], 1, True, 128),
+@pytest.mark.parametrize("lens,heads,width,causal,rows", [
+    ([16001], 40, 128, True, 256), ([1100, 900, 1300, 796], 32, 128, True, 256), ([784, 816], 16, 72, False, 256),
+    ([2048], 16, 128, True, 128), ([8192], 4, 128, True, 128), ([100, 100, 100], 8, 128, True, 128), ([784], 16, 72, False, 128),
+    ([0, 5, 0], 1, 128, True, 128), ([], 1, 128, True, 128),
+    ([784] * 5, 8, 128, False, 128), ([300] * 8, 8, 128, True, 256),        # the last wave decides
+    ([16384], 4, 128, True, 256), ([16384], 4, 192, True, 128), ([4096], 32, 192, True, 256),
 ])
-def test_query_rows_per_block(lens, heads, causal, rows):
-    """Many blocks take two tiles each; where the longest block would decide, each takes one."""
-    assert K.attn_tile_rows(lens, heads, causal, 148) == rows
+def test_query_rows_per_block(lens, heads, width, causal, rows):
+    """Many blocks take two tiles each; where the longest blocks would decide, or the last wave, each takes one."""
+    assert K.attn_tile_rows(lens, heads, causal, 148, width) == rows
 
 
 def test_pair_table_covers_the_same_rows():

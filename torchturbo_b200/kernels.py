@@ -594,28 +594,35 @@ def q_tile_rows(cu_seqlens, block: int = 128) -> list:
     return rows
 
 
-def attn_tile_rows(lens, heads: int, causal: bool, sms: int) -> int:
+def attn_tile_rows(lens, heads: int, causal: bool, sms: int, width: int = 128) -> int:
     """Query rows that a thread block of the forward kernel takes (the `block` of `build_q_tiles`): two tiles of 128 rows where
-    that fills the GPU, one where the longest block of the launch would then be what everything waits for.
+    that is faster, one where the longest blocks of the launch, or the last of their waves, would then be what everything waits for.
 
-    Compared are the estimates of both launches in thousands of clocks: the longest block against the sum of all blocks over
-    the SMs.  A kv block costs 2.05 with one query tile and 3.35 with two (16001 tokens, 40 heads: 2442 us and 2110 us), and
-    every block 8 more to start and end.  Measured, one tile / two: 8192 tokens x 4 heads 76 / 121 us, 2048 x 16 31 / 39,
-    2048 x 24 46 / 39, 2048 x 32 54 / 46, 4 documents of 4096 x 32 82 / 68; full attention, 784 tokens x 16 heads 17 / 23,
-    two such documents 29 / 25."""
+    Compared are the estimates of both launches in thousands of clocks, the larger of two bounds: the work of an SM, and, since of
+    the j * sms + 1 longest blocks one SM takes j + 1, that many times the shortest of these.  A kv block and a thread block cost,
+    with one query tile and with two, 2.05 + 8 and 3.2 + 8 for query / key heads up to 128 wide, 2.05 + 10 and 3.8 + 9 for 192 (half
+    as much again for the scores, and one V stage when both tiles are there).  Fitted to 680 measured launches (widths 64, 72, 128
+    and 192, one to 32 documents of 17 to 16384 tokens, 1 to 128 heads): of what the better of the two takes the choice loses 0.1 %
+    on average.  One tile / two in us: 16001 tokens x 40 heads 3383 / 2795, 192 wide 3346 / 3397; 8192 x 8 148 / 128, 192 wide
+    150 / 147; 16384 x 4, 192 wide 285 / 299; 2048 x 16 26 / 34; 5 documents of 784 x 8, full attention 26 / 31 (160 longer blocks
+    are two waves on 148 SMs, as are 280 shorter ones); 8 of 300 x 8 14 / 10."""
+    per_kv, per_block = ((2.05, 3.2), (8.0, 8.0)) if width <= 128 else ((2.05, 3.8), (10.0, 9.0))
 
-    def launch(step: int, per_block: float) -> float:
-        longest = total = 0.0
+    def launch(step: int) -> float:
+        cost, start = per_kv[step - 1], per_block[step - 1]
+        blocks, of = [], {}                                          # of one head; of a document with so many tiles
         for n in lens:
             tiles = (n + 127) // 128
-            entries = (tiles + step - 1) // step
-            # entry i of a causal document sees min(step (i + 1), tiles) blocks, each entry of a full one all of them
-            blocks = step * entries * (entries - 1) // 2 + tiles if causal and tiles else entries * tiles
-            total += blocks * per_block + 8.0 * entries
-            longest = max(longest, tiles * per_block + 8.0)
-        return max(longest, total * heads / sms)
+            if tiles not in of:
+                # entry i of a causal document sees min(step (i + 1), tiles) kv blocks, each entry of a full one all of them
+                seen = range(step, tiles + step, step) if causal else [tiles] * ((tiles + step - 1) // step)
+                of[tiles] = [min(kv, tiles) * cost + start for kv in seen]
+            blocks += of[tiles]
+        blocks.sort(reverse=True)
+        waves = [(j + 1) * blocks[first // heads] for j, first in enumerate(range(0, len(blocks) * heads, sms))]
+        return max(sum(blocks) * heads / sms, *waves, 0.0)
 
-    return 256 if launch(2, 3.35) < launch(1, 2.05) else 128
+    return 256 if launch(2) < launch(1) else 128
 
 
 def _covered(rows) -> tuple[int, int]:

@@ -32,10 +32,10 @@ class _Tiles:
         self.lens = [max(b - a, 0) for a, b in zip(offs[:-1], offs[1:])]
         self._tile_rows: dict = {}
 
-    def tile_rows(self, heads: int, causal: bool) -> int:
-        key = (heads, causal)
+    def tile_rows(self, heads: int, causal: bool, width: int) -> int:
+        key = (heads, causal, width > 128)
         if key not in self._tile_rows:
-            self._tile_rows[key] = K.attn_tile_rows(self.lens, heads, causal, K.num_sms(self.cu.device.index))
+            self._tile_rows[key] = K.attn_tile_rows(self.lens, heads, causal, K.num_sms(self.cu.device.index), width)
         return self._tile_rows[key]
 
 
@@ -49,7 +49,7 @@ class FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens, max_seqlen, causal, scale, want_ml):
         tiles = _tiles_for(cu_seqlens, q.device)
-        block = tiles.tile_rows(q.shape[1], causal)
+        block = tiles.tile_rows(q.shape[1], causal, q.shape[2])
         out, lse, ml = K.attn_fwd(q, k, v, tiles.q[block], scale=scale, causal=causal, want_max_logit=want_ml, rows=tiles.rows,
                                   tile_rows=block)
         ctx.save_for_backward(q, k, v, out, lse)
