@@ -77,7 +77,75 @@ def test_both_tile_counts(rows, causal, D, Hq, Hk, rising):
     bound = 2.0 ** -8 * (mag + ref.abs()) + 1e-4 * mag + 1e-6
     assert ((out.float() - ref).abs() <= bound)[: cu[-1]].all()
     assert (lse[:, : cu[-1]] - ref_lse[:, : cu[-1]]).abs().max() < 1e-4 * max(1.0, float(ref_lse[:, : cu[-1]].abs().max()))
-    top = max(float((q[a:b].float().transpose(0, 1) @ k[a:b].float().repeat_interleave(Hq // Hk, 1).permute(1, 2, 0) * scale)
-                    .masked_fill(torch.ones(b - a, b - a, dtype=torch.bool, device="cuda").triu(1) & causal, -math.inf).max())
-              for a, b in zip(cu[:-1], cu[1:]))
-    assert abs(float(ml.max()) - top) <= 1e-4 * max(1.0, abs(top))
+    top = torch.stack([(q[a:b].float().transpose(0, 1) @ k[a:b].float().repeat_interleave(Hq // Hk, 1).permute(1, 2, 0) * scale)
+                       .masked_fill(torch.ones(b - a, b - a, dtype=torch.bool, device="cuda").triu(1) & causal, -math.inf).amax((1, 2))
+                       for a, b in zip(cu[:-1], cu[1:])]).amax(0)
+    assert ml.shape == (Hq,) and bool(((ml - top).abs() <= 1e-4 * top.abs().clamp(min=1.0)).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [128, 256])
+@pytest.mark.parametrize("D", [128, 192])
+def test_maximum_in_any_tile(rows, D):
+    """The per-head maximum logit, placed in the first tile of a pair, in the second, and in a document's last rows."""
+    T, H, scale = 700, 6, D ** -0.5
+    g = torch.Generator("cuda").manual_seed(D)
+    q, k, v = (torch.randn(T, H, d, generator=g, device="cuda").bfloat16() for d in (D, D, 128))
+    for h, t in enumerate((0, 127, 128, 255, 384, 699)):
+        q[t, h] = k[t, h] * 4
+    cu = torch.tensor([0, T], dtype=torch.int32)
+    _, _, ml = K.attn_fwd(q, k, v, K.build_q_tiles(cu, rows).cuda(), scale=scale, causal=True, want_max_logit=True, rows=(0, T), tile_rows=rows)
+    top = (q.float().transpose(0, 1) @ k.float().permute(1, 2, 0) * scale).masked_fill(
+        torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), -math.inf).amax((1, 2))
+    assert bool(((ml - top).abs() <= 1e-4 * top.abs()).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [128, 256])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("D", [72, 128, 192])
+def test_longer_documents(rows, causal, D):
+    """More blocks than stages many times over, and a last entry of one tile or of two, the second of them cut."""
+    lens, H, Dv = [2048 + 3, 1664, 2304 + 200], 2, min(D, 128)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    g = torch.Generator("cuda").manual_seed(D + rows)
+    q, k, v = (torch.randn(cu[-1], H, d, generator=g, device="cuda").bfloat16() for d in (D, D, Dv))
+    scale = D ** -0.5
+    out, lse, _ = K.attn_fwd(q, k, v, K.build_q_tiles(torch.tensor(cu, dtype=torch.int32), rows).cuda(), scale=scale, causal=causal,
+                             rows=(0, cu[-1]), tile_rows=rows)
+    torch.cuda.synchronize()
+    assert K.attn_status()[0] == 0
+    ref, mag, ref_lse = _reference(q, k, torch.nn.functional.pad(v, (0, 128 - Dv)), cu, causal, scale)
+    ref, mag = ref[..., :Dv], mag[..., :Dv]
+    assert bool(((out.float() - ref).abs() <= 2.0 ** -8 * (mag + ref.abs()) + 1e-4 * mag + 1e-6).all())     # as above
+    assert (lse - ref_lse).abs().max() < 1e-4 * float(ref_lse.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [128, 192])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
+def test_values_that_are_not_finite(D, where, value):
+    """One element that is not finite spoils the rows that see it, and no other, with one query tile per block and with two."""
+    T, H, scale, at = 900, 2, D ** -0.5, 300
+    g = torch.Generator("cuda").manual_seed(D)
+    args = {n: torch.randn(T, H, d, generator=g, device="cuda").bfloat16() for n, d in (("q", D), ("k", D), ("v", 128))}
+    clean = {n: t.clone() for n, t in args.items()}
+    args[where][at, 1, 5] = value
+    cu = torch.tensor([0, 256, T], dtype=torch.int32)
+    got = {}
+    for rows in (128, 256):
+        table = K.build_q_tiles(cu, rows).cuda()
+        got[rows], ok = (K.attn_fwd(*(t[n] for n in "qkv"), table, scale=scale, causal=True, rows=(0, T), tile_rows=rows)[0].float()
+                         for t in (args, clean))
+        torch.cuda.synchronize()
+        assert K.attn_status()[0] == 0
+        touched = torch.zeros(T, H, dtype=torch.bool, device="cuda")
+        touched[at: at + 1 if where == "q" else T, 1] = True
+        if where == "v":      # the row block of the key at hand multiplies it by zero as well: 0 x inf is not a number
+            touched[256:, 1] = True
+        assert torch.equal(got[rows][~touched], ok[~touched])
+    assert bool(((got[128] == got[256]) | (got[128].isnan() & got[256].isnan())).all())
+    assert not bool(got[256][at:, 1].isfinite().all())

@@ -50,6 +50,11 @@ def test_dense(K, M, N, Kd, a_mn, b_mn):
     assert float((out - (base + ref)).abs().max()) <= _sum_error(Kd) + 2.0 ** -15       # and one rounding of a sum below 512
     res = _rand(M, N)
     _check(K.gemm(*args, residual=res, **kw), ref + res.double(), Kd)
+    half = torch.tensor([-0.375], device="cuda")
+    _check(K.gemm(*args, alpha=half, **kw), -0.375 * ref, Kd)
+    out = base.clone()
+    K.gemm(*args, out=out, accumulate=True, alpha=half, **kw)
+    assert float((out - (base - 0.375 * ref)).abs().max()) <= _sum_error(Kd) + 2.0 ** -15
     wide = torch.full((M, N + 16), 7.0, device="cuda", dtype=torch.bfloat16)     # rows further apart: nothing beside them is written
     K.gemm(*args, out=wide[:, :N], **kw)
     _check(wide[:, :N], ref, Kd)
