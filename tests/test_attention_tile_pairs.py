@@ -19,6 +19,17 @@ def test_query_rows_per_block(lens, heads, width, causal, rows):
     assert K.attn_tile_rows(lens, heads, causal, 148, width) == rows
 
 
+def test_benchmark_takes_the_table_of_the_operator(monkeypatch):
+    from torchturbo_b200.benchmarks import attention_bench
+
+    monkeypatch.setattr(K, "num_sms", lambda *_: 148)
+    monkeypatch.setattr(torch.Tensor, "cuda", lambda self: self)
+    cu = torch.tensor([0, 1000, 4000, 8192], dtype=torch.int32)
+    for heads, width, rows in ((32, 128, 256), (1, 128, 128), (1, 192, 128)):
+        table = attention_bench._forward_table(cu, [1000, 3000, 4192], heads, width)
+        assert table["tile_rows"] == rows and torch.equal(table["q_tiles_dev"], K.build_q_tiles(cu, rows)) and table["rows"] == (0, 8192)
+
+
 def test_pair_table_covers_the_same_rows():
     cu = torch.tensor([3, 3, 4, 260, 516, 773, 1000], dtype=torch.int32)
     one, two = (K.build_q_tiles(cu, b).tolist() for b in (128, 256))

@@ -9,6 +9,12 @@ from .. import kernels as K
 from .kernel_bench import peaks, time_fn
 
 
+def _forward_table(cu, docs, heads, width):
+    """The query rows per block that the operator chooses for this batch, and the table for it."""
+    block = K.attn_tile_rows(docs, heads, True, K.num_sms(), width)
+    return dict(q_tiles_dev=K.build_q_tiles(cu, block).cuda(), tile_rows=block, rows=(0, sum(docs)))
+
+
 def bench_attention():
     pk = peaks()
     rows = []
@@ -21,8 +27,9 @@ def bench_attention():
         cu = torch.tensor([0] + list(torch.tensor(docs).cumsum(0)), dtype=torch.int32)
         tiles = K.build_q_tiles(cu).cuda()
         fl = sum(4.0 * L * L * Hq * D / 2 for L in docs)
-        t, _ = time_fn(lambda: K.attn_fwd(q, k, v, tiles, scale=D ** -0.5, causal=True))
-        row = dict(op="attn_fwd_causal", T=T, Hq=Hq, Hk=Hk, docs=docs, ms=t, tflops=fl / t / 1e9,
+        fwd = _forward_table(cu, docs, Hq, D)
+        t, _ = time_fn(lambda: K.attn_fwd(q, k, v, scale=D ** -0.5, causal=True, **fwd))
+        row = dict(op="attn_fwd_causal", T=T, Hq=Hq, Hk=Hk, docs=docs, tile_rows=fwd["tile_rows"], ms=t, tflops=fl / t / 1e9,
                    frac_of_peak=fl / t / 1e9 / pk["tflops"], peak_src=pk["src"])
         try:
             from flash_attn import flash_attn_varlen_func
@@ -37,7 +44,7 @@ def bench_attention():
         rows.append(row)
         print(json.dumps(row), flush=True)
         # backward: the whole call (row dot products, the tcgen05 kernel, fp32 -> bf16 casts of dQ / dK / dV)
-        out, lse, _ = K.attn_fwd(q, k, v, tiles, scale=D ** -0.5, causal=True)
+        out, lse, _ = K.attn_fwd(q, k, v, scale=D ** -0.5, causal=True, **fwd)
         dout = torch.randn_like(out)
         kv_tiles = K.build_kv_tiles(cu).cuda()
         tb, _ = time_fn(lambda: K.attn_bwd(dout, q, k, v, out, lse, kv_tiles, scale=D ** -0.5, causal=True))
@@ -69,11 +76,12 @@ def bench_attention():
         tiles, kv_tiles = K.build_q_tiles(cu).cuda(), K.build_kv_tiles(cu).cuda()
         fl = sum(2.0 * L * L * H * (192 + 128) / 2 for L in docs)
         sc = 192 ** -0.5
-        t, _ = time_fn(lambda: K.attn_fwd(q, k, v, tiles, scale=sc, causal=True))
-        out, lse, _ = K.attn_fwd(q, k, v, tiles, scale=sc, causal=True)
+        fwd = _forward_table(cu, docs, H, 192)
+        t, _ = time_fn(lambda: K.attn_fwd(q, k, v, scale=sc, causal=True, **fwd))
+        out, lse, _ = K.attn_fwd(q, k, v, scale=sc, causal=True, **fwd)
         dout = torch.randn_like(out)
         tb, _ = time_fn(lambda: K.attn_bwd(dout, q, k, v, out, lse, kv_tiles, scale=sc, causal=True, q_tiles_dev=tiles))
-        row = dict(op="mla_attn_fwd_bwd_causal", T=T, H=H, docs=docs, fwd_ms=t, bwd_ms=tb, fwd_tflops=fl / t / 1e9,
+        row = dict(op="mla_attn_fwd_bwd_causal", T=T, H=H, docs=docs, tile_rows=fwd["tile_rows"], fwd_ms=t, bwd_ms=tb, fwd_tflops=fl / t / 1e9,
                    bwd_tflops=2.5 * fl / tb / 1e9, fwd_frac_of_peak=fl / t / 1e9 / pk["tflops"],
                    bwd_frac_of_peak=2.5 * fl / tb / 1e9 / pk["tflops"], peak_src=pk["src"])
         try:
