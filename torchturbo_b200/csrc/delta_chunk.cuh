@@ -17,16 +17,16 @@
 // never to the bf16 inputs.  Two terms and three products on both-fp32 products left dg 4 to 14 and dbeta 13 to 16 times as
 // far from 64 bits as fp32 products; now dbeta, gx and gS are closer than those and dg within 1.5 times of them.
 //
-// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.15 ms, out 0.13, bwd_pre 0.09, bwd_post 0.57 (0.60
+// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.15 ms, out 0.13, bwd_pre 0.09, bwd_post 0.58 (0.60
 // when every warp split again the fp32 tiles that it shares with three others); with two-term operands and sums kept in the tensor
 // cores' accumulators 0.14, 0.11, 0.09 and 0.45.  A gated-delta-net layer forward + backward takes 2.5 ms, against 10.4 when the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and
 // gathers over materialised [chunk, 64, 64 .. 128] tensors.
 //
 // Why mma.sync and not tcgen05: the products are 64 x 64 x 128 at most, each feeds the next through registers and shared
 // memory, and their operands are built element by element (splits, decays).  What bounds them, from the counters of the same
-// case: bwd_post moves 0.69 GB (0.11 ms at the copy rate) and kept the tensor pipe 33 % active with 12,000 mma.sync per chunk
-// and head before its planes; one CTA of 16 warps filled 43 % of the issue slots, and its warps waited for the tensor pipe, for results of their own
-// instructions, at barriers between the phases and for loads in similar shares.  out and prep: tensor pipe 30 and 14 %, issue
+// case: bwd_post moves 0.69 GB (0.11 ms at the copy rate) and keeps the tensor pipe 34 % active with 12,000 mma.sync per chunk
+// and head; one CTA of 16 warps fills 29 % of the issue slots (43 before its planes), and its warps wait for the tensor pipe, for
+// results of their own instructions, at barriers between the phases and for loads in similar shares.  out and prep: tensor pipe 30 and 14 %, issue
 // slots 49 and 44 %, traffic a third and a quarter of their time.  So neither memory nor the tensor pipe is full: it is the chain
 // of phases on one CTA per SM.  That splitting once took only 4 % off bwd_post says the same.
 #pragma once
