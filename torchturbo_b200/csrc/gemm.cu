@@ -67,6 +67,18 @@ struct EpFuse {
   int ret_rows;               // rows of every rank's return buffer (tags at or past it are refused)
 };
 
+// n / d for 0 <= n < 2^31 by a multiplication: with 2^s >= d and m = ceil(2^(31 + s) / d), m d exceeds 2^(31 + s) by less than 2^s, so
+// that n m / 2^(31 + s) stays below the next whole number.
+struct FastDiv {
+  uint32_t mul, shift;
+  __device__ __forceinline__ int operator()(int n) const { return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> shift); }
+};
+static FastDiv fast_div(int d) {
+  uint32_t s = 0;
+  while ((1ull << s) < static_cast<uint64_t>(d)) ++s;
+  return FastDiv{static_cast<uint32_t>(((1ull << (31 + s)) + d - 1) / d), 31 + s};
+}
+
 struct GemmParams {
   EpFuse ep;
   int M, N, K;   // per-problem extents (N = output columns; for SwiGLU N = F)
@@ -86,6 +98,8 @@ struct GemmParams {
   __nv_bfloat16* preact;  // optional [M, ld_preact] receives gate|up
   long long ld_preact;
   const float* alpha;     // optional device scalar multiplied into the product (plain stores)
+  int tma_out;            // plain bf16 rows: stored by the copy engine through the map of C
+  FastDiv by_group, by_band, by_rest;   // tile counts: of a group, of a whole band, rows of the last band
   int k_splits, kb_per_split;  // > 1: "group" g covers k-blocks [g, g + 1) * kb_per_split of one product, stored at C[g]
 };
 
@@ -121,7 +135,8 @@ __device__ __forceinline__ uint32_t epi_piece_addr64(uint32_t base, int row, int
 
 template <int BN, bool A_MN, bool B_MN, int EPI, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS_PUSH, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+            const GemmParams p) {
   using L = SmemLayout<BN, PAIR>;
   constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -185,26 +200,40 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // its n-tiles are walked (an m-fastest walk over all m-tiles re-read A from DRAM once per n-tile column).
   // A pair's tile has 256 rows, so its bands have half as many; `mt` is the 128-row tile of this CTA.
   constexpr int RASTER_M = PAIR ? 8 : 16;
-  auto decode = [&](int t, int& g, int& mt, int& nt) {
-    g = t / tiles_per_group;
-    const int r = t - g * tiles_per_group;
-    const int per_band = RASTER_M * p.n_tiles;
-    const int band = r / per_band;
-    const int m_base = band * RASTER_M;
-    const int band_rows = (p.m_tiles - m_base) < RASTER_M ? (p.m_tiles - m_base) : RASTER_M;
-    const int w = r - band * per_band;
-    nt = w / band_rows;
-    mt = m_base + w - nt * band_rows;
-    if (PAIR) mt = 2 * mt + rank;
+  // What a tile reads from memory (its expert, or the row range of its group) is asked for a tile ahead: a tile of a grouped weight
+  // gradient at 256 rows an expert is 2600 clocks of products, and the load in front of them was 400 to 800.
+  struct Tile {
+    int g, mt, nt;    // mt: 128-row tile of this CTA
+    int a, b;         // grouped-M: a = expert; grouped-K: row range
   };
+  auto fetch = [&](int t) {
+    Tile x{0, 0, 0, 0, 0};
+    if (t >= total_tiles) return x;
+    x.g = p.by_group(t);
+    const int r = t - x.g * tiles_per_group;
+    const int band = p.by_band(r);
+    const int m_base = band * RASTER_M;
+    const int w = r - band * RASTER_M * p.n_tiles;
+    const int left = p.m_tiles - m_base;
+    x.nt = left < RASTER_M ? p.by_rest(w) : w / RASTER_M;
+    x.mt = m_base + w - x.nt * (left < RASTER_M ? left : RASTER_M);
+    if (PAIR) x.mt = 2 * x.mt + rank;
+    if (p.tile_group) {
+      x.a = __ldg(p.tile_group + x.mt);
+    } else if (p.groups_k > 0) {
+      x.a = __ldg(p.group_rows + x.g);
+      x.b = __ldg(p.group_rows + x.g + 1);
+    }
+    return x;
+  };
+  auto unused = [&](const Tile& x) { return p.tile_group != nullptr && x.a < 0; };
   // k-range of a tile: dense -> [0, K); split -> its share of [0, K); grouped-K -> rows of group g.
-  auto krange = [&](int g, int& k0, int& nkb) {
+  auto krange = [&](const Tile& x, int& k0, int& nkb) {
     if (p.groups_k > 0) {
-      int r0 = p.group_rows[g], r1 = p.group_rows[g + 1];
-      k0 = r0;
-      nkb = (r1 - r0) / BK;
+      k0 = x.a;
+      nkb = (x.b - x.a) / BK;
     } else if (p.k_splits > 1) {
-      const int kb0 = g * p.kb_per_split;
+      const int kb0 = x.g * p.kb_per_split;
       k0 = kb0 * BK;
       nkb = min(p.kb_per_split, (p.K + BK - 1) / BK - kb0);
     } else {
@@ -218,11 +247,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     int stage = 0;
     uint32_t phase = 0;
     // all k-blocks of one tile; run by one thread
-    auto load_tile = [&](int g, int mt, int nt, int bgroup) -> bool {
+    auto load_tile = [&](const Tile& x) -> bool {
       int k0, nkb;
-      krange(g, k0, nkb);
-      const int m0 = mt * BM;
-      const int n0 = nt * (EPI == EPI_SWIGLU ? BN / 2 : BN);
+      krange(x, k0, nkb);
+      const int m0 = x.mt * BM;
+      const int n0 = x.nt * (EPI == EPI_SWIGLU ? BN / 2 : BN);
+      const int bgroup = p.tile_group ? x.a : 0;
       for (int kb = 0; kb < nkb; ++kb) {
         if (!mbar_wait(&empty[stage], phase ^ 1, KID_GEMM, 1)) return false;
         uint8_t* sa = smem + stage * L::STAGE_BYTES;
@@ -277,15 +307,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       if (elect_one()) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        for (int t = walker; t < total_tiles; t += walkers) {
-          int g, mt, nt;
-          decode(t, g, mt, nt);
-          int bgroup = 0;
-          if (p.tile_group) {
-            bgroup = p.tile_group[mt];
-            if (bgroup < 0) continue;
-          }
-          if (!load_tile(g, mt, nt, bgroup)) break;
+        Tile x = fetch(walker), next;
+        for (int t = walker; t < total_tiles; t += walkers, x = next) {
+          next = fetch(t + walkers);
+          if (!unused(x) && !load_tile(x)) break;
         }
         // The leading CTA's products release the stages of both CTAs.  The last releases, which no load waits for, have to be here
         // before this CTA may end: each stage is waited for once more (at once for one that was never used).
@@ -305,9 +330,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const int* my_flags = reinterpret_cast<const int*>(p.ep.peers.base[p.ep.rank] + p.ep.off_flags);
       bool ok = true;
       for (int t = walker; t < total_tiles && ok; t += walkers) {
-        int g, mt, nt;
-        decode(t, g, mt, nt);
-        const int bgroup = p.tile_group[mt];
+        const Tile x = fetch(t);
+        const int bgroup = x.a;
         if (bgroup < 0) continue;
         if (!((s_landed[bgroup >> 5] >> (bgroup & 31)) & 1u)) {
           bool mine = true;
@@ -320,7 +344,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
         if (lane == 0) {
           fence_proxy_async_all();
-          ok = load_tile(g, mt, nt, bgroup);
+          ok = load_tile(x);
         }
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       }
@@ -337,11 +361,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = walker; t < total_tiles && ok; t += walkers) {
-        int g, mt, nt, k0, nkb;
-        decode(t, g, mt, nt);
-        if (p.tile_group && p.tile_group[mt] < 0) continue;
-        krange(g, k0, nkb);
+      Tile x = fetch(walker), next;
+      for (int t = walker; t < total_tiles && ok; t += walkers, x = next) {
+        int k0, nkb;
+        next = fetch(t + walkers);
+        if (unused(x)) continue;
+        krange(x, k0, nkb);
         if (!mbar_wait(&tempty[acc], acc_phase ^ 1, KID_GEMM, 2)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
@@ -376,53 +401,115 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (int t = walker; t < total_tiles && ok; t += walkers) {
-      int g, mt, nt, k0, nkb;
-      decode(t, g, mt, nt);
-      if (p.tile_group && p.tile_group[mt] < 0) continue;
-      krange(g, k0, nkb);
-      if (!mbar_wait(&tfull[acc], acc_phase, KID_GEMM, 4, consumer_budget)) { ok = false; break; }
-      tc_fence_after();
-      const int row = mt * BM + lane_group * 32 + lane;
+    Tile x = fetch(walker), next;
+    for (int t = walker; t < total_tiles && ok; t += walkers, x = next) {
+      int k0, nkb;
+      next = fetch(t + walkers);
+      if (unused(x)) continue;
+      krange(x, k0, nkb);
+      const int g = x.g, nt = x.nt;
+      const int row_base = x.mt * BM + lane_group * 32;
+      const int row = row_base + lane;
       const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(lane_group * 32) << 16);
+      const long long gbase = static_cast<long long>(g) * p.c_group_stride;
+      if (!mbar_wait(&tfull[acc], acc_phase, KID_GEMM, 4, consumer_budget)) { ok = false; break; }
+      tc_fence_after();
+      auto release = [&]() {      // the accumulator has been read
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_cluster(leader_addr(&tempty[acc]));
+          else mbar_arrive(&tempty[acc]);
+        }
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      };
 
+      if (EPI == EPI_STORE && p.tma_out) {
+        // Plain bf16 rows, 64 columns at a time: parked as bf16 (128 bytes a row, the copy engine's swizzle) and handed to the copy
+        // engine, which clips at the edges of C.  An SM's ordinary stores leave at 32 bytes a clock however they are shaped, and a warp
+        // that issues them waits: 2500 clocks of a tile's epilogue, which was 5000 with the decoding of the tile, against 2600 of
+        // products for a grouped weight gradient at 256 rows an expert.  Before -> now: 128 of those, 2048 x 1536 and 768 x 2048,
+        // 305 -> 282 and 157 -> 148 us (805 MB of results: 268 us at the 3.0 TB/s that a plain fill writes); 3000 x 4304 x 1152
+        // 31 -> 27; 2048^3 18.6 -> 17; 300 x 2048 x 512 10.4 -> 8.5.
+        constexpr int CH = BN / 32 / (EPI_WARPS / 4);
+        const float alpha = p.alpha ? __ldg(p.alpha) : 1.f;
+        uint8_t* stage_at = epi_stage + (warp - 2) * L::EPI_STAGE_BYTES;
+        const uint32_t st = smem_u32(stage_at);
+        const int first = nt * BN + col_half * CH * 32;
+        bool held = true;
+#pragma unroll 1
+        for (int c = 0; c < CH; c += 2) {
+          const int col0 = first + c * 32;
+          if (col0 >= p.N || row_base >= p.M) break;      // uniform across the warp
+          uint32_t v[2][32];
+          if (nkb > 0) {
+            tmem_ld_32x32b_x32(t_row + (col_half * CH + c) * 32, v[0]);
+            tmem_ld_32x32b_x32(t_row + (col_half * CH + c) * 32 + 32, v[1]);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 64; ++i) v[i >> 5][i & 31] = 0u;
+          }
+          if (c + 2 >= CH) {
+            release();
+            held = false;
+          }
+          if (p.alpha) {
+#pragma unroll
+            for (int i = 0; i < 64; ++i) v[i >> 5][i & 31] = __float_as_uint(__uint_as_float(v[i >> 5][i & 31]) * alpha);
+          }
+          if (lane == 0) bulk_wait_read_all();      // the copy engine has read what was parked before
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int y = (8 * i + 2 * e) & 31;
+              w[e] = pack_bf16(__uint_as_float(v[i >> 2][y]), __uint_as_float(v[i >> 2][y + 1]));
+            }
+            st_shared_v4(epi_piece_addr(st, lane, i), w[0], w[1], w[2], w[3]);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmC, stage_at, col0, row_base, g);
+            bulk_commit_group();
+          }
+        }
+        if (held) release();
+        continue;
+      }
       if (EPI == EPI_STORE) {
         const int n0 = nt * BN;
         uint8_t* cbase = reinterpret_cast<uint8_t*>(p.C);
-        const long long coff = static_cast<long long>(g) * p.c_group_stride + static_cast<long long>(row) * p.ldc;
-        // bf16 output: first element of the four rows this lane stores in the row-major pass (null = skip the row).
-        // With the scatter epilogue a row goes to the rank it came from, at the entry its tag names.
-        __nv_bfloat16* rowptr[4] = {nullptr, nullptr, nullptr, nullptr};
-        if (!p.c_fp32) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int rr = mt * BM + lane_group * 32 + (lane >> 2) + 8 * j;
-            if (rr >= p.M) continue;
-            if (p.ep.scat_on) {
-              const int tag = __ldcg(p.ep.row_tag + rr);
-              if (tag >= 0) {
-                // a tag that names no rank or no entry (rows that never landed) must not become an address
-                if ((tag >> EP_TAG_SHIFT) < p.ep.W && (tag & EP_TAG_MASK) < p.ep.ret_rows)
-                  rowptr[j] = reinterpret_cast<__nv_bfloat16*>(p.ep.peers.base[tag >> EP_TAG_SHIFT] + p.ep.off_ret) +
-                              static_cast<long long>(tag & EP_TAG_MASK) * p.ldc;
-                else
-                  atomicCAS(p.ep.status, 0, 3);
-              }
-            } else {
-              rowptr[j] = reinterpret_cast<__nv_bfloat16*>(cbase) + static_cast<long long>(g) * p.c_group_stride +
-                          static_cast<long long>(rr) * p.ldc;
-            }
-          }
-          if (p.ep.scat_on && p.ep.row_val && nt == 0 && col_half == 0 && row_ok) {
-            const int tag = __ldcg(p.ep.row_tag + row);
-            if (tag >= 0 && (tag >> EP_TAG_SHIFT) < p.ep.W && (tag & EP_TAG_MASK) < p.ep.ret_rows)
-              reinterpret_cast<float*>(p.ep.peers.base[tag >> EP_TAG_SHIFT] + p.ep.off_ret_vals)[tag & EP_TAG_MASK] =
-                  p.ep.row_val[row];
-          }
-        }
+        const long long coff = gbase + static_cast<long long>(row) * p.ldc;
         constexpr int CH = BN / 32 / (EPI_WARPS / 4);
         const float alpha = p.alpha ? __ldg(p.alpha) : 1.f;
+        const uint32_t st = smem_u32(epi_stage + (warp - 2) * L::EPI_STAGE_BYTES);
+        // first element of output row `rr` (null = skip it); with the scatter epilogue a row goes to the rank it came from, at the
+        // entry its tag names
+        auto tag_of = [&](int rr) { return rr < p.M ? (p.ep.scat_on ? __ldcg(p.ep.row_tag + rr) : 0) : -1; };
+        auto row_dst = [&](int rr, int tag) -> __nv_bfloat16* {
+          if (tag < 0) return nullptr;
+          if (!p.ep.scat_on) return reinterpret_cast<__nv_bfloat16*>(cbase) + gbase + static_cast<long long>(rr) * p.ldc;
+          // a tag that names no rank or no entry (rows that never landed) must not become an address
+          if ((tag >> EP_TAG_SHIFT) < p.ep.W && (tag & EP_TAG_MASK) < p.ep.ret_rows)
+            return reinterpret_cast<__nv_bfloat16*>(p.ep.peers.base[tag >> EP_TAG_SHIFT] + p.ep.off_ret) +
+                   static_cast<long long>(tag & EP_TAG_MASK) * p.ldc;
+          atomicCAS(p.ep.status, 0, 3);
+          return nullptr;
+        };
+        if (p.ep.scat_on && p.ep.row_val && nt == 0 && col_half == 0 && row_ok) {
+          const int tag = __ldcg(p.ep.row_tag + row);
+          if (tag >= 0 && (tag >> EP_TAG_SHIFT) < p.ep.W && (tag & EP_TAG_MASK) < p.ep.ret_rows)
+            reinterpret_cast<float*>(p.ep.peers.base[tag >> EP_TAG_SHIFT] + p.ep.off_ret_vals)[tag & EP_TAG_MASK] =
+                p.ep.row_val[row];
+        }
+        int tag[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) tag[j] = tag_of(row_base + (lane >> 2) + 8 * j);
 #pragma unroll 1
         for (int c = col_half * CH; c < (col_half + 1) * CH; ++c) {
           const int col0 = n0 + c * 32;
@@ -441,79 +528,67 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           const bool full_chunk = (col0 + 32 <= p.N);
           if (full_chunk) {
-            // warp-uniform branch: every lane takes part in the transposition, rows past M are skipped on the way out
-            const uint32_t st = smem_u32(epi_stage + (warp - 2) * L::EPI_STAGE_BYTES);
+            // warp-uniform branch: every lane takes part in the transposition, rows past M are skipped on the way out; what
+            // is added and the parked rows are read ahead of the first store (sums into an fp32 gradient of 128 experts, 2048 x
+            // 1536 of 256 rows each: 1965 -> 822 us; every store waited for its own two loads before)
             __syncwarp();  // the previous chunk's readers are done with the staging area
-            if (!p.c_fp32 && !p.residual && !p.accumulate) {
-              // nothing is added in fp32: the chunk is parked as bf16, half the shared-memory traffic (grouped weight gradients,
-              // whose tiles are mostly epilogue, 342 -> 287 and 185 -> 150 us for 128 experts of 256 rows, 2048 x 1536 and 768 x 2048)
-              const int q = lane & 3;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                uint32_t w[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) w[e] = pack_bf16(__uint_as_float(v[8 * i + 2 * e]), __uint_as_float(v[8 * i + 2 * e + 1]));
-                st_shared_v4(epi_piece_addr64(st, lane, i), w[0], w[1], w[2], w[3]);
-              }
-              __syncwarp();
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                if (rowptr[j] == nullptr) continue;
-                uint4 w;
-                ld_shared_v4(epi_piece_addr64(st, (lane >> 2) + 8 * j, q), w.x, w.y, w.z, w.w);
-                *reinterpret_cast<uint4*>(rowptr[j] + col0 + 8 * q) = w;
-              }
-              continue;
-            }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               st_shared_v4(epi_piece_addr(st, lane, i), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
             __syncwarp();
-            const int row_base = mt * BM + lane_group * 32;
-            const long long gbase = static_cast<long long>(g) * p.c_group_stride;
             if (p.c_fp32) {
-              const int q = lane & 7;
+              const int q = lane & 7, r0 = row_base + (lane >> 3);
+              float* dst = reinterpret_cast<float*>(cbase) + gbase + static_cast<long long>(r0) * p.ldc + col0 + 4 * q;
+              float4 o[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
-                const int r = (lane >> 3) + 4 * j;
-                if (row_base + r >= p.M) continue;
                 uint32_t w0, w1, w2, w3;
-                ld_shared_v4(epi_piece_addr(st, r, q), w0, w1, w2, w3);
-                float4 o = make_float4(__uint_as_float(w0), __uint_as_float(w1), __uint_as_float(w2), __uint_as_float(w3));
-                float* dst = reinterpret_cast<float*>(cbase) + gbase + static_cast<long long>(row_base + r) * p.ldc + col0 + 4 * q;
-                if (p.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(dst);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4*>(dst) = o;
+                ld_shared_v4(epi_piece_addr(st, (lane >> 3) + 4 * j, q), w0, w1, w2, w3);
+                o[j] = make_float4(__uint_as_float(w0), __uint_as_float(w1), __uint_as_float(w2), __uint_as_float(w3));
               }
+              if (p.accumulate) {
+                float4 old[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  if (r0 + 4 * j < p.M) old[j] = *reinterpret_cast<const float4*>(dst + 4 * j * p.ldc);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { o[j].x += old[j].x; o[j].y += old[j].y; o[j].z += old[j].z; o[j].w += old[j].w; }
+              }
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (r0 + 4 * j < p.M) *reinterpret_cast<float4*>(dst + 4 * j * p.ldc) = o[j];
             } else {
-              const int q = lane & 3;
+              const int q = lane & 3, r0 = row_base + (lane >> 2);
+              __nv_bfloat16* dst[4];
+              uint4 res[4], old[4];
+              float f[4][8];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const int r = (lane >> 2) + 8 * j;
-                if (rowptr[j] == nullptr) continue;
-                uint32_t w[8];
-                ld_shared_v4(epi_piece_addr(st, r, 2 * q), w[0], w[1], w[2], w[3]);
-                ld_shared_v4(epi_piece_addr(st, r, 2 * q + 1), w[4], w[5], w[6], w[7]);
-                float f[8];
+                dst[j] = row_dst(r0 + 8 * j, tag[j]);
+                if (dst[j] == nullptr) continue;
+                dst[j] += col0 + 8 * q;
+                if (p.residual) res[j] = *reinterpret_cast<const uint4*>(p.residual + static_cast<long long>(r0 + 8 * j) * p.ldr + col0 + 8 * q);
+                if (p.accumulate) old[j] = *reinterpret_cast<const uint4*>(dst[j]);
+              }
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(w[e]);
-                __nv_bfloat16* dst = rowptr[j] + col0 + 8 * q;
-                if (p.residual) {
-                  const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + static_cast<long long>(row_base + r) * p.ldr + col0 + 8 * q);
-                  const float2 a = unpack_bf16(rr.x), b = unpack_bf16(rr.y), c2 = unpack_bf16(rr.z), d = unpack_bf16(rr.w);
-                  f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y; f[4] += c2.x; f[5] += c2.y; f[6] += d.x; f[7] += d.y;
-                }
-                if (p.accumulate) {
-                  const uint4 rr = *reinterpret_cast<const uint4*>(dst);
-                  const float2 a = unpack_bf16(rr.x), b = unpack_bf16(rr.y), c2 = unpack_bf16(rr.z), d = unpack_bf16(rr.w);
-                  f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y; f[4] += c2.x; f[5] += c2.y; f[6] += d.x; f[7] += d.y;
-                }
-                uint4 o;
-                o.x = pack_bf16(f[0], f[1]); o.y = pack_bf16(f[2], f[3]);
-                o.z = pack_bf16(f[4], f[5]); o.w = pack_bf16(f[6], f[7]);
-                *reinterpret_cast<uint4*>(dst) = o;
+              for (int j = 0; j < 4; ++j) {
+                uint32_t w[8];
+                ld_shared_v4(epi_piece_addr(st, (lane >> 2) + 8 * j, 2 * q), w[0], w[1], w[2], w[3]);
+                ld_shared_v4(epi_piece_addr(st, (lane >> 2) + 8 * j, 2 * q + 1), w[4], w[5], w[6], w[7]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[j][e] = __uint_as_float(w[e]);
+              }
+              auto add = [](float (&x)[8], const uint4& u) {
+                const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c2 = unpack_bf16(u.z), d = unpack_bf16(u.w);
+                x[0] += a.x; x[1] += a.y; x[2] += b.x; x[3] += b.y; x[4] += c2.x; x[5] += c2.y; x[6] += d.x; x[7] += d.y;
+              };
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (dst[j] == nullptr) continue;
+                if (p.residual) add(f[j], res[j]);
+                if (p.accumulate) add(f[j], old[j]);
+                *reinterpret_cast<uint4*>(dst[j]) = make_uint4(pack_bf16(f[j][0], f[j][1]), pack_bf16(f[j][2], f[j][3]),
+                                                               pack_bf16(f[j][4], f[j][5]), pack_bf16(f[j][6], f[j][7]));
               }
             }
             continue;
@@ -521,62 +596,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           if (!row_ok) continue;
           if (p.c_fp32) {
             float* dst = reinterpret_cast<float*>(cbase) + coff + col0;
-            if (full_chunk) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                float4 o = make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
-                                       __uint_as_float(v[i + 3]));
-                if (p.accumulate) {
-                  float4 old = *reinterpret_cast<float4*>(dst + i);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4*>(dst + i) = o;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {  // constant indices keep v[] in registers
-                if (col0 + i < p.N) {
-                  float o = __uint_as_float(v[i]);
-                  if (p.accumulate) o += dst[i];
-                  dst[i] = o;
-                }
+            for (int i = 0; i < 32; ++i) {  // constant indices keep v[] in registers
+              if (col0 + i < p.N) {
+                float o = __uint_as_float(v[i]);
+                if (p.accumulate) o += dst[i];
+                dst[i] = o;
               }
             }
           } else {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(cbase) + coff + col0;
             const __nv_bfloat16* res = p.residual ? p.residual + static_cast<long long>(row) * p.ldr + col0 : nullptr;
-            if (full_chunk) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                float f[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[i + j]);
-                if (res) {
-                  uint4 r = *reinterpret_cast<const uint4*>(res + i);
-                  float2 a = unpack_bf16(r.x), b = unpack_bf16(r.y), c2 = unpack_bf16(r.z), d = unpack_bf16(r.w);
-                  f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y;
-                  f[4] += c2.x; f[5] += c2.y; f[6] += d.x; f[7] += d.y;
-                }
-                if (p.accumulate) {
-                  uint4 r = *reinterpret_cast<const uint4*>(dst + i);
-                  float2 a = unpack_bf16(r.x), b = unpack_bf16(r.y), c2 = unpack_bf16(r.z), d = unpack_bf16(r.w);
-                  f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y;
-                  f[4] += c2.x; f[5] += c2.y; f[6] += d.x; f[7] += d.y;
-                }
-                uint4 o;
-                o.x = pack_bf16(f[0], f[1]); o.y = pack_bf16(f[2], f[3]);
-                o.z = pack_bf16(f[4], f[5]); o.w = pack_bf16(f[6], f[7]);
-                *reinterpret_cast<uint4*>(dst + i) = o;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                if (col0 + i < p.N) {
-                  float o = __uint_as_float(v[i]);
-                  if (res) o += __bfloat162float(res[i]);
-                  if (p.accumulate) o += __bfloat162float(dst[i]);
-                  dst[i] = __float2bfloat16(o);
-                }
+            for (int i = 0; i < 32; ++i) {
+              if (col0 + i < p.N) {
+                float o = __uint_as_float(v[i]);
+                if (res) o += __bfloat162float(res[i]);
+                if (p.accumulate) o += __bfloat162float(dst[i]);
+                dst[i] = __float2bfloat16(o);
               }
             }
           }
@@ -616,8 +653,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               pu[j / 2] = pack_bf16(u0, u1);
             }
             const uint32_t st = smem_u32(epi_stage + (warp - 2) * L::EPI_STAGE_BYTES);
-            const int row_base = mt * BM + lane_group * 32;
-            const int q = lane & 3;
+            const int q = lane & 3, r0 = row_base + (lane >> 2);
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(r0) * p.ldc + col0 + 8 * q;
+            __nv_bfloat16* pdst = pre ? p.preact + static_cast<long long>(r0) * p.ld_preact + col0 + 8 * q : nullptr;
+            // parked rows are read ahead of the first store of a round
+            uint4 x[4], y[4];
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -627,15 +667,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const int r = (lane >> 2) + 8 * j;
-              if (row_base + r >= p.M) continue;
-              uint4 w;
-              ld_shared_v4(epi_piece_addr64(st, r, q), w.x, w.y, w.z, w.w);
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row_base + r) * p.ldc + col0 + 8 * q) = w;
-              if (pre) {
-                ld_shared_v4(epi_piece_addr64(st + 2048, r, q), w.x, w.y, w.z, w.w);
-                *reinterpret_cast<uint4*>(p.preact + static_cast<long long>(row_base + r) * p.ld_preact + col0 + 8 * q) = w;
-              }
+              ld_shared_v4(epi_piece_addr64(st, (lane >> 2) + 8 * j, q), x[j].x, x[j].y, x[j].z, x[j].w);
+              if (pre) ld_shared_v4(epi_piece_addr64(st + 2048, (lane >> 2) + 8 * j, q), y[j].x, y[j].y, y[j].z, y[j].w);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (r0 + 8 * j >= p.M) continue;
+              *reinterpret_cast<uint4*>(dst + 8 * j * p.ldc) = x[j];
+              if (pre) *reinterpret_cast<uint4*>(pdst + 8 * j * p.ld_preact) = y[j];
             }
             if (pre) {
               __syncwarp();
@@ -644,13 +683,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 st_shared_v4(epi_piece_addr64(st, lane, i), pu[4 * i], pu[4 * i + 1], pu[4 * i + 2], pu[4 * i + 3]);
               __syncwarp();
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int r = (lane >> 2) + 8 * j;
-                if (row_base + r >= p.M) continue;
-                uint4 w;
-                ld_shared_v4(epi_piece_addr64(st, r, q), w.x, w.y, w.z, w.w);
-                *reinterpret_cast<uint4*>(p.preact + static_cast<long long>(row_base + r) * p.ld_preact + p.F + col0 + 8 * q) = w;
-              }
+              for (int j = 0; j < 4; ++j) ld_shared_v4(epi_piece_addr64(st, (lane >> 2) + 8 * j, q), x[j].x, x[j].y, x[j].z, x[j].w);
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (r0 + 8 * j < p.M) *reinterpret_cast<uint4*>(pdst + 8 * j * p.ld_preact + p.F) = x[j];
             }
             continue;
           }
@@ -671,14 +707,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (PAIR) mbar_arrive_cluster(leader_addr(&tempty[acc]));
-        else mbar_arrive(&tempty[acc]);
-      }
-      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      release();
     }
+    if (EPI == EPI_STORE && p.tma_out && lane == 0) bulk_wait_all();
     if (p.ep.scat_on) __threadfence_system();   // this thread's peer stores are ordered before the "returned" flag
   } else if (p.ep.push_on) {
     // ------------------------------------------------------------ push warps (warps 10..11)
@@ -856,7 +887,7 @@ split_sum_kernel(const float* __restrict__ ws, int splits, int M, int N, void* C
 template <int BN, bool A_MN, bool B_MN, int EPI, bool PAIR>
 static int launch(const GemmArgs& a, cudaStream_t stream) {
   using L = SmemLayout<BN, PAIR>;
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
   // ---- A map (2D)
   {
     uint64_t dims[2];
@@ -947,15 +978,31 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
     p.c_fp32 = 1; p.accumulate = 0; p.residual = nullptr; p.alpha = nullptr;
   }
 
+  const long long total = static_cast<long long>(p.m_tiles) * p.n_tiles * (p.groups_k > 0 ? p.groups_k : p.k_splits);
+  if (total <= 0) return 0;
+  if (total >= (1ll << 31) - 65536) return 910;
+  // ---- C map (3D, last dim = group)
+  tmC = tmA;       // placeholder where nothing is stored through it
+  p.tma_out = EPI == EPI_STORE && !split && !a.c_fp32 && !a.residual && !a.accumulate && !p.ep.scat_on && a.M > 0 && a.N > 0 &&
+              (a.groups_k == 0 || a.c_group_stride % 8 == 0);
+  if (p.tma_out) {
+    const uint64_t dims[3] = {static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.groups_k > 0 ? a.groups_k : 1)};
+    const uint64_t str[2] = {static_cast<uint64_t>(a.ldc) * 2, static_cast<uint64_t>(a.groups_k > 0 ? a.c_group_stride : a.ldc * a.M) * 2};
+    const uint32_t box[3] = {64, 32, 1};
+    int r = make_tmap_bf16(&tmC, a.C, 3, dims, str, box);
+    if (r) return 30000 + r;
+  }
+  constexpr int RASTER_M = PAIR ? 8 : 16;
+  p.by_group = fast_div(p.m_tiles * p.n_tiles);
+  p.by_band = fast_div(RASTER_M * p.n_tiles);
+  p.by_rest = fast_div(p.m_tiles % RASTER_M ? p.m_tiles % RASTER_M : 1);
+
   auto kfn = gemm_kernel<BN, A_MN, B_MN, EPI, PAIR>;
   static bool smem_done[16] = {};
   {
     const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), L::TOTAL, smem_done);
     if (e != cudaSuccess) return 300 + static_cast<int>(e);
   }
-  long long total = static_cast<long long>(p.m_tiles) * p.n_tiles * (p.groups_k > 0 ? p.groups_k : p.k_splits);
-  if (total <= 0) return 0;
-  if (total >= (1ll << 31) - 65536) return 910;
   if (PAIR) {
     const int pairs = static_cast<int>(total < a.num_sms / 2 ? total : a.num_sms / 2);
     cudaLaunchConfig_t cfg{};
@@ -968,11 +1015,11 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tmA, tmB, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tmA, tmB, tmC, p);
     if (e != cudaSuccess) return 400 + static_cast<int>(e);
   } else {
     const int grid = static_cast<int>(total < a.num_sms ? total : a.num_sms);
-    kfn<<<grid, p.ep.push_on ? GEMM_THREADS_PUSH : GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, p);
+    kfn<<<grid, p.ep.push_on ? GEMM_THREADS_PUSH : GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmC, p);
   }
   if (split) {
     const long long n = static_cast<long long>(a.M) * (a.N / 4);
@@ -994,7 +1041,9 @@ static int launch(const GemmArgs& a, cudaStream_t stream) {
 //  * short runs do not make up for the handshakes between the two at the first loads and the last stores: 32 k-blocks per CTA
 //    (2048^3) 21 -> 23 us, 47 (3456 x 1152 x 3000) the same, 68 (3000 x 1152 x 4304) 39 -> 35;
 //  * grouped weight gradients have few k-blocks per tile (four at 256 rows per expert), so a tile is mostly its epilogue, and the
-//    epilogue of one half waits for the other's: 128 x 2048 x 1536 and 128 x 768 x 2048 of 256 rows 287 -> 350 and 150 -> 186.
+//    epilogue of one half waits for the other's: 128 x 2048 x 1536 and 128 x 768 x 2048 of 256 rows 282 -> 300 and 148 -> 176;
+//  * experts' rows in 256-row tiles: an odd number of 128-row tiles leaves half a pair idle, which takes back what the shared loads
+//    save (128 experts of 256 rows on average 250 -> 257, of exactly 192 rows 213 -> 198).
 static bool pays_in_pairs(const GemmArgs& a) {
   if (a.tile_group || a.ep || a.groups_k > 0 || a.M <= BM || a.num_sms < 2) return false;
   const long long nt = a.epi == EPI_SWIGLU ? (a.N + 127) / 128 : (a.N + 255) / 256;
