@@ -6,23 +6,31 @@
 //
 // One CTA owns one 128-row KV tile of one document for one *query* head; K_j and V_j stay resident in shared memory
 // and dK_j / dV_j accumulate in TMEM over every 64-row query tile that can see the KV tile.  With grouped-query
-// attention the CTAs of the query heads that share a KV head add their dK / dV into fp32 accumulators with vector
-// atomics (splitting by query head keeps the longest CTA short: a causal KV tile near the start of a long document
+// attention the CTAs of the query heads that share a KV head add their dK / dV into fp32 accumulators by TMA reductions
+// (splitting by query head keeps the longest CTA short: a causal KV tile near the start of a long document
 // is seen by every later query tile).  Per query-tile iteration, all on tcgen05 with M = 128:
 //     S^T  = K_j  Q_i^T          [kv, q]     (K-major  x K-major)
 //     dP^T = V_j  dO_i^T         [kv, q]     (K-major  x K-major)
-//     P^T  = exp2(S^T c - lse_q),  dS^T = P^T (dP^T - Delta_q) scale        (one thread per kv row, bf16 -> smem)
-//     dV  += P^T  dO_i           [kv, d]     (K-major  x MN-major)
+//     P^T  = exp2(S^T c - lse_q),  dS^T = P^T (dP^T - Delta_q) scale        (one thread per kv row, P -> TMEM, dS -> smem)
+//     dV  += P^T  dO_i           [kv, d]     (TMEM     x MN-major)
 //     dK  += dS^T Q_i            [kv, d]     (K-major  x MN-major)
 //     dQ^T = K_j^T dS^T          [d, q]      (MN-major x MN-major)  -> transposed through shared memory and added
 //                                            into the fp32 dQ buffer by one TMA reduction per tile (the L2 does the adds)
 // Warp roles: 0 TMA producer, 1 MMA issuer, 2-9 softmax/dS, 10-13 dQ read-out.  The softmax of a tile is the longest
 // dependent chain of an iteration (TMEM read, 64 exponentials per kv row, two bf16 tiles to shared memory), so two
 // warpgroups share it: warps 2-5 take query columns 0-31 of every kv row, warps 6-9 columns 32-63 (a warp may read
-// the TMEM lanes 32 (warp % 4) .. +31 at any column).  P^T / dS^T (shared memory) and dQ^T (TMEM) are double-buffered:
-// the softmax warps of query tile i+1 run while the tensor cores still consume the P^T / dS^T of tile i, and the dQ
-// read-out of tile i overlaps the dQ^T MMAs of tile i+1.  Waits are bounded; on timeout the roles drain to the final
+// the TMEM lanes 32 (warp % 4) .. +31 at any column).  P^T (TMEM) and dS^T (shared memory; one buffer with 192-wide heads) are
+// double-buffered: the softmax warps of query tile i+1 run while the tensor cores still consume the P^T / dS^T of tile i, and the
+// dQ read-out of tile i overlaps the products of tile i+1.  Waits are bounded; on timeout the roles drain to the final
 // barrier, TMEM is freed and the status word records where the wait gave up.
+//
+// What bounds it: 2300 clocks per pair of tiles, of which the products need 1280 at the tensor rate and 1500 with the 192 KB that
+// they read through shared memory (another 112 KB are written and read by the other roles); the softmax warps' chain is 1800.  It
+// was 3300: P^T in shared memory left room for two Q / dO stages only, whose refill was waited for (700); the row statistics were
+// waited for at the top of every iteration (700); masks and dS stores between the exponentials kept them from overlapping; and
+// every CTA ended with 9700 clocks of 16-byte atomics (7500 now, all of it traffic of 128 KB of sums).  Whole call in us, before ->
+// now: 4096 tokens in four documents, 32 / 4 heads 355 -> 296, bit-reproducible 703 -> 475; 8192 tokens, 32 / 8 heads 1070 -> 893;
+// 192 / 128-wide heads, 4096 x 16 295 -> 245; five documents of 600, 16 heads of 72, full attention 101 -> 89; 300 x 8 29 -> 26.
 //
 // Replaces flash-attn 2's backward used through the reference attention interface
 // (models/modules/attention/interface.py:114-158).
@@ -40,10 +48,10 @@ struct AttnBwdParams {
   const int* kv_tiles;   // [n_tiles, 3]: first kv row, document start, document end
   const float* lse;      // [Hq, T]
   const float* delta;    // [Hq, T]  rowsum(dO * O)
-  float* dq_acc;         // [T, Hq, D] fp32, zero-initialised
+  float* dq_acc;         // [T, Hq, D] fp32, zero before the kernel
   __nv_bfloat16* dk;     // [T, Hk, D]   written directly when Hq == Hk
   __nv_bfloat16* dv;     // [T, Hk, D]
-  float* dk_acc;         // [T, Hk, D] fp32, zero-initialised (used when Hq > Hk)
+  float* dk_acc;         // [T, Hk, D] fp32, zero before the kernel (used when Hq > Hk)
   float* dv_acc;
   int Hq, Hk;
   int D, Dv;             // width of query / key heads and of value heads
@@ -57,23 +65,29 @@ template <int DQK, bool WITH_DQ>
 struct BwdSmem {
   static constexpr int K_BYTES = 128 * DQK * 2;     // K tile: DQK / 64 panels of 16 KB
   static constexpr int Q_BYTES = 64 * DQK * 2;      // Q tile: DQK / 64 panels of 8 KB
+  static constexpr int STAGES = 3;                  // Q / dO tiles on their way or in use
+  static constexpr int DS_BUFS = DQK == 128 ? 2 : 1;
   static constexpr int K = 0;
   static constexpr int V = K + K_BYTES;             // 32 KB
-  static constexpr int Q0 = V + 32768;              // 2 x Q_BYTES
-  static constexpr int DO0 = Q0 + 2 * Q_BYTES;      // 2 x 16 KB
-  static constexpr int PT = DO0 + 2 * 16384;        // 2 x 16 KB  P^T  [128 kv][64 q]
-  static constexpr int DST = PT + 2 * 16384;        // 2 x 16 KB  dS^T [128 kv][64 q]
-  static constexpr int DQS = DST + 2 * 16384;       // 32 KB  dQ tile [64 q][128 d] fp32, source of the TMA reduction
-  static constexpr int LSE = DQS + (WITH_DQ ? 32768 : 0);   // float [2][64]
-  static constexpr int DELTA = LSE + 2 * 64 * 4;    // float [2][64]
-  static constexpr int BARS = DELTA + 2 * 64 * 4;
-  static constexpr int TOTAL = BARS + 256 + 1024;
+  static constexpr int Q0 = V + 32768;
+  static constexpr int DO0 = Q0 + STAGES * Q_BYTES;
+  static constexpr int DST = DO0 + STAGES * 16384;  // 16 KB each: dS^T [128 kv][64 q]
+  static constexpr int DQS = DST + DS_BUFS * 16384; // 32 KB  dQ tile [64 q][128 d] fp32, source of the TMA reduction
+  static constexpr int STAT = DQS + (WITH_DQ ? 32768 : 0);  // float [2][lse, delta][128]: two iterations' rows, two buffers
+  static constexpr int BARS = STAT + 2 * 2 * 128 * 4;
+  static constexpr int TOTAL = BARS + 256;
+  static_assert(TOTAL <= 232448, "one CTA per SM");
+  static_assert(DST >= 8 * 16384, "the tiles before dS^T hold dK and dV in fp32 at the end");
 };
 
 __device__ __forceinline__ float bw_exp2(float x) {
   float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// two pairs of fp32 from shared memory; volatile without a memory clobber: stays behind the waits, free among the arithmetic
+__device__ __forceinline__ void ld_shared_pairs(uint32_t addr, uint64_t& a, uint64_t& b) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
 
 // Warp-collective: 32 consecutive fp32 columns of two accumulators, both loads in flight before the one wait.
@@ -107,7 +121,8 @@ template <int DQK, bool WITH_DQ, bool FULL>
 __global__ void __launch_bounds__(448, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                 const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV,
+                const AttnBwdParams p) {
   static_assert(DQK == 128 || !WITH_DQ, "the fused dQ path exists for 128-wide heads only");
   using BwdSmem = ttb::BwdSmem<DQK, WITH_DQ>;
   const int D = FULL ? DQK : p.D, Dv = FULL ? BW_D : p.Dv;
@@ -116,24 +131,27 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     else tma_load_3d(dst, map, bar, col, head, row);
   };
   constexpr int NP = DQK / 64, Q_BYTES = BwdSmem::Q_BYTES;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];      // swizzled tiles; there is no room to align them by hand
+  if (smem_u32(smem) & 1023) {
+    if (threadIdx.x == 0) set_status(KID_ATTN_BWD, 12, blockIdx.x);
+    return;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BwdSmem::BARS);
   uint64_t* kv_full = bars + 0;
-  uint64_t* qdo_full = bars + 1;    // [2]
-  uint64_t* qdo_empty = bars + 3;   // [2]
-  uint64_t* st_full = bars + 5;
-  uint64_t* st_empty = bars + 6;
-  uint64_t* pds_full = bars + 7;    // [2]
-  uint64_t* pds_empty = bars + 9;   // [2]
-  uint64_t* dq_full = bars + 11;    // [2]
-  uint64_t* dq_empty = bars + 13;   // [2]
+  constexpr int STAGES = BwdSmem::STAGES;
+  uint64_t* qdo_full = bars + 1;    // [3]
+  uint64_t* qdo_empty = bars + 4;   // [3]
+  uint64_t* st_full = bars + 7;
+  uint64_t* st_empty = bars + 8;
+  uint64_t* pds_full = bars + 9;    // [2]
+  uint64_t* pds_empty = bars + 11;  // [2]
+  uint64_t* dq_full = bars + 13;
+  uint64_t* dq_empty = bars + 14;
   uint64_t* acc_full = bars + 15;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* s_dead = reinterpret_cast<volatile int*>(bars + 17);   // a softmax warp's wait gave up
   volatile int* s_dead_dq = reinterpret_cast<volatile int*>(bars + 18);  // a dQ warp's wait gave up
-  float* s_lse = reinterpret_cast<float*>(smem + BwdSmem::LSE);
-  float* s_delta = reinterpret_cast<float*>(smem + BwdSmem::DELTA);
+  float* s_stat = reinterpret_cast<float*>(smem + BwdSmem::STAT);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Launch order.  With dQ in this kernel, tiles vary fastest: the CTAs of one head run together and share its Q / dO
@@ -157,12 +175,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 1); }
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 1); }
     mbar_init(st_full, 1); mbar_init(st_empty, 8);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&pds_full[i], 8); mbar_init(&pds_empty[i], 1);
-      mbar_init(&dq_full[i], 1); mbar_init(&dq_empty[i], 4);
-    }
+    for (int i = 0; i < 2; ++i) { mbar_init(&pds_full[i], 8); mbar_init(&pds_empty[i], 1); }
+    mbar_init(dq_full, 1); mbar_init(dq_empty, 4);
     mbar_init(acc_full, 1);
     *s_dead = 0;
     *s_dead_dq = 0;
@@ -178,9 +194,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tm_ST = tmem_base;          // 64 cols
   const uint32_t tm_DPT = tmem_base + 64;    // 64 cols
-  const uint32_t tm_DQT = tmem_base + 128;   // 2 x 64 cols (form with dQ)
-  const uint32_t tm_DV = tmem_base + (WITH_DQ ? 256 : 128);    // 128 cols
-  const uint32_t tm_DK = tmem_base + (WITH_DQ ? 384 : 256);    // DQK cols
+  const uint32_t tm_PT = tmem_base + 128;    // 2 x 32 cols: P^T as packed bf16, the A operand of dV
+  const uint32_t tm_DQT = tmem_base + 192;   // 64 cols (form with dQ)
+  const uint32_t tm_DV = tmem_base + (WITH_DQ ? 256 : 192);    // 128 cols
+  const uint32_t tm_DK = tmem_base + (WITH_DQ ? 384 : 320);    // DQK cols
 
   auto it_head = [&](int it) { return p.group_loop ? hq + it / n_qt : hq; };
   auto it_q0 = [&](int it) { return q_first + (p.group_loop ? it % n_qt : it) * BW_Q; };
@@ -194,9 +211,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int pn = 0; pn < NP; ++pn) load_head(smem + BwdSmem::K + pn * 16384, &tmK, kv_full, pn * 64, hk, DQK, kv0);
       load_head(smem + BwdSmem::V, &tmV, kv_full, 0, hk, 128, kv0);
       load_head(smem + BwdSmem::V + 16384, &tmV, kv_full, 64, hk, 128, kv0);
+      int st = 0;
+      uint32_t ph = 0;
       for (int it = 0; it < n_it; ++it) {
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
         if (!mbar_wait(&qdo_empty[st], ph ^ 1, KID_ATTN_BWD, 1)) break;
         const int h = it_head(it), q0 = it_q0(it);
         mbar_expect_tx(&qdo_full[st], Q_BYTES + 16384);
@@ -206,6 +223,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int pn = 0; pn < NP; ++pn) load_head(sq + pn * 8192, &tmQ, &qdo_full[st], pn * 64, h, DQK, q0);
         load_head(sd, &tmDO, &qdo_full[st], 0, h, 128, q0);
         load_head(sd + 8192, &tmDO, &qdo_full[st], 64, h, 128, q0);
+        if (++st == STAGES) { st = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
@@ -221,13 +239,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // operands read along their rows (K-major) and, where a product reduces over rows, across them (MN-major)
       const SmemDesc dK = make_smem_desc2(smem_u32(smem + BwdSmem::K), 16, 1024), dV = make_smem_desc2(smem_u32(smem + BwdSmem::V), 16, 1024);
       const SmemDesc dQ = make_smem_desc2(smem_u32(smem + BwdSmem::Q0), 16, 1024), dDO = make_smem_desc2(smem_u32(smem + BwdSmem::DO0), 16, 1024);
-      const SmemDesc dPT = make_smem_desc2(smem_u32(smem + BwdSmem::PT), 16, 1024), dDST = make_smem_desc2(smem_u32(smem + BwdSmem::DST), 16, 1024);
+      const SmemDesc dDST = make_smem_desc2(smem_u32(smem + BwdSmem::DST), 16, 1024);
       const SmemDesc dKt = make_smem_desc2(smem_u32(smem + BwdSmem::K), 16384, 1024), dDSt = make_smem_desc2(smem_u32(smem + BwdSmem::DST), 8192, 1024);
       const SmemDesc dQt = make_smem_desc2(smem_u32(smem + BwdSmem::Q0), 8192, 1024), dDOt = make_smem_desc2(smem_u32(smem + BwdSmem::DO0), 8192, 1024);
       bool ok = mbar_wait(kv_full, 0, KID_ATTN_BWD, 2);
+      int st_s = 0, st = 0;          // stage of the tile whose scores are formed / whose gradients are
+      uint32_t ph_s = 0;
       auto issue_scores = [&](int it) -> bool {
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
+        const int st = st_s;
+        const uint32_t ph = ph_s;
+        if (++st_s == STAGES) { st_s = 0; ph_s ^= 1; }
         if (!mbar_wait(&qdo_full[st], ph, KID_ATTN_BWD, 3)) return false;
         if (!mbar_wait(st_empty, (it & 1) ^ 1, KID_ATTN_BWD, 4)) return false;
         tc_fence_after();
@@ -252,34 +273,34 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (it + 1 < n_it) {
           if (!issue_scores(it + 1)) { ok = false; break; }
         }
-        const int st = it & 1;
-        const uint32_t ph2 = (it >> 1) & 1;
-        if (!mbar_wait(&pds_full[st], ph2, KID_ATTN_BWD, 5)) { ok = false; break; }
-        if (WITH_DQ) {
-          if (!mbar_wait(&dq_empty[st], ph2 ^ 1, KID_ATTN_BWD, 6)) { ok = false; break; }
-        }
+        const int b = it & 1, db = it % BwdSmem::DS_BUFS;
+        if (!mbar_wait(&pds_full[b], (it >> 1) & 1, KID_ATTN_BWD, 5)) { ok = false; break; }
         tc_fence_after();
-        const SmemDesc pt = desc_at(dPT, st * 16384), dst = desc_at(dDST, st * 16384), dst_t = desc_at(dDSt, st * 16384);
+        const SmemDesc dst = desc_at(dDST, db * 16384), dst_t = desc_at(dDSt, db * 16384);
         const SmemDesc q_t = desc_at(dQt, st * Q_BYTES), do_t = desc_at(dDOt, st * 16384);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {  // reduction over q = 64
-          // A: P^T / dS^T K-major single panel; B: dO / Q as [q rows][d] MN-major, d panels 8 KB apart
-          umma_ss_w(leader, tm_DV, desc_at(pt, kk * 32), desc_at(do_t, kk * 2048), id_acc, (it | kk) != 0);
+          // A: P^T from tensor memory (16 queries are 8 columns), dS^T K-major single panel; B: dO / Q as [q rows][d] MN-major, d
+          // panels 8 KB apart
+          umma_ts_w(leader, tm_DV, tm_PT + b * 32 + kk * 8, desc_at(do_t, kk * 2048), id_acc, (it | kk) != 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           umma_ss_w(leader, tm_DK, desc_at(dst, kk * 32), desc_at(q_t, kk * 2048), id_dk, (it | kk) != 0);
         }
         umma_commit_w(leader, &qdo_empty[st]);
+        if (++st == STAGES) st = 0;
         if (WITH_DQ) {
+          if (!mbar_wait(dq_empty, (it & 1) ^ 1, KID_ATTN_BWD, 6)) { ok = false; break; }
+          tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {  // reduction over kv = 128
             // A: K^T from the K tile ([kv rows][d], MN-major, d panels 16 KB apart); B: dS^T ([kv rows][q]) MN-major
-            umma_ss_w(leader, tm_DQT + st * 64, desc_at(dKt, kk * 2048), desc_at(dst_t, kk * 2048), id_dq, kk != 0);
+            umma_ss_w(leader, tm_DQT, desc_at(dKt, kk * 2048), desc_at(dst_t, kk * 2048), id_dq, kk != 0);
           }
-          umma_commit_w(leader, &dq_full[st]);
+          umma_commit_w(leader, dq_full);
         }
-        umma_commit_w(leader, &pds_empty[st]);
+        umma_commit_w(leader, &pds_empty[b]);
       }
       if (ok) umma_commit_w(leader, acc_full);
     }
@@ -293,30 +314,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const float c = p.scale * 1.4426950408889634f;
     const int tid = threadIdx.x - 64;  // 0..255 inside the two groups
     bool ok = true;
-    // lse / delta of the 64 query rows of an iteration are staged one iteration ahead (double-buffered); the global
-    // load is issued at the top of the iteration before and stored at its end
-    auto fetch = [&](int it) -> float {
-      const int q0s = it_q0(it);
-      if (tid < 64) {
-        const int q = q0s + tid;
-        return (q < de) ? -p.lse[static_cast<long long>(it_head(it)) * p.T + q] * 1.4426950408889634f : -INFINITY;
-      }
-      if (tid < 128) {
-        const int q = q0s + tid - 64;
-        return (q < de) ? -p.delta[static_cast<long long>(it_head(it)) * p.T + q] * p.scale : 0.f;
-      }
-      return 0.f;
+    // lse / delta of the 128 query rows of two iterations are staged two iterations ahead, one value a thread (double-buffered).  The
+    // load is issued before the two and its value is touched only after them: with the factors applied where it was loaded, every
+    // iteration began with the load's latency, a third of its time.
+    const int srow = tid & 127;
+    const bool is_lse = tid < 128;
+    const float* stat = is_lse ? p.lse : p.delta;
+    int h_n = hq, q0_n = q_first;              // head and first query row of the iteration to be staged or done next
+    auto advance = [&](int& h, int& q0) {
+      q0 += BW_Q;
+      if (q0 >= de) { q0 = q_first; ++h; }
     };
-    auto put = [&](int it, float v) {
-      if (tid < 64) s_lse[(it & 1) * 64 + tid] = v;
-      else if (tid < 128) s_delta[(it & 1) * 64 + tid - 64] = v;
+    int q_mine = 0;                            // this thread's row of the two iterations that are staged
+    auto fetch = [&](int h, int q0) {          // the second one may lie past the last iteration: its rows are loaded and not used
+      if (srow >= 64) advance(h, q0);
+      q_mine = q0 + (srow & 63);
+      float v;                                 // volatile: the compiler would move a plain load down to the use of its value
+      asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(stat + static_cast<long long>(min(h, p.Hq - 1)) * p.T + min(q_mine, de - 1)));
+      return v;
     };
-    if (n_it > 0) put(0, fetch(0));
+    auto put = [&](int pair, float v) {
+      const bool in = q_mine < de;
+      s_stat[(pair & 1) * 256 + tid] = is_lse ? (in ? -v * 1.4426950408889634f : -INFINITY) : (in ? -v * p.scale : 0.f);
+    };
+    put(0, fetch(h_n, q0_n));
     asm volatile("bar.sync 1, 256;" ::: "memory");
     // one iteration; false when a wait gave up (the caller still joins the group barrier, so no warp is left in it)
     auto body = [&](int it) -> bool {
-      const int q0 = it_q0(it);
-      const float staged = (it + 1 < n_it) ? fetch(it + 1) : 0.f;
+      const int q0 = q0_n;
+      advance(h_n, q0_n);
       if (!mbar_wait(st_full, it & 1, KID_ATTN_BWD, 7)) return false;
       tc_fence_after();
       float s[32], dp[32];
@@ -325,100 +351,136 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(st_empty);
-      const float* lse = s_lse + (it & 1) * 64 + half * 32;
-      const float* dl = s_delta + (it & 1) * 64 + half * 32;
+      const uint32_t lse = smem_u32(s_stat) + (((it >> 1) & 1) * 256 + (it & 1) * 64 + half * 32) * 4, dl = lse + 512;
       const int qh = q0 + half * 32;
       const bool need_mask = (q0 + BW_Q > de) || (kv0 + BW_KV > de) || (p.causal && kv0 + BW_KV - 1 > qh);
-      // the tile that used this P^T / dS^T buffer two iterations ago must have been consumed (a fresh barrier passes)
+      // The tiles that used these buffers must have been consumed: P^T two iterations ago (a fresh barrier passes), and dS^T, where
+      // it has one buffer, by the iteration before, whose products were issued before the scores of this one were read.
       if (!mbar_wait(&pds_empty[it & 1], ((it >> 1) & 1) ^ 1, KID_ATTN_BWD, 8)) return false;
-      uint8_t* sPT = smem + BwdSmem::PT + (it & 1) * 16384;
-      uint8_t* sDST = smem + BwdSmem::DST + (it & 1) * 16384;
+      if (BwdSmem::DS_BUFS == 1 && it > 0 && !mbar_wait(&pds_empty[(it - 1) & 1], ((it - 1) >> 1) & 1, KID_ATTN_BWD, 11)) return false;
+      tc_fence_after();
       // two columns per instruction; the staged row statistics are -lse log2(e) and -Delta scale
       const uint64_t cc = f2_pack(c, c), sc2 = f2_pack(p.scale, p.scale);
+      uint32_t wp[16], wd[16];
+      // Masked tiles have their own copy (a branch around every pair of columns kept their chains of exponential, product and
+      // conversion from overlapping), and dS is stored behind all of them for the same reason.
+      auto columns = [&](auto masked) {
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        uint32_t wp[4], wd[4];
-        const ulonglong2 l01 = *reinterpret_cast<const ulonglong2*>(lse + ch * 8), l23 = *reinterpret_cast<const ulonglong2*>(lse + ch * 8 + 4);
-        const ulonglong2 d01 = *reinterpret_cast<const ulonglong2*>(dl + ch * 8), d23 = *reinterpret_cast<const ulonglong2*>(dl + ch * 8 + 4);
-        const uint64_t lv[4] = {l01.x, l01.y, l23.x, l23.y};
-        const uint64_t dlv[4] = {d01.x, d01.y, d23.x, d23.y};
+        for (int ch = 0; ch < 4; ++ch) {
+          uint64_t lv[4], dlv[4];
+          ld_shared_pairs(lse + ch * 32, lv[0], lv[1]);
+          ld_shared_pairs(lse + ch * 32 + 16, lv[2], lv[3]);
+          ld_shared_pairs(dl + ch * 32, dlv[0], dlv[1]);
+          ld_shared_pairs(dl + ch * 32 + 16, dlv[2], dlv[3]);
 #pragma unroll
-        for (int qq = 0; qq < 4; ++qq) {
-          const int col = ch * 8 + qq * 2;
-          float a0, a1;
-          f2_unpack(f2_fma(f2_pack(s[col], s[col + 1]), cc, lv[qq]), a0, a1);
-          float p0 = bw_exp2(a0), p1 = bw_exp2(a1);
-          if (need_mask) {
-            const int q = qh + col;
-            p0 = (kv_ok && q < de && (!p.causal || kv <= q)) ? p0 : 0.f;
-            p1 = (kv_ok && q + 1 < de && (!p.causal || kv <= q + 1)) ? p1 : 0.f;
+          for (int qq = 0; qq < 4; ++qq) {
+            const int col = ch * 8 + qq * 2;
+            float a0, a1;
+            f2_unpack(f2_fma(f2_pack(s[col], s[col + 1]), cc, lv[qq]), a0, a1);
+            float p0 = bw_exp2(a0), p1 = bw_exp2(a1);
+            if (decltype(masked)::value) {
+              const int q = qh + col;
+              p0 = (kv_ok && q < de && (!p.causal || kv <= q)) ? p0 : 0.f;
+              p1 = (kv_ok && q + 1 < de && (!p.causal || kv <= q + 1)) ? p1 : 0.f;
+            }
+            float d0, d1;
+            f2_unpack(f2_mul(f2_pack(p0, p1), f2_fma(f2_pack(dp[col], dp[col + 1]), sc2, dlv[qq])), d0, d1);
+            wp[ch * 4 + qq] = pack_bf16(p0, p1);
+            wd[ch * 4 + qq] = pack_bf16(d0, d1);
           }
-          float d0, d1;
-          f2_unpack(f2_mul(f2_pack(p0, p1), f2_fma(f2_pack(dp[col], dp[col + 1]), sc2, dlv[qq])), d0, d1);
-          wp[qq] = pack_bf16(p0, p1);
-          wd[qq] = pack_bf16(d0, d1);
         }
-        const int off = row * 128 + (((half * 4 + ch) ^ (row & 7)) * 16);
-        *reinterpret_cast<uint4*>(sPT + off) = make_uint4(wp[0], wp[1], wp[2], wp[3]);
-        *reinterpret_cast<uint4*>(sDST + off) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-      }
+      };
+      if (need_mask) columns(std::true_type{});
+      else columns(std::false_type{});
+      const uint32_t ds_row = smem_u32(smem + BwdSmem::DST) + (it % BwdSmem::DS_BUFS) * 16384 + row * 128;
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch)
+        st_shared_v4(ds_row + (((half * 4 + ch) ^ (row & 7)) * 16), wd[4 * ch], wd[4 * ch + 1], wd[4 * ch + 2], wd[4 * ch + 3]);
+      tmem_st_32x32b_x16(tm_PT + (it & 1) * 32 + half * 16 + (static_cast<uint32_t>(lg * 32) << 16), wp);
+      tmem_st_wait();
+      tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pds_full[it & 1]);
-      if (it + 1 < n_it) put(it + 1, staged);
       return true;
     };
-    for (int it = 0; it < n_it; ++it) {
-      if (!body(it)) { *s_dead = 1; ok = false; }
+    for (int it = 0; it < n_it; it += 2) {
+      int h_2 = h_n, q0_2 = q0_n;
+      advance(h_2, q0_2);
+      advance(h_2, q0_2);
+      const float staged = fetch(h_2, q0_2);   // past the last iteration too: some row of this head
+      if (!body(it) || (it + 1 < n_it && !body(it + 1))) { *s_dead = 1; ok = false; }
+      put((it >> 1) + 1, staged);
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (*s_dead) { ok = false; break; }
     }
-    // ---- epilogue: dK / dV of this tile
-    if (ok && n_it > 0) ok = mbar_wait(acc_full, 0, KID_ATTN_BWD, 9);
+    // ---- epilogue: dV (columns 0-31 group) or dK (the other) of this warp's 32 kv rows, by way of shared memory and the copy engine.
+    // All products have retired, so that K, V and the Q / dO stages are free: 16 KB per warp.  The rows lie kilobytes apart in
+    // memory, and a thread that adds its own row 16 bytes at a time held the CTA up for 9700 clocks.
+    if (ok) ok = mbar_wait(acc_full, 0, KID_ATTN_BWD, 9);       // a kv tile is seen by its own rows at least
     if (ok) {
       tc_fence_after();
-      const uint32_t lane_off = static_cast<uint32_t>(lg * 32) << 16;
-      {
-        const int which = half;                  // columns 0-31 group: dV, the other group: dK
-        const int width = which == 0 ? Dv : D;
-        const long long off = (static_cast<long long>(kv) * p.Hk + hk) * width;
-        __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + off;
-        float* acc = (which == 0 ? p.dv_acc : p.dk_acc) + off;
-        const uint32_t tm = (which == 0 ? tm_DV : tm_DK) + lane_off;
+      const int which = half, width = which == 0 ? Dv : D;
+      const CUtensorMap* map = which == 0 ? &tmDV : &tmDK;
+      const uint32_t tm = (which == 0 ? tm_DV : tm_DK) + (static_cast<uint32_t>(lg * 32) << 16);
+      const int row0 = kv0 + lg * 32;
+      const bool sums = G > 1 && !p.group_loop;
+      uint8_t* tile = smem + (which * 4 + lg) * 16384;
+      if (sums) {
+        // fp32, 32 columns a box; rows past the document are other documents', to which zeros are added
 #pragma unroll 1
         for (int cb = 0; cb * 32 < width; ++cb) {
           uint32_t v[32];
-          if (n_it > 0) {
-            tmem_ld_32x32b_x32(tm + cb * 32, v);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0u;
+          tmem_ld_32x32b_x32(tm + cb * 32, v);
+          tmem_ld_wait();
+          uint8_t* box = tile + (cb & 3) * 4096;
+          if (cb == 4) {                        // 192-wide heads: the first boxes once more
+            if (lane == 0) bulk_wait_read_all();
+            __syncwarp();
           }
-          if (kv_ok) {
-            if (G == 1 || p.group_loop) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                if (cb * 32 + i >= width) continue;
-                uint4 w;
-                w.x = pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-                w.y = pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
-                w.z = pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5]));
-                w.w = pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7]));
-                *reinterpret_cast<uint4*>(dst + cb * 32 + i) = w;
-              }
-            } else {
+          for (int i = 0; i < 8; ++i) {
+            uint4 w = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            if (!kv_ok) w = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(box + lane * 128 + ((i ^ (lane & 7)) << 4)) = w;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (FULL) tma_reduce_add_2d(map, box, hk * width + cb * 32, row0);
+            else tma_reduce_add_3d(map, box, cb * 32, hk, row0);
+            bulk_commit_group();
+          }
+        }
+      } else {
+        const bool whole = row0 + 32 <= de;     // no row of another document, which its own CTA writes
+#pragma unroll 1
+        for (int cb = 0; cb * 64 < width; ++cb) {
+          uint32_t v[2][32];
+          tmem_ld_32x32b_x32(tm + cb * 64, v[0]);
+          tmem_ld_32x32b_x32(tm + cb * 64 + 32, v[1]);
+          tmem_ld_wait();
+          uint8_t* box = tile + cb * 4096;
+          __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + (static_cast<long long>(kv) * p.Hk + hk) * width + cb * 64;
 #pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                if (cb * 32 + i >= width) continue;
-                atomicAdd(reinterpret_cast<float4*>(acc + cb * 32 + i),
-                          make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
-                                      __uint_as_float(v[i + 3])));
-              }
+          for (int i = 0; i < 8; ++i) {
+            const float* f = reinterpret_cast<const float*>(&v[i >> 2][(i & 3) * 8]);
+            uint4 w = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+            if (whole) *reinterpret_cast<uint4*>(box + lane * 128 + ((i ^ (lane & 7)) << 4)) = w;
+            else if (kv_ok && cb * 64 + i * 8 < width) *reinterpret_cast<uint4*>(dst + i * 8) = w;
+          }
+          if (whole) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (FULL) tma_store_2d(map, box, hk * width + cb * 64, row0);
+              else tma_store_3d(map, box, cb * 64, hk, row0);
+              bulk_commit_group();
             }
           }
         }
       }
+      if (lane == 0) bulk_wait_read_all();      // shared memory may go; the grid's end waits for the rest
     }
   } else if (WITH_DQ) {
     // ---------------------------------------------------------------- dQ read-out (thread = head-dim index d)
@@ -431,13 +493,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int it = 0; it < n_it; ++it) {
       const int q0 = it_q0(it);
       float v[64];
-      if (alive && !mbar_wait(&dq_full[it & 1], (it >> 1) & 1, KID_ATTN_BWD, 10)) { alive = false; *s_dead_dq = 1; }
+      if (alive && !mbar_wait(dq_full, it & 1, KID_ATTN_BWD, 10)) { alive = false; *s_dead_dq = 1; }
       if (alive) {
         tc_fence_after();
-        tmem_ld64(tm_DQT + (it & 1) * 64 + (static_cast<uint32_t>(lg * 32) << 16), v);
+        tmem_ld64(tm_DQT + (static_cast<uint32_t>(lg * 32) << 16), v);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&dq_empty[it & 1]);
+        if (lane == 0) mbar_arrive(dq_empty);
       }
       // the reduction of the previous tile has finished reading the staging tile
       if (it > 0 && tid_dq == 0) bulk_wait_read_all();
@@ -467,10 +529,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
-// delta[h, t] = sum_d dO[t,h,d] * O[t,h,d].  Sixteen lanes and 16-byte loads per (t, h): 22 -> 16 us for 4096 x 32 rows.
+// fp32 accumulators that a launch clears on the way
+struct Cleared {
+  float4* at[3];
+  long long vecs[3];
+};
+
+// delta[h, t] = sum_d dO[t,h,d] * O[t,h,d].  Sixteen lanes and 16-byte loads per (t, h): 22 -> 16 us for 4096 x 32 rows.  The kernel
+// reads only, so the accumulators of the kernels behind it are cleared here (71 MB in that case, 12 us as a launch of their own).
 __global__ void __launch_bounds__(256)
 attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                      float* __restrict__ delta, long long T, int Hq, int Dv) {
+                      float* __restrict__ delta, long long T, int Hq, int Dv, const Cleared z) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < z.vecs[r]; i += static_cast<long long>(gridDim.x) * blockDim.x)
+      z.at[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
   long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
   const int l = threadIdx.x & 15;
   const bool ok = row < T * Hq;
@@ -510,23 +583,24 @@ using namespace ttb;
 
 template <int DQK, bool WITH_DQ, bool FULL>
 static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv,
-                           const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, cudaStream_t stream) {
+                           const CUtensorMap& tdq, const CUtensorMap& tdk, const CUtensorMap& tdv, const AttnBwdParams& p, int n_tiles,
+                           cudaStream_t stream) {
   static bool smem_done[16] = {};
   using Smem = ttb::BwdSmem<DQK, WITH_DQ>;
   const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(attn_bwd_kernel<DQK, WITH_DQ, FULL>), Smem::TOTAL, smem_done);
   if (e != cudaSuccess) return 300 + static_cast<int>(e);
   const int heads = p.group_loop ? p.Hk : p.Hq;
   dim3 grid(WITH_DQ ? n_tiles : heads, WITH_DQ ? heads : n_tiles);
-  attn_bwd_kernel<DQK, WITH_DQ, FULL><<<grid, WITH_DQ ? 448 : 320, Smem::TOTAL, stream>>>(tq, tdo, tk, tv, tdq, p);
+  attn_bwd_kernel<DQK, WITH_DQ, FULL><<<grid, WITH_DQ ? 448 : 320, Smem::TOTAL, stream>>>(tq, tdo, tk, tv, tdq, tdk, tdv, p);
   return 0;
 }
 
 // q: [T, Hq, D] contiguous; dout, out: [T, Hq, Dv] contiguous; k: [T, Hk, D] (ldk); v: [T, Hk, Dv] (ldv, may be strided); D and
 // Dv up to 128 in multiples of 8, or D = 192 with Dv = 128.  delta fp32 [Hq*T] scratch (left filled with rowsum(dO * O) for the query-major dQ pass).
-// with_dq != 0 (D <= 128 only): dQ too, reduced into dq_acc (fp32 [T*Hq*D], zero-initialised) and cast to dq;
+// with_dq != 0 (D <= 128 only): dQ too, reduced into dq_acc (fp32 [T*Hq*D], cleared here) and cast to dq;
 // with_dq == 0: dK and dV only (dq_acc and dq unused); with_dq == 2: the same with one CTA per kv head looping over the
 // query heads of its group, so that dK / dV are written once and without atomics (no accumulators needed).  dk: [T, Hk, D], dv: [T, Hk, Dv]; with Hq > Hk the fp32
-// accumulators dk_acc / dv_acc (zero-initialised, same shapes) are required.
+// accumulators dk_acc / dv_acc (cleared here, same shapes) are required.
 TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const void* v, long long ldv, const void* out,
                             const void* dout, const float* lse, float* delta, float* dq_acc, float* dk_acc,
                             float* dv_acc, void* dq, void* dk, void* dv, const int* kv_tiles, int n_tiles, long long T, int Hq, int Hk, int D, int Dv, float scale,
@@ -539,8 +613,19 @@ TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const v
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
   if (T == 0 || n_tiles == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15) return 906;
+  const bool grouped = Hq != Hk && !group_loop;
+  if (with_dq && (dq_acc == nullptr || dq == nullptr)) return 905;
+  if (grouped && (dk_acc == nullptr || dv_acc == nullptr)) return 903;
+  const long long n[3] = {with_dq ? T * Hq * D : 0, grouped ? T * Hk * D : 0, grouped ? T * Hk * Dv : 0};
+  float* acc[3] = {dq_acc, dk_acc, dv_acc};
+  Cleared cleared;
+  for (int i = 0; i < 3; ++i) {
+    if (reinterpret_cast<uintptr_t>(acc[i]) & 15) return 906;
+    cleared.at[i] = reinterpret_cast<float4*>(acc[i]);
+    cleared.vecs[i] = n[i] / 4;
+  }
   attn_bwd_delta_kernel<<<(unsigned)((T * Hq + 15) / 16), 256, 0, stream>>>((const __nv_bfloat16*)dout,
-                                                                        (const __nv_bfloat16*)out, delta, T, Hq, Dv);
+                                                                        (const __nv_bfloat16*)out, delta, T, Hq, Dv, cleared);
   const bool full = D >= 128 && Dv == BW_D;
   const auto map = full ? make_rows_map : make_heads_map;
   CUtensorMap tq, tdo, tk, tv;
@@ -550,7 +635,6 @@ TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const v
   if (map(&tv, v, T, ldv, Hk, Dv, 128)) return 104;
   CUtensorMap tdq = tq;   // placeholder in the form without dQ
   if (with_dq) {
-    if (dq_acc == nullptr || dq == nullptr) return 905;
     // the staging tile's rows, clipped to the head where it is narrower
     const uint64_t dims2[2] = {static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T)};
     const uint64_t dims3[3] = {static_cast<uint64_t>(D), static_cast<uint64_t>(Hq), static_cast<uint64_t>(T)};
@@ -558,26 +642,36 @@ TTB_EXPORT int ttb_attn_bwd(const void* q, const void* k, long long ldk, const v
     const uint32_t box2[2] = {static_cast<uint32_t>(BW_D), 64}, box3[3] = {static_cast<uint32_t>(BW_D), 1, 64};
     if (full ? make_tmap_f32_linear(&tdq, dq_acc, 2, dims2, str + 1, box2) : make_tmap_f32_linear(&tdq, dq_acc, 3, dims3, str, box3)) return 105;
   }
-  if (Hq != Hk && !group_loop && (dk_acc == nullptr || dv_acc == nullptr)) return 903;
+  // dK / dV: boxes of 32 rows and 128 bytes, fp32 sums or bf16 results
+  CUtensorMap tdk, tdv;
+  auto out_map = [&](CUtensorMap* m, float* acc, void* res, int width) {
+    const int size = grouped ? 4 : 2;
+    const uint64_t dims2[2] = {static_cast<uint64_t>(Hk) * width, static_cast<uint64_t>(T)};
+    const uint64_t dims3[3] = {static_cast<uint64_t>(width), static_cast<uint64_t>(Hk), static_cast<uint64_t>(T)};
+    const uint64_t str[2] = {static_cast<uint64_t>(width) * size, static_cast<uint64_t>(Hk) * width * size};
+    const uint32_t box2[2] = {static_cast<uint32_t>(128 / size), 32}, box3[3] = {static_cast<uint32_t>(128 / size), 1, 32};
+    return make_tmap_typed(m, grouped ? static_cast<const void*>(acc) : res, full ? 2 : 3, full ? dims2 : dims3, full ? str + 1 : str,
+                           full ? box2 : box3, grouped ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                           CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  if (out_map(&tdk, dk_acc, dk, D)) return 106;
+  if (out_map(&tdv, dv_acc, dv, Dv)) return 107;
   AttnBwdParams p{kv_tiles, lse, delta, dq_acc, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_acc, dv_acc, Hq, Hk, D, Dv, T, scale, causal, group_loop};
   auto run = [&](auto is_full) {
     constexpr bool FULL = decltype(is_full)::value;
-    return with_dq ? launch_attn_bwd<128, true, FULL>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
-                   : launch_attn_bwd<128, false, FULL>(tq, tdo, tk, tv, tdq, p, n_tiles, stream);
+    return with_dq ? launch_attn_bwd<128, true, FULL>(tq, tdo, tk, tv, tdq, tdk, tdv, p, n_tiles, stream)
+                   : launch_attn_bwd<128, false, FULL>(tq, tdo, tk, tv, tdq, tdk, tdv, p, n_tiles, stream);
   };
-  const int rc = D == 192 ? launch_attn_bwd<192, false, true>(tq, tdo, tk, tv, tdq, p, n_tiles, stream)
+  const int rc = D == 192 ? launch_attn_bwd<192, false, true>(tq, tdo, tk, tv, tdq, tdk, tdv, p, n_tiles, stream)
                           : (full ? run(std::true_type{}) : run(std::false_type{}));
   if (rc) return rc;
   // fp32 accumulators -> bf16; the ones that lie back to back on both sides go in one launch
-  const bool grouped = Hq != Hk && !group_loop;
-  const long long n[3] = {with_dq ? T * Hq * D : 0, grouped ? T * Hk * D : 0, grouped ? T * Hk * Dv : 0};
-  const float* src[3] = {dq_acc, dk_acc, dv_acc};
   __nv_bfloat16* dst[3] = {(__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv};
   for (int i = 0; i < 3;) {
     long long run = n[i];
     int j = i + 1;
-    while (j < 3 && run > 0 && src[j] == src[i] + run && dst[j] == dst[i] + run) run += n[j++];
-    if (run > 0) attn_bwd_cast_kernel<<<(unsigned)((run / 8 + 255) / 256), 256, 0, stream>>>(src[i], dst[i], run);
+    while (j < 3 && run > 0 && acc[j] == acc[i] + run && dst[j] == dst[i] + run) run += n[j++];
+    if (run > 0) attn_bwd_cast_kernel<<<(unsigned)((run / 8 + 255) / 256), 256, 0, stream>>>(acc[i], dst[i], run);
     i = j;
   }
   cudaError_t e = cudaGetLastError();

@@ -491,10 +491,10 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Tensor dq_acc, dk_acc, dv_acc, dq, dk, dv;
     const bool grouped = Hq != Hk && !deterministic;
     if (grouped) {
-      // query heads of a group add into fp32 accumulators, converted at the end; accumulators and results lie back to back, so
-      // that they are cleared and converted by one launch each
+      // query heads of a group add into fp32 accumulators, cleared by the first launch and converted by the last; accumulators and
+      // results lie back to back, so that they are converted in one
       const long long nq = split ? 0 : T * Hq * D, nk = T * Hk * D, nv = T * Hk * Dv;
-      const Tensor acc = at::zeros({nq + nk + nv}, f), res = at::empty({nq + nk + nv}, dt);
+      const Tensor acc = at::empty({nq + nk + nv}, f), res = at::empty({nq + nk + nv}, dt);
       auto part = [T](const Tensor& t, long long first, long long H, long long W) { return t.narrow(0, first, T * H * W).view({T, H, W}); };
       if (split) {
         dq = empty_rows(q);
@@ -505,7 +505,7 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
       dk_acc = part(acc, nq, Hk, D); dk = part(res, nq, Hk, D);
       dv_acc = part(acc, nq + nk, Hk, Dv); dv = part(res, nq + nk, Hk, Dv);
     } else {
-      if (!split) dq_acc = at::zeros({T, Hq, D}, f);
+      if (!split) dq_acc = at::empty({T, Hq, D}, f);
       dq = empty_rows(q);
       if (split) zero_outside(dq, lo, hi);
       dk = at::empty({T, Hk, D}, dt); zero_outside(dk, lo, hi);
