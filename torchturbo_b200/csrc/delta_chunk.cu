@@ -35,14 +35,14 @@ delta_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __restric
   dc_load_gates(p, row0, n, h, sG, sB);
   dc_wait();
   __syncthreads();
-  dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
-  dc_row_norms<256>(sK, sRk, p.l2, 1.f);
+  dc_row_norms<256>(sQ, sRq, p.scale, sK, sRk, 1.f, p.l2);
   if (warp == 0) dc_cumsum(sG, lane);
   __syncthreads();
   if (tid < DC_C) sW[tid] = sB[tid] * sRk[tid] * expf(sG[tid]);
   if (tid == 0) decay[hc] = expf(sG[DC_C - 1]);
 
-  const int mi = warp & 3, m0 = mi * 16, g = lane >> 2, t2 = (lane & 3) * 2;
+  // rows 16 mi: the work on a triangle grows with mi, so the two warps of a scheduler (warp, warp + 4) take rows that add up
+  const int mi = warp < 4 ? warp : 7 - warp, m0 = mi * 16, g = lane >> 2, t2 = (lane & 3) * 2;
   {
     // scores: warps 0-3 k k^T -> L, warps 4-7 q k^T -> A, 16 rows each
     const bool is_q = warp >= 4;
@@ -367,17 +367,18 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
     }
   };
 
-  dc_load_rows<NT>(sQ, p.q + row0 * p.q_t + h / p.rep * p.q_h, p.q_t, n);
-  dc_load_rows<NT>(sK, p.k + row0 * p.k_t + h / p.rep * p.k_h, p.k_t, n);
-  dc_load_rows<NT>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
-  dc_load_gates(p, row0, n, h, sG, sB);
   float4 va[4], vb[4];
   {
+    // what does not depend on the chunk's rows is asked for first
     float4 vt[2];
     fetch(va, dX + hc * DC_C * DC_D);
     fetch(vb, X + hc * DC_C * DC_D);
 #pragma unroll
     for (int e = 0; e < 2; ++e) vt[e] = __ldg(reinterpret_cast<const float4*>(Tg + hc * DC_C * DC_C) + tid + e * NT);
+    dc_load_rows<NT>(sQ, p.q + row0 * p.q_t + h / p.rep * p.q_h, p.q_t, n);
+    dc_load_rows<NT>(sK, p.k + row0 * p.k_t + h / p.rep * p.k_h, p.k_t, n);
+    dc_load_rows<NT>(sDO, dO + (static_cast<long long>(row0) * p.H + h) * DC_D, static_cast<long long>(p.H) * DC_D, n);
+    dc_load_gates(p, row0, n, h, sG, sB);
     store(sW, va);
     store(sX, vb);
 #pragma unroll
@@ -389,8 +390,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   fetch_half(va, St + st_at, 0);                 // the first half of S is on its way while db is formed
   dc_wait();
   __syncthreads();
-  dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
-  dc_row_norms<NT>(sK, sRk, p.l2, 1.f);
+  dc_row_norms<NT>(sQ, sRq, p.scale, sK, sRk, 1.f, p.l2);
   if (warp == 0) dc_cumsum(sG, lane);
   __syncthreads();
   if (tid < DC_C) {
@@ -400,7 +400,8 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   }
   // Warp tile: 16 rows x 32 neighbouring columns, so that a row's sums are four quarters of 32 channels.  (16 columns of each half
   // of the 128 gave the same products but other roundings of those sums: 3e-4 in the 2-norm of a layer's bf16 gradients.)
-  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 16, c0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int mi = warp >> 2, cq = dc_block_col(warp);
+  const int m0 = mi * 16, n0 = cq * 16, c0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
   const int i0 = m0 + g, i1 = i0 + 8;
   auto col_of = [&](int nt) { return c0 + nt * 8 + t2; };
   // sums over a row's 128 channels: four lanes, then four warps (added in a fixed order at the end)
@@ -409,6 +410,14 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
   for (int x = 0; x < 6; ++x) part[x][0] = part[x][1] = 0.f;
   // ---- db = T^T dx; dv = beta db
   {
+    uint32_t vv[4][2];                           // this thread's v values, on their way during the product
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int i = rr ? i1 : i0;
+        vv[nt][rr] = i < n ? __ldg(reinterpret_cast<const uint32_t*>(p.v + (row0 + i) * p.v_t + h * p.v_h + col_of(nt))) : 0u;
+      }
     float acc[4][4] = {};
     for (int kk = mi; kk < 4; ++kk) {
       uint32_t a[3][4];
@@ -434,7 +443,7 @@ delta_bwd_post_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ dO
         const float x = acc[nt][2 * rr], y = acc[nt][2 * rr + 1], be = rr ? be1 : be0;
         dc_put(sDB + i * DC_QS + col, DQ_PL, x, y);
         if (i < n) {
-          const float2 v = unpack_bf16(__ldg(reinterpret_cast<const uint32_t*>(p.v + (row0 + i) * p.v_t + h * p.v_h + col)));
+          const float2 v = unpack_bf16(vv[nt][rr]);
           part[0][rr] += x * v.x + y * v.y;
           *reinterpret_cast<uint32_t*>(dV + (static_cast<long long>(row0 + i) * p.H + h) * DC_D + col) = pack_bf16(x * be, y * be);
         }

@@ -253,17 +253,49 @@ __device__ __forceinline__ void dc_load_f32(float* s, int ld, const float* src, 
     dc_copy16(s + r * ld + c, src + static_cast<long long>(r) * src_ld + c, 16);
   }
 }
-// 1 / |row| of a tile (or 1 without normalisation), times `mul`
+// 1 / |row| of a tile (or 1 without normalisation), times `mul`.  All of a warp's rows are summed before the first result is written,
+// so that their shuffles overlap; with two tiles in one call those of both.
 template <int NT>
-__device__ __forceinline__ void dc_row_norms(const __nv_bfloat16* s, float* out, int l2, float mul) {
+__device__ __forceinline__ void dc_row_squares(const __nv_bfloat16* s, float (&ss)[DC_C * 32 / NT]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = warp; r < DC_C; r += NT / 32) {
-    const uint2 u = *reinterpret_cast<const uint2*>(s + r * DC_QS + lane * 4);
+#pragma unroll
+  for (int x = 0; x < DC_C * 32 / NT; ++x) {
+    const uint2 u = *reinterpret_cast<const uint2*>(s + (warp + x * (NT / 32)) * DC_QS + lane * 4);
     const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
-    const float ss = warp_sum(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
-    if (lane == 0) out[r] = l2 ? rsqrtf(ss + 1e-6f) * mul : mul;
+    ss[x] = a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
   }
 }
+template <int NT>
+__device__ __forceinline__ void dc_row_norms(const __nv_bfloat16* s, float* out, int l2, float mul) {
+  float ss[DC_C * 32 / NT];
+  dc_row_squares<NT>(s, ss);
+#pragma unroll
+  for (int x = 0; x < DC_C * 32 / NT; ++x) ss[x] = warp_sum(ss[x]);
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int x = 0; x < DC_C * 32 / NT; ++x) out[(threadIdx.x >> 5) + x * (NT / 32)] = l2 ? rsqrtf(ss[x] + 1e-6f) * mul : mul;
+  }
+}
+template <int NT>
+__device__ __forceinline__ void dc_row_norms(const __nv_bfloat16* s0, float* out0, float mul0, const __nv_bfloat16* s1, float* out1, float mul1, int l2) {
+  float a[DC_C * 32 / NT], b[DC_C * 32 / NT];
+  dc_row_squares<NT>(s0, a);
+  dc_row_squares<NT>(s1, b);
+#pragma unroll
+  for (int x = 0; x < DC_C * 32 / NT; ++x) { a[x] = warp_sum(a[x]); b[x] = warp_sum(b[x]); }
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int x = 0; x < DC_C * 32 / NT; ++x) {
+      const int r = (threadIdx.x >> 5) + x * (NT / 32);
+      out0[r] = l2 ? rsqrtf(a[x] + 1e-6f) * mul0 : mul0;
+      out1[r] = l2 ? rsqrtf(b[x] + 1e-6f) * mul1 : mul1;
+    }
+  }
+}
+// Sixteen warps on 4 x 4 blocks of a 64-row triangle: warp w takes block row w / 4 and this block column.  The work on a triangle grows
+// (or falls) with the row, and blocks above the diagonal have none, so the four warps of a scheduler (w % 4) are one of each row, with two
+// or three blocks on or below the diagonal.  With the rows dealt out by w % 4 one scheduler had all of the longest.
+__device__ __forceinline__ int dc_block_col(int warp) { return (0xE493D2E4u >> ((warp >> 2) * 8 + (warp & 3) * 2)) & 3; }
 // inclusive cumulative sum of 64 values, by one warp
 __device__ __forceinline__ void dc_cumsum(float* s, int lane) {
   const float a = s[2 * lane], b = s[2 * lane + 1];

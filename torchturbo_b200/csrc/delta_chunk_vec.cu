@@ -83,8 +83,7 @@ delta_vec_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __res
   dc_load_rows<256>(sK, p.k + row0 * p.k_t + h * p.k_h, p.k_t, n);
   if (tid < DC_C) sB[tid] = tid < n ? __ldg(p.beta + static_cast<long long>(row0 + tid) * p.H + h) : 0.f;
   dv_cumsum<256>(p, sG, DV_G, row0, n, h);
-  dc_row_norms<256>(sQ, sRq, p.l2, p.scale);
-  dc_row_norms<256>(sK, sRk, p.l2, 1.f);
+  dc_row_norms<256>(sQ, sRq, p.scale, sK, sRk, 1.f, p.l2);
   if (tid < DC_D) {
     const float gl = sG[(DC_C - 1) * DV_G + tid];
     sGL[tid] = gl;
@@ -188,7 +187,7 @@ delta_vec_prep_kernel(const DeltaChunkIn p, float* __restrict__ Tg, float* __res
     }
   }
   // ---- u = (T beta) v and w = T (beta k^ e^G)
-  const int mi = warp & 3, m0 = mi * 16, g = lane >> 2, t2 = (lane & 3) * 2, n0 = (warp >> 2) * 64;
+  const int mi = warp < 4 ? warp : 7 - warp, m0 = mi * 16, g = lane >> 2, t2 = (lane & 3) * 2, n0 = (warp >> 2) * 64;
   {
     float acc[8][4] = {};
     for (int kk = 0; kk <= mi; ++kk) {
@@ -416,12 +415,19 @@ delta_vec_score_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
   dc_load_f32<NT, DC_C, DC_D>(sX, DV_A, X + hc * DC_C * DC_D, DC_D);
   if (tid < DC_C) sB[tid] = tid < n ? __ldg(p.beta + static_cast<long long>(row0 + tid) * p.H + h) : 0.f;
   dv_cumsum<NT>(p, sG, DV_G, row0, n, h);
-  dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
-  dc_row_norms<NT>(sK, sRk, p.l2, 1.f);
+  dc_row_norms<NT>(sQ, sRq, p.scale, sK, sRk, 1.f, p.l2);
   __syncthreads();
-  const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int mi = warp >> 2, cq = dc_block_col(warp), m0 = mi * 16, n0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
   const int i0 = m0 + g, i1 = i0 + 8;
   {
+    uint32_t vv[4][2];                           // this thread's v values, on their way during the product
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int i = rr ? i1 : i0;
+        vv[nt][rr] = i < n ? __ldg(reinterpret_cast<const uint32_t*>(p.v + (row0 + i) * p.v_t + h * p.v_h + n0 + nt * 8 + t2)) : 0u;
+      }
     float acc[4][4] = {}, part[2] = {0.f, 0.f};
     for (int kk = mi; kk < 4; ++kk) {
       uint32_t a[3][4];
@@ -443,7 +449,7 @@ delta_vec_score_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
         *reinterpret_cast<float2*>(sDB + i * DV_A + col) = make_float2(x, y);
         *reinterpret_cast<float2*>(DB + (hc * DC_C + i) * DC_D + col) = make_float2(x, y);
         if (i < n) {
-          const float2 v = unpack_bf16(__ldg(reinterpret_cast<const uint32_t*>(p.v + (row0 + i) * p.v_t + h * p.v_h + col)));
+          const float2 v = unpack_bf16(vv[nt][rr]);
           part[rr] += x * v.x + y * v.y;
           *reinterpret_cast<uint32_t*>(dV + (static_cast<long long>(row0 + i) * p.H + h) * DC_D + col) = pack_bf16(x * be, y * be);
         }
@@ -589,8 +595,7 @@ delta_vec_state_kernel(const DeltaChunkIn p, const __nv_bfloat16* __restrict__ d
   dc_load_f32<NT, DC_C, DC_D>(sDB, DV_A, DB + hc * DC_C * DC_D, DC_D);
   if (tid < DC_C) sB[tid] = tid < n ? __ldg(p.beta + static_cast<long long>(row0 + tid) * p.H + h) : 0.f;
   dv_cumsum<NT>(p, sG, DV_G, row0, n, h);
-  dc_row_norms<NT>(sQ, sRq, p.l2, p.scale);
-  dc_row_norms<NT>(sK, sRk, p.l2, 1.f);
+  dc_row_norms<NT>(sQ, sRq, p.scale, sK, sRk, 1.f, p.l2);
   __syncthreads();
   const int mi = warp & 3, m0 = mi * 16, cq = warp >> 2, n0 = cq * 32, g = lane >> 2, t2 = (lane & 3) * 2;
   const int i0 = m0 + g, i1 = i0 + 8;
