@@ -1,0 +1,52 @@
+"""The chunk recurrence of the delta rule over many short, empty and unequal sequences (more than the blocks of a launch, more than are
+sorted by length), with every combination of a first state and added gradients, against 64 bits."""
+import pytest
+import torch
+
+
+def _scan(a, b, u, dec, init, add, lens, reverse, s1, s2):
+    a, b, u, dec = (t.double() for t in (a, b, u, dec))
+    H, NC, ns = u.shape[0], u.shape[1], len(lens)
+    if dec.dim() == 2:
+        dec = dec[..., None].expand(H, NC, 128)
+    X, states = torch.zeros_like(u), torch.zeros(H, NC + ns, 128, 128, dtype=torch.float64, device=u.device)
+    c0 = 0
+    for s, n in enumerate(lens):
+        order = range(c0 + n - 1, c0 - 1, -1) if reverse else range(c0, c0 + n)
+        first = (c0 + n if reverse else c0) + s
+        S = add[:, first].double() if reverse else init[:, s].double() if init is not None else torch.zeros_like(states[:, 0])
+        states[:, first] = S
+        for c in order:
+            slot = (c if reverse else c + 1) + s
+            X[:, c] = u[:, c] + s1 * a[:, c] @ S
+            S = dec[:, c, :, None] * S + s2 * b[:, c].transpose(1, 2) @ X[:, c] + (add[:, slot].double() if add is not None else 0)
+            states[:, slot] = S
+        c0 += n
+    return X, states
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H, lens", [(1, [1]), (2, [3, 0, 5]), (3, [i % 4 for i in range(40)]), (5, [2] * 17), (1, [0] * 33 + [6])])
+@pytest.mark.parametrize("vec", [False, True])
+@pytest.mark.parametrize("with_init, with_add, reverse", [(False, False, False), (True, False, False), (False, True, False), (True, True, False),
+                                                          (False, True, True)])
+def test_against_64_bits(H, lens, vec, with_init, with_add, reverse):
+    from torchturbo_b200 import kernels as K
+
+    NC, ns, g = sum(lens), len(lens), torch.Generator("cuda").manual_seed(len(lens))
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    a, b = (rnd(H, NC, 64, 128) * 0.03).bfloat16(), (rnd(H, NC, 64, 128) * 0.03).bfloat16()
+    u, dec = rnd(H, NC, 64, 128), torch.rand(*((H, NC, 128) if vec else (H, NC)), device="cuda", generator=g)
+    init = rnd(H, ns, 128, 128) if with_init else None
+    add = rnd(H, NC + ns, 128, 128) if with_add else None
+    cu = torch.tensor([0] + lens).cumsum(0)
+    seq = torch.stack((cu[:-1], torch.tensor(lens)), 1).to(torch.int32).cuda()
+    s1, s2 = (1.0, -1.0) if reverse else (-1.0, 1.0)
+    x, states = K.delta_state_scan(a, b, u, dec, init, add, seq, reverse=reverse, s1=s1, s2=s2)
+    want_x, want_s = _scan(a, b, u, dec, init, add, lens, reverse, s1, s2)
+    # S and X enter the products rounded to bf16 (2^-9 of each element), a chunk after the other, and nothing grows from chunk to chunk
+    bound = 2.0 ** -8 * max(lens)
+    for got, want in ((x, want_x), (states, want_s)):
+        assert (got.double() - want).norm() <= bound * want.norm()
+    again = K.delta_state_scan(a, b, u, dec, init, add, seq, reverse=reverse, s1=s1, s2=s2)
+    assert torch.equal(x, again[0]) and torch.equal(states, again[1])

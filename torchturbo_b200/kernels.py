@@ -656,6 +656,8 @@ def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, r
     if add is not None:
         add = add.contiguous()
         assert add.shape == (H, NC + nseq, 128, 128) and add.dtype == torch.float32
+    # the copy engine moves whole rows: tensors that start between 16-byte boundaries are copied
+    u, decay, init, add, seq_chunks_dev = (t if t is None or t.data_ptr() % 16 == 0 else t.clone() for t in (u, decay, init, add, seq_chunks_dev))
     x = torch.empty_like(u)
     states = torch.empty(H, NC + nseq, 128, 128, dtype=torch.float32, device=u.device)
     _check(lib().ttb_delta_state_scan(_p(a_tiles), _p(b_tiles), _p(u), _p(x), _p(decay), C.c_int(int(decay.dim() == 3)),
