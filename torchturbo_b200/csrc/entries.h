@@ -57,6 +57,9 @@ TTB_EXPORT int ttb_qknorm_rope_fwd(const void*, long long, int, int, int, const 
 TTB_EXPORT int ttb_qknorm_rope_bwd(const void*, const void*, const void*, const void*, long long, int, int, int, const void*,
                             const void*, const float*, const float*, const float*, void*, long long, float*, void*, int, long
                             long, int, int, void*);
+TTB_EXPORT int ttb_qkv_rope_fwd(const void*, const void*, const float*, const float*, void*, void*, void*, long long, int, int, int, void*);
+TTB_EXPORT int ttb_qkv_rope_bwd(const void*, const void*, const void*, const float*, const float*, void*, float*, void*, int, long long, int,
+                            int, int, void*);
 TTB_EXPORT int ttb_rope(const void*, long long, long long, const float*, const float*, void*, long long, int, int, float,
                             void*);
 TTB_EXPORT int ttb_swiglu_fwd(const void*, long long, void*, long long, const float*, long long, int, const int*, void*);

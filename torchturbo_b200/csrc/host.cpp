@@ -382,6 +382,42 @@ PyObject* qknorm_rope_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   });
 }
 
+PyObject* qkv_rope_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 5);
+    const Tensor &x = in.tensor(), &bias = in.tensor();
+    const int heads = static_cast<int>(in.integer());
+    const Tensor &cos = in.tensor(), &sin = in.tensor();
+    const long long T = x.size(0), D = x.size(1) / (3 * heads);
+    need(x.dim() == 2 && x.is_contiguous() && bias.is_contiguous() && bias.numel() == x.size(1) && D * 3 * heads == x.size(1), "a row is q, k and v of all heads");
+    const auto dt = x.scalar_type();
+    const Tensor q = empty({T, heads, D}, dt, x), k = empty({T, heads, D}, dt, x), v = empty({T, heads, D}, dt, x);
+    launch("ttb_qkv_rope_fwd", 1, [&](void* st) {
+      return ttb_qkv_rope_fwd(at_(x), at_(bias), f32(cos), f32(sin), to_(q), to_(k), to_(v), T, heads, static_cast<int>(D / 2),
+                              static_cast<int>(std::max<long long>(1, std::min<long long>(T, 4 * sms(x)))), st);
+    });
+    return wrap_all(q, k, v);
+  });
+}
+
+PyObject* qkv_rope_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 6);
+    const Tensor &dq = in.tensor(), &dk = in.tensor(), &dv = in.tensor(), &cos = in.tensor(), &sin = in.tensor();
+    const bool f32out = in.flag();
+    const long long T = dq.size(0), heads = dq.size(1), D = dq.size(2), W = 3 * heads * D;
+    need(dq.is_contiguous() && dk.is_contiguous() && dv.is_contiguous() && dk.sizes() == dq.sizes() && dv.sizes() == dq.sizes(), "gradients of one shape");
+    const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(T, 2 * sms(dq))));
+    const Tensor dx = empty({T, W}, dq.scalar_type(), dq), part = empty({grid, W}, at::kFloat, dq);
+    const Tensor db = T ? empty({W}, out_type(f32out), dq) : at::zeros({W}, plain(dq).dtype(out_type(f32out)));
+    launch("ttb_qkv_rope_bwd", 2, [&](void* st) {
+      return ttb_qkv_rope_bwd(at_(dq), at_(dk), at_(dv), f32(cos), f32(sin), to_(dx), f32w(part), to_(db), !f32out, T, static_cast<int>(heads),
+                              static_cast<int>(D / 2), grid, st);
+    });
+    return wrap_all(dx, db);
+  });
+}
+
 PyObject* rope(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args in(args, n, 4);
@@ -541,7 +577,7 @@ PyObject* launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_From
 
 #define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ENTRY(setup), ENTRY(launches), ENTRY(gemm), ENTRY(rmsnorm_fwd), ENTRY(rmsnorm_bwd), ENTRY(layernorm_fwd), ENTRY(layernorm_bwd),
-                         ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(rope), ENTRY(swiglu_fwd),
+                         ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(rope), ENTRY(swiglu_fwd),
                          ENTRY(swiglu_bwd), ENTRY(attn_fwd), ENTRY(attn_bwd), {nullptr, nullptr, 0, nullptr}};
 #undef ENTRY
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "ttb_host", nullptr, -1, methods};

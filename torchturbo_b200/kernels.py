@@ -315,6 +315,16 @@ def qknorm_rope_bwd(dq, dk, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dq
     return host().qknorm_rope_bwd(dq, dk, dv, qkv, n_q, n_kv, head_dim, wq, wk, cos, sin, rstd, dqkv, use_norm, dw_dtype != torch.bfloat16)
 
 
+def qkv_rope_fwd(x, bias, heads, cos, sin):
+    """x: [T, 3 * heads * D] -> q, k = RoPE(x + bias), v = x + bias, each [T, heads, D]; cos, sin fp32 [T, D / 2]."""
+    return host().qkv_rope_fwd(x, bias, heads, cos, sin)
+
+
+def qkv_rope_bwd(dq, dk, dv, cos, sin, db_dtype=torch.float32):
+    """Returns (dx [T, 3 * heads * D], dbias in ``db_dtype``: fp32 or bf16)."""
+    return host().qkv_rope_bwd(dq, dk, dv, cos, sin, db_dtype != torch.bfloat16)
+
+
 def rope(x, cos, sin, sign: float = 1.0):
     """Half-rotation RoPE of bf16 [T, heads, D] (channels contiguous); cos, sin fp32 [T, D / 2].  ``sign=-1`` rotates back."""
     return host().rope(x, cos, sin, sign)

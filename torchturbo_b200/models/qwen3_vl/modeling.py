@@ -113,14 +113,12 @@ class VisionBlock(nn.Module):
         self.act = _ACTS[getattr(cfg, "hidden_act", "gelu_pytorch_tanh")]
 
     def forward(self, x, cos, sin, cu, max_len):
-        """Biases, GELU and residual adds ride on `ops.bias_act` (one pass after each GEMM), the norms on
-        `ops.layer_norm`; attention is full (non-causal) over each frame's patches."""
+        """Biases, GELU and residual adds ride on `ops.bias_act` (one pass after each GEMM) and, with the rotary embedding, on
+        `ops.qkv_bias_rope`, the norms on `ops.layer_norm`; attention is full (non-causal) over each frame's patches."""
         P = x.shape[0]
         a, m = self.attn, self.mlp
         h = ops.layer_norm(x, self.norm1.weight, self.norm1.bias, self.norm1.eps)
-        qkv = ops.bias_act(ops.linear(h, a.qkv.weight), a.qkv.bias).view(P, 3, self.n_heads, self.head_dim)
-        q, k, v = qkv[:, 0], qkv[:, 1], qkv[:, 2]
-        q, k = ops.rotary_position_embedding(q, cos, sin), ops.rotary_position_embedding(k, cos, sin)
+        q, k, v = ops.qkv_bias_rope(ops.linear(h, a.qkv.weight), a.qkv.bias, self.n_heads, cos, sin)
         o = ops.attention(q.contiguous(), k.contiguous(), v.contiguous(), cu, max_len, causal=False,
                           scale=1.0 / math.sqrt(self.head_dim))
         x = ops.bias_act(ops.linear(o.reshape(P, -1), a.proj.weight), a.proj.bias, residual=x)

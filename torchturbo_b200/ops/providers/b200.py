@@ -441,6 +441,40 @@ class B200RoPE(_B200Op):
         return RopeFn.apply(x, _aligned(cos.float()), _aligned(sin.float()), 1.0)
 
 
+class QKVBiasRopeFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, bias, heads, cos, sin):
+        ctx.save_for_backward(bias, cos, sin)
+        ctx.heads = heads
+        return K.qkv_rope_fwd(x, bias, heads, cos, sin)
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        bias, cos, sin = ctx.saved_tensors
+        if torch.is_grad_enabled():              # a graph of the gradient is wanted: by way of the separate operations
+            dx = torch.stack((RopeFn.apply(dq, cos, sin, -1.0), RopeFn.apply(dk, cos, sin, -1.0), dv), 1).flatten(1)
+            return dx, dx.float().sum(0).to(bias.dtype), None, None, None
+        dx, db = K.qkv_rope_bwd(_aligned(dq), _aligned(dk), _aligned(dv), cos, sin, db_dtype=bias.dtype)
+        return dx, db, None, None, None
+
+
+@_custom("qkv_bias_rope", "b200_qkv_bias_rope")
+class B200QKVBiasRope(_B200Op):
+    """One pass each way between the projection and the attention kernel, which takes the three results as they are."""
+
+    parts = {"bias_act", "rotary_position_embedding"}
+
+    def __call__(self, x, bias, heads, cos, sin):
+        from ..ops import get_or_create_ops
+
+        W = x.shape[-1]
+        if not self.parts.isdisjoint(get_or_create_ops().overrides) or not _ok(x, bias) or x.dim() != 2 or W % (24 * heads) or W > 8 * 2048 or bias.shape != (W,) \
+                or cos.shape != (x.shape[0], W // (6 * heads)) or sin.shape != cos.shape or not (cos.is_cuda and sin.is_cuda) \
+                or cos.requires_grad or sin.requires_grad or not _eager(x, bias, cos, sin):
+            return N.TorchQKVBiasRope()(x, bias, heads, cos, sin)
+        return QKVBiasRopeFn.apply(_aligned(x), _aligned(bias), heads, _aligned(cos.float()), _aligned(sin.float()))
+
+
 # ------------------------------------------------------------------------------------------------
 # MoE: router, permutation, experts
 # ------------------------------------------------------------------------------------------------

@@ -88,6 +88,17 @@ class TorchBiasAct(OpImpl):
         return bias_act_ref(x, bias, act, residual)
 
 
+@_native("qkv_bias_rope")
+class TorchQKVBiasRope(OpImpl):
+    """Bias of a fused `[q | k | v]` projection, split into heads, rotary embedding of q and k: three `[T, heads, D]` tensors."""
+
+    def __call__(self, x, bias, heads, cos, sin):
+        from ..ops import ops
+
+        q, k, v = ops.bias_act(x, bias).view(x.shape[0], 3, heads, -1).unbind(1)
+        return ops.rotary_position_embedding(q, cos, sin), ops.rotary_position_embedding(k, cos, sin), v
+
+
 def swiglu_ref(x, probs=None):
     gate, up = x.chunk(2, dim=-1)
     y = F.silu(gate) * up
