@@ -50,3 +50,21 @@ def test_against_64_bits(H, lens, vec, with_init, with_add, reverse):
         assert (got.double() - want).norm() <= bound * want.norm()
     again = K.delta_state_scan(a, b, u, dec, init, add, seq, reverse=reverse, s1=s1, s2=s2)
     assert torch.equal(x, again[0]) and torch.equal(states, again[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H, lens", [(2, [3, 0, 5]), (3, [i % 4 for i in range(40)])])
+def test_a_first_state_of_zero_is_not_read(H, lens):
+    from torchturbo_b200 import kernels as K
+
+    NC, ns, g = sum(lens), len(lens), torch.Generator("cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    a, b = (rnd(H, NC, 64, 128) * 0.03).bfloat16(), (rnd(H, NC, 64, 128) * 0.03).bfloat16()
+    u, dec, add = rnd(H, NC, 64, 128), torch.rand(H, NC, device="cuda", generator=g), rnd(H, NC + ns, 128, 128)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    seq = torch.stack((cu[:-1], torch.tensor(lens)), 1).to(torch.int32).cuda()
+    last = (cu[1:] + torch.arange(ns)).cuda()
+    kw = dict(reverse=True, s1=1.0, s2=-1.0)
+    want = K.delta_state_scan(a, b, u, dec, None, add.index_fill(1, last, 0.0), seq, **kw)
+    got = K.delta_state_scan(a, b, u, dec, None, add.index_fill(1, last, float("nan")), seq, zero_first=True, **kw)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

@@ -48,7 +48,8 @@ struct DeltaStateParams {
   const float* decay;    // [H, NC] or [H, NC, 128]
   const int* seq_chunks; // [nseq, 2]: first chunk, number of chunks
   int nseq, H, NC, items;
-  int vec, reverse, add, init;
+  int vec, reverse, add;
+  int first;             // state before the first chunk: 0 zero, 1 from `add` (reverse), 2 from `init`
   float s1, s2;
 };
 
@@ -148,7 +149,7 @@ delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const int slot = (p.reverse ? x.c0 + x.n - 1 - i : x.c0 + i + 1) + x.seq;
     return (x.h * slots + slot) * DS_D;
   };
-  const bool first_loaded = p.reverse || p.init;      // the state before the first chunk comes from memory, else it is zero
+  const bool first_loaded = p.first != 0;
   const bool gated = p.add || first_loaded;           // the loading warp hands out the places of the states, with or without data in them
   // counters of this role's chunks (t) and states (g: one more per item); slot = count & 1, phase = (count >> 1) & 1
   uint32_t t = 0, g = 0;
@@ -173,7 +174,7 @@ delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           return true;
         };
         if (gated) {
-          ok = p.reverse ? hand_out(&tmG, state_row(x, -1)) : hand_out(p.init ? &tmI : nullptr, (x.h * p.nseq + x.seq) * DS_D);
+          ok = p.first == 1 ? hand_out(&tmG, state_row(x, -1)) : hand_out(p.first ? &tmI : nullptr, (x.h * p.nseq + x.seq) * DS_D);
           if (!ok) break;
         }
         ++g;
@@ -380,7 +381,8 @@ delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 using namespace ttb;
 
 // A, B: bf16 [H * NC * 64, 128] (chunk-major rows); U, X: fp32 [H, NC, 64, 128]; decay fp32 [H, NC] or [H, NC, 128];
-// init fp32 [H, nseq, 128, 128] or null; add, states fp32 [H, NC + nseq, 128, 128] (add may be null when forward).
+// init fp32 [H, nseq, 128, 128] or null; add, states fp32 [H, NC + nseq, 128, 128] (add may be null when forward).  reverse: 0, 1, or
+// 2 for a first state of zero, whose slot of `add` is then not read.
 TTB_EXPORT int ttb_delta_state_scan(const void* A, const void* B, const float* U, float* X, const float* decay, int vec,
                                     const float* init, const float* add, float* states, const int* seq_chunks, int nseq,
                                     int H, int NC, int reverse, float s1, float s2, void* stream_ptr) {
@@ -407,7 +409,8 @@ TTB_EXPORT int ttb_delta_state_scan(const void* A, const void* B, const float* U
   }
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 301;
-  DeltaStateParams p{decay, seq_chunks, nseq, H, NC, static_cast<int>(items), vec, reverse, add != nullptr, init != nullptr && !reverse, s1, s2};
+  DeltaStateParams p{decay, seq_chunks, nseq, H, NC, static_cast<int>(items), vec, reverse != 0, add != nullptr,
+                     reverse == 1 ? 1 : !reverse && init ? 2 : 0, s1, s2};
   static bool done[16] = {};
   const cudaError_t es = ensure_dynamic_smem(reinterpret_cast<const void*>(delta_state_kernel), DsSmem::TOTAL, done);
   if (es != cudaSuccess) return 300 + static_cast<int>(es);

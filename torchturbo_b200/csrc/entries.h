@@ -57,6 +57,10 @@ TTB_EXPORT int ttb_qknorm_rope_fwd(const void*, long long, int, int, int, const 
 TTB_EXPORT int ttb_qknorm_rope_bwd(const void*, const void*, const void*, const void*, long long, int, int, int, const void*,
                             const void*, const float*, const float*, const float*, void*, long long, float*, void*, int, long
                             long, int, int, void*);
+TTB_EXPORT int ttb_gdn_gate_fwd(const void*, long long, const void*, long long, const void*, int, const void*, int, float*, float*, long long,
+                            int, void*);
+TTB_EXPORT int ttb_gdn_gate_bwd(const float*, const float*, const void*, long long, const void*, int, const void*, int, const float*, void*,
+                            void*, float*, void*, int, long long, int, int, void*);
 TTB_EXPORT int ttb_qkv_rope_fwd(const void*, const void*, const float*, const float*, void*, void*, void*, long long, int, int, int, void*);
 TTB_EXPORT int ttb_qkv_rope_bwd(const void*, const void*, const void*, const float*, const float*, void*, float*, void*, int, long long, int,
                             int, int, void*);

@@ -161,6 +161,57 @@ kda_gate_bwd_kernel(const float* __restrict__ dd, const __nv_bfloat16* __restric
   part[(blockIdx.y * 2 + 1) * step + col] = sum_a;
 }
 
+// ============================================================================
+// Gates of a gated delta net, per head, from the two raw projections (bf16 [rows, H], any row stride):
+//   g = -exp(A_h) softplus(a + dt_h),   beta = sigmoid(b),   fp32 [rows, H]
+// The backward returns da and db and the sums behind d(A) and d(dt).  131,000 elements for 4096 tokens and 32 heads are no work for the
+// chip: what counts is the number of launches, one forward and two backward here, ten and fifteen in torch (4096 x 32: 47 -> 4 us and
+// 65 -> 9 us with their gaps).  The same fp32 functions as torch's, softplus the identity above 20.
+// ============================================================================
+__global__ void __launch_bounds__(256)
+gdn_gate_fwd_kernel(const __nv_bfloat16* __restrict__ a, long long a_t, const __nv_bfloat16* __restrict__ b, long long b_t,
+                    const void* __restrict__ A, int a_bf16, const void* __restrict__ dt, int dt_bf16, float* __restrict__ g,
+                    float* __restrict__ beta, long long rows, int H) {
+  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= rows * H) return;
+  const long long r = idx / H;
+  const int h = static_cast<int>(idx - r * H);
+  const float x = __bfloat162float(a[r * a_t + h]) + load_scalar(dt, h, dt_bf16), y = __bfloat162float(b[r * b_t + h]);
+  g[idx] = -expf(load_scalar(A, h, a_bf16)) * (x > 20.f ? x : log1pf(expf(x)));
+  beta[idx] = 1.f / (1.f + expf(-y));
+}
+
+// 32 heads and a share of the rows per block; part: fp32 [blocks, 2, H], d(A) then d(dt)
+__global__ void __launch_bounds__(256)
+gdn_gate_bwd_kernel(const float* __restrict__ dg, const float* __restrict__ dbeta, const __nv_bfloat16* __restrict__ a, long long a_t,
+                    const void* __restrict__ A, int a_bf16, const void* __restrict__ dt, int dt_bf16, const float* __restrict__ beta,
+                    __nv_bfloat16* __restrict__ da, __nv_bfloat16* __restrict__ db, float* __restrict__ part, long long rows, int H) {
+  __shared__ float red[2][8][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, h = blockIdx.x * 32 + x;
+  float sum_a = 0.f, sum_dt = 0.f;
+  if (h < H) {
+    const float e = expf(load_scalar(A, h, a_bf16)), t = load_scalar(dt, h, dt_bf16);
+    for (long long r = static_cast<long long>(blockIdx.y) * 8 + y; r < rows; r += static_cast<long long>(gridDim.y) * 8) {
+      const float z = __bfloat162float(a[r * a_t + h]) + t, d = dg[r * H + h], s = beta[r * H + h], ez = expf(z);
+      const bool linear = z > 20.f;
+      const float dz = -d * e * (linear ? 1.f : ez / (ez + 1.f));
+      sum_a += -d * e * (linear ? z : log1pf(ez));
+      sum_dt += dz;
+      da[r * H + h] = __float2bfloat16(dz);
+      db[r * H + h] = __float2bfloat16(dbeta[r * H + h] * (1.f - s) * s);
+    }
+  }
+  red[0][y][x] = sum_a;
+  red[1][y][x] = sum_dt;
+  __syncthreads();
+  if (y < 2 && h < H) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += red[y][i][x];
+    part[(static_cast<long long>(blockIdx.y) * 2 + y) * H + h] = s;
+  }
+}
+
 }  // namespace ttb
 
 using namespace ttb;
@@ -234,5 +285,26 @@ TTB_EXPORT int ttb_kda_gate_bwd(const float* dd, const void* g, const void* A, i
   kda_gate_bwd_kernel<<<dim3(H, blocks), 128, 0, STREAM(stream)>>>(dd, (const __nv_bfloat16*)g, A, a_bf16, dt, dt_bf16,
                                                                   (__nv_bfloat16*)dg, part, rows, H, bounded, bound, per);
   colsum(part, sums, 0, blocks, 2 * H * 128, STREAM(stream));
+  LAUNCH_RET();
+}
+
+// a, b: bf16 [rows, H] with row strides a_t, b_t; A, dt: [H] fp32 or bf16; g, beta: fp32 [rows, H]
+TTB_EXPORT int ttb_gdn_gate_fwd(const void* a, long long a_t, const void* b, long long b_t, const void* A, int a_bf16, const void* dt, int dt_bf16,
+                                float* g, float* beta, long long rows, int H, void* stream) {
+  const long long n = rows * H;
+  if (n == 0) return 0;
+  gdn_gate_fwd_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, STREAM(stream)>>>((const __nv_bfloat16*)a, a_t, (const __nv_bfloat16*)b, b_t, A,
+                                                                                       a_bf16, dt, dt_bf16, g, beta, rows, H);
+  LAUNCH_RET();
+}
+
+// da, db: bf16 [rows, H] contiguous; part: fp32 [blocks, 2, H]; sums: [2, H] (d(A), d(dt)), fp32 or bf16
+TTB_EXPORT int ttb_gdn_gate_bwd(const float* dg, const float* dbeta, const void* a, long long a_t, const void* A, int a_bf16, const void* dt,
+                                int dt_bf16, const float* beta, void* da, void* db, float* part, void* sums, int out_bf16, long long rows, int H,
+                                int blocks, void* stream) {
+  if (rows == 0 || H == 0) return 0;
+  gdn_gate_bwd_kernel<<<dim3((H + 31) / 32, blocks), 256, 0, STREAM(stream)>>>(dg, dbeta, (const __nv_bfloat16*)a, a_t, A, a_bf16, dt, dt_bf16, beta,
+                                                                             (__nv_bfloat16*)da, (__nv_bfloat16*)db, part, rows, H);
+  colsum(part, sums, out_bf16, blocks, 2 * H, STREAM(stream));
   LAUNCH_RET();
 }

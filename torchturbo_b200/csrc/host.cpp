@@ -465,6 +465,45 @@ PyObject* swiglu_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// gates of a gated delta net
+// ---------------------------------------------------------------------------------------------
+bool plain_type(const Tensor& t) { return is_bf16(t) || t.scalar_type() == at::kFloat; }
+
+PyObject* gdn_gate_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 4);
+    const Tensor &a = in.tensor(), &b = in.tensor(), &A = in.tensor(), &dt = in.tensor();
+    const long long T = a.size(0), H = a.size(1);
+    need(is_bf16(a) && is_bf16(b) && b.sizes() == a.sizes() && (H == 1 || (a.stride(1) == 1 && b.stride(1) == 1)), "projections: bf16 rows of heads");
+    need(A.numel() == H && dt.numel() == H && A.is_contiguous() && dt.is_contiguous() && plain_type(A) && plain_type(dt), "one value per head");
+    const Tensor g = empty({T, H}, at::kFloat, a), beta = empty({T, H}, at::kFloat, a);
+    launch("ttb_gdn_gate_fwd", 1, [&](void* st) {
+      return ttb_gdn_gate_fwd(at_(a), a.stride(0), at_(b), b.stride(0), at_(A), is_bf16(A), at_(dt), is_bf16(dt), f32w(g), f32w(beta), T,
+                              static_cast<int>(H), st);
+    });
+    return wrap_all(g, beta);
+  });
+}
+
+PyObject* gdn_gate_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 7);
+    const Tensor &dg = in.tensor(), &dbeta = in.tensor(), &a = in.tensor(), &A = in.tensor(), &dt = in.tensor(), &beta = in.tensor();
+    const bool f32out = in.flag();
+    const long long T = a.size(0), H = a.size(1);
+    need(dg.is_contiguous() && dbeta.is_contiguous() && dg.scalar_type() == at::kFloat && dbeta.scalar_type() == at::kFloat, "gradients: fp32 rows of heads");
+    const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((T + 7) / 8, 2 * sms(a))));
+    const Tensor da = empty({T, H}, at::kBFloat16, a), db = empty({T, H}, at::kBFloat16, a), part = empty({blocks, 2, H}, at::kFloat, a);
+    const Tensor sums = T ? empty({2, H}, out_type(f32out), a) : at::zeros({2, H}, plain(a).dtype(out_type(f32out)));
+    launch("ttb_gdn_gate_bwd", 2, [&](void* st) {
+      return ttb_gdn_gate_bwd(f32(dg), f32(dbeta), at_(a), a.stride(0), at_(A), is_bf16(A), at_(dt), is_bf16(dt), f32(beta), to_(da), to_(db),
+                              f32w(part), to_(sums), !f32out, T, static_cast<int>(H), blocks, st);
+    });
+    return wrap_all(da, db, sums.select(0, 0), sums.select(0, 1));
+  });
+}
+
+// ---------------------------------------------------------------------------------------------
 // attention
 // ---------------------------------------------------------------------------------------------
 // Rows that no sequence covers read as zero; [lo, hi) = covered rows, lo < 0 = unknown.
@@ -577,7 +616,8 @@ PyObject* launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_From
 
 #define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ENTRY(setup), ENTRY(launches), ENTRY(gemm), ENTRY(rmsnorm_fwd), ENTRY(rmsnorm_bwd), ENTRY(layernorm_fwd), ENTRY(layernorm_bwd),
-                         ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(rope), ENTRY(swiglu_fwd),
+                         ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(gdn_gate_fwd),
+                         ENTRY(gdn_gate_bwd), ENTRY(rope), ENTRY(swiglu_fwd),
                          ENTRY(swiglu_bwd), ENTRY(attn_fwd), ENTRY(attn_bwd), {nullptr, nullptr, 0, nullptr}};
 #undef ENTRY
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "ttb_host", nullptr, -1, methods};

@@ -359,6 +359,16 @@ def kda_gate_bwd(dd, g, A_log, dt_bias, lower_bound):
     return dg, sums[0], sums[1].view(H, D)
 
 
+def gdn_gate_fwd(a, b, A_log, dt_bias):
+    """(g = -exp(A_log) softplus(a + dt_bias), beta = sigmoid(b)), fp32 [T, H], of bf16 projections [T, H]."""
+    return host().gdn_gate_fwd(a, b, A_log, dt_bias)
+
+
+def gdn_gate_bwd(dg, dbeta, a, A_log, dt_bias, beta, dtype=torch.float32):
+    """(da, db bf16, d(A_log), d(dt_bias) in ``dtype``: fp32 or bf16)."""
+    return host().gdn_gate_bwd(dg, dbeta, a, A_log, dt_bias, beta, dtype != torch.bfloat16)
+
+
 # --------------------------------------------------------------------------------------
 # SwiGLU
 # --------------------------------------------------------------------------------------
@@ -649,10 +659,11 @@ def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_ls
     return host().attn_fwd(q, k, v, q_tiles_dev, scale, causal, want_lse, want_max_logit, *_covered(rows), tile_rows)
 
 
-def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, reverse: bool, s1: float, s2: float):
+def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, reverse: bool, s1: float, s2: float, zero_first: bool = False):
     """Chunk-state recurrence of the delta rule (csrc/delta_state.cu).  `a_tiles`, `b_tiles`: bf16 [H, NC, 64, 128];
     `u`: fp32 [H, NC, 64, 128]; `decay`: fp32 [H, NC] or [H, NC, 128]; `init`: fp32 [H, nseq, 128, 128] or None;
-    `add`: fp32 [H, NC + nseq, 128, 128] (required when `reverse`); `seq_chunks_dev`: int32 [nseq, 2].
+    `add`: fp32 [H, NC + nseq, 128, 128] (required when `reverse`); `seq_chunks_dev`: int32 [nseq, 2].  A reverse pass starts from the
+    last slots of `add`, with `zero_first` from zero (those slots are not read).
     Returns (x fp32 [H, NC, 64, 128], states fp32 [H, NC + nseq, 128, 128])."""
     H, NC, Cc, D = u.shape
     nseq = seq_chunks_dev.shape[0]
@@ -672,7 +683,7 @@ def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, r
     states = torch.empty(H, NC + nseq, 128, 128, dtype=torch.float32, device=u.device)
     _check(lib().ttb_delta_state_scan(_p(a_tiles), _p(b_tiles), _p(u), _p(x), _p(decay), C.c_int(int(decay.dim() == 3)),
                                       _p(init), _p(add), _p(states), _p(seq_chunks_dev), C.c_int(nseq), C.c_int(H),
-                                      C.c_int(NC), C.c_int(int(reverse)), C.c_float(s1), C.c_float(s2), _stream()),
+                                      C.c_int(NC), C.c_int((2 if zero_first else 1) if reverse else 0), C.c_float(s1), C.c_float(s2), _stream()),
            "ttb_delta_state_scan")
     return x, states
 

@@ -22,7 +22,6 @@ from typing import Any, Optional
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
 from ...ops import ops
 from .attention.ulysses import gather_heads_scatter_seq, gather_seq_scatter_heads, ulysses_attention
@@ -159,10 +158,8 @@ class GatedDeltaNet(nn.Module):
         sp, r = ctx.sp_size, ctx.sp_rank
         if sp > 1 and (self.n_k % sp or self.n_v % sp):
             raise ValueError(f"linear-attention heads ({self.n_k} key / {self.n_v} value) must divide by sp={sp}")
-        qkv = ops.linear(x, self.in_proj_qkv.weight)
-        z = ops.linear(x, self.in_proj_z.weight).view(T, self.n_v, self.dv)
-        b = ops.linear(x, self.in_proj_b.weight)
-        a = ops.linear(x, self.in_proj_a.weight)
+        qkv, z, b, a = ops.linears(x, self.in_proj_qkv.weight, self.in_proj_z.weight, self.in_proj_b.weight, self.in_proj_a.weight)
+        z = z.view(T, self.n_v, self.dv)
         w = self.conv1d.weight.squeeze(1)
         A_log, dt_bias = self.A_log, self.dt_bias
         Tg, hk, hv = T, self.n_k, self.n_v
@@ -183,8 +180,8 @@ class GatedDeltaNet(nn.Module):
         # views of the one row (an index into the batch dimension would cost a cleared buffer and a copy in the backward)
         q, k, v = mixed.squeeze(0).split([hk * self.dk, hk * self.dk, hv * self.dv], dim=-1)
         q, k, v = q.reshape(1, Tg, hk, self.dk), k.reshape(1, Tg, hk, self.dk), v.reshape(1, Tg, hv, self.dv)
-        beta = torch.sigmoid(b.float()).unsqueeze(0)
-        g = (-A_log.float().exp() * F.softplus(a.float() + dt_bias.float())).unsqueeze(0)
+        g, beta = ops.gdn_gates(a, b, A_log, dt_bias)
+        g, beta = g.unsqueeze(0), beta.unsqueeze(0)
         shared = dict(heads_per_key=hv // hk) if hv // hk > 1 else {}        # every key head serves hv / hk value heads
         o, _ = ops.gated_delta_rule(q, k, v, g, beta, use_qk_l2norm_in_kernel=True, cu_seqlens=cu, **shared)
         o = o.squeeze(0)                                                    # [Tg, hv, dv]

@@ -92,6 +92,73 @@ class B200Linear(_B200Op):
         return LinearFn.apply(x, weight, residual)
 
 
+class LinearsFn(torch.autograd.Function):
+    """Several projections of the same rows.  Their input gradients add up in the products' epilogues instead of in passes of their
+    own, and projections of up to 64 columns share one product each way: alone, each is a product of a fraction of a tile.  4096 x
+    2048 rows onto 8192 + 4096 + 32 + 32 columns: the three sums took 24 us, the narrow products 64 of which 50 are left."""
+
+    NARROW = 64
+
+    @staticmethod
+    def forward(ctx, x, *ws):
+        x2 = x.reshape(-1, x.shape[-1])
+        narrow = [i for i, w in enumerate(ws) if w.shape[0] <= LinearsFn.NARROW]
+        if len(narrow) < 2:
+            narrow = []
+        joint = torch.cat([ws[i] for i in narrow]) if narrow else None
+        ys = [None if i in narrow else K.gemm(x2, w) for i, w in enumerate(ws)]
+        for i, y in zip(narrow, K.gemm(x2, joint).split([ws[i].shape[0] for i in narrow], 1) if narrow else ()):
+            ys[i] = y
+        ctx.save_for_backward(x2, joint, *ws)
+        ctx.narrow, ctx.x_shape = narrow, x.shape
+        ctx.set_materialize_grads(False)
+        return tuple(y.view(*x.shape[:-1], y.shape[1]) for y in ys)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x2, joint, *ws = ctx.saved_tensors
+        dx, dws, parts = None, [None] * len(ws), []
+        for i, (dy, w) in enumerate(zip(dys, ws)):
+            if i not in ctx.narrow and dy is not None:
+                parts.append((i, _rows(dy), w))
+        live = [i for i in ctx.narrow if dys[i] is not None]
+        if live:
+            whole = len(live) == len(ctx.narrow)
+            dy = torch.cat([_rows(dys[i]) for i in live], 1)
+            parts.append((live, dy, joint if whole else torch.cat([ws[i] for i in live])))
+        # the first product writes dx, the others add to it; the shortest first, as a long one hides its sums behind its products
+        for i, dy, w in sorted(parts, key=lambda part: part[1].shape[1]):
+            if ctx.needs_input_grad[0]:
+                dx = K.gemm(dy, w, b_mn=True) if dx is None else K.gemm(dy, w, b_mn=True, out=dx, accumulate=True)
+            if not isinstance(i, list):
+                if ctx.needs_input_grad[1 + i]:
+                    dws[i] = _weight_grad(w, dy, x2)
+                continue
+            sizes = [ws[n].shape[0] for n in i]
+            if any(getattr(ws[n], "main_grad", None) is not None or not ctx.needs_input_grad[1 + n] for n in i):
+                for n, d in zip(i, dy.split(sizes, 1)):
+                    if ctx.needs_input_grad[1 + n]:
+                        dws[n] = _weight_grad(ws[n], d, x2)
+            else:
+                for n, d in zip(i, K.gemm(dy, x2, a_mn=True, b_mn=True).split(sizes)):
+                    dws[n] = d
+        return (dx.view(ctx.x_shape) if dx is not None else None, *dws)
+
+
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    return t.reshape(-1, t.shape[-1]).contiguous()
+
+
+@_custom("linears", "tcgen05_linears")
+class B200Linears(_B200Op):
+    def __call__(self, x, *weights):
+        from ..ops import get_or_create_ops
+
+        if "linear" in get_or_create_ops().overrides or not _ok(x, *weights) or x.shape[-1] % 8 or any(w.shape[0] % 8 for w in weights):
+            return N.TorchLinears()(x, *weights)
+        return LinearsFn.apply(x, *weights)
+
+
 class RouterGatingFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):

@@ -30,8 +30,8 @@ from ... import kernels as K
 from ...runtime import TurboDevice
 from ..base import OpImpl, OpImplKind
 from ..registry import register_op
-from .b200 import _aligned
-from .native_linear_attention import _bounds, kda_gate, l2norm, repeat_key_heads
+from .b200 import _aligned, _eager
+from .native_linear_attention import _bounds, gdn_gates_ref, kda_gate, l2norm, repeat_key_heads
 
 CHUNK = 64
 
@@ -112,7 +112,7 @@ class ChunkDelta(torch.autograd.Function):
     or None; `tables` = (seq_chunks, chunk_rows, last slots, first slots) on the device."""
 
     @staticmethod
-    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2):
+    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2, want_final):
         seq, chunk_rows, last, first = tables
         kw = dict(l2=l2, scale=scale)
         T, A, u, w, k_out, decay = K.delta_prep(q, k, v, g, beta, chunk_rows, **kw)
@@ -121,7 +121,7 @@ class ChunkDelta(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, g, beta, T, A, w, k_out, decay, x, states, seq, chunk_rows, last, first)
         ctx.meta = (kw, init is not None)
         ctx.set_materialize_grads(False)
-        return o, states.index_select(1, last)
+        return o, (states.index_select(1, last) if want_final else None)
 
     @staticmethod
     @torch.autograd.function.once_differentiable
@@ -130,13 +130,11 @@ class ChunkDelta(torch.autograd.Function):
         kw, has_init = ctx.meta
         do = _aligned(do) if do is not None else torch.zeros(v.shape, dtype=v.dtype, device=v.device)
         gx, gs = K.delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, seq.shape[0], **kw)
-        if dfinal is None:
-            gs.index_fill_(1, last, 0.0)
-        else:
+        if dfinal is not None:
             gs.index_copy_(1, last, dfinal.contiguous())
-        dx, ds = K.delta_state_scan(k_out, w, gx, decay, None, gs, seq, reverse=True, s1=1.0, s2=-1.0)
+        dx, ds = K.delta_state_scan(k_out, w, gx, decay, None, gs, seq, reverse=True, s1=1.0, s2=-1.0, zero_first=dfinal is None)
         dq, dk, dv, dg, dbeta = K.delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, ds, **kw)
-        return dq, dk, dv, dg, dbeta, (ds.index_select(1, first) if has_init else None), None, None, None
+        return dq, dk, dv, dg, dbeta, (ds.index_select(1, first) if has_init else None), None, None, None, None
 
 
 def _rows_for_kernel(t: torch.Tensor, R: int) -> torch.Tensor:
@@ -250,7 +248,7 @@ def chunk_delta_rule_batched(q, k, v, g, beta, scale=None, initial_state=None, o
         tables = _chunk_tables(segs, C, dev)
         init = initial_state.float().transpose(0, 1).contiguous() if initial_state is not None else None
         o, final = ChunkDelta.apply(*(_rows_for_kernel(t, R) for t in (q, k, v)), g.float().reshape(R, *g.shape[2:]).contiguous(),
-                                    beta.float().reshape(R, H).contiguous(), init, tables, float(scale), bool(use_qk_l2norm))
+                                    beta.float().reshape(R, H).contiguous(), init, tables, float(scale), bool(use_qk_l2norm), bool(output_final_state))
         return o.view(B, T, H, V), (final.transpose(0, 1).contiguous() if output_final_state else None)
     q, k = (repeat_key_heads(t, heads_per_key) for t in (q, k))
     qf, kf, vf, gf, bf = (t.float() for t in (q, k, v, g, beta))
@@ -352,8 +350,43 @@ def _gate(g, A_log, dt_bias, lower_bound):
     return kda_gate(g, A_log, dt_bias, lower_bound)
 
 
+class GDNGatesFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, a, b, A_log, dt_bias):
+        g, beta = K.gdn_gate_fwd(a, b, A_log, dt_bias)
+        ctx.save_for_backward(a, b, A_log, dt_bias, beta)
+        return g, beta
+
+    @staticmethod
+    def backward(ctx, dg, dbeta):
+        a, b, A_log, dt_bias, beta = ctx.saved_tensors
+        if torch.is_grad_enabled():              # a graph of the gradient is wanted: by way of the separate operations
+            needs = ctx.needs_input_grad
+            given = [t for t, n in zip((a, b, A_log, dt_bias), needs) if n]
+            grads = iter(torch.autograd.grad(gdn_gates_ref(a, b, A_log, dt_bias), given, (dg, dbeta), create_graph=True, allow_unused=True))
+            return tuple(next(grads) if n else None for n in needs)
+        same = A_log.dtype == dt_bias.dtype
+        da, db, dA, dd = K.gdn_gate_bwd(dg.contiguous(), dbeta.contiguous(), a, A_log, dt_bias, beta, A_log.dtype if same else torch.float32)
+        return da, db, dA.to(A_log.dtype), dd.to(dt_bias.dtype)
+
+
 def _register(op_name: str, impl_name: str):
     return register_op(op_name=op_name, impl_name=impl_name, kind=OpImplKind.CUSTOM, priority=100, devices=(TurboDevice.CUDA,))
+
+
+@_register("gdn_gates", "b200_gdn_gates")
+class B200GDNGates(OpImpl):
+    """One launch forward and two backward (projections may be columns of a wider matrix)."""
+
+    def available(self) -> bool:
+        return K.available()
+
+    def __call__(self, a, b, A_log, dt_bias):
+        plain, H = (torch.bfloat16, torch.float32), a.shape[-1]
+        if not (a.dim() == 2 and b.shape == a.shape and H > 0 and all(t.is_cuda and t.dtype == torch.bfloat16 and t.stride(1) == 1 for t in (a, b))
+                and all(t.is_cuda and t.dtype in plain and t.shape == (H,) for t in (A_log, dt_bias)) and _eager(a, b, A_log, dt_bias)):
+            return gdn_gates_ref(a, b, A_log, dt_bias)
+        return GDNGatesFn.apply(a, b, A_log.contiguous(), dt_bias.contiguous())
 
 
 @_register("gated_delta_rule", "b200_chunk_gated_delta_rule")

@@ -142,6 +142,16 @@ class TorchLinear(OpImpl):
         return y + residual if residual is not None else y
 
 
+@_native("linears")
+class TorchLinears(OpImpl):
+    """Several projections of the same rows: `(x @ w^T for w in weights)`."""
+
+    def __call__(self, x, *weights):
+        from ..ops import ops
+
+        return tuple(ops.linear(x, w) for w in weights)
+
+
 @_native("router_gating")
 class TorchRouterGating(OpImpl):
     """Router logits `x @ W^T` returned in fp32."""

@@ -231,6 +231,18 @@ def repeat_key_heads(t, heads_per_key: int):
     return t.unsqueeze(3).expand(B, T, H, heads_per_key, Kd).reshape(B, T, H * heads_per_key, Kd)
 
 
+def gdn_gates_ref(a, b, A_log, dt_bias):
+    return -A_log.float().exp() * F.softplus(a.float() + dt_bias.float()), torch.sigmoid(b.float())
+
+
+@_native("gdn_gates", "torch_gdn_gates")
+class TorchGDNGates(OpImpl):
+    """Log decay `-exp(A_log) softplus(a + dt_bias)` and step size `sigmoid(b)` of a gated delta net, fp32 `[T, H]`."""
+
+    def __call__(self, a, b, A_log, dt_bias):
+        return gdn_gates_ref(a, b, A_log, dt_bias)
+
+
 @_native("gated_delta_rule", "torch_chunk_gated_delta_rule")
 class TorchGatedDeltaRule(OpImpl):
     """q, k: [B, T, H / heads_per_key, K], each head serving `heads_per_key` value heads in a row; v: [B, T, H, V]."""
