@@ -38,16 +38,6 @@ constexpr int DC_C = 64;
 constexpr int DC_D = 128;
 constexpr int DC_QS = 136;   // row stride (elements) of bf16 tiles: 272 bytes, ldmatrix rows fall on distinct banks
 
-struct DeltaChunkIn {
-  const __nv_bfloat16 *q, *k, *v;                      // row r, head h, channel c at [r * *_t + h * *_h + c]
-  long long q_t, q_h, k_t, k_h, v_t, v_h;
-  const float *g, *beta;                               // log decay [rows, H] or [rows, H, 128]; step size [rows, H]
-  const int* chunk_rows;                               // [NC, 3]: first row, rows (1 .. 64), sequence
-  int H, NC, l2;
-  float scale;
-  int rep;                                             // value heads per key head: head h reads q and k of head h / rep
-};
-
 __device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t b0, const uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])

@@ -1,6 +1,7 @@
 // C entry points that csrc/host.cpp calls and the argument structure of the GEMM, declared once for both sides: every kernel source
 // includes this (through common.cuh), so a definition whose parameters differ from what the launch functions pass does not compile.
 #pragma once
+#include <cuda_bf16.h>
 
 #define TTB_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -40,6 +41,17 @@ struct GemmArgs {
   int k_splits;
 };
 
+// inputs of the chunk-parallel delta-rule kernels (delta_chunk.cuh)
+struct DeltaChunkIn {
+  const __nv_bfloat16 *q, *k, *v;                      // row r, head h, channel c at [r * *_t + h * *_h + c]
+  long long q_t, q_h, k_t, k_h, v_t, v_h;
+  const float *g, *beta;                               // log decay [rows, H] or [rows, H, 128]; step size [rows, H]
+  const int* chunk_rows;                               // [NC, 3]: first row, rows (1 .. 64), sequence
+  int H, NC, l2;
+  float scale;
+  int rep;                                             // value heads per key head: head h reads q and k of head h / rep
+};
+
 }  // namespace ttb
 
 TTB_EXPORT int ttb_gemm_bf16(const ttb::GemmArgs*, void*);
@@ -57,6 +69,23 @@ TTB_EXPORT int ttb_qknorm_rope_fwd(const void*, long long, int, int, int, const 
 TTB_EXPORT int ttb_qknorm_rope_bwd(const void*, const void*, const void*, const void*, long long, int, int, int, const void*,
                             const void*, const float*, const float*, const float*, void*, long long, float*, void*, int, long
                             long, int, int, void*);
+TTB_EXPORT int ttb_delta_prep(const ttb::DeltaChunkIn*, float*, float*, float*, void*, void*, float*, void*);
+TTB_EXPORT int ttb_delta_out(const ttb::DeltaChunkIn*, const float*, const float*, const float*, int, void*, void*);
+TTB_EXPORT int ttb_delta_bwd_pre(const ttb::DeltaChunkIn*, const void*, const float*, int, float*, float*, void*);
+TTB_EXPORT int ttb_delta_bwd_post(const ttb::DeltaChunkIn*, const void*, const float*, const float*, const float*, const float*, const float*, int,
+                            void*, void*, void*, float*, float*, void*);
+TTB_EXPORT int ttb_delta_vec_prep(const ttb::DeltaChunkIn*, float*, float*, float*, void*, void*, float*, void*);
+TTB_EXPORT int ttb_delta_vec_out(const ttb::DeltaChunkIn*, const float*, const float*, const float*, int, void*, void*);
+TTB_EXPORT int ttb_delta_vec_bwd_pre(const ttb::DeltaChunkIn*, const void*, const float*, int, float*, float*, void*);
+TTB_EXPORT int ttb_delta_vec_bwd_post(const ttb::DeltaChunkIn*, const void*, const float*, const float*, const float*, const float*, const float*,
+                            int, void*, void*, void*, float*, float*, float*, void*);
+TTB_EXPORT int ttb_delta_head_sum(const void*, const void*, void*, void*, long long, int, void*);
+TTB_EXPORT int ttb_delta_state_scan(const void*, const void*, const float*, float*, const float*, int, const float*, const float*, float*,
+                            const int*, int, int, int, int, float, float, void*);
+TTB_EXPORT int ttb_kda_gate_row_blocks(long long, int);
+TTB_EXPORT int ttb_kda_gate_fwd(const void*, const void*, int, const void*, int, float*, long long, int, int, float, void*);
+TTB_EXPORT int ttb_kda_gate_bwd(const float*, const void*, const void*, int, const void*, int, void*, float*, float*, long long, int, int, float,
+                            void*);
 TTB_EXPORT int ttb_gdn_gate_fwd(const void*, long long, const void*, long long, const void*, int, const void*, int, float*, float*, long long,
                             int, void*);
 TTB_EXPORT int ttb_gdn_gate_bwd(const float*, const float*, const void*, long long, const void*, int, const void*, int, const float*, void*,

@@ -504,6 +504,196 @@ PyObject* gdn_gate_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Kimi delta attention gate
+// ---------------------------------------------------------------------------------------------
+PyObject* kda_gate_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 5);
+    const Tensor &g = in.tensor(), &A = in.tensor();
+    const Tensor dt = in.optional();
+    const bool bounded = in.flag();
+    const double bound = in.real();
+    const Tensor out = empty(g.sizes(), at::kFloat, g);
+    launch("ttb_kda_gate_fwd", 1, [&](void* st) {
+      return ttb_kda_gate_fwd(at_(g), at_(A), is_bf16(A), at_(dt), dt.defined() && is_bf16(dt), f32w(out), g.size(0), static_cast<int>(g.size(1)),
+                              bounded, static_cast<float>(bound), st);
+    });
+    return wrap(out);
+  });
+}
+
+PyObject* kda_gate_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 6);
+    const Tensor &dd = in.tensor(), &g = in.tensor(), &A = in.tensor();
+    const Tensor dt = in.optional();
+    const bool bounded = in.flag();
+    const double bound = in.real();
+    const long long R = g.size(0), H = g.size(1), D = g.size(2);
+    const int blocks = ttb_kda_gate_row_blocks(R, static_cast<int>(H));
+    const Tensor dg = empty_rows(g), part = empty({std::max(blocks, 1), 2, H * D}, at::kFloat, g);
+    const Tensor sums = R ? empty({2, H * D}, at::kFloat, g) : at::zeros({2, H * D}, plain(g).dtype(at::kFloat));
+    launch("ttb_kda_gate_bwd", 2, [&](void* st) {
+      return ttb_kda_gate_bwd(f32(dd), at_(g), at_(A), is_bf16(A), at_(dt), dt.defined() && is_bf16(dt), to_(dg), f32w(part), f32w(sums), R,
+                              static_cast<int>(H), bounded, static_cast<float>(bound), st);
+    });
+    return wrap_all(dg, sums.select(0, 0), sums.select(0, 1).view({H, D}));
+  });
+}
+
+// ---------------------------------------------------------------------------------------------
+// delta rule
+// ---------------------------------------------------------------------------------------------
+// q, k, v, g, beta, chunk_rows of a call and what the kernels make of them (kernels.delta_prep)
+struct DeltaIn {
+  const Tensor &q, &k, &v, &g, &beta, &rows;
+  ttb::DeltaChunkIn in{};
+  explicit DeltaIn(Args& a) : q(a.tensor()), k(a.tensor()), v(a.tensor()), g(a.tensor()), beta(a.tensor()), rows(a.tensor()) {}
+  // l2 and scale are a call's last arguments
+  const ttb::DeltaChunkIn* fill(Args& a) {
+    const bool l2 = a.flag();
+    const double scale = a.real();
+    need(v.dim() == 3 && q.dim() == 3 && k.dim() == 3 && rows.dim() == 2, "rows of heads");
+    const long long R = v.size(0), H = v.size(1), Hk = q.size(1);
+    check_device(q);
+    auto heads = [&](const Tensor& t, long long n) { return is_bf16(t) && t.size(0) == R && t.size(1) == n && t.size(2) == 128 && t.stride(2) == 1; };
+    need(heads(q, Hk) && heads(k, Hk) && heads(v, H), "q, k, v: bf16 rows of 128-wide heads");
+    need(Hk > 0 && H % Hk == 0 && (Hk == H || g.dim() == 2), "key heads");
+    need(g.scalar_type() == at::kFloat && g.is_contiguous() && (g.dim() == 2 || (g.dim() == 3 && g.size(2) == 128)) && g.size(0) == R && g.size(1) == H, "log decay");
+    need(beta.scalar_type() == at::kFloat && beta.is_contiguous() && beta.dim() == 2 && beta.size(0) == R && beta.size(1) == H, "step size");
+    need(rows.scalar_type() == at::kInt && rows.is_contiguous() && rows.size(1) == 3, "chunk table");
+    auto bf = [](const Tensor& t) { return static_cast<const __nv_bfloat16*>(at_(t)); };
+    in.q = bf(q); in.k = bf(k); in.v = bf(v);
+    in.q_t = q.stride(0); in.q_h = q.stride(1);
+    in.k_t = k.stride(0); in.k_h = k.stride(1);
+    in.v_t = v.stride(0); in.v_h = v.stride(1);
+    in.g = f32(g); in.beta = f32(beta); in.chunk_rows = i32(rows);
+    in.H = static_cast<int>(H); in.NC = static_cast<int>(rows.size(0)); in.l2 = l2; in.scale = static_cast<float>(scale);
+    in.rep = static_cast<int>(H / Hk);
+    return &in;
+  }
+  bool vec() const { return g.dim() == 3; }
+};
+
+PyObject* delta_prep(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 8);
+    DeltaIn d(in);
+    const ttb::DeltaChunkIn* a = d.fill(in);
+    const long long H = a->H, NC = a->NC;
+    const Tensor tri = empty({2, H, NC, 64, 64}, at::kFloat, d.q), u = empty({H, NC, 64, 128}, at::kFloat, d.q);
+    const Tensor wk = empty({2, H, NC, 64, 128}, at::kBFloat16, d.q), decay = d.vec() ? empty({H, NC, 128}, at::kFloat, d.q) : empty({H, NC}, at::kFloat, d.q);
+    const Tensor T = tri.select(0, 0), A = tri.select(0, 1), w = wk.select(0, 0), k_out = wk.select(0, 1);
+    launch(d.vec() ? "ttb_delta_vec_prep" : "ttb_delta_prep", 1, [&](void* st) {
+      return (d.vec() ? ttb_delta_vec_prep : ttb_delta_prep)(a, f32w(T), f32w(A), f32w(u), to_(w), to_(k_out), f32w(decay), st);
+    });
+    return wrap_all(T, A, u, w, k_out, decay);
+  });
+}
+
+PyObject* delta_out(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 11);
+    DeltaIn d(in);
+    const Tensor &A = in.tensor(), &x = in.tensor(), &states = in.tensor();
+    const ttb::DeltaChunkIn* a = d.fill(in);
+    const Tensor o = empty(d.v.sizes(), at::kBFloat16, d.q);
+    launch(d.vec() ? "ttb_delta_vec_out" : "ttb_delta_out", 1, [&](void* st) {
+      return (d.vec() ? ttb_delta_vec_out : ttb_delta_out)(a, f32(A), f32(x), f32(states), static_cast<int>(states.size(1)) - a->NC, to_(o), st);
+    });
+    return wrap(o);
+  });
+}
+
+PyObject* delta_bwd_pre(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 11);
+    DeltaIn d(in);
+    const Tensor &dout = in.tensor(), &A = in.tensor();
+    const int nseq = static_cast<int>(in.integer());
+    const ttb::DeltaChunkIn* a = d.fill(in);
+    need(dout.is_contiguous() && is_bf16(dout) && dout.sizes() == d.v.sizes(), "the gradient has v's shape");
+    const Tensor gx = empty({a->H, a->NC, 64, 128}, at::kFloat, d.q), gs = empty({a->H, a->NC + nseq, 128, 128}, at::kFloat, d.q);
+    launch(d.vec() ? "ttb_delta_vec_bwd_pre" : "ttb_delta_bwd_pre", 1, [&](void* st) {
+      return (d.vec() ? ttb_delta_vec_bwd_pre : ttb_delta_bwd_pre)(a, at_(dout), f32(A), nseq, f32w(gx), f32w(gs), st);
+    });
+    return wrap_all(gx, gs);
+  });
+}
+
+PyObject* delta_bwd_post(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 14);
+    DeltaIn d(in);
+    const Tensor &dout = in.tensor(), &T = in.tensor(), &x = in.tensor(), &dx = in.tensor(), &states = in.tensor(), &dstates = in.tensor();
+    const ttb::DeltaChunkIn* a = d.fill(in);
+    need(dout.is_contiguous() && is_bf16(dout) && dout.sizes() == d.v.sizes(), "the gradient has v's shape");
+    const int nseq = static_cast<int>(states.size(1)) - a->NC;
+    Tensor dq = empty(d.v.sizes(), at::kBFloat16, d.q), dk = empty(d.v.sizes(), at::kBFloat16, d.q);     // of every value head
+    const Tensor dv = empty(d.v.sizes(), at::kBFloat16, d.q), dg = empty(d.g.sizes(), at::kFloat, d.q), db = empty(d.beta.sizes(), at::kFloat, d.q);
+    if (d.vec()) {
+      // held until the launches are queued: a pointer alone would let another thread of this stream be given the block first
+      const Tensor scratch = empty({4, x.size(0), x.size(1), x.size(2), x.size(3)}, at::kFloat, d.q);
+      launch("ttb_delta_vec_bwd_post", 2, [&](void* st) {
+        return ttb_delta_vec_bwd_post(a, at_(dout), f32(T), f32(x), f32(dx), f32(states), f32(dstates), nseq, to_(dq), to_(dk), to_(dv), f32w(dg),
+                                      f32w(db), f32w(scratch), st);
+      });
+    } else {
+      launch("ttb_delta_bwd_post", 1, [&](void* st) {
+        return ttb_delta_bwd_post(a, at_(dout), f32(T), f32(x), f32(dx), f32(states), f32(dstates), nseq, to_(dq), to_(dk), to_(dv), f32w(dg),
+                                  f32w(db), st);
+      });
+    }
+    if (a->rep > 1) {
+      const Tensor sq = empty(d.q.sizes(), at::kBFloat16, d.q), sk = empty(d.q.sizes(), at::kBFloat16, d.q);
+      launch("ttb_delta_head_sum", 1, [&](void* st) {
+        return ttb_delta_head_sum(at_(dq), at_(dk), to_(sq), to_(sk), d.q.size(0) * d.q.size(1), a->rep, st);
+      });
+      dq = sq;
+      dk = sk;
+    }
+    return wrap_all(dq, dk, dv, dg, db);
+  });
+}
+
+PyObject* delta_state_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 10);
+    const Tensor &a = in.tensor(), &b = in.tensor(), &u0 = in.tensor(), &decay0 = in.tensor();
+    const Tensor init0 = in.optional(), add0 = in.optional();
+    const Tensor& seq0 = in.tensor();
+    const int reverse = static_cast<int>(in.integer());
+    const double s1 = in.real(), s2 = in.real();
+    need(u0.dim() == 4 && seq0.dim() == 2 && (decay0.dim() == 2 || decay0.dim() == 3), "chunks of 64 rows");
+    const long long H = u0.size(0), NC = u0.size(1), nseq = seq0.size(0);
+    need(u0.size(2) == 64 && u0.size(3) == 128 && a.sizes() == u0.sizes() && b.sizes() == u0.sizes(), "chunks of 64 rows");
+    need(is_bf16(a) && is_bf16(b) && u0.scalar_type() == at::kFloat && a.is_contiguous() && b.is_contiguous() && u0.is_contiguous(), "operands");
+    need(decay0.is_contiguous() && decay0.scalar_type() == at::kFloat && decay0.size(0) == H && decay0.size(1) == NC, "decay");
+    need(seq0.scalar_type() == at::kInt && seq0.is_contiguous() && seq0.size(1) == 2, "sequence table");
+    check_device(u0);
+    // the copy engine moves whole rows: tensors that start between 16-byte boundaries are copied
+    auto placed = [](const Tensor& t) {
+      if (!t.defined()) return t;
+      const Tensor c = t.contiguous();
+      return reinterpret_cast<uintptr_t>(c.const_data_ptr()) % 16 ? c.clone() : c;
+    };
+    const Tensor u = placed(u0), decay = placed(decay0), init = placed(init0), add = placed(add0), seq = placed(seq0);
+    auto states_like = [&](const Tensor& t, long long slots) {
+      return t.scalar_type() == at::kFloat && t.dim() == 4 && t.size(0) == H && t.size(1) == slots && t.size(2) == 128 && t.size(3) == 128;
+    };
+    need(!init.defined() || states_like(init, nseq), "first states");
+    need(!add.defined() || states_like(add, NC + nseq), "added gradients");
+    const Tensor x = empty_rows(u), states = empty({H, NC + nseq, 128, 128}, at::kFloat, u);
+    launch("ttb_delta_state_scan", 1, [&](void* st) {
+      return ttb_delta_state_scan(at_(a), at_(b), f32(u), f32w(x), f32(decay), decay.dim() == 3, f32(init), f32(add), f32w(states), i32(seq),
+                                  static_cast<int>(nseq), static_cast<int>(H), static_cast<int>(NC), reverse, static_cast<float>(s1),
+                                  static_cast<float>(s2), st);
+    });
+    return wrap_all(x, states);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------
 // attention
 // ---------------------------------------------------------------------------------------------
 // Rows that no sequence covers read as zero; [lo, hi) = covered rows, lo < 0 = unknown.
@@ -617,7 +807,8 @@ PyObject* launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_From
 #define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ENTRY(setup), ENTRY(launches), ENTRY(gemm), ENTRY(rmsnorm_fwd), ENTRY(rmsnorm_bwd), ENTRY(layernorm_fwd), ENTRY(layernorm_bwd),
                          ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(gdn_gate_fwd),
-                         ENTRY(gdn_gate_bwd), ENTRY(rope), ENTRY(swiglu_fwd),
+                         ENTRY(gdn_gate_bwd), ENTRY(kda_gate_fwd), ENTRY(kda_gate_bwd), ENTRY(delta_prep), ENTRY(delta_out), ENTRY(delta_bwd_pre),
+                         ENTRY(delta_bwd_post), ENTRY(delta_state_scan), ENTRY(rope), ENTRY(swiglu_fwd),
                          ENTRY(swiglu_bwd), ENTRY(attn_fwd), ENTRY(attn_bwd), {nullptr, nullptr, 0, nullptr}};
 #undef ENTRY
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "ttb_host", nullptr, -1, methods};

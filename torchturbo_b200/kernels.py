@@ -96,8 +96,8 @@ def host():
 
 # kernels launched per C entry point (used to report how many of this library's kernels ran in a region)
 _LAUNCHES_PER_CALL = {"ttb_gated_rmsnorm_bwd": 2, "ttb_causal_conv1d_bwd": 2,
-                      "ttb_causal_conv1d_row_blocks": 0, "ttb_kda_gate_bwd": 2, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
-                      "ttb_ep_combine_all": 3, "ttb_delta_vec_bwd_post": 2, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
+                      "ttb_causal_conv1d_row_blocks": 0, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
+                      "ttb_ep_combine_all": 3, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
                       "ttb_gemm_status": 0}
 LAUNCH_COUNT = 0
 
@@ -333,30 +333,14 @@ def rope(x, cos, sin, sign: float = 1.0):
 # --------------------------------------------------------------------------------------
 # Kimi delta attention gate
 # --------------------------------------------------------------------------------------
-def _gate_args(g, A_log, dt_bias, lower_bound):
-    half = torch.bfloat16
-    return (_p(g), _p(A_log), C.c_int(int(A_log.dtype == half)), _p(dt_bias), C.c_int(int(dt_bias is not None and dt_bias.dtype == half))), \
-        (C.c_longlong(g.shape[0]), C.c_int(g.shape[1]), C.c_int(int(lower_bound is not None)), C.c_float(lower_bound or 0.0), _stream())
-
-
 def kda_gate_fwd(g, A_log, dt_bias, lower_bound):
     """Log decay fp32 [rows, H, 128] from the bf16 projection `g`; A_log [H] and dt_bias [H * 128] (or None) in bf16 or fp32."""
-    out = torch.empty(g.shape, dtype=torch.float32, device=g.device)
-    head, tail = _gate_args(g, A_log, dt_bias, lower_bound)
-    _check(lib().ttb_kda_gate_fwd(*head, _p(out), *tail), "ttb_kda_gate_fwd")
-    return out
+    return host().kda_gate_fwd(g, A_log, dt_bias, lower_bound is not None, lower_bound or 0.0)
 
 
 def kda_gate_bwd(dd, g, A_log, dt_bias, lower_bound):
     """(dg bf16, d(dt) fp32 [H * 128], channel sums of d(A_log) fp32 [H, 128])."""
-    R, H, D = g.shape
-    dg = torch.empty_like(g)
-    blocks = int(lib().ttb_kda_gate_row_blocks(C.c_longlong(R), C.c_int(H)))
-    part = torch.empty(max(blocks, 1), 2, H * D, dtype=torch.float32, device=g.device)
-    sums = (torch.empty if R else torch.zeros)(2, H * D, dtype=torch.float32, device=g.device)
-    head, tail = _gate_args(g, A_log, dt_bias, lower_bound)
-    _check(lib().ttb_kda_gate_bwd(_p(dd), *head, _p(dg), _p(part), _p(sums), *tail), "ttb_kda_gate_bwd")
-    return dg, sums[0], sums[1].view(H, D)
+    return host().kda_gate_bwd(dd, g, A_log, dt_bias, lower_bound is not None, lower_bound or 0.0)
 
 
 def gdn_gate_fwd(a, b, A_log, dt_bias):
@@ -665,109 +649,32 @@ def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, r
     `add`: fp32 [H, NC + nseq, 128, 128] (required when `reverse`); `seq_chunks_dev`: int32 [nseq, 2].  A reverse pass starts from the
     last slots of `add`, with `zero_first` from zero (those slots are not read).
     Returns (x fp32 [H, NC, 64, 128], states fp32 [H, NC + nseq, 128, 128])."""
-    H, NC, Cc, D = u.shape
-    nseq = seq_chunks_dev.shape[0]
-    assert Cc == 64 and D == 128 and a_tiles.shape == u.shape and b_tiles.shape == u.shape
-    assert a_tiles.dtype == torch.bfloat16 and b_tiles.dtype == torch.bfloat16 and u.dtype == torch.float32
-    assert a_tiles.is_contiguous() and b_tiles.is_contiguous() and u.is_contiguous() and decay.is_contiguous()
-    assert decay.dtype == torch.float32 and decay.shape[:2] == (H, NC) and decay.dim() in (2, 3)
-    if init is not None:
-        init = init.contiguous()
-        assert init.shape == (H, nseq, 128, 128) and init.dtype == torch.float32
-    if add is not None:
-        add = add.contiguous()
-        assert add.shape == (H, NC + nseq, 128, 128) and add.dtype == torch.float32
-    # the copy engine moves whole rows: tensors that start between 16-byte boundaries are copied
-    u, decay, init, add, seq_chunks_dev = (t if t is None or t.data_ptr() % 16 == 0 else t.clone() for t in (u, decay, init, add, seq_chunks_dev))
-    x = torch.empty_like(u)
-    states = torch.empty(H, NC + nseq, 128, 128, dtype=torch.float32, device=u.device)
-    _check(lib().ttb_delta_state_scan(_p(a_tiles), _p(b_tiles), _p(u), _p(x), _p(decay), C.c_int(int(decay.dim() == 3)),
-                                      _p(init), _p(add), _p(states), _p(seq_chunks_dev), C.c_int(nseq), C.c_int(H),
-                                      C.c_int(NC), C.c_int((2 if zero_first else 1) if reverse else 0), C.c_float(s1), C.c_float(s2), _stream()),
-           "ttb_delta_state_scan")
-    return x, states
+    return host().delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, (2 if zero_first else 1) if reverse else 0, s1, s2)
 
 
-class _DeltaChunkIn(C.Structure):
-    """`struct DeltaChunkIn` of csrc/delta_chunk.cu."""
-
-    _fields_ = [("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p),
-                ("q_t", C.c_longlong), ("q_h", C.c_longlong), ("k_t", C.c_longlong), ("k_h", C.c_longlong),
-                ("v_t", C.c_longlong), ("v_h", C.c_longlong),
-                ("g", C.c_void_p), ("beta", C.c_void_p), ("chunk_rows", C.c_void_p),
-                ("H", C.c_int), ("NC", C.c_int), ("l2", C.c_int), ("scale", C.c_float), ("rep", C.c_int)]
-
-
-def _delta_in(q, k, v, g, beta, chunk_rows, l2: bool, scale: float) -> _DeltaChunkIn:
-    """v: bf16 [rows, H, 128]; q, k: the same or, with one decay per head, of H / rep heads that serve rep value heads each (any
-    row / head stride that keeps 16-byte alignment); g: fp32 [rows, H]
-    or [rows, H, 128] (one decay per head, or per head and channel); beta: fp32 [rows, H]; chunk_rows: int32 [NC, 3] on the device (first row, number of rows, sequence of every chunk)."""
-    R, H, _ = v.shape
-    Hk = q.shape[1]
-    check_device(q)
-    for t, heads in ((q, Hk), (k, Hk), (v, H)):
-        assert t.dtype == torch.bfloat16 and t.shape == (R, heads, 128) and t.stride(2) == 1
-    assert H % Hk == 0 and (Hk == H or g.dim() == 2)
-    assert g.dtype == torch.float32 and g.shape in ((R, H), (R, H, 128)) and g.is_contiguous()
-    assert beta.dtype == torch.float32 and beta.shape == (R, H) and beta.is_contiguous()
-    assert chunk_rows.dtype == torch.int32 and chunk_rows.is_contiguous() and chunk_rows.shape[1] == 3
-    return _DeltaChunkIn(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0), k.stride(1),
-                         v.stride(0), v.stride(1), g.data_ptr(), beta.data_ptr(), chunk_rows.data_ptr(), H,
-                         chunk_rows.shape[0], int(l2), scale, H // Hk)
-
-
-def _delta_call(step: str, g, *args) -> None:
-    name = f"ttb_delta_{'vec_' if g.dim() == 3 else ''}{step}"
-    _check(getattr(lib(), name)(*args), name)
-
-
+# Inputs of the chunk kernels: v: bf16 [rows, H, 128]; q, k: the same or, with one decay per head, of H / rep heads that serve rep value
+# heads each (any row / head stride that keeps 16-byte alignment); g: fp32 [rows, H] or [rows, H, 128] (one decay per head, or per head
+# and channel); beta: fp32 [rows, H]; chunk_rows: int32 [NC, 3] on the device (first row, number of rows, sequence of every chunk).
 def delta_prep(q, k, v, g, beta, chunk_rows, *, l2: bool, scale: float):
     """Chunk-parallel operands of the gated delta rule (csrc/delta_chunk.cu).  Returns (T, A fp32 [H, NC, 64, 64],
     u fp32 [H, NC, 64, 128], w, k_out bf16 [H, NC, 64, 128], decay fp32 [H, NC] or [H, NC, 128])."""
-    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    H, NC, dev = a.H, a.NC, q.device
-    tri = torch.empty(2, H, NC, 64, 64, dtype=torch.float32, device=dev)
-    u = torch.empty(H, NC, 64, 128, dtype=torch.float32, device=dev)
-    wk = torch.empty(2, H, NC, 64, 128, dtype=torch.bfloat16, device=dev)
-    decay = torch.empty(H, NC, *g.shape[2:], dtype=torch.float32, device=dev)
-    _delta_call("prep", g, C.byref(a), _p(tri[0]), _p(tri[1]), _p(u), _p(wk[0]), _p(wk[1]), _p(decay), _stream())
-    return tri[0], tri[1], u, wk[0], wk[1], decay
+    return host().delta_prep(q, k, v, g, beta, chunk_rows, l2, scale)
 
 
 def delta_out(q, k, v, g, beta, chunk_rows, A, x, states, *, l2: bool, scale: float):
     """o bf16 [rows, H, 128] from the new values `x` and the chunk-start states of the recurrence."""
-    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    o = torch.empty(v.shape, dtype=torch.bfloat16, device=q.device)
-    _delta_call("out", g, C.byref(a), _p(A), _p(x), _p(states), C.c_int(states.shape[1] - a.NC), _p(o), _stream())
-    return o
+    return host().delta_out(q, k, v, g, beta, chunk_rows, A, x, states, l2, scale)
 
 
 def delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq: int, *, l2: bool, scale: float):
     """Gradients that reach the recurrence directly: (gx like x, gS [H, NC + nseq, 128, 128]; the slots behind the last
     chunk of a sequence are left to the caller)."""
-    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    assert do.is_contiguous() and do.dtype == torch.bfloat16 and do.shape == v.shape
-    gx = torch.empty(a.H, a.NC, 64, 128, dtype=torch.float32, device=q.device)
-    gs = torch.empty(a.H, a.NC + nseq, 128, 128, dtype=torch.float32, device=q.device)
-    _delta_call("bwd_pre", g, C.byref(a), _p(do), _p(A), C.c_int(nseq), _p(gx), _p(gs), _stream())
-    return gx, gs
+    return host().delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq, l2, scale)
 
 
 def delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, *, l2: bool, scale: float):
     """(dq, dk bf16 like q, dv bf16 [rows, H, 128], dg like g, dbeta fp32 [rows, H])."""
-    a = _delta_in(q, k, v, g, beta, chunk_rows, l2, scale)
-    dq, dk, dv = (torch.empty(v.shape, dtype=torch.bfloat16, device=q.device) for _ in range(3))   # of every value head
-    dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
-    # held until the launches are queued: a pointer alone would let another thread of this stream be given the block first
-    scratch = torch.empty(4, *x.shape, dtype=torch.float32, device=q.device) if g.dim() == 3 else None
-    _delta_call("bwd_post", g, C.byref(a), _p(do), _p(T), _p(x), _p(dx), _p(states), _p(dstates), C.c_int(states.shape[1] - a.NC),
-                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta),
-                *([_p(scratch)] if scratch is not None else []), _stream())
-    if a.rep > 1:
-        per_head, (dq, dk) = (dq, dk), (torch.empty(q.shape, dtype=torch.bfloat16, device=q.device) for _ in range(2))
-        _check(lib().ttb_delta_head_sum(_p(per_head[0]), _p(per_head[1]), _p(dq), _p(dk), C.c_longlong(q.shape[0] * q.shape[1]),
-                                        C.c_int(a.rep), _stream()), "ttb_delta_head_sum")
-    return dq, dk, dv, dg, dbeta
+    return host().delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, l2, scale)
 
 
 # --------------------------------------------------------------------------------------

@@ -131,7 +131,7 @@ class ChunkDelta(torch.autograd.Function):
         do = _aligned(do) if do is not None else torch.zeros(v.shape, dtype=v.dtype, device=v.device)
         gx, gs = K.delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, seq.shape[0], **kw)
         if dfinal is not None:
-            gs.index_copy_(1, last, dfinal.contiguous())
+            gs.index_copy_(1, last.long(), dfinal.contiguous())
         dx, ds = K.delta_state_scan(k_out, w, gx, decay, None, gs, seq, reverse=True, s1=1.0, s2=-1.0, zero_first=dfinal is None)
         dq, dk, dv, dg, dbeta = K.delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, ds, **kw)
         return dq, dk, dv, dg, dbeta, (ds.index_select(1, first) if has_init else None), None, None, None, None
@@ -161,7 +161,7 @@ def _chunk_tables(segs, C: int, device):
     host = torch.tensor(seq + rows + last + first, dtype=torch.int32).pin_memory()
     dev = host.to(device, non_blocking=True)
     seq_d, rows_d, slots_d = dev.split([2 * nseq, 3 * c, 2 * nseq])
-    last_d, first_d = slots_d.long().split(nseq)
+    last_d, first_d = slots_d.split(nseq)
     return seq_d.view(nseq, 2), rows_d.view(c, 3), last_d, first_d
 
 
