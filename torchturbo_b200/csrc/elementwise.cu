@@ -1308,13 +1308,30 @@ sqnorm_kernel(const AdamMeta* __restrict__ meta, const int2* __restrict__ chunks
   if (end > t.numel) end = t.numel;
   float s = 0.f;
   const bool aligned = (reinterpret_cast<uintptr_t>(t.g) & 15) == 0;
-  const long long n8 = (aligned && t.g_is_bf16) ? ((end - start) / 8) : 0;
-  for (long long q = threadIdx.x; q < n8; q += blockDim.x) {
-    const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(t.g) + start + q * 8);
-    const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
-    s += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y;
+  // Sixteen bytes a load, and four loads of a thread on their way at a time: fp32 gradients, which went by single
+  // words, 72 -> 53 us for 60 M and 328 -> 238 us (6.7 TB/s) for 400 M; bf16 ones had their 16 bytes before (35 and 137 us).
+  long long done = 0;
+  if (aligned && t.g_is_bf16) {
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(t.g) + start);
+    const int n8 = static_cast<int>((end - start) / 8);
+#pragma unroll 4
+    for (int q = threadIdx.x; q < n8; q += 256) {
+      const uint4 u = __ldg(src + q);
+      const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+      s += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y;
+    }
+    done = static_cast<long long>(n8) * 8;
+  } else if (aligned) {
+    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(t.g) + start);
+    const int n4 = static_cast<int>((end - start) / 4);
+#pragma unroll 4
+    for (int q = threadIdx.x; q < n4; q += 256) {
+      const float4 u = __ldg(src + q);
+      s += u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w;
+    }
+    done = static_cast<long long>(n4) * 4;
   }
-  for (long long i = start + n8 * 8 + threadIdx.x; i < end; i += blockDim.x) {
+  for (long long i = start + done + threadIdx.x; i < end; i += 256) {
     float g = t.g_is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(t.g)[i])
                           : reinterpret_cast<const float*>(t.g)[i];
     s += g * g;
