@@ -462,10 +462,12 @@ constexpr int CONV_MAX_W = 8;   // widest supported filter
 // Filters of up to four taps (every linear-attention layer): a thread owns 4 channels (8 would spill the window), walks its rows four
 // at a time with the next four rows' loads already issued, and keeps the taps' window in registers, so that x (and dy) are read
 // once.  One pass each way: the backward adds every dpre row into the W rows of dx that it reaches while they are still in registers
-// (the W - 1 rows behind a block are recomputed by it), which saves writing and re-reading dpre.  What bounds it is the issue of its
-// arithmetic (two exponentials and 48 products per element pair), so steps in which every tap of every row counts run without the
-// checks, and products go two channels at a time.  4096 x 8192, W = 4: forward 59 -> 45 -> 41 us, backward 180 (two kernels) -> 136
-// -> 102 us; 31 us of it would be memory.
+// (the W - 1 rows behind a block are recomputed by it), which saves writing and re-reading dpre.  Steps in which every tap of every row
+// counts run without the checks, and products go two channels at a time.  The next rows' loads have to be held in place: as plain
+// conditional loads they drew the unpacking of their row with them, so that a thread waited for memory at every step, which was most of
+// the backward's time.  What bounds it now is the issue of its arithmetic (two exponentials and 48 products per element pair).
+// 4096 x 8192, W = 4, from cold caches with the column sums: forward 47 -> 41 us, backward 132 -> 79; 16384 x 6144: 121 -> 100 and
+// 343 -> 179; 2047 x 3072: 16 and 50 -> 36 (memory alone: 22 and 33 us for the first).
 constexpr int CONV_ROWS = 4;    // rows per step
 
 __device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
@@ -474,6 +476,18 @@ __device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
 }
 __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&f)[4]) {
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+}
+
+// Loads that stay where they are written: the compiler otherwise moves the unpacking of a row up to its load, and the thread waits there
+__device__ __forceinline__ uint2 load_here(const __nv_bfloat16* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int load_here(const int* p) {
+  int v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
 }
 
 // c += a * b for two neighbouring channels (one instruction; each half rounds as an fma of its own)
@@ -527,10 +541,10 @@ causal_conv1d_w4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   auto fetch = [&](long long t0) {
 #pragma unroll
     for (int u = 0; u < CONV_ROWS; ++u) {
-      const bool in = t0 + u < re;
-      nx[u] = in ? *reinterpret_cast<const uint2*>(x + (t0 + u) * D + c) : zero;
-      if (BWD) ng[u] = in ? *reinterpret_cast<const uint2*>(dy + (t0 + u) * D + c) : zero;
-      nf[u] = in ? seq_start[t0 + u] : 0;
+      const long long t = t0 + u < re ? t0 + u : re - 1;     // (rows from `re` on are loaded for nothing)
+      nx[u] = load_here(x + t * D + c);
+      if (BWD) ng[u] = load_here(dy + t * D + c);
+      nf[u] = load_here(seq_start + t);
     }
   };
   fetch(r0);
@@ -1510,12 +1524,14 @@ TTB_EXPORT int ttb_bias_act_bwd(const void* dy, const void* x, const void* bias,
   LAUNCH_RET();
 }
 
-// a thread owns 4 channels of a filter of up to four taps, else 8
-static void conv_grid(long long T, int D, int W, int& threads, dim3& grid, int& rows_per_block) {
+// A thread owns 4 channels of a filter of up to four taps, else 8.  Blocks per SM: up to four taps, whole waves of what an SM holds, one
+// of the backward (4; its rows of overlap and column sums grow with the number of blocks: 8, 12 and 24 per SM take 85, 91 and 109 us
+// against 79) and two of the forward (12; 41 us, one wave 42, and 100 against 104 us for 16384 x 6144).
+static void conv_grid(long long T, int D, int W, bool bwd, int& threads, dim3& grid, int& rows_per_block) {
   const int vec = W <= 4 ? D / 4 : D / 8;
   threads = vec >= 128 ? 128 : ((vec + 31) / 32) * 32;
   const int gx = (vec + threads - 1) / threads;
-  long long want = (148LL * 8 + gx - 1) / gx;      // about eight blocks per SM in total
+  long long want = W <= 4 ? 148LL * (bwd ? 4 : 12) / gx : (148LL * 8 + gx - 1) / gx;
   if (want > T) want = T;
   if (want < 1) want = 1;
   rows_per_block = static_cast<int>((T + want - 1) / want);
@@ -1528,7 +1544,7 @@ TTB_EXPORT int ttb_causal_conv1d_fwd(const void* x, const void* w, const void* b
   if (T == 0) return 0;
   int threads, rpb;
   dim3 grid;
-  conv_grid(T, D, W, threads, grid, rpb);
+  conv_grid(T, D, W, false, threads, grid, rpb);
   if (W <= 4)
     causal_conv1d_w4_kernel<false><<<grid, threads, 0, STREAM(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
         (const __nv_bfloat16*)bias, seq_start, nullptr, (__nv_bfloat16*)y, nullptr, T, D, W, silu, rpb);
@@ -1542,7 +1558,7 @@ TTB_EXPORT int ttb_causal_conv1d_fwd(const void* x, const void* w, const void* b
 TTB_EXPORT int ttb_causal_conv1d_row_blocks(long long T, int D, int W) {
   int threads, rpb;
   dim3 grid;
-  conv_grid(T > 0 ? T : 1, D, W, threads, grid, rpb);
+  conv_grid(T > 0 ? T : 1, D, W, true, threads, grid, rpb);
   return static_cast<int>(grid.y);
 }
 
@@ -1553,7 +1569,7 @@ TTB_EXPORT int ttb_causal_conv1d_bwd(const void* dy, const void* x, const void* 
   if (T == 0) return 0;
   int threads, rpb;
   dim3 grid;
-  conv_grid(T, D, W, threads, grid, rpb);
+  conv_grid(T, D, W, true, threads, grid, rpb);
   if (W <= 4) {
     causal_conv1d_w4_kernel<true><<<grid, threads, 0, STREAM(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
         (const __nv_bfloat16*)bias, seq_start, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, part, T, D, W, silu, rpb);
