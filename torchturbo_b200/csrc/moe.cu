@@ -13,6 +13,7 @@
 //    GEMM never straddles experts and the host never learns the split sizes.
 //    Contract: ops/moe.py:10-46, ops/providers/native/moe_permutation.py:24-126.
 #include "common.cuh"
+#include <type_traits>
 
 namespace ttb {
 
@@ -22,43 +23,38 @@ constexpr int SEG_ALIGN = 128;
 
 enum ScoreFn : int { SOFTMAX_PRE = 0, SOFTMAX_POST = 1, SIGMOID = 2 };
 
-struct ArgMax {
-  float v;
-  int i;
-};
-__device__ __forceinline__ ArgMax warp_argmax(float v, int i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    float ov = __shfl_xor_sync(0xffffffffu, v, o);
-    int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
-  }
-  return {v, i};
+// Floats as integers in the same order; NaN ranks with -inf (it never wins, but something is always selected), a denormal is zero.
+// Zero stands for "none": no float maps to it.
+__device__ __forceinline__ unsigned rank_key(float v) {
+  unsigned u = __float_as_uint(v == v ? v : -INFINITY);
+  if ((u & 0x7fffffffu) < 0x00800000u) u = 0;
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
 }
 
-// Select top-k of `sel` (values per lane: expert id = j*32 + lane).  Returns ids through out_idx[k]
-// (identical on every lane) in descending order.
-__device__ __forceinline__ void warp_topk(const float (&sel)[MAX_E_PER_LANE], int epl, int E, int k, int lane,
-                                          int (&out_idx)[MAX_K]) {
-  unsigned taken = 0;
-  for (int r = 0; r < k; ++r) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
+// Top-k of `sel` (value j of a lane belongs to expert j * 32 + lane), in descending order, the lower id first among equals: lane r
+// returns the r-th id, 0x7fffffff where there is none left.  A round is two warp reductions over integers; as ten shuffles of value and
+// id, with the ids in an array that a loop of unknown length indexes, the selection was most of the router's time (below).
+template <int EPL>
+__device__ __forceinline__ int warp_topk(const float (&sel)[EPL], int E, int k, int lane) {
+  unsigned key[EPL];
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
-      if (j < epl) {
-        int e = j * 32 + lane;
-        if (e < E && !((taken >> j) & 1u)) {
-          float v = sel[j];
-          if (!(v == v)) v = -INFINITY;   // NaN never wins a comparison: rank it last instead of selecting nothing
-          if (v > bv || (v == bv && e < bi)) { bv = v; bi = e; }
-        }
-      }
-    }
-    ArgMax am = warp_argmax(bv, bi);
-    out_idx[r] = am.i;
-    if ((am.i & 31) == lane && am.i < E) taken |= 1u << (am.i >> 5);
+  for (int j = 0; j < EPL; ++j) key[j] = j * 32 + lane < E ? rank_key(sel[j]) : 0u;
+  int mine = 0x7fffffff;
+  for (int r = 0; r < k; ++r) {
+    unsigned best = key[0];
+    int bj = 0;
+#pragma unroll
+    for (int j = 1; j < EPL; ++j)
+      if (key[j] > best) { best = key[j]; bj = j; }
+    const unsigned top = __reduce_max_sync(0xffffffffu, best);
+    const unsigned e = best == top && best != 0u ? bj * 32 + lane : 0x7fffffff;
+    const unsigned first = __reduce_min_sync(0xffffffffu, e);
+    if (lane == r) mine = static_cast<int>(first);
+#pragma unroll
+    for (int j = 0; j < EPL; ++j)
+      if (first == j * 32 + lane) key[j] = 0u;
   }
+  return mine;
 }
 
 struct RouterParams {
@@ -76,37 +72,40 @@ struct RouterParams {
   float scaling;
 };
 
-__global__ void router_fwd_kernel(const RouterParams p) {
+// One warp per token, with the lanes' slots known at compile time (EPL = 1, 2, 4 or 8 for up to 32, 64, 128 or 256 experts).  Bound by the
+// chain of the selection's rounds.  4096 tokens, eight of 128 experts: 23 -> 12 us; 16384 tokens, 256 experts, with a bias: 105 -> 54;
+// 300 tokens, four of 64: 6.2 -> 3.0.
+template <int EPL>
+__global__ void __launch_bounds__(256) router_fwd_kernel(const RouterParams p) {
   extern __shared__ float s_scores[];  // [E] block partial
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
-  const int epl = (p.E + 31) / 32;
   if (p.score_partial) {
     for (int i = threadIdx.x; i < p.E; i += blockDim.x) s_scores[i] = 0.f;
     __syncthreads();
   }
   for (long long t = static_cast<long long>(blockIdx.x) * wpb + wib; t < p.T;
        t += static_cast<long long>(gridDim.x) * wpb) {
-    float lg[MAX_E_PER_LANE], sc[MAX_E_PER_LANE], sel[MAX_E_PER_LANE];
+    float lg[EPL], sc[EPL], sel[EPL];
     float mx = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       int e = j * 32 + lane;
-      lg[j] = (j < epl && e < p.E) ? p.logits[t * p.E + e] : -INFINITY;
+      lg[j] = (e < p.E) ? p.logits[t * p.E + e] : -INFINITY;
       mx = fmaxf(mx, lg[j]);
     }
     mx = warp_max(mx);
     float se = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) se += (lg[j] == -INFINITY) ? 0.f : __expf(lg[j] - mx);
+    for (int j = 0; j < EPL; ++j) se += (lg[j] == -INFINITY) ? 0.f : __expf(lg[j] - mx);
     se = warp_sum(se);
     const float lse = mx + logf(se);
     if (p.lse && lane == 0) p.lse[t] = lse;
     // normalised scores used by the aux loss (and by SOFTMAX_PRE / SIGMOID routing)
     float ssum = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       if (lg[j] == -INFINITY) { sc[j] = 0.f; continue; }
       sc[j] = (p.score_fn == SIGMOID) ? 1.f / (1.f + __expf(-lg[j])) : __expf(lg[j] - lse);
       ssum += sc[j];
@@ -114,7 +113,7 @@ __global__ void router_fwd_kernel(const RouterParams p) {
     if (p.score_fn == SIGMOID) ssum = warp_sum(ssum);
     // selection values
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       int e = j * 32 + lane;
       float base = (p.score_fn == SOFTMAX_POST) ? lg[j] : sc[j];
       if (lg[j] == -INFINITY) base = -INFINITY;
@@ -123,21 +122,15 @@ __global__ void router_fwd_kernel(const RouterParams p) {
       // outside [0, E).  As -inf a NaN row selects the lowest expert ids; its weights stay NaN and reach the loss.
       sel[j] = (base == base) ? base : -INFINITY;
     }
-    int idx[MAX_K];
-    warp_topk(sel, epl, p.E, p.k, lane, idx);
+    const int chosen = warp_topk<EPL>(sel, p.E, p.k, lane);
     // routing weights
     float w = 0.f;  // lane r (< k) holds weight r
     {
       float raw = -INFINITY;
-      for (int r = 0; r < p.k; ++r) {
-        int e = idx[r];
-        // value lives on lane (e & 31), slot (e >> 5): broadcast it
-        float vv = 0.f;
 #pragma unroll
-        for (int j = 0; j < MAX_E_PER_LANE; ++j)
-          if (j == (e >> 5)) vv = (p.score_fn == SOFTMAX_POST) ? lg[j] : sc[j];
-        vv = __shfl_sync(0xffffffffu, vv, e & 31);
-        if (lane == r) raw = vv;
+      for (int j = 0; j < EPL; ++j) {
+        const float vv = __shfl_sync(0xffffffffu, p.score_fn == SOFTMAX_POST ? lg[j] : sc[j], chosen & 31);
+        if (lane < p.k && j == (chosen >> 5)) raw = vv;
       }
       if (p.score_fn == SOFTMAX_POST) {
         float m2 = warp_max(raw);
@@ -153,37 +146,28 @@ __global__ void router_fwd_kernel(const RouterParams p) {
       }
       w *= p.scaling;
     }
-    for (int r = 0; r < p.k; ++r) {
-      if (lane == r) {
-        const int e_sel = idx[r] < p.E ? idx[r] : p.E - 1;   // k > number of selectable experts: stay in range
-        p.topk_idx[t * p.k + r] = e_sel;
-        p.topk_prob[t * p.k + r] = w;
-        if (p.counts) atomicAdd(&p.counts[e_sel], 1);
-      }
+    const int e_sel = chosen < p.E ? chosen : p.E - 1;   // k > number of selectable experts: stay in range
+    if (lane < p.k) {
+      p.topk_idx[t * p.k + lane] = e_sel;
+      p.topk_prob[t * p.k + lane] = w;
+      if (p.counts) atomicAdd(&p.counts[e_sel], 1);
     }
     // aux statistics: bias-free top-k over normalised scores, padding excluded
     const bool valid = p.valid_mask ? (p.valid_mask[t] != 0) : true;
     if ((p.score_partial || p.aux_counts) && valid) {
-      float nsc[MAX_E_PER_LANE];
+      float nsc[EPL];
       const float inv = (p.score_fn == SIGMOID) ? 1.f / (ssum + 1e-20f) : 1.f;
 #pragma unroll
-      for (int j = 0; j < MAX_E_PER_LANE; ++j) nsc[j] = (lg[j] == -INFINITY) ? -INFINITY : sc[j] * inv;
+      for (int j = 0; j < EPL; ++j) nsc[j] = (lg[j] == -INFINITY) ? -INFINITY : sc[j] * inv;
       if (p.aux_counts) {
-        int aidx[MAX_K];
-        if (p.expert_bias) {
-          warp_topk(nsc, epl, p.E, p.k, lane, aidx);
-        } else {
-#pragma unroll
-          for (int r = 0; r < MAX_K; ++r) aidx[r] = idx[r];
-        }
-        for (int r = 0; r < p.k; ++r)
-          if (lane == r) atomicAdd(&p.aux_counts[aidx[r] < p.E ? aidx[r] : p.E - 1], 1);
+        const int picked = p.expert_bias ? warp_topk<EPL>(nsc, p.E, p.k, lane) : chosen;
+        if (lane < p.k) atomicAdd(&p.aux_counts[picked < p.E ? picked : p.E - 1], 1);
       }
       if (p.score_partial) {
 #pragma unroll
-        for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+        for (int j = 0; j < EPL; ++j) {
           int e = j * 32 + lane;
-          if (j < epl && e < p.E) atomicAdd(&s_scores[e], nsc[j]);
+          if (e < p.E) atomicAdd(&s_scores[e], nsc[j]);
         }
       }
     }
@@ -210,18 +194,18 @@ struct RouterBwdParams {
   float scaling;
 };
 
-__global__ void router_bwd_kernel(const RouterBwdParams p) {
+template <int EPL>
+__global__ void __launch_bounds__(256) router_bwd_kernel(const RouterBwdParams p) {
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
-  const int epl = (p.E + 31) / 32;
   for (long long t = static_cast<long long>(blockIdx.x) * wpb + (threadIdx.x >> 5); t < p.T;
        t += static_cast<long long>(gridDim.x) * wpb) {
-    float lg[MAX_E_PER_LANE], sc[MAX_E_PER_LANE], ds[MAX_E_PER_LANE], dl[MAX_E_PER_LANE];
+    float lg[EPL], sc[EPL], ds[EPL], dl[EPL];
     float mx = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       int e = j * 32 + lane;
-      lg[j] = (j < epl && e < p.E) ? p.logits[t * p.E + e] : -INFINITY;
+      lg[j] = (e < p.E) ? p.logits[t * p.E + e] : -INFINITY;
       mx = fmaxf(mx, lg[j]);
       ds[j] = 0.f;
       dl[j] = 0.f;
@@ -229,12 +213,12 @@ __global__ void router_bwd_kernel(const RouterBwdParams p) {
     mx = warp_max(mx);
     float se = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) se += (lg[j] == -INFINITY) ? 0.f : __expf(lg[j] - mx);
+    for (int j = 0; j < EPL; ++j) se += (lg[j] == -INFINITY) ? 0.f : __expf(lg[j] - mx);
     se = warp_sum(se);
     const float lse = mx + logf(se);
     float ssum = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       if (lg[j] == -INFINITY) { sc[j] = 0.f; continue; }
       sc[j] = (p.score_fn == SIGMOID) ? 1.f / (1.f + __expf(-lg[j])) : __expf(lg[j] - lse);
       ssum += sc[j];
@@ -261,7 +245,7 @@ __global__ void router_bwd_kernel(const RouterBwdParams p) {
             int e = __shfl_sync(0xffffffffu, my_e, r);
             float vv = 0.f;
 #pragma unroll
-            for (int j = 0; j < MAX_E_PER_LANE; ++j)
+            for (int j = 0; j < EPL; ++j)
               if (j == (e >> 5)) vv = sc[j];
             vv = __shfl_sync(0xffffffffu, vv, e & 31);
             if (lane == r) sraw = vv;
@@ -279,7 +263,7 @@ __global__ void router_bwd_kernel(const RouterBwdParams p) {
         float g = __shfl_sync(0xffffffffu, g_sel, r);
         if ((e & 31) == lane) {
 #pragma unroll
-          for (int j = 0; j < MAX_E_PER_LANE; ++j)
+          for (int j = 0; j < EPL; ++j)
             if (j == (e >> 5)) {
               if (p.score_fn == SOFTMAX_POST) dl[j] += g; else ds[j] += g;
             }
@@ -293,47 +277,47 @@ __global__ void router_bwd_kernel(const RouterBwdParams p) {
         const float Sall = ssum + 1e-20f;
         float dot = 0.f;
 #pragma unroll
-        for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+        for (int j = 0; j < EPL; ++j) {
           int e = j * 32 + lane;
-          if (j < epl && e < p.E) dot += p.aux_grad[e] * sc[j] / Sall;
+          if (e < p.E) dot += p.aux_grad[e] * sc[j] / Sall;
         }
         dot = warp_sum(dot);
 #pragma unroll
-        for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+        for (int j = 0; j < EPL; ++j) {
           int e = j * 32 + lane;
-          if (j < epl && e < p.E) ds[j] += (p.aux_grad[e] - dot) / Sall;
+          if (e < p.E) ds[j] += (p.aux_grad[e] - dot) / Sall;
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+        for (int j = 0; j < EPL; ++j) {
           int e = j * 32 + lane;
-          if (j < epl && e < p.E) ds[j] += p.aux_grad[e];
+          if (e < p.E) ds[j] += p.aux_grad[e];
         }
       }
     }
     // ---- score -> logit jacobian
     if (p.score_fn == SIGMOID) {
 #pragma unroll
-      for (int j = 0; j < MAX_E_PER_LANE; ++j) dl[j] += ds[j] * sc[j] * (1.f - sc[j]);
+      for (int j = 0; j < EPL; ++j) dl[j] += ds[j] * sc[j] * (1.f - sc[j]);
     } else {
       float dot = 0.f;
 #pragma unroll
-      for (int j = 0; j < MAX_E_PER_LANE; ++j) dot += ds[j] * sc[j];
+      for (int j = 0; j < EPL; ++j) dot += ds[j] * sc[j];
       dot = warp_sum(dot);
 #pragma unroll
-      for (int j = 0; j < MAX_E_PER_LANE; ++j) dl[j] += sc[j] * (ds[j] - dot);
+      for (int j = 0; j < EPL; ++j) dl[j] += sc[j] * (ds[j] - dot);
     }
     // ---- logsumexp gradient (z-loss): d(lse)/dl = softmax(l)
     if (p.dlse) {
       const float zc = p.dlse[t];
 #pragma unroll
-      for (int j = 0; j < MAX_E_PER_LANE; ++j)
+      for (int j = 0; j < EPL; ++j)
         if (lg[j] != -INFINITY) dl[j] += zc * __expf(lg[j] - lse);
     }
 #pragma unroll
-    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       int e = j * 32 + lane;
-      if (j < epl && e < p.E) p.dlogits[t * p.E + e] = dl[j];
+      if (e < p.E) p.dlogits[t * p.E + e] = dl[j];
     }
   }
 }
@@ -591,6 +575,14 @@ using namespace ttb;
 #define STREAM(s) reinterpret_cast<cudaStream_t>(s)
 #define LAUNCH_RET() do { cudaError_t e__ = cudaGetLastError(); return e__ == cudaSuccess ? 0 : 400 + (int)e__; } while (0)
 
+template <typename F>
+static void by_slots(int E, F launch) {
+  if (E <= 32) launch(std::integral_constant<int, 1>{});
+  else if (E <= 64) launch(std::integral_constant<int, 2>{});
+  else if (E <= 128) launch(std::integral_constant<int, 4>{});
+  else launch(std::integral_constant<int, 8>{});
+}
+
 // score_partial: [grid, E] scratch; score_sum: [E] output (may be null together with score_partial)
 TTB_EXPORT int ttb_router_fwd(const float* logits, const float* expert_bias, const unsigned char* valid_mask,
                               int* topk_idx, float* topk_prob, float* lse, float* score_partial, float* score_sum,
@@ -602,7 +594,7 @@ TTB_EXPORT int ttb_router_fwd(const float* logits, const float* expert_bias, con
                  score_fn, scaling};
   const long long need = (T + 7) / 8;
   if (grid > need) grid = (int)need;
-  router_fwd_kernel<<<grid, 256, E * sizeof(float), STREAM(stream)>>>(p);
+  by_slots(E, [&](auto slots) { router_fwd_kernel<decltype(slots)::value><<<grid, 256, E * sizeof(float), STREAM(stream)>>>(p); });
   if (score_partial && score_sum)
     colsum_f32_kernel<<<(E + 31) / 32, 1024, 0, STREAM(stream)>>>(score_partial, score_sum, grid, E);
   LAUNCH_RET();
@@ -618,7 +610,7 @@ TTB_EXPORT int ttb_router_bwd(const float* logits, const int* topk_idx, const fl
                     scaling};
   long long grid = (T + 7) / 8;
   if (grid > 4096) grid = 4096;
-  router_bwd_kernel<<<(unsigned)grid, 256, 0, STREAM(stream)>>>(p);
+  by_slots(E, [&](auto slots) { router_bwd_kernel<decltype(slots)::value><<<(unsigned)grid, 256, 0, STREAM(stream)>>>(p); });
   LAUNCH_RET();
 }
 
