@@ -9,15 +9,25 @@ namespace ttb {
 // Gated RMSNorm of short rows (head widths of the linear-attention layers): y = bf16(n * act(gate)) with
 // n = bf16(bf16(x * rstd) * w), H = 8 L channels held by L lanes, so a warp normalises 32 / L rows with shuffles only.
 //   dn = bf16(dy * act(gate)), dgate = dy * n * act'(gate), dx and dw as in the plain norm with dn in the place of dy
-// Every rounding of the separate kernels (norm, fp32 product, cast) is kept.  131072 rows of 128 (100 and 168 MB) take 30 us
-// forward and 47 us backward, 24 and 37 with approximate exponentials and divisions; the plain norm's block per row alone took
-// 380 us backward on them.
+// Every rounding of the separate kernels (norm, fp32 product, cast) is kept.  A thread has its next row's loads under way while it works on
+// one: 131072 rows of 128 (100 and 168 MB) from cold caches 37 -> 35 us forward and 62 -> 52 us backward with its column sums (memory
+// alone: 16 and 27).  What is left over that is exponentials and divisions at full precision (approximate ones saved 6 and 10 us).
 // ============================================================================
 template <int L>
 __device__ __forceinline__ float lane_group_sum(float v) {
 #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+// eight values of a row that is still on its way: the load stays here, the unpacking where the row is used
+__device__ __forceinline__ uint4 load_here(const __nv_bfloat16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
@@ -31,10 +41,20 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_fwd_kernel(const __nv_bfloa
   load8(w + c, wf);
   // all lanes of a warp stay in the loop (the shuffles name the whole warp); rows past the end are computed and dropped
   const long long last = (R + ROWS - 1) / ROWS * ROWS;
-  for (long long row = static_cast<long long>(blockIdx.x) * ROWS + threadIdx.x / L; row < last; row += static_cast<long long>(gridDim.x) * ROWS) {
+  const long long step = static_cast<long long>(gridDim.x) * ROWS;
+  long long row = static_cast<long long>(blockIdx.x) * ROWS + threadIdx.x / L;
+  uint4 nx, ng;
+  auto fetch = [&](long long r) {      // (a row past the end is loaded as the last one)
+    const long long at = (r < R ? r : R - 1) * H + c;
+    nx = load_here(x + at); ng = load_here(gate + at);
+  };
+  fetch(row);
+  for (; row < last; row += step) {
     const bool ok = row < R;
-    float f[8] = {}, g[8] = {};
-    if (ok) { load8(x + row * H + c, f); load8(gate + row * H + c, g); }
+    const uint4 cx = nx, cg = ng;
+    if (row + step < last) fetch(row + step);
+    float f[8], g[8];
+    unpack8(cx, f); unpack8(cg, g);
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
@@ -62,16 +82,23 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
   float wf[8], dw[8] = {};
   load8(w + c, wf);
   const long long last = (R + ROWS - 1) / ROWS * ROWS;
-  for (long long row = static_cast<long long>(blockIdx.x) * ROWS + r0; row < last; row += static_cast<long long>(gridDim.x) * ROWS) {
+  const long long step = static_cast<long long>(gridDim.x) * ROWS;
+  long long row = static_cast<long long>(blockIdx.x) * ROWS + r0;
+  uint4 nx, ng, nd;
+  float nr;
+  auto fetch = [&](long long r) {
+    const long long k = r < R ? r : R - 1, at = k * H + c;
+    nx = load_here(x + at); ng = load_here(gate + at); nd = load_here(dy + at);
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(nr) : "l"(rstd_in + k));
+  };
+  fetch(row);
+  for (; row < last; row += step) {
     const bool ok = row < R;
-    float f[8] = {}, g[8] = {}, d[8] = {};
-    float rstd = 0.f;
-    if (ok) {
-      load8(x + row * H + c, f);
-      load8(gate + row * H + c, g);
-      load8(dy + row * H + c, d);
-      rstd = rstd_in[row];
-    }
+    const uint4 cx = nx, cg = ng, cd = nd;
+    const float rstd = nr;
+    if (row + step < last) fetch(row + step);
+    float f[8], g[8], d[8];
+    unpack8(cx, f); unpack8(cg, g); unpack8(cd, d);
     float dot = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -81,7 +108,7 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
       g[j] = d[j] * n * slope;
       f[j] *= rstd;
       const float dn = round_bf16(d[j] * act);
-      dw[j] += dn * f[j];
+      if (ok) dw[j] += dn * f[j];
       d[j] = dn * wf[j];
       dot += d[j] * f[j];
     }
