@@ -17,10 +17,11 @@
 // never to the bf16 inputs.  Two terms and three products on both-fp32 products left dg 4 to 14 and dbeta 13 to 16 times as
 // far from 64 bits as fp32 products; now dbeta, gx and gS are closer than those and dg within 1.5 times of them.
 //
-// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.15 ms, out 0.13, bwd_pre 0.09, bwd_post 0.58 (0.60
-// when every warp split again the fp32 tiles that it shares with three others); with two-term operands and sums kept in the tensor
-// cores' accumulators 0.14, 0.11, 0.09 and 0.45.  A gated-delta-net layer forward + backward takes 2.5 ms, against 10.4 when the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and
-// gathers over materialised [chunk, 64, 64 .. 128] tensors.
+// Measured (4096 tokens, 32 heads, four documents, one pass): prep 0.13 ms, out 0.13, bwd_pre 0.09, bwd_post 0.50 (0.15, 0.14, 0.10 and
+// 0.58 before the row norms ran beside the loads and the loads that need no row before the rows' own; 0.60 when every warp split
+// again the fp32 tiles that it shares with three others).  A gated-delta-net layer forward + backward takes 2.0 ms, against 10.4 when
+// the chunk-parallel part was about 250 launches of fp32 products, element-wise passes and gathers over materialised
+// [chunk, 64, 64 .. 128] tensors.
 //
 // Why mma.sync and not tcgen05: the products are 64 x 64 x 128 at most, each feeds the next through registers and shared
 // memory, and their operands are built element by element (splits, decays).  What bounds them, from the counters of the same

@@ -6,7 +6,7 @@ The chunked evaluation splits into work that is parallel over chunks and one rec
       G = cumsum(g) inside the chunk,  D_ij = exp(G_i - G_j) (i >= j)
       T = (I + strict_lower(k beta k^T . D))^-1,  u = T (beta v),  w = T (beta k e^G)
       q_in = q e^G,  k_out = k e^(G_last - G),  d = e^(G_last)
-  recurrence (the `delta_state` tcgen05 kernel, two or four CTAs per sequence and head, which own columns of the state;
+  recurrence (the `delta_state` tcgen05 kernel, whose work items are 32 columns of the state of a sequence and head;
   forward and reverse):
       v_new_c = u_c - w_c S_c,        S_{c+1} = d_c (.) S_c + k_out_c^T v_new_c
   chunk-parallel again:
