@@ -101,3 +101,29 @@ def test_layouts(rows, cols):
         t.start()
         t.join()
         same(box[0], "thread")
+
+
+@pytest.mark.gpu
+def test_tensors_without_storage_are_an_error_and_not_a_crash():
+    """Batched gradients have no address: the launch function finds out while it holds no interpreter lock."""
+    x = torch.randn(16, 64, device="cuda").bfloat16()
+    seen = []
+
+    class Probe(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, t):
+            return t.float().sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            with pytest.raises((RuntimeError, AssertionError)):
+                K.rmsnorm_fwd(x * g.bfloat16(), x[0], 1e-6)
+            with pytest.raises((RuntimeError, AssertionError)):
+                K.gemm(x * g.bfloat16(), x)
+            seen.append(True)
+            return x * g.bfloat16()
+
+    leaf = x.clone().requires_grad_(True)
+    torch.autograd.grad(Probe.apply(leaf), leaf, torch.tensor([1.0, 2.0], device="cuda"), is_grads_batched=True)
+    assert seen
+    assert K.gemm(x, x).shape == (16, 16)

@@ -111,14 +111,22 @@ void check_device(const Tensor& t) {
                              "; call torch.cuda.set_device() for this process before using the ops");
 }
 
+// Gives the interpreter lock up for its lifetime.  An object, because a call may leave by an exception (the address of a tensor that has
+// no storage, such as the batched gradients of `is_grads_batched`), and whoever turns that into a Python error needs the lock.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 // Runs a C entry on the current stream without the interpreter lock.
 template <typename F>
 void launch(const char* what, int kernels, F call) {
   void* stream = c10::cuda::getCurrentCUDAStream().stream();
   int code;
-  Py_BEGIN_ALLOW_THREADS
-  code = call(stream);
-  Py_END_ALLOW_THREADS
+  {
+    const Unlocked without_lock;
+    code = call(stream);
+  }
   if (code != 0) fail(g_kernel_error, std::string(what) + " failed with code " + std::to_string(code));
   g_launches.fetch_add(kernels, std::memory_order_relaxed);
 }
@@ -138,6 +146,7 @@ PyObject* wrap_all(const Ts&... ts) {
 // rows x last dimension
 Tensor rows2d(const Tensor& t) { return t.dim() == 2 ? t.contiguous() : t.reshape({-1, t.size(-1)}).contiguous(); }
 Tensor like_shape(const Tensor& t2, const Tensor& x) { return x.dim() == 2 ? t2 : t2.view(x.sizes()); }
+int kda_gate_row_blocks(long long rows, int heads) { return ttb_kda_gate_row_blocks(rows, heads); }
 int row_blocks(long long rows, const Tensor& t) { return static_cast<int>(std::max<long long>(1, std::min<long long>(rows, 2 * sms(t)))); }
 at::ScalarType out_type(bool f32out) { return f32out ? at::kFloat : at::kBFloat16; }
 
@@ -555,7 +564,7 @@ PyObject* kda_gate_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const bool bounded = in.flag();
     const double bound = in.real();
     const long long R = g.size(0), H = g.size(1), D = g.size(2);
-    const int blocks = ttb_kda_gate_row_blocks(R, static_cast<int>(H));
+    const int blocks = kda_gate_row_blocks(R, static_cast<int>(H));
     const Tensor dg = empty_rows(g), part = empty({std::max(blocks, 1), 2, H * D}, at::kFloat, g);
     const Tensor sums = R ? empty({2, H * D}, at::kFloat, g) : at::zeros({2, H * D}, plain(g).dtype(at::kFloat));
     launch("ttb_kda_gate_bwd", 2, [&](void* st) {
@@ -610,7 +619,8 @@ PyObject* delta_prep(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Tensor wk = empty({2, H, NC, 64, 128}, at::kBFloat16, d.q), decay = d.vec() ? empty({H, NC, 128}, at::kFloat, d.q) : empty({H, NC}, at::kFloat, d.q);
     const Tensor T = tri.select(0, 0), A = tri.select(0, 1), w = wk.select(0, 0), k_out = wk.select(0, 1);
     launch(d.vec() ? "ttb_delta_vec_prep" : "ttb_delta_prep", 1, [&](void* st) {
-      return (d.vec() ? ttb_delta_vec_prep : ttb_delta_prep)(a, f32w(T), f32w(A), f32w(u), to_(w), to_(k_out), f32w(decay), st);
+      if (d.vec()) return ttb_delta_vec_prep(a, f32w(T), f32w(A), f32w(u), to_(w), to_(k_out), f32w(decay), st);
+      return ttb_delta_prep(a, f32w(T), f32w(A), f32w(u), to_(w), to_(k_out), f32w(decay), st);
     });
     return wrap_all(T, A, u, w, k_out, decay);
   });
@@ -624,7 +634,8 @@ PyObject* delta_out(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const ttb::DeltaChunkIn* a = d.fill(in);
     const Tensor o = empty(d.v.sizes(), at::kBFloat16, d.q);
     launch(d.vec() ? "ttb_delta_vec_out" : "ttb_delta_out", 1, [&](void* st) {
-      return (d.vec() ? ttb_delta_vec_out : ttb_delta_out)(a, f32(A), f32(x), f32(states), static_cast<int>(states.size(1)) - a->NC, to_(o), st);
+      if (d.vec()) return ttb_delta_vec_out(a, f32(A), f32(x), f32(states), static_cast<int>(states.size(1)) - a->NC, to_(o), st);
+      return ttb_delta_out(a, f32(A), f32(x), f32(states), static_cast<int>(states.size(1)) - a->NC, to_(o), st);
     });
     return wrap(o);
   });
@@ -640,7 +651,8 @@ PyObject* delta_bwd_pre(PyObject*, PyObject* const* args, Py_ssize_t n) {
     need(dout.is_contiguous() && is_bf16(dout) && dout.sizes() == d.v.sizes(), "the gradient has v's shape");
     const Tensor gx = empty({a->H, a->NC, 64, 128}, at::kFloat, d.q), gs = empty({a->H, a->NC + nseq, 128, 128}, at::kFloat, d.q);
     launch(d.vec() ? "ttb_delta_vec_bwd_pre" : "ttb_delta_bwd_pre", 1, [&](void* st) {
-      return (d.vec() ? ttb_delta_vec_bwd_pre : ttb_delta_bwd_pre)(a, at_(dout), f32(A), nseq, f32w(gx), f32w(gs), st);
+      if (d.vec()) return ttb_delta_vec_bwd_pre(a, at_(dout), f32(A), nseq, f32w(gx), f32w(gs), st);
+      return ttb_delta_bwd_pre(a, at_(dout), f32(A), nseq, f32w(gx), f32w(gs), st);
     });
     return wrap_all(gx, gs);
   });
