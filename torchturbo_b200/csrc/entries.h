@@ -82,6 +82,7 @@ TTB_EXPORT int ttb_delta_vec_bwd_post(const ttb::DeltaChunkIn*, const void*, con
 TTB_EXPORT int ttb_delta_head_sum(const void*, const void*, void*, void*, long long, int, void*);
 TTB_EXPORT int ttb_delta_state_scan(const void*, const void*, const float*, float*, const float*, int, const float*, const float*, float*,
                             const int*, int, int, int, int, float, float, void*);
+TTB_EXPORT int ttb_scale(const void*, int, const float*, void*, int, long long, int, void*);
 TTB_EXPORT int ttb_copy_words(void*, const void*, long long, void*);
 TTB_EXPORT int ttb_kda_gate_row_blocks(long long, int);
 TTB_EXPORT int ttb_kda_gate_fwd(const void*, const void*, int, const void*, int, float*, long long, int, int, float, void*);

@@ -514,6 +514,24 @@ PyObject* gdn_gate_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// a tensor times a factor on the device
+// ---------------------------------------------------------------------------------------------
+PyObject* scale(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Args in(args, n, 3);
+    const Tensor &x = in.tensor(), &g = in.tensor();
+    const bool bf16 = in.flag();
+    check_device(x);
+    check_device(g);
+    need(x.is_contiguous() && (is_bf16(x) || x.scalar_type() == at::kFloat), "scale: a contiguous bf16 or fp32 tensor");
+    need(g.numel() == 1 && g.scalar_type() == at::kFloat, "scale: one fp32 factor");
+    const Tensor out = empty(x.sizes(), bf16 ? at::kBFloat16 : at::kFloat, x);
+    launch("ttb_scale", 1, [&](void* st) { return ttb_scale(at_(x), is_bf16(x), f32(g), to_(out), bf16, x.numel(), sms(x), st); });
+    return wrap(out);
+  });
+}
+
+// ---------------------------------------------------------------------------------------------
 // tables between pinned host memory and the device
 // ---------------------------------------------------------------------------------------------
 PyObject* copy_words(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -844,7 +862,7 @@ PyObject* launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_From
 #define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ENTRY(setup), ENTRY(launches), ENTRY(gemm), ENTRY(rmsnorm_fwd), ENTRY(rmsnorm_bwd), ENTRY(layernorm_fwd), ENTRY(layernorm_bwd),
                          ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(gdn_gate_fwd),
-                         ENTRY(gdn_gate_bwd), ENTRY(copy_words), ENTRY(kda_gate_fwd), ENTRY(kda_gate_bwd), ENTRY(delta_prep), ENTRY(delta_out), ENTRY(delta_bwd_pre),
+                         ENTRY(gdn_gate_bwd), ENTRY(scale), ENTRY(copy_words), ENTRY(kda_gate_fwd), ENTRY(kda_gate_bwd), ENTRY(delta_prep), ENTRY(delta_out), ENTRY(delta_bwd_pre),
                          ENTRY(delta_bwd_post), ENTRY(delta_state_scan), ENTRY(rope), ENTRY(swiglu_fwd),
                          ENTRY(swiglu_bwd), ENTRY(attn_fwd), ENTRY(attn_bwd), {nullptr, nullptr, 0, nullptr}};
 #undef ENTRY

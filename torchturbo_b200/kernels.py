@@ -464,6 +464,12 @@ def adamw_step(plan: MultiTensorPlan, *, lr, beta1, beta2, eps, weight_decay, st
                            C.c_float(bc2_sqrt), _p(clip), C.c_float(grad_prescale), _stream()), "ttb_adamw")
 
 
+def scale(x: torch.Tensor, factor: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """`(x.float() * factor).to(dtype)` in one pass: x contiguous bf16 or fp32, factor one fp32 value on the device, dtype bf16 or fp32."""
+    assert dtype in (torch.bfloat16, torch.float32)
+    return host().scale(x, factor, dtype == torch.bfloat16)
+
+
 # --------------------------------------------------------------------------------------
 # MoE router / permutation
 # --------------------------------------------------------------------------------------

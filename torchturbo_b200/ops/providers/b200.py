@@ -470,11 +470,12 @@ def _rope_rows(x: torch.Tensor) -> torch.Tensor:
 
 
 def _eager(*tensors) -> bool:
-    """Ordinary tensors outside tracers, function transforms and forward-mode differentiation.  An operator that has always
+    """Ordinary tensors outside tracers, function transforms, batched gradients and forward-mode differentiation.  An operator that has always
     been made of torch operations stays so for everything else."""
     return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active()
                 or torch._C._get_dispatch_mode(torch._C._TorchDispatchModeKey.PROXY) is not None) and all(
-        type(t) in (torch.Tensor, torch.nn.Parameter) and forward_ad.unpack_dual(t).tangent is None for t in tensors)
+        type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t) and forward_ad.unpack_dual(t).tangent is None
+        for t in tensors)
 
 
 class RopeFn(torch.autograd.Function):
@@ -728,6 +729,14 @@ class B200GroupedMatmul(_B200Op):
 # ------------------------------------------------------------------------------------------------
 # losses
 # ------------------------------------------------------------------------------------------------
+def _scaled(x, g, dtype):
+    """A loss's saved gradient times the loss's own; what a graph or a transform of the gradient has to see stays torch operations."""
+    if (torch.is_grad_enabled() or not _eager(x, g) or not x.is_cuda or g.device != x.device or not x.is_contiguous()
+            or x.dtype not in (BF16, torch.float32) or dtype not in (BF16, torch.float32)):
+        return (x.float() * g).to(dtype)
+    return K.scale(x, g.float(), dtype)
+
+
 class CrossEntropyFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, labels):
@@ -741,7 +750,7 @@ class CrossEntropyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (grad,) = ctx.saved_tensors
-        return (grad.float() * g).to(ctx.dtype).view(ctx.shape), None
+        return _scaled(grad, g, ctx.dtype).view(ctx.shape), None
 
 
 @_custom("cross_entropy_loss", "b200_cross_entropy")
@@ -813,8 +822,8 @@ class LinearCrossEntropyFn(torch.autograd.Function):
                 gw = K.gemm(dlogits, h2, a_mn=True, b_mn=True, out_dtype=wdtype, alpha=g.float().reshape(1))
         else:
             dh, dw = ctx.saved_tensors
-            gw = (dw * g).to(wdtype) if dw is not None else None
-        gh = (dh * g.to(dh.dtype)).view(shape) if dh is not None else None
+            gw = _scaled(dw, g, wdtype) if dw is not None else None
+        gh = _scaled(dh, g, dh.dtype).view(shape) if dh is not None else None
         return gh, gw, None, None
 
 
