@@ -72,14 +72,9 @@ TTB_EXPORT int ttb_qknorm_rope_bwd(const void*, const void*, const void*, const 
 TTB_EXPORT int ttb_delta_prep(const ttb::DeltaChunkIn*, float*, float*, float*, void*, void*, float*, void*);
 TTB_EXPORT int ttb_delta_out(const ttb::DeltaChunkIn*, const float*, const float*, const float*, int, void*, void*);
 TTB_EXPORT int ttb_delta_bwd_pre(const ttb::DeltaChunkIn*, const void*, const float*, int, float*, float*, void*);
-TTB_EXPORT int ttb_delta_bwd_post(const ttb::DeltaChunkIn*, const void*, const float*, const float*, const float*, const float*, const float*, int,
-                            void*, void*, void*, float*, float*, void*);
 TTB_EXPORT int ttb_delta_vec_prep(const ttb::DeltaChunkIn*, float*, float*, float*, void*, void*, float*, void*);
 TTB_EXPORT int ttb_delta_vec_out(const ttb::DeltaChunkIn*, const float*, const float*, const float*, int, void*, void*);
 TTB_EXPORT int ttb_delta_vec_bwd_pre(const ttb::DeltaChunkIn*, const void*, const float*, int, float*, float*, void*);
-TTB_EXPORT int ttb_delta_vec_bwd_post(const ttb::DeltaChunkIn*, const void*, const float*, const float*, const float*, const float*, const float*,
-                            int, void*, void*, void*, float*, float*, float*, void*);
-TTB_EXPORT int ttb_delta_head_sum(const void*, const void*, void*, void*, long long, int, void*);
 TTB_EXPORT int ttb_delta_state_scan(const void*, const void*, const float*, float*, const float*, int, const float*, const float*, float*,
                             const int*, int, int, int, int, float, float, void*);
 TTB_EXPORT int ttb_scale(const void*, int, const float*, void*, int, long long, int, void*);

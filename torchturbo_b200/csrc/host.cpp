@@ -676,41 +676,6 @@ PyObject* delta_bwd_pre(PyObject*, PyObject* const* args, Py_ssize_t n) {
   });
 }
 
-PyObject* delta_bwd_post(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  return guarded([&]() -> PyObject* {
-    Args in(args, n, 14);
-    DeltaIn d(in);
-    const Tensor &dout = in.tensor(), &T = in.tensor(), &x = in.tensor(), &dx = in.tensor(), &states = in.tensor(), &dstates = in.tensor();
-    const ttb::DeltaChunkIn* a = d.fill(in);
-    need(dout.is_contiguous() && is_bf16(dout) && dout.sizes() == d.v.sizes(), "the gradient has v's shape");
-    const int nseq = static_cast<int>(states.size(1)) - a->NC;
-    Tensor dq = empty(d.v.sizes(), at::kBFloat16, d.q), dk = empty(d.v.sizes(), at::kBFloat16, d.q);     // of every value head
-    const Tensor dv = empty(d.v.sizes(), at::kBFloat16, d.q), dg = empty(d.g.sizes(), at::kFloat, d.q), db = empty(d.beta.sizes(), at::kFloat, d.q);
-    if (d.vec()) {
-      // held until the launches are queued: a pointer alone would let another thread of this stream be given the block first
-      const Tensor scratch = empty({4, x.size(0), x.size(1), x.size(2), x.size(3)}, at::kFloat, d.q);
-      launch("ttb_delta_vec_bwd_post", 2, [&](void* st) {
-        return ttb_delta_vec_bwd_post(a, at_(dout), f32(T), f32(x), f32(dx), f32(states), f32(dstates), nseq, to_(dq), to_(dk), to_(dv), f32w(dg),
-                                      f32w(db), f32w(scratch), st);
-      });
-    } else {
-      launch("ttb_delta_bwd_post", 1, [&](void* st) {
-        return ttb_delta_bwd_post(a, at_(dout), f32(T), f32(x), f32(dx), f32(states), f32(dstates), nseq, to_(dq), to_(dk), to_(dv), f32w(dg),
-                                  f32w(db), st);
-      });
-    }
-    if (a->rep > 1) {
-      const Tensor sq = empty(d.q.sizes(), at::kBFloat16, d.q), sk = empty(d.q.sizes(), at::kBFloat16, d.q);
-      launch("ttb_delta_head_sum", 1, [&](void* st) {
-        return ttb_delta_head_sum(at_(dq), at_(dk), to_(sq), to_(sk), d.q.size(0) * d.q.size(1), a->rep, st);
-      });
-      dq = sq;
-      dk = sk;
-    }
-    return wrap_all(dq, dk, dv, dg, db);
-  });
-}
-
 PyObject* delta_state_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     Args in(args, n, 10);
@@ -863,7 +828,7 @@ PyObject* launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_From
 PyMethodDef methods[] = {ENTRY(setup), ENTRY(launches), ENTRY(gemm), ENTRY(rmsnorm_fwd), ENTRY(rmsnorm_bwd), ENTRY(layernorm_fwd), ENTRY(layernorm_bwd),
                          ENTRY(bias_act_fwd), ENTRY(bias_act_bwd), ENTRY(qknorm_rope_fwd), ENTRY(qknorm_rope_bwd), ENTRY(qkv_rope_fwd), ENTRY(qkv_rope_bwd), ENTRY(gdn_gate_fwd),
                          ENTRY(gdn_gate_bwd), ENTRY(scale), ENTRY(copy_words), ENTRY(kda_gate_fwd), ENTRY(kda_gate_bwd), ENTRY(delta_prep), ENTRY(delta_out), ENTRY(delta_bwd_pre),
-                         ENTRY(delta_bwd_post), ENTRY(delta_state_scan), ENTRY(rope), ENTRY(swiglu_fwd),
+                         ENTRY(delta_state_scan), ENTRY(rope), ENTRY(swiglu_fwd),
                          ENTRY(swiglu_bwd), ENTRY(attn_fwd), ENTRY(attn_bwd), {nullptr, nullptr, 0, nullptr}};
 #undef ENTRY
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "ttb_host", nullptr, -1, methods};

@@ -97,7 +97,7 @@ def host():
 # kernels launched per C entry point (used to report how many of this library's kernels ran in a region)
 _LAUNCHES_PER_CALL = {"ttb_gated_rmsnorm_bwd": 2, "ttb_causal_conv1d_bwd": 2,
                       "ttb_causal_conv1d_row_blocks": 0, "ttb_ep_dispatch_all": 5, "ttb_ep_dispatch_rows": 3,
-                      "ttb_ep_combine_all": 3, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
+                      "ttb_ep_combine_all": 3, "ttb_delta_vec_bwd_post": 2, "ttb_ep_combine_vals": 4, "ttb_ep_prepare": 3, "ttb_ep_prepare_bwd": 1, "ttb_router_fwd": 2, "ttb_perm_index": 3, "ttb_perm_scatter": 2,
                       "ttb_gemm_status": 0}
 LAUNCH_COUNT = 0
 
@@ -685,9 +685,41 @@ def delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq: int, *, l2: bool, s
     return host().delta_bwd_pre(q, k, v, g, beta, chunk_rows, do, A, nseq, l2, scale)
 
 
+class _DeltaChunkIn(C.Structure):
+    """`struct DeltaChunkIn` of csrc/entries.h."""
+
+    _fields_ = [("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p),
+                ("q_t", C.c_longlong), ("q_h", C.c_longlong), ("k_t", C.c_longlong), ("k_h", C.c_longlong),
+                ("v_t", C.c_longlong), ("v_h", C.c_longlong),
+                ("g", C.c_void_p), ("beta", C.c_void_p), ("chunk_rows", C.c_void_p),
+                ("H", C.c_int), ("NC", C.c_int), ("l2", C.c_int), ("scale", C.c_float), ("rep", C.c_int)]
+
+
 def delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, *, l2: bool, scale: float):
     """(dq, dk bf16 like q, dv bf16 [rows, H, 128], dg like g, dbeta fp32 [rows, H])."""
-    return host().delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, dstates, l2, scale)
+    R, H, _ = v.shape
+    Hk, NC = q.shape[1], chunk_rows.shape[0]
+    check_device(q)
+    for t, heads in ((q, Hk), (k, Hk), (v, H)):
+        assert t.dtype == torch.bfloat16 and t.shape == (R, heads, 128) and t.stride(2) == 1
+    assert H % Hk == 0 and (Hk == H or g.dim() == 2)
+    assert g.dtype == torch.float32 and g.shape in ((R, H), (R, H, 128)) and g.is_contiguous()
+    assert beta.dtype == torch.float32 and beta.shape == (R, H) and beta.is_contiguous()
+    assert chunk_rows.dtype == torch.int32 and chunk_rows.is_contiguous() and chunk_rows.shape[1] == 3
+    a = _DeltaChunkIn(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0), k.stride(1), v.stride(0), v.stride(1),
+                      g.data_ptr(), beta.data_ptr(), chunk_rows.data_ptr(), H, NC, int(l2), scale, H // Hk)
+    dq, dk, dv = (torch.empty(v.shape, dtype=torch.bfloat16, device=q.device) for _ in range(3))   # of every value head
+    dg, dbeta = torch.empty_like(g), torch.empty_like(beta)
+    # held until the launches are queued: a pointer alone would let another thread of this stream be given the block first
+    scratch = torch.empty(4, *x.shape, dtype=torch.float32, device=q.device) if g.dim() == 3 else None
+    name = "ttb_delta_vec_bwd_post" if g.dim() == 3 else "ttb_delta_bwd_post"
+    _check(getattr(lib(), name)(C.byref(a), _p(do), _p(T), _p(x), _p(dx), _p(states), _p(dstates), C.c_int(states.shape[1] - NC),
+                                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta), *([_p(scratch)] if scratch is not None else []), _stream()), name)
+    if H > Hk:
+        per_head, (dq, dk) = (dq, dk), (torch.empty(q.shape, dtype=torch.bfloat16, device=q.device) for _ in range(2))
+        _check(lib().ttb_delta_head_sum(_p(per_head[0]), _p(per_head[1]), _p(dq), _p(dk), C.c_longlong(R * Hk), C.c_int(H // Hk), _stream()),
+               "ttb_delta_head_sum")
+    return dq, dk, dv, dg, dbeta
 
 
 # --------------------------------------------------------------------------------------

@@ -112,7 +112,7 @@ class ChunkDelta(torch.autograd.Function):
     or None; `tables` = (seq_chunks, chunk_rows, last slots, first slots) on the device."""
 
     @staticmethod
-    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2, want_final):
+    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2, want_final=True):
         seq, chunk_rows, last, first = tables
         kw = dict(l2=l2, scale=scale)
         T, A, u, w, k_out, decay = K.delta_prep(q, k, v, g, beta, chunk_rows, **kw)
