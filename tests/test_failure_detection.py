@@ -50,6 +50,7 @@ def _w_heartbeat(rank, world):
     hb.beat(step=0)
     dist.barrier()
     assert hb.stale_ranks() == [] and hb.last((rank + 1) % world)[0] == 0
+    dist.barrier()          # nobody beats again before both have looked
     if rank == 1:
         # this rank "dies" between steps: no kernel or collective of it is in flight, it just stops beating
         time.sleep(15.0)
