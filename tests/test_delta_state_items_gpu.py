@@ -68,3 +68,29 @@ def test_a_first_state_of_zero_is_not_read(H, lens):
     want = K.delta_state_scan(a, b, u, dec, None, add.index_fill(1, last, 0.0), seq, **kw)
     got = K.delta_state_scan(a, b, u, dec, None, add.index_fill(1, last, float("nan")), seq, zero_first=True, **kw)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H, lens", [(1, [1]), (2, [1, 0, 1]), (3, [1] * 40), (5, [2] * 17), (30, [3, 3, 2, 3]), (148, [2]), (60, [2] * 4), (37, [4] * 7)])
+@pytest.mark.parametrize("vec", [False, True])
+@pytest.mark.parametrize("with_init", [False, True])
+def test_forward_with_the_longest_sequence_known(H, lens, vec, with_init):
+    """Sequences of one chunk, and pairs of heads and sequences that fill the chip once or twice, take the other form of the forward pass."""
+    from torchturbo_b200 import kernels as K
+
+    NC, ns, g = sum(lens), len(lens), torch.Generator("cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    a, b = (rnd(H, NC, 64, 128) * 0.03).bfloat16(), (rnd(H, NC, 64, 128) * 0.03).bfloat16()
+    u, dec = rnd(H, NC, 64, 128), torch.rand(*((H, NC, 128) if vec else (H, NC)), device="cuda", generator=g)
+    init = rnd(H, ns, 128, 128) if with_init else None
+    cu = torch.tensor([0] + lens).cumsum(0)
+    seq = torch.stack((cu[:-1], torch.tensor(lens)), 1).to(torch.int32).cuda()
+    kw = dict(reverse=False, s1=-1.0, s2=1.0)
+    x, states = K.delta_state_scan(a, b, u, dec, init, None, seq, longest=max(lens), **kw)
+    want_x, want_s = _scan(a, b, u, dec, init, None, lens, False, -1.0, 1.0)
+    bound = 2.0 ** -8 * max(lens)                   # as above
+    for got, want in ((x, want_x), (states, want_s)):
+        assert (got.double() - want).norm() <= bound * want.norm()
+    other = K.delta_state_scan(a, b, u, dec, init, None, seq, **kw)
+    assert torch.equal(x, other[0]) and torch.equal(states, other[1])
+    assert K.status() == (0, 0)

@@ -26,9 +26,10 @@
 // added values did not fit into registers, and the decay was waited for; with one pair of warps for X and S it was 3700 and 4300.
 // CTAs stay and walk the (sequence, head, column group) items, longest sequences first: the loads of the next item overlap the end of
 // the last, and a short sequence does not pay for barriers and tensor memory.
+// Forward passes whose CTAs would leave a last wave partly empty take the form without any of that (`wide_pays`, below).
 // Forward and reverse in us, before -> now: 32 heads, 4096 tokens in four documents (the longest 44 chunks) 140 + 252 -> 94 + 104, in
-// one document 155 + 288 -> 105 + 113 (203 MB written each way, 68 at the rate of a fill), in four equal ones 66 + 114 -> 74 + 85, in 64
-// of one chunk 96 + 163 -> 86 + 129; 8 heads with decay vectors, 2047 tokens 47 + 77 -> 33 + 37.
+// one document 155 + 288 -> 105 + 113 (203 MB written each way, 68 at the rate of a fill), in four equal ones 70 + 117 -> 70 + 91, in 64
+// of one chunk 100 + 167 -> 88 + 127; 8 heads with decay vectors, 2047 tokens 47 + 77 -> 33 + 37.
 // Every wait is bounded; on a timeout the roles drain to the final barrier, TMEM is freed and the status word records
 // kernel / site.
 //
@@ -376,16 +377,224 @@ delta_state_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   }
 }
 
+// Forward pass in CTAs of 64 columns whose threads load U and store X and the states themselves: warps 0, 1, 4, 5 hold the state and form X
+// (warps 4 and 5 K-entries 64-127 and tokens 32-63), 2 loads the operands (two stages), 3 issues the products.
+struct DsWideParams {
+  const float *U, *decay, *init;
+  float *X, *states;
+  const int* seq_chunks;
+  int nseq, NC, vec;
+  float s1, s2;
+};
+
+struct DsWideSmem {
+  static constexpr int V = 64;                           // value columns
+  static constexpr int ST_PANEL = V * 128;               // S^T bf16 [64 v][64 k] per panel, two panels
+  static constexpr int ST = 0;
+  static constexpr int XT = ST + 2 * ST_PANEL;           // X^T bf16 [64 v][64 c]
+  static constexpr int A = XT + V * 128;                 // 2 x 16 KB  A_c [64 c][128 k] (also behind the short tiles above)
+  static constexpr int B = A + 2 * 16384;                // 2 x 16 KB  B_c [64 c][128 k]
+  static constexpr int DEC = B + 2 * 16384;              // float [128]
+  static constexpr int BARS = DEC + 512;
+  static constexpr int TOTAL = BARS + 256 + 1024;
+};
+
+__global__ void __launch_bounds__(192, 2)
+delta_state_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const DsWideParams p) {
+  using L = DsWideSmem;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
+  uint64_t *ab_full = bars, *ab_empty = bars + 2;        // [2]
+  uint64_t *st_ready = bars + 4, *acc1_full = bars + 5, *x_ready = bars + 6, *acc2_full = bars + 7;      // as above
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  volatile int* s_dead = reinterpret_cast<volatile int*>(bars + 9);      // a state warp's wait gave up
+  float* s_dec = reinterpret_cast<float*>(smem + L::DEC);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * L::V, slots = p.NC + p.nseq;
+  const int c0 = p.seq_chunks[seq * 2], n = p.seq_chunks[seq * 2 + 1];
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) { mbar_init(&ab_full[i], 1); mbar_init(&ab_empty[i], 1); }
+    mbar_init(st_ready, 4); mbar_init(acc1_full, 1); mbar_init(x_ready, 4); mbar_init(acc2_full, 1);
+    *s_dead = 0;
+    mbar_fence_init();
+  }
+  if (warp == 3) {
+    tmem_alloc(tmem_slot, 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot, tm1 = tmem_base, tm2 = tmem_base + 128;
+
+  if (warp == 2) {
+    if (elect_one()) {
+      tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
+      for (int i = 0; i < n; ++i) {
+        const int st = i & 1, row0 = (h * p.NC + c0 + i) * DS_C;
+        if (!mbar_wait(&ab_empty[st], ((i >> 1) & 1) ^ 1, KID_DELTA_STATE, 17)) break;
+        mbar_expect_tx(&ab_full[st], 32768);
+        uint8_t *sa = smem + L::A + st * 16384, *sb = smem + L::B + st * 16384;
+        tma_load_2d(sa, &tmA, &ab_full[st], 0, row0);
+        tma_load_2d(sa + 8192, &tmA, &ab_full[st], 64, row0);
+        tma_load_2d(sb, &tmB, &ab_full[st], 0, row0);
+        tma_load_2d(sb + 8192, &tmB, &ab_full[st], 64, row0);
+      }
+    }
+  } else if (warp == 3) {
+    constexpr uint32_t id1 = make_idesc_bf16(128, 64, false, false), id2 = make_idesc_bf16(128, 128, false, true);
+    if (elect_one()) {
+      const uint32_t sST = smem_u32(smem + L::ST), sXT = smem_u32(smem + L::XT);
+      for (int i = 0; i < n; ++i) {
+        const int st = i & 1;
+        if (!mbar_wait(&ab_full[st], (i >> 1) & 1, KID_DELTA_STATE, 18)) break;
+        if (!mbar_wait(st_ready, i & 1, KID_DELTA_STATE, 19)) break;
+        tc_fence_after();
+        const uint32_t sA = smem_u32(smem + L::A + st * 16384), sB = smem_u32(smem + L::B + st * 16384);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)    // reduction over k = 128
+          umma_ss(tm1, make_smem_desc(sST + (kk >> 2) * L::ST_PANEL + (kk & 3) * 32, 16, 1024),
+                  make_smem_desc(sA + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id1, kk != 0);
+        umma_commit(acc1_full);
+        if (!mbar_wait(x_ready, i & 1, KID_DELTA_STATE, 20)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)    // reduction over the 64 tokens of the chunk
+          umma_ss(tm2, make_smem_desc(sXT + kk * 32, 16, 1024), make_smem_desc(sB + kk * 2048, 8192, 1024), id2, kk != 0);
+        umma_commit(acc2_full);
+        umma_commit(&ab_empty[st]);
+      }
+    }
+  } else {
+    const int half = warp >> 2, vl = (warp & 3) * 32 + lane, v = v0 + vl, k0 = half * 64, t0 = half * 32;   // this thread's column, K-entries, tokens
+    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    uint8_t *sST = smem + L::ST + half * L::ST_PANEL + vl * 128, *sXT = smem + L::XT + vl * 128;
+    float S[64], u[32];
+    auto state_at = [&](int slot) { return p.states + ((static_cast<long long>(h) * slots + slot) * DS_D + k0) * DS_D + v; };
+    auto row_at = [&](int i) { return ((static_cast<long long>(h) * p.NC + c0 + i) * DS_C + t0) * DS_D + v; };
+    auto signal = [&](uint64_t* bar) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto publish = [&]() {
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch)
+        *reinterpret_cast<uint4*>(sST + ((ch ^ (lane & 7)) * 16)) = make_uint4(pack_bf16(S[ch * 8 + 0], S[ch * 8 + 1]), pack_bf16(S[ch * 8 + 2], S[ch * 8 + 3]),
+                                                                               pack_bf16(S[ch * 8 + 4], S[ch * 8 + 5]), pack_bf16(S[ch * 8 + 6], S[ch * 8 + 7]));
+      signal(st_ready);
+    };
+    auto fetch_u = [&](int i) {
+      const float* src = p.U + row_at(i);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) u[j] = __ldg(src + j * DS_D);
+    };
+    {
+      const float* src = p.init ? p.init + ((static_cast<long long>(h) * p.nseq + seq) * DS_D + k0) * DS_D + v : nullptr;
+      float* dst = state_at(c0 + seq);
+#pragma unroll
+      for (int k = 0; k < 64; ++k) S[k] = src ? __ldg(src + k * DS_D) : 0.f;
+#pragma unroll
+      for (int k = 0; k < 64; ++k) dst[k * DS_D] = S[k];
+    }
+    if (n > 0) {
+      publish();
+      fetch_u(0);
+    }
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      // the decay is asked for ahead of the first wait: a load behind the second one would be on the chain
+      const long long chunk = static_cast<long long>(h) * p.NC + c0 + i;
+      const float dec = __ldg(p.decay + (p.vec ? chunk * DS_D + half * L::V + vl : chunk));
+      if (ok && mbar_wait(acc1_full, i & 1, KID_DELTA_STATE, 21)) {
+        tc_fence_after();
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tm1 + t0 + lanes, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) u[j] = fmaf(p.s1, __uint_as_float(r[j]), u[j]);
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+          *reinterpret_cast<uint4*>(sXT + (((half * 4 + ch) ^ (lane & 7)) * 16)) =
+              make_uint4(pack_bf16(p.s2 * u[ch * 8 + 0], p.s2 * u[ch * 8 + 1]), pack_bf16(p.s2 * u[ch * 8 + 2], p.s2 * u[ch * 8 + 3]),
+                         pack_bf16(p.s2 * u[ch * 8 + 4], p.s2 * u[ch * 8 + 5]), pack_bf16(p.s2 * u[ch * 8 + 6], p.s2 * u[ch * 8 + 7]));
+        tc_fence_before();
+        signal(x_ready);
+        // off the chain, while the second product runs: X goes out, the next U comes in, and a decay vector is staged for all threads (its
+        // last readers have published the state that this chunk's first product waited for)
+        float* xout = p.X + row_at(i);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) xout[j * DS_D] = u[j];
+        if (i + 1 < n) fetch_u(i + 1);
+        if (p.vec) s_dec[half * L::V + vl] = dec;
+      } else {
+        *s_dead = 1;
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");     // the decay vector is staged; a failed wait is published
+      if (*s_dead) break;
+      if (!mbar_wait(acc2_full, i & 1, KID_DELTA_STATE, 22)) {
+        ok = false;
+        continue;                                        // to the barrier of the next chunk, which the other warps wait at
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int cb = 0; cb < 2; ++cb) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tm2 + k0 + cb * 32 + lanes, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int k = cb * 32 + j;
+          S[k] = fmaf(p.vec ? s_dec[k0 + k] : dec, S[k], __uint_as_float(r[j]));
+        }
+      }
+      tc_fence_before();
+      if (i + 1 < n) publish();
+      float* dst = state_at(c0 + i + 1 + seq);
+#pragma unroll
+      for (int k = 0; k < 64; ++k) dst[k * DS_D] = S[k];
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 3) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 256);
+  }
+}
+
+// Whether a forward pass takes the form with 64 columns a CTA (the same bits).  It moves less through shared memory per column, so that two
+// of its CTAs hold an SM up less, but its chain is longer (2.3 us a chunk alone on an SM, 1.5 with 32 columns).  `places` CTAs of either
+// form run at once; the lines are those of sequence-and-head pairs at 148 SMs, times in us for 32 and for 64 columns:
+//  * 75 to 148 pairs: all of its CTAs run at once, where a last wave of the other form's is partly empty, if no sequence is much
+//    longer than the others (those of the last wave are the shortest): 32 heads with four of 16 chunks 78 and 70, of 24 110 and 100, with
+//    three of 21 88 and 81.  Lengths with a mean of 0.83 of the longest 92 and 88, of 0.71 115 and 123; 80 pairs at 0.80 76 and 78, 96 at 0.88
+//    82 and 84, whose shorter last wave is less of a loss;
+//  * 223 to 259: two full waves against three and a bit: 240 pairs of 24 chunks 203 and 195, 256 205 and 203, 288 219 and 231;
+//  * sequences of one chunk, which have no chain: 64 pairs 12.3 and 10.2, 128 14.3 and 12.3, 256 20.5 and 18.4; the same from 600 on.
+// Outside these it is 1.0 to 1.5 times slower (1 pair to 74: 1.4; 160 to 192: 1.1; 320: 1.1).
+static bool wide_pays(int nseq, int H, int NC, int longest, long long places) {
+  const long long pairs = static_cast<long long>(nseq) * H;
+  if (longest <= 0 || H > 65535) return false;
+  if (longest == 1) return pairs <= 2 * places;
+  if (10ll * NC < (8 * pairs < 3 * places ? 9ll : 8ll) * longest * nseq) return false;
+  return (2 * pairs <= places && 4 * pairs > places) || (4 * pairs > 3 * places && 8 * pairs <= 7 * places);
+}
+
 }  // namespace ttb
 
 using namespace ttb;
 
 // A, B: bf16 [H * NC * 64, 128] (chunk-major rows); U, X: fp32 [H, NC, 64, 128]; decay fp32 [H, NC] or [H, NC, 128];
 // init fp32 [H, nseq, 128, 128] or null; add, states fp32 [H, NC + nseq, 128, 128] (add may be null when forward).  reverse: 0, 1, or
-// 2 for a first state of zero, whose slot of `add` is then not read.
+// 2 for a first state of zero, whose slot of `add` is then not read.  longest: chunks of the longest sequence (0: not known).
 TTB_EXPORT int ttb_delta_state_scan(const void* A, const void* B, const float* U, float* X, const float* decay, int vec,
                                     const float* init, const float* add, float* states, const int* seq_chunks, int nseq,
-                                    int H, int NC, int reverse, float s1, float s2, void* stream_ptr) {
+                                    int H, int NC, int longest, int reverse, float s1, float s2, void* stream_ptr) {
   if (nseq <= 0 || H <= 0 || NC <= 0) return 0;
   if (reverse && add == nullptr) return 911;
   const long long items = static_cast<long long>(DS_D / DS_V) * H * nseq;
@@ -409,6 +618,15 @@ TTB_EXPORT int ttb_delta_state_scan(const void* A, const void* B, const float* U
   }
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 301;
+  if (!reverse && add == nullptr && wide_pays(nseq, H, NC, longest, 2ll * sms)) {
+    const DsWideParams w{U, decay, init, X, states, seq_chunks, nseq, NC, vec, s1, s2};
+    static bool wide_done[16] = {};
+    const cudaError_t es = ensure_dynamic_smem(reinterpret_cast<const void*>(delta_state_wide_kernel), DsWideSmem::TOTAL, wide_done);
+    if (es != cudaSuccess) return 300 + static_cast<int>(es);
+    delta_state_wide_kernel<<<dim3(nseq, H, DS_D / DsWideSmem::V), 192, DsWideSmem::TOTAL, stream>>>(ta, tb, w);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : 400 + (int)e;
+  }
   DeltaStateParams p{decay, seq_chunks, nseq, H, NC, static_cast<int>(items), vec, reverse != 0, add != nullptr,
                      reverse == 1 ? 1 : !reverse && init ? 2 : 0, s1, s2};
   static bool done[16] = {};

@@ -76,7 +76,7 @@ TTB_EXPORT int ttb_delta_vec_prep(const ttb::DeltaChunkIn*, float*, float*, floa
 TTB_EXPORT int ttb_delta_vec_out(const ttb::DeltaChunkIn*, const float*, const float*, const float*, int, void*, void*);
 TTB_EXPORT int ttb_delta_vec_bwd_pre(const ttb::DeltaChunkIn*, const void*, const float*, int, float*, float*, void*);
 TTB_EXPORT int ttb_delta_state_scan(const void*, const void*, const float*, float*, const float*, int, const float*, const float*, float*,
-                            const int*, int, int, int, int, float, float, void*);
+                            const int*, int, int, int, int, int, float, float, void*);
 TTB_EXPORT int ttb_scale(const void*, int, const float*, void*, int, long long, int, void*);
 TTB_EXPORT int ttb_copy_words(void*, const void*, long long, void*);
 TTB_EXPORT int ttb_kda_gate_row_blocks(long long, int);

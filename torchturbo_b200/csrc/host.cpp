@@ -678,12 +678,13 @@ PyObject* delta_bwd_pre(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 PyObject* delta_state_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    Args in(args, n, 10);
+    Args in(args, n, 11);
     const Tensor &a = in.tensor(), &b = in.tensor(), &u0 = in.tensor(), &decay0 = in.tensor();
     const Tensor init0 = in.optional(), add0 = in.optional();
     const Tensor& seq0 = in.tensor();
     const int reverse = static_cast<int>(in.integer());
     const double s1 = in.real(), s2 = in.real();
+    const int longest = static_cast<int>(in.integer());
     need(u0.dim() == 4 && seq0.dim() == 2 && (decay0.dim() == 2 || decay0.dim() == 3), "chunks of 64 rows");
     const long long H = u0.size(0), NC = u0.size(1), nseq = seq0.size(0);
     need(u0.size(2) == 64 && u0.size(3) == 128 && a.sizes() == u0.sizes() && b.sizes() == u0.sizes(), "chunks of 64 rows");
@@ -706,7 +707,7 @@ PyObject* delta_state_scan(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Tensor x = empty_rows(u), states = empty({H, NC + nseq, 128, 128}, at::kFloat, u);
     launch("ttb_delta_state_scan", 1, [&](void* st) {
       return ttb_delta_state_scan(at_(a), at_(b), f32(u), f32w(x), f32(decay), decay.dim() == 3, f32(init), f32(add), f32w(states), i32(seq),
-                                  static_cast<int>(nseq), static_cast<int>(H), static_cast<int>(NC), reverse, static_cast<float>(s1),
+                                  static_cast<int>(nseq), static_cast<int>(H), static_cast<int>(NC), longest, reverse, static_cast<float>(s1),
                                   static_cast<float>(s2), st);
     });
     return wrap_all(x, states);

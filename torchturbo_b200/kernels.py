@@ -656,13 +656,16 @@ def attn_fwd(q, k, v, q_tiles_dev, *, scale: float, causal: bool = True, want_ls
     return host().attn_fwd(q, k, v, q_tiles_dev, scale, causal, want_lse, want_max_logit, *_covered(rows), tile_rows)
 
 
-def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, reverse: bool, s1: float, s2: float, zero_first: bool = False):
+def delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, *, reverse: bool, s1: float, s2: float, zero_first: bool = False,
+                     longest: int = 0):
     """Chunk-state recurrence of the delta rule (csrc/delta_state.cu).  `a_tiles`, `b_tiles`: bf16 [H, NC, 64, 128];
     `u`: fp32 [H, NC, 64, 128]; `decay`: fp32 [H, NC] or [H, NC, 128]; `init`: fp32 [H, nseq, 128, 128] or None;
     `add`: fp32 [H, NC + nseq, 128, 128] (required when `reverse`); `seq_chunks_dev`: int32 [nseq, 2].  A reverse pass starts from the
     last slots of `add`, with `zero_first` from zero (those slots are not read).
+    ``longest``: chunks of the longest sequence, which the choice between the kernel's forms goes by (0: not known).
     Returns (x fp32 [H, NC, 64, 128], states fp32 [H, NC + nseq, 128, 128])."""
-    return host().delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, (2 if zero_first else 1) if reverse else 0, s1, s2)
+    return host().delta_state_scan(a_tiles, b_tiles, u, decay, init, add, seq_chunks_dev, (2 if zero_first else 1) if reverse else 0, s1, s2,
+                                   longest)
 
 
 # Inputs of the chunk kernels: v: bf16 [rows, H, 128]; q, k: the same or, with one decay per head, of H / rep heads that serve rep value

@@ -75,7 +75,8 @@ class StateScan(torch.autograd.Function):
         wb, kb = w.to(torch.bfloat16).contiguous(), k_out.to(torch.bfloat16).contiguous()
         u = u.contiguous()
         decay = decay.contiguous()
-        x, states = K.delta_state_scan(wb, kb, u, decay, init, None, seq_dev, reverse=False, s1=-1.0, s2=1.0)
+        x, states = K.delta_state_scan(wb, kb, u, decay, init, None, seq_dev, reverse=False, s1=-1.0, s2=1.0,
+                                       longest=max((n for _, n in seq_chunks), default=0))
         ctx.save_for_backward(wb, kb, decay, x, states, seq_dev)
         ctx.seq_chunks = seq_chunks
         ctx.has_init = init is not None
@@ -112,11 +113,11 @@ class ChunkDelta(torch.autograd.Function):
     or None; `tables` = (seq_chunks, chunk_rows, last slots, first slots) on the device."""
 
     @staticmethod
-    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2, want_final=True):
+    def forward(ctx, q, k, v, g, beta, init, tables, scale, l2, want_final=True, longest=0):
         seq, chunk_rows, last, first = tables
         kw = dict(l2=l2, scale=scale)
         T, A, u, w, k_out, decay = K.delta_prep(q, k, v, g, beta, chunk_rows, **kw)
-        x, states = K.delta_state_scan(w, k_out, u, decay, init, None, seq, reverse=False, s1=-1.0, s2=1.0)
+        x, states = K.delta_state_scan(w, k_out, u, decay, init, None, seq, reverse=False, s1=-1.0, s2=1.0, longest=longest)
         o = K.delta_out(q, k, v, g, beta, chunk_rows, A, x, states, **kw)
         ctx.save_for_backward(q, k, v, g, beta, T, A, w, k_out, decay, x, states, seq, chunk_rows, last, first)
         ctx.meta = (kw, init is not None)
@@ -134,7 +135,7 @@ class ChunkDelta(torch.autograd.Function):
             gs.index_copy_(1, last.long(), dfinal.contiguous())
         dx, ds = K.delta_state_scan(k_out, w, gx, decay, None, gs, seq, reverse=True, s1=1.0, s2=-1.0, zero_first=dfinal is None)
         dq, dk, dv, dg, dbeta = K.delta_bwd_post(q, k, v, g, beta, chunk_rows, do, T, x, dx, states, ds, **kw)
-        return dq, dk, dv, dg, dbeta, (ds.index_select(1, first) if has_init else None), None, None, None, None
+        return dq, dk, dv, dg, dbeta, (ds.index_select(1, first) if has_init else None), None, None, None, None, None
 
 
 def _rows_for_kernel(t: torch.Tensor, R: int) -> torch.Tensor:
@@ -248,7 +249,8 @@ def chunk_delta_rule_batched(q, k, v, g, beta, scale=None, initial_state=None, o
         tables = _chunk_tables(segs, C, dev)
         init = initial_state.float().transpose(0, 1).contiguous() if initial_state is not None else None
         o, final = ChunkDelta.apply(*(_rows_for_kernel(t, R) for t in (q, k, v)), g.float().reshape(R, *g.shape[2:]).contiguous(),
-                                    beta.float().reshape(R, H).contiguous(), init, tables, float(scale), bool(use_qk_l2norm), bool(output_final_state))
+                                    beta.float().reshape(R, H).contiguous(), init, tables, float(scale), bool(use_qk_l2norm), bool(output_final_state),
+                                    max((b - a + C - 1 for _, a, b in segs), default=0) // C)
         return o.view(B, T, H, V), (final.transpose(0, 1).contiguous() if output_final_state else None)
     q, k = (repeat_key_heads(t, heads_per_key) for t in (q, k))
     qf, kf, vf, gf, bf = (t.float() for t in (q, k, v, g, beta))
