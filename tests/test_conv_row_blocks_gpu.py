@@ -50,3 +50,9 @@ def test_rows(T, D, W):
     for got, ref, size, rounded in ((y, want[0], want[3], 0.0), (dx, want[1], want[4], 2.0 ** -8)):
         assert ((got.double().cpu() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * (2.0 ** -17 + rounded * (1 + 2.0 ** -8)) + 1e-30).all()
     assert ((dw.double().cpu() - want[2]).abs() <= want[5] * 2.0 ** -17 + 1e-30).all()
+
+
+@pytest.mark.parametrize("T, D", [(2, 8200), (63, 8200), (300, 8200), (1190, 512), (1776, 1032), (6000, 2056)])
+def test_rows_of_a_block(T, D):
+    """Blocks of one to three rows, of one or more whole steps, and (the last) of as many as fill the chip twice."""
+    test_rows(T, D, 4)

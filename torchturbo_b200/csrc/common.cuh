@@ -521,6 +521,13 @@ inline int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const ui
 }
 
 // fp32 tiles without swizzle (rows of the box contiguous in shared memory): TMA reductions
+// SMs of the current device
+inline int device_sms() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+  return n;
+}
+
 inline int make_tmap_f32_linear(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                                 const uint64_t* strides_bytes, const uint32_t* box) {
   return make_tmap_typed(out, base, rank, dims, strides_bytes, box, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, CU_TENSOR_MAP_SWIZZLE_NONE);

@@ -1560,15 +1560,24 @@ TTB_EXPORT int ttb_bias_act_bwd(const void* dy, const void* x, const void* bias,
 
 // A thread owns 4 channels of a filter of up to four taps, else 8.  Blocks per SM: up to four taps, whole waves of what an SM holds, one
 // of the backward (4; its rows of overlap and column sums grow with the number of blocks: 8, 12 and 24 per SM take 85, 91 and 109 us
-// against 79) and two of the forward (12; 41 us, one wave 42, and 100 against 104 us for 16384 x 6144).
+// against 79) and two of the forward (12; 41 us, one wave 42, and 100 against 104 us for 16384 x 6144).  Where two waves of the forward
+// leave a block less than 14 rows, of which three more are read before the first, it is one wave of whole steps of four rows, and fewer
+// rows only where there would not be a block for every SM.  Two waves -> this, inputs from memory: 4096 x 512 7.7 -> 6.2 us, 300 x 8192
+// 8.5 -> 6.8, 2047 x 1024 7.8 -> 6.1, 1001 x 3072 8.4 -> 7.5, 64 x 12288 6.9 -> 3.8, 16 x 512 2.0 (two rows a block 2.2); 15 rows with two
+// waves 17.4 (2047 x 6144), with one 17.8.
 static void conv_grid(long long T, int D, int W, bool bwd, int& threads, dim3& grid, int& rows_per_block) {
   const int vec = W <= 4 ? D / 4 : D / 8;
   threads = vec >= 128 ? 128 : ((vec + 31) / 32) * 32;
   const int gx = (vec + threads - 1) / threads;
-  long long want = W <= 4 ? 148LL * (bwd ? 4 : 12) / gx : (148LL * 8 + gx - 1) / gx;
+  const long long sms = device_sms();
+  long long want = W <= 4 ? sms * (bwd ? 4 : 12) / gx : (sms * 8 + gx - 1) / gx;
   if (want > T) want = T;
   if (want < 1) want = 1;
   rows_per_block = static_cast<int>((T + want - 1) / want);
+  if (W <= 4 && !bwd && rows_per_block < 14) {
+    const long long steps = (T * gx + sms * 6 * CONV_ROWS - 1) / (sms * 6 * CONV_ROWS), each = (T * gx + sms - 1) / sms;
+    rows_per_block = static_cast<int>(steps * CONV_ROWS < each ? steps * CONV_ROWS : each);
+  }
   grid = dim3(gx, static_cast<unsigned>((T + rows_per_block - 1) / rows_per_block));
 }
 
