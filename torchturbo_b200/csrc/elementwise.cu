@@ -1126,10 +1126,13 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long lon
 // Writes per-row loss (0 for ignored rows) and, when dlogits != nullptr, the gradient
 // (softmax - onehot) * grad_scale[0] in bf16 (may alias a bf16 logits buffer).
 // Bound by memory: the rows in flight (two blocks per SM, 90 MB of 151936 logits) and the gradients just written share the L2, and what a
-// row's second pass finds there no more is read again.  So that pass walks the row from its end, where it was read last, and marks what
-// it reads and writes as the first to leave: 4096 x 151936 bf16, gradient in place, 518 -> 473 us (from the end alone 489, marks alone
-// 488; one read and one write at the rate of a copy: 408), 1024 rows 148 -> 133, 32000 logits 113 -> 115.  With a third fewer
-// instructions it takes the same time; 512 threads per block take 514 us, and 102 with 32000 logits.
+// row's second pass finds there no more is read again.  Where that happens (LONG) the pass walks the row from its end, where it was read
+// last, and marks what it reads and writes as the first to leave: 4096 x 151936 bf16, gradient in place, 518 -> 473 us (from the end
+// alone 489, marks alone 488; one read and one write at the rate of a copy: 408), 1024 rows 148 -> 133.  Shorter rows are still there,
+// and the plain order is the faster one: in place, plain and LONG, 4096 x 32000 111 and 113 us, x 80000 245 and 257, x 112000 350 and
+// 356, x 116000 373 and 371, x 128256 411 and 403; with a gradient of its own, which takes L2 as well, x 80000 249 and 256, x 84000 270
+// and 268, x 100352 328 and 311.  With a third fewer instructions it takes the same time; 512 threads per block take 514 us, and 102 with
+// 32000 logits.
 // ============================================================================
 template <typename TL>
 __device__ __forceinline__ float ld_logit(const TL* p, long long i);
@@ -1141,7 +1144,8 @@ __device__ __forceinline__ float ld_logit<__nv_bfloat16>(const __nv_bfloat16* p,
 }
 
 constexpr int CE_THREADS = 1024;
-template <typename TL>
+static bool ce_long(int V, bool in_place) { return V >= (in_place ? 114000 : 84000); }      // the measured lines, above
+template <typename TL, bool LONG>
 __global__ void __launch_bounds__(CE_THREADS)
 cross_entropy_kernel(const TL* __restrict__ logits, long long ldl, const long long* __restrict__ labels,
                      float* __restrict__ loss_rows, float* __restrict__ lse_rows, __nv_bfloat16* dlogits, long long ldd,
@@ -1202,9 +1206,9 @@ cross_entropy_kernel(const TL* __restrict__ logits, long long ldl, const long lo
     if (vec) {
       const __nv_bfloat16* lb = reinterpret_cast<const __nv_bfloat16*>(lr);
       constexpr int STEP = CE_THREADS * 8;
-      for (int c = (V - 1) / STEP * STEP + threadIdx.x * 8; c >= 0; c -= STEP) {
-        if (c >= V) continue;
-        const uint4 u = __ldcs(reinterpret_cast<const uint4*>(lb + c));
+      for (int c = (LONG ? (V - 1) / STEP * STEP : 0) + threadIdx.x * 8; LONG ? c >= 0 : c < V; c += LONG ? -STEP : STEP) {
+        if (LONG && c >= V) continue;
+        const uint4 u = LONG ? __ldcs(reinterpret_cast<const uint4*>(lb + c)) : *reinterpret_cast<const uint4*>(lb + c);
         const float2 a = unpack_bf16(u.x), b2 = unpack_bf16(u.y), c2 = unpack_bf16(u.z), d = unpack_bf16(u.w);
         float f[8] = {a.x, a.y, b2.x, b2.y, c2.x, c2.y, d.x, d.y};
         const int hit = static_cast<int>(label) - c;
@@ -1216,7 +1220,8 @@ cross_entropy_kernel(const TL* __restrict__ logits, long long ldl, const long lo
         }
         uint4 o;
         o.x = pack_bf16(f[0], f[1]); o.y = pack_bf16(f[2], f[3]); o.z = pack_bf16(f[4], f[5]); o.w = pack_bf16(f[6], f[7]);
-        __stcs(reinterpret_cast<uint4*>(dlogits + r * ldd + c), o);
+        if (LONG) __stcs(reinterpret_cast<uint4*>(dlogits + r * ldd + c), o);
+        else *reinterpret_cast<uint4*>(dlogits + r * ldd + c) = o;
       }
     } else {
       for (int c = threadIdx.x; c < V; c += CE_THREADS) {
@@ -1684,14 +1689,13 @@ TTB_EXPORT int ttb_cross_entropy(const void* logits, int logits_fp32, long long 
                                  float* loss_rows, float* lse_rows, void* dlogits, long long ldd,
                                  const float* grad_scale, float grad_scale_host, long long R, int V, void* stream) {
   if (R == 0) return 0;
-  if (logits_fp32)
-    cross_entropy_kernel<float><<<(unsigned)R, CE_THREADS, 0, STREAM(stream)>>>(
-        (const float*)logits, ldl, labels, loss_rows, lse_rows, (__nv_bfloat16*)dlogits, ldd, grad_scale,
-        grad_scale_host, V);
-  else
-    cross_entropy_kernel<__nv_bfloat16><<<(unsigned)R, CE_THREADS, 0, STREAM(stream)>>>(
-        (const __nv_bfloat16*)logits, ldl, labels, loss_rows, lse_rows, (__nv_bfloat16*)dlogits, ldd, grad_scale,
-        grad_scale_host, V);
+  auto run = [&](auto kernel, auto* rows) {
+    kernel<<<(unsigned)R, CE_THREADS, 0, STREAM(stream)>>>(rows, ldl, labels, loss_rows, lse_rows, (__nv_bfloat16*)dlogits, ldd, grad_scale,
+                                                           grad_scale_host, V);
+  };
+  if (logits_fp32) run(cross_entropy_kernel<float, false>, (const float*)logits);
+  else if (ce_long(V, dlogits == logits)) run(cross_entropy_kernel<__nv_bfloat16, true>, (const __nv_bfloat16*)logits);
+  else run(cross_entropy_kernel<__nv_bfloat16, false>, (const __nv_bfloat16*)logits);
   LAUNCH_RET();
 }
 
