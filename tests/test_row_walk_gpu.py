@@ -57,3 +57,17 @@ def test_bias_and_activation(T, C):
     # the kernel's error function and exponential are good to 2^-18 of their argument's scale (|z| < 12)
     assert ((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + dy.double().abs() * 2.0 ** -14).all()
     assert ((db.double() - want.sum(0)).abs() <= 2.0 ** -8 * want.sum(0).abs() + dy.double().abs().sum(0) * 2.0 ** -14).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [2, 148, 149, 296, 301, 591])
+@pytest.mark.parametrize("H", [264, 2048, 4104, 8192])
+def test_norms_with_a_row_or_two_for_a_block(T, H):
+    test_norms(T, H)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [2, 296])
+@pytest.mark.parametrize("C", [4304, 16384])
+def test_bias_and_activation_with_a_row_for_a_block(T, C):
+    test_bias_and_activation(T, C)

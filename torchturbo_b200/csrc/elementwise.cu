@@ -48,17 +48,23 @@ __device__ __forceinline__ void block_sums(float (&v)[N], float* red) {
 // 136 with two; 2850 x 1152 LayerNorm 18.3 and 16.5); blocks of more than 512 threads run one to an SM, and a second of them would only
 // start when the first has ended (1000 x 8192 30 us with two, 23 with one).
 static int row_threads(int cols) { return cols / 8 > 1024 ? 1024 : (cols / 8 + 31) / 32 * 32; }
+// Blocks of one row each do not walk: what prepares a next row costs 0.15 us, of 3.0 (8 x 512) to 5.1 (61 x 2048).  Rows that leave an SM
+// for each stay apart also where blocks are large (8 x 8192 10.3 us with two a block, 9.2 so).
 struct RowPlan {
   int grid, threads;
-  bool two;
+  bool two, walk;
 };
 static RowPlan row_plan(long long rows, int cols, int grid) {
-  RowPlan p{grid, row_threads(cols), false};
-  if (p.threads > 512) p.grid = (grid + 1) / 2;
+  RowPlan p{grid, row_threads(cols), false, false};
+  if (p.threads > 512 && rows > device_sms()) p.grid = (grid + 1) / 2;
+  if (p.threads <= 256 && rows > grid && rows < 2ll * grid) p.grid = static_cast<int>((rows + 1) / 2);
   if (p.grid > rows) p.grid = static_cast<int>(rows);
-  p.two = p.threads <= 256 && rows >= 2ll * p.grid;
+  p.two = p.threads <= 256 && rows > p.grid;
+  p.walk = rows > p.grid;
   return p;
 }
+// the form of a row kernel that a plan asks for
+#define ROW_KERNEL(name, plan) ((plan).two ? name<2, true> : (plan).walk ? name<1, true> : name<1, false>)
 __device__ __forceinline__ float block_max(float v, float* red) {
   v = warp_max(v);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -138,7 +144,7 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 // reduction a row took two memory latencies.  With the column sum, before -> now: 16384 x 4096 189 -> 97 us (5.5 TB/s), 4096 x 8192
 // 101 -> 59, 4096 x 2048 21 -> 19; LayerNorm 16384 x 4096 254 -> 107, 2850 x 1152 18.6 -> 16.5.
 //   dx = rstd * (g - xhat * mean(g * xhat)),  g = dy * w,  xhat = x * rstd   (+ dres_in)
-template <int ROWS>
+template <int ROWS, bool WALK>
 __global__ void __launch_bounds__(ROWS == 1 ? 1024 : 256)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dx,
@@ -168,7 +174,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   };
   load(blockIdx.x);
   const long long step = static_cast<long long>(ROWS) * gridDim.x;
-  for (long long first = blockIdx.x; first < T; first += step) {
+  for (long long first = blockIdx.x; first < T; first += WALK ? step : T) {
     float xh[ROWS][8], g[ROWS][8], dot[ROWS], r[ROWS];
     uint4 rs[ROWS];
 #pragma unroll
@@ -193,7 +199,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
         }
       }
     }
-    load(first + step);
+    if (WALK) load(first + step);
     block_sums<ROWS>(dot, red);
 #pragma unroll
     for (int k = 0; k < ROWS; ++k) {
@@ -284,7 +290,7 @@ __global__ void layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const 
   }
 }
 
-template <int ROWS>
+template <int ROWS, bool WALK>
 __global__ void __launch_bounds__(ROWS == 1 ? 1024 : 256)
 layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
@@ -314,7 +320,7 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   };
   load(blockIdx.x);
   const long long step = static_cast<long long>(ROWS) * gridDim.x;
-  for (long long first = blockIdx.x; first < T; first += step) {
+  for (long long first = blockIdx.x; first < T; first += WALK ? step : T) {
     float xh[ROWS][8], g[ROWS][8], sums[2 * ROWS], rstd[ROWS];
 #pragma unroll
     for (int k = 0; k < ROWS; ++k) {
@@ -339,7 +345,7 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
       sums[2 * k] = sg;
       sums[2 * k + 1] = sgx;
     }
-    load(first + step);
+    if (WALK) load(first + step);
     block_sums<2 * ROWS>(sums, red);
 #pragma unroll
     for (int k = 0; k < ROWS; ++k) {
@@ -409,6 +415,7 @@ __global__ void bias_act_fwd_kernel(const __nv_bfloat16* __restrict__ x, const _
 
 // Blocks walk rows of up to 8192 columns (blockIdx.y: which), eight columns a thread, the next row's loads ahead of this one's arithmetic.
 // With the column sum, GELU, before -> now: 2850 x 4304 25 -> 21 us, 16384 x 4096 108 -> 74, 2000 x 16384 107 -> 54.
+template <bool WALK>
 __global__ void __launch_bounds__(1024)
 bias_act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ bias,
                     __nv_bfloat16* __restrict__ dx, float* __restrict__ part, long long R, int C, int act) {
@@ -424,9 +431,9 @@ bias_act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
     if (act) xu = *reinterpret_cast<const uint4*>(x + row * C + c);
   };
   load(blockIdx.x);
-  for (long long row = blockIdx.x; row < R; row += gridDim.x) {
+  for (long long row = blockIdx.x; row < R; row += WALK ? gridDim.x : R) {
     const uint32_t ds[4] = {du.x, du.y, du.z, du.w}, xs[4] = {xu.x, xu.y, xu.z, xu.w};
-    load(row + gridDim.x);
+    if (WALK) load(row + gridDim.x);
     uint32_t o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1451,7 +1458,7 @@ TTB_EXPORT int ttb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
   const RowPlan plan = row_plan(T, H, grid);
   grid = plan.grid;
   auto DY = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
-  (plan.two ? rmsnorm_bwd_kernel<2> : rmsnorm_bwd_kernel<1>)<<<grid, plan.threads, 0, STREAM(stream)>>>(
+  ROW_KERNEL(rmsnorm_bwd_kernel, plan)<<<grid, plan.threads, 0, STREAM(stream)>>>(
       DY, X, W, rstd, (const __nv_bfloat16*)dres_in, (__nv_bfloat16*)dx, dw_partial, T, H, one_plus_w);
   colsum(dw_partial, dw_out, dw_bf16, grid, H, STREAM(stream));
   LAUNCH_RET();
@@ -1480,7 +1487,7 @@ TTB_EXPORT int ttb_layernorm_bwd(const void* dy, const void* x, const void* w, c
   const RowPlan plan = row_plan(T, H, grid);
   grid = plan.grid;
   auto DY = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
-  (plan.two ? layernorm_bwd_kernel<2> : layernorm_bwd_kernel<1>)<<<grid, plan.threads, 0, STREAM(stream)>>>(DY, X, W, mean, rstd,
+  ROW_KERNEL(layernorm_bwd_kernel, plan)<<<grid, plan.threads, 0, STREAM(stream)>>>(DY, X, W, mean, rstd,
                                                                                                        (__nv_bfloat16*)dx, part, T, H);
   colsum(part, dwdb_out, out_bf16, grid, 2 * H, STREAM(stream));
   LAUNCH_RET();
@@ -1557,8 +1564,8 @@ TTB_EXPORT int ttb_bias_act_bwd(const void* dy, const void* x, const void* bias,
   if (C > 16384) return 902;
   if (grid > R) grid = (int)R;
   const int threads = row_threads(C > 8192 ? (C + 15) / 16 * 8 : C);
-  bias_act_bwd_kernel<<<dim3(grid, C > 8192 ? 2 : 1), threads, 0, STREAM(stream)>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                                                                                 (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, part, R, C, act);
+  (R > grid ? bias_act_bwd_kernel<true> : bias_act_bwd_kernel<false>)<<<dim3(grid, C > 8192 ? 2 : 1), threads, 0, STREAM(stream)>>>(
+      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, part, R, C, act);
   colsum(part, dbias_out, out_bf16, grid, C, STREAM(stream));
   LAUNCH_RET();
 }
@@ -1787,7 +1794,7 @@ TTB_EXPORT int ttb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void
   auto DY = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
   // every block writes its full row of `scratch` (H floats), and the column sum below reads exactly rows [0, grid):
   // nothing has to be cleared between calls
-  (plan.two ? rmsnorm_bwd_kernel<2> : rmsnorm_bwd_kernel<1>)<<<grid, plan.threads, 0, STREAM(stream)>>>(
+  ROW_KERNEL(rmsnorm_bwd_kernel, plan)<<<grid, plan.threads, 0, STREAM(stream)>>>(
       DY, X, W, rstd, (const __nv_bfloat16*)dres_in, (__nv_bfloat16*)dx, scratch, T, H, one_plus_w);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return TTB_NOALLOC_ERR_LAUNCH_DX + static_cast<int>(e);
