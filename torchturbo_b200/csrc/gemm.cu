@@ -488,12 +488,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         constexpr int CH = BN / 32 / (EPI_WARPS / 4);
         const float alpha = p.alpha ? __ldg(p.alpha) : 1.f;
         const uint32_t st = smem_u32(epi_stage + (warp - 2) * L::EPI_STAGE_BYTES);
-        // first element of output row `rr` (null = skip it); with the scatter epilogue a row goes to the rank it came from, at the
-        // entry its tag names
-        auto tag_of = [&](int rr) { return rr < p.M ? (p.ep.scat_on ? __ldcg(p.ep.row_tag + rr) : 0) : -1; };
-        auto row_dst = [&](int rr, int tag) -> __nv_bfloat16* {
-          if (tag < 0) return nullptr;
+        // bf16 output: first element of the four rows that this lane stores in the row-major pass (null = skip it); with the scatter
+        // epilogue a row goes to the rank it came from, at the entry its tag names
+        auto row_dst = [&](int rr) -> __nv_bfloat16* {
+          if (rr >= p.M || p.c_fp32) return nullptr;
           if (!p.ep.scat_on) return reinterpret_cast<__nv_bfloat16*>(cbase) + gbase + static_cast<long long>(rr) * p.ldc;
+          const int tag = __ldcg(p.ep.row_tag + rr);
+          if (tag < 0) return nullptr;
           // a tag that names no rank or no entry (rows that never landed) must not become an address
           if ((tag >> EP_TAG_SHIFT) < p.ep.W && (tag & EP_TAG_MASK) < p.ep.ret_rows)
             return reinterpret_cast<__nv_bfloat16*>(p.ep.peers.base[tag >> EP_TAG_SHIFT] + p.ep.off_ret) +
@@ -507,9 +508,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             reinterpret_cast<float*>(p.ep.peers.base[tag >> EP_TAG_SHIFT] + p.ep.off_ret_vals)[tag & EP_TAG_MASK] =
                 p.ep.row_val[row];
         }
-        int tag[4];
+        __nv_bfloat16* rowptr[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tag[j] = tag_of(row_base + (lane >> 2) + 8 * j);
+        for (int j = 0; j < 4; ++j) rowptr[j] = row_dst(row_base + (lane >> 2) + 8 * j);
 #pragma unroll 1
         for (int c = col_half * CH; c < (col_half + 1) * CH; ++c) {
           const int col0 = n0 + c * 32;
@@ -532,6 +533,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             // is added and the parked rows are read ahead of the first store (sums into an fp32 gradient of 128 experts, 2048 x
             // 1536 of 256 rows each: 1965 -> 822 us; every store waited for its own two loads before)
             __syncwarp();  // the previous chunk's readers are done with the staging area
+            if (p.ep.scat_on) {
+              // nothing is added in fp32: parked as bf16, half the shared-memory traffic (second product of 4096 tokens, one rank to itself,
+              // parked as fp32 and as bf16: 128 experts, eight a token, 768 to 2048, 153 and 143 us; 16, four a token, 512 to 1024, 54 and 46)
+              const int q = lane & 3;
+              uint4 o[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) w[e] = pack_bf16(__uint_as_float(v[8 * i + 2 * e]), __uint_as_float(v[8 * i + 2 * e + 1]));
+                st_shared_v4(epi_piece_addr64(st, lane, i), w[0], w[1], w[2], w[3]);
+              }
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 4; ++j) ld_shared_v4(epi_piece_addr64(st, (lane >> 2) + 8 * j, q), o[j].x, o[j].y, o[j].z, o[j].w);
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (rowptr[j] != nullptr) *reinterpret_cast<uint4*>(rowptr[j] + col0 + 8 * q) = o[j];
+              continue;
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               st_shared_v4(epi_piece_addr(st, lane, i), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
@@ -564,7 +585,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               float f[4][8];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                dst[j] = row_dst(r0 + 8 * j, tag[j]);
+                dst[j] = rowptr[j];
                 if (dst[j] == nullptr) continue;
                 dst[j] += col0 + 8 * q;
                 if (p.residual) res[j] = *reinterpret_cast<const uint4*>(p.residual + static_cast<long long>(r0 + 8 * j) * p.ldr + col0 + 8 * q);
