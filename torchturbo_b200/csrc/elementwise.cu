@@ -1138,7 +1138,8 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long lon
 // alone 489, marks alone 488; one read and one write at the rate of a copy: 408), 1024 rows 148 -> 133.  Shorter rows are still there,
 // and the plain order is the faster one: in place, plain and LONG, 4096 x 32000 111 and 113 us, x 80000 245 and 257, x 112000 350 and
 // 356, x 116000 373 and 371, x 128256 411 and 403; with a gradient of its own, which takes L2 as well, x 80000 249 and 256, x 84000 270
-// and 268, x 100352 328 and 311.  With a third fewer instructions it takes the same time; 512 threads per block take 514 us, and 102 with
+// and 268, x 100352 328 and 311 (300 to 600 rows whose logits and gradients just fill the L2 are an exception: 600 x 40000 27.0 and
+// 25.7).  With a third fewer instructions it takes the same time; 512 threads per block take 514 us, and 102 with
 // 32000 logits.
 // ============================================================================
 template <typename TL>
