@@ -378,7 +378,8 @@ def _register(op_name: str, impl_name: str):
 
 @_register("gdn_gates", "b200_gdn_gates")
 class B200GDNGates(OpImpl):
-    """One launch forward and two backward (projections may be columns of a wider matrix)."""
+    """One launch forward and two backward.  Projections may be columns of a wider matrix, but next to one another: `a` and `b` as
+    sequence parallelism leaves them, alternating in memory, take torch operations."""
 
     def available(self) -> bool:
         return K.available()
