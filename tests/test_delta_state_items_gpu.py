@@ -71,7 +71,7 @@ def test_a_first_state_of_zero_is_not_read(H, lens):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("H, lens", [(1, [1]), (2, [1, 0, 1]), (3, [1] * 40), (5, [2] * 17), (30, [3, 3, 2, 3]), (148, [2]), (60, [2] * 4), (37, [4] * 7)])
+@pytest.mark.parametrize("H, lens", [(1, [1]), (2, [1, 0, 1]), (3, [1] * 40), (5, [2] * 17), (30, [3, 3, 2, 3]), (148, [2]), (60, [2] * 4), (37, [4] * 7), (32, [4, 3, 3, 3])])
 @pytest.mark.parametrize("vec", [False, True])
 @pytest.mark.parametrize("with_init", [False, True])
 def test_forward_with_the_longest_sequence_known(H, lens, vec, with_init):

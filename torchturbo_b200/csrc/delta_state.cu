@@ -574,15 +574,18 @@ delta_state_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 //    longer than the others (those of the last wave are the shortest): 32 heads with four of 16 chunks 78 and 70, of 24 110 and 100, with
 //    three of 21 88 and 81.  Lengths with a mean of 0.83 of the longest 92 and 88, of 0.71 115 and 123; 80 pairs at 0.80 76 and 78, 96 at 0.88
 //    82 and 84, whose shorter last wave is less of a loss;
-//  * 223 to 259: two full waves against three and a bit: 240 pairs of 24 chunks 203 and 195, 256 205 and 203, 288 219 and 231;
-//  * sequences of one chunk, which have no chain: 64 pairs 12.3 and 10.2, 128 14.3 and 12.3, 256 20.5 and 18.4; the same from 600 on.
+//  * 223 to 259: two full waves against three and a bit: 240 pairs of 24 chunks 203 and 195, 256 205 and 203, 288 219 and 231; with a mean of
+//    0.89 of the longest 224 170 and 168, but 256 170 and 176;
+//  * sequences of one chunk, which have no chain: 64 pairs 12.3 and 10.2, 128 14.3 and 12.3, 256 20.5 and 18.4; 512 29.7 and 30.7, with first
+//    states 35.8 and 38.9.
 // Outside these it is 1.0 to 1.5 times slower (1 pair to 74: 1.4; 160 to 192: 1.1; 320: 1.1).
 static bool wide_pays(int nseq, int H, int NC, int longest, long long places) {
   const long long pairs = static_cast<long long>(nseq) * H;
   if (longest <= 0 || H > 65535) return false;
-  if (longest == 1) return pairs <= 2 * places;
-  if (10ll * NC < (8 * pairs < 3 * places ? 9ll : 8ll) * longest * nseq) return false;
-  return (2 * pairs <= places && 4 * pairs > places) || (4 * pairs > 3 * places && 8 * pairs <= 7 * places);
+  if (longest == 1) return pairs <= places;
+  const long long mean = 20ll * NC, top = static_cast<long long>(longest) * nseq;      // of the lengths, in twentieths, and the longest
+  if (2 * pairs <= places) return 4 * pairs > places && mean >= (8 * pairs < 3 * places ? 18 : 16) * top;
+  return 4 * pairs > 3 * places && 8 * pairs <= 7 * places && mean >= 19 * top;
 }
 
 }  // namespace ttb
